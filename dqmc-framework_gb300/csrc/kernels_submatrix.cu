@@ -36,6 +36,7 @@
 #include <cstdint>
 
 #include "dqmc_device.cuh"
+#include "oz_tc.cuh"
 #include "ozaki.cuh"
 #include "tcgen05.cuh"
 
@@ -51,7 +52,7 @@ constexpr int OZS = 6, OZB = 7;  // 6 slices of 7 bits; group sums < 2^22 for K 
 // tensor-core tiles: 128 rows x 32 columns, K = 32 in two chunks of 16
 constexpr int TM = 128, TN = 32;
 constexpr int A_BYTES = OZS * 2 * TM * 32;  // A operand: [slice][chunk][128 lines x 16 k]
-constexpr int B_BYTES = OZS * 2 * TN * 32;  // one B tile: [slice][chunk][32 lines x 16 k]
+constexpr int B_BYTES = OZS * 2 * TN * 32;  // one B tile: [chunk][slice][32 lines x 16 k]
 constexpr int NBB = 3;                      // B tiles in flight (loads run two tiles ahead)
 constexpr int ACC_COLS = OZS * TN;          // TMEM columns of one accumulator (6 weight groups)
 constexpr unsigned TMEM_COLS = 512;         // two accumulators
@@ -218,7 +219,6 @@ __device__ void sub_gemm(const SubTC& tc, unsigned& gt, unsigned& nA, const unsi
   if (tid >= kSubThreads) {
     // ---- producer (one thread; its warp reconverges before the final barrier)
     if (tid == kSubThreads) {
-      constexpr uint32_t idesc = tc::idesc_bf16(TM, TN);
       auto load_b = [&](int t) {
         const unsigned u = gt + t;
         const int cb = cb_of(t), bb = (int)(u % NBB);
@@ -228,7 +228,7 @@ __device__ void sub_gemm(const SubTC& tc, unsigned& gt, unsigned& nA, const unsi
         tc::mbar_expect_tx(&tc.ldB[bb], OZS * nk * TN * 32);
         for (int s2 = 0; s2 < OZS; ++s2)
           for (int kk = 0; kk < nk; ++kk)
-            tc::bulk_g2s(dst + (s2 * 2 + kk) * TN * 32,
+            tc::bulk_g2s(dst + (kk * OZS + s2) * TN * 32,
                          bG + s2 * b_sst + ((long long)kk * b_nlb + cb * (TN / 8)) * 128, TN * 32, &tc.ldB[bb]);
       };
       auto issue = [&](int t) {  // A if a new row block, then the MMAs of tile t
@@ -251,14 +251,10 @@ __device__ void sub_gemm(const SubTC& tc, unsigned& gt, unsigned& nA, const unsi
         tc::fence_after();
         const unsigned sa = tc::su32(tc.A), sb = tc::su32(tc.B + bb * B_BYTES);
         for (int kk = 0; kk < nk; ++kk)
-  #pragma unroll
-          for (int i = 0; i < OZS; ++i) {
-            const uint64_t ad = tc::desc(sa + (i * 2 + kk) * TM * 32, 128, 256);
-  #pragma unroll
-            for (int jj = 0; jj < OZS - i; ++jj)
-              tc::mma(tc.tmem + (unsigned)(acc * ACC_COLS + (i + jj) * TN), ad,
-                      tc::desc(sb + (jj * 2 + kk) * TN * 32, 128, 256), idesc, kk > 0 || i > 0);
-          }
+#pragma unroll
+          for (int i = 0; i < OZS; ++i)
+            oztc::mma_row<OZS, TM, TN>(tc.tmem + (unsigned)(acc * ACC_COLS), sa + (i * 2 + kk) * TM * 32,
+                                       sb + kk * OZS * TN * 32, i, kk > 0 || i > 0);
         tc::commit(&tc.mmab[acc]);
         tc::commit(&tc.bfree[bb]);
       };

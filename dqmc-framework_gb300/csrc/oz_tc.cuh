@@ -6,11 +6,11 @@
 // 256 bytes, so that the 16-deep chunk of one slice over a tile's MT (or NT)
 // consecutive lines is one contiguous range of MT * 32 bytes.  One thread
 // streams the chunks with bulk asynchronous copies into a ring of NS stages
-// (each completing on its own mbarrier's byte count), issues the S (S+1) / 2
-// MMAs of a chunk (slice pair (i, j) accumulates into weight group i + j, S
-// groups of NT FP32 columns in TMEM) and refills a stage once the MMAs that read
-// it have completed (their commit mbarrier): NS - 1 chunks are in flight while
-// the tensor core works.  Every wait is bounded; on a timeout the loop stops,
+// (each completing on its own mbarrier's byte count), issues the MMAs of the
+// S (S+1) / 2 slice pairs of a chunk (slice pair (i, j) accumulates into weight
+// group i + j, S groups of NT FP32 columns in TMEM; mma_row) and refills a stage
+// once the MMAs that read it have completed (their commit mbarrier): NS - 1
+// chunks are in flight while the tensor core works.  Every wait is bounded; on a timeout the loop stops,
 // waits (bounded) for the copies it issued and reports the failure.
 #pragma once
 #include <cstdint>
@@ -22,6 +22,27 @@ namespace oztc {
 
 // bytes of one stage: S slices of an MT x 16 A chunk and an NT x 16 B chunk
 __host__ __device__ constexpr int stage_bytes(int S, int MT, int NT) { return S * (MT + NT) * 16 * 2; }
+
+// The MMAs of A slice i with the B slices 0 .. S-1-i of one 16-deep chunk.  The B slices lie
+// side by side in shared memory (NT lines of 32 bytes each, 8-line groups 256 bytes apart), and
+// pair (i, j) accumulates into the NT columns of group i + j, so B slices j, j+1, ... and their
+// accumulators are consecutive: they form one operand of (S - i) NT lines, issued as MMAs of up
+// to 256 columns.  The tensor core reads A from shared memory once per MMA, which bounds MMAs of
+// 32 columns; each group still receives its pairs in order of i, so the sums are those of one
+// MMA per pair.  Against one MMA of NT columns per pair: a pair of half-sweeps of 128 walkers,
+// 16 x 16, beta = 10 went from 902 to 826 ms, 8 walkers of 24 x 24 with dynamic measurement from
+// 291 to 264 ms, 6 walkers of 16 x 16 (few enough to be bound by the decisions) from 99.6 to 95.4.
+template <int S, int MT, int NT>
+__device__ __forceinline__ void mma_row(unsigned taddr, unsigned sa, unsigned sb, int i, bool accum) {
+  // K-major core matrices: 128 bytes apart along k, 8-line groups 256 bytes apart
+  const uint64_t ad = tc::desc(sa, 128, 256);
+  const int cols = (S - i) * NT;
+#pragma unroll
+  for (int n0 = 0; n0 < S * NT; n0 += 256)
+    if (n0 < cols)
+      tc::mma(taddr + (unsigned)(i * NT + n0), ad, tc::desc(sb + n0 * 32, 128, 256),
+              tc::idesc_bf16(MT, cols - n0 < 256 ? cols - n0 : 256), accum);
+}
 
 // Thread-only main loop.  a0 / b0: slice 0 of the tile's first line block at
 // chunk 0; consecutive slices sstride elements apart, consecutive chunks cstep.
@@ -35,7 +56,6 @@ __device__ int mainloop(unsigned char* tsm, unsigned long long* full, unsigned l
                         const unsigned short* a0, const unsigned short* b0, long long sstride, long long cstep,
                         int nch, bool& ok, int land_limit = 1 << 24) {
   constexpr int A_SL = MT * 32, B_SL = NT * 32, STAGE = stage_bytes(S, MT, NT);
-  constexpr uint32_t idesc = tc::idesc_bf16(MT, NT);
   auto produce = [&](int c, int st) {
     unsigned char* sA = tsm + st * STAGE;
     unsigned char* sB = sA + S * A_SL;
@@ -56,13 +76,8 @@ __device__ int mainloop(unsigned char* tsm, unsigned long long* full, unsigned l
     tc::fence_after();
     const unsigned sa = tc::su32(tsm + st * STAGE), sb = sa + S * A_SL;
 #pragma unroll
-    for (int i = 0; i < S; ++i) {
-      // K-major core matrices: 128 bytes apart along k, 8-line groups 256 bytes apart
-      const uint64_t ad = tc::desc(sa + i * A_SL, 128, 256);
-#pragma unroll
-      for (int jj = 0; jj < S - i; ++jj)
-        tc::mma(taddr + (unsigned)((i + jj) * NT), ad, tc::desc(sb + jj * B_SL, 128, 256), idesc, c > 0 || i > 0);
-    }
+    for (int i = 0; i < S; ++i)
+      mma_row<S, MT, NT>(taddr, sa + i * A_SL, sb, i, c > 0 || i > 0);
     tc::commit(&done[st]);
     last = c;
     if (c >= 1 && c - 1 + NS < nch) {  // the stage of chunk c - 1 is free once its MMAs completed
