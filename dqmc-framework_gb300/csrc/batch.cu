@@ -604,6 +604,12 @@ int dqmc_batch_create(const dqmc_walker_desc* descs, int n, const dqmc_batch_opt
     // checkerboard/square.cpp:34-49 (note its exp(+0.5 dtau mu) sign)
     plaq(h.cbP, std::cosh(dtau * d.hopping_t), std::sinh(dtau * d.hopping_t), std::exp(0.5 * dtau * d.mu));
     plaq(h.cbI, std::cosh(-dtau * d.hopping_t), std::sinh(-dtau * d.hopping_t), std::exp(-0.5 * dtau * d.mu));
+    h.cb_h = std::tanh(dtau * d.hopping_t);
+    for (int inv = 0; inv < 2; ++inv) {
+      const double f = inv ? h.cbI[0] : h.cbP[0];  // exp(+-dtau mu / 2) cosh^2
+      h.cb_e[inv][0] = h.e_pa * (f * f);
+      h.cb_e[inv][1] = h.e_ma * (f * f);
+    }
     h.G = reinterpret_cast<double*>(base + off[w].G);
     h.chain = reinterpret_cast<double*>(base + off[w].chain);
     const bool gen = N > kMaxSmemN || o.precision == DQMC_MIXED || o.hbm;

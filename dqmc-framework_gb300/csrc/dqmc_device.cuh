@@ -42,6 +42,9 @@ struct WalkerDev {
   // ratio constants indexed by [s>0 ? 0 : 1]: exp(-2 alpha s) - 1, exp(+2 alpha s) - 1, exp(2 alpha s)
   double cm[2], cp[2], ex2[2];
   double cbP[16], cbI[16];   // checkerboard plaquettes exp(+dtau t h) e^{0.5 dtau mu}, inverse
+  // the plaquette as f c^2 [[1, h], [h, 1]] (x) [[1, h], [h, 1]]: h (its inverse has -h), and
+  // exp(+alpha), exp(-alpha) times (f c^2)^2 of the two passes of a product ([1]: of the inverse)
+  double cb_h, cb_e[2][2];
   double* G;                 // [2][N*N]
   double* chain;             // [S][N*N] (general walkers: [2][S][N*N], ping-pong)
   double* work;              // general walkers: GEMM temporary [S][N*N]

@@ -17,6 +17,8 @@
 //   push_kernel     src/svd_stack.cpp:34-61 (stack push; QRP replaces dgesvd).
 //   greens_kernel   include/utils/numerical_stable.hpp:34-239 (stable G, wrap error).
 #include <cuda_runtime.h>
+
+#include <algorithm>
 #include <cstdint>
 
 #include "dqmc_device.cuh"
@@ -74,8 +76,10 @@ __device__ double block_max(double v, double* red) {
 __device__ __forceinline__ int spin_sign(const WalkerDev& w, int spin) {
   return (w.model == 0 && spin == 1) ? -1 : 1;
 }
-// exp(+/- alpha) for the product sgn * s
-__device__ __forceinline__ double bdiag(const WalkerDev& w, int sgn_times_s) {
+// exp(+/- alpha) for the product sgn * s, with the checkerboard products' constant factor folded
+// in when fold (inv: of the products with exp(+dtau K))
+__device__ __forceinline__ double bdiag(const WalkerDev& w, int sgn_times_s, int inv, bool fold) {
+  if (fold && w.cb) return w.cb_e[inv][sgn_times_s > 0 ? 0 : 1];
   return sgn_times_s > 0 ? w.e_pa : w.e_ma;
 }
 
@@ -97,9 +101,39 @@ __device__ __forceinline__ void plaq_sites(int L, int q, int parity, int (&idx)[
   idx[3] = x1 + L * y1;
 }
 
-// pre: scale inputs by d[row] (d from the scale table sd, null = none); post likewise on outputs
-__device__ void cb_left(double* M, int ld, int N, int L, int parity, const double* P,
-                        const double* pre, const double* post) {
+// The plaquette matrix is f c^2 [[1, h], [h, 1]] (x) [[1, h], [h, 1]] with c = cosh, h = tanh of
+// +-dtau t: applied as two butterflies of 8 FMAs on the plaquette's 4 values instead of a 4 x 4
+// product of 4 multiplies and 12 FMAs (an FP64 warp instruction holds its pipe for 64 cycles,
+// and the passes are half of a checkerboard slice's FP64 work).  The factors f c^2 of a product's
+// two passes are folded into the diagonal scale of the product (bdiag).
+__device__ __forceinline__ void plaq_apply(double (&v)[4], double h) {
+  const double a0 = fma(h, v[1], v[0]), a1 = fma(h, v[0], v[1]);
+  const double a2 = fma(h, v[3], v[2]), a3 = fma(h, v[2], v[3]);
+  v[0] = fma(h, a2, a0);
+  v[1] = fma(h, a3, a1);
+  v[2] = fma(h, a0, a2);
+  v[3] = fma(h, a1, a3);
+}
+
+// The plain 4 x 4 product: the set-up keeps it, because the sign it takes from an LU of the
+// initial G is rounding noise once G has eigenvalues below its rounding (8 x 8 at beta = 8), and
+// a given seed has to keep its sign.
+__device__ __forceinline__ void plaq_product(double (&v)[4], const double* P) {
+  double o[4];
+#pragma unroll
+  for (int a = 0; a < 4; ++a) {
+    o[a] = P[a * 4 + 0] * v[0];
+    o[a] = fma(P[a * 4 + 1], v[1], o[a]);
+    o[a] = fma(P[a * 4 + 2], v[2], o[a]);
+    o[a] = fma(P[a * 4 + 3], v[3], o[a]);
+  }
+#pragma unroll
+  for (int a = 0; a < 4; ++a) v[a] = o[a];
+}
+
+// pre: scale inputs by pre[row] (null = none); post likewise on outputs; P: plain product
+__device__ void cb_left(double* M, int ld, int N, int L, int parity, double h, const double* pre,
+                        const double* post, const double* P = nullptr) {
   const int nq = (L >> 1) * (L >> 1);
   for (int it = threadIdx.x; it < nq * N; it += kThreads) {
     const int q = it % nq, c = it / nq;
@@ -111,20 +145,18 @@ __device__ void cb_left(double* M, int ld, int N, int L, int parity, const doubl
       v[a] = at(M, ld, idx[a], c);
       if (pre) v[a] *= pre[idx[a]];
     }
+    if (P) plaq_product(v, P);
+    else plaq_apply(v, h);
 #pragma unroll
     for (int a = 0; a < 4; ++a) {
-      double o = P[a * 4 + 0] * v[0];
-      o = fma(P[a * 4 + 1], v[1], o);
-      o = fma(P[a * 4 + 2], v[2], o);
-      o = fma(P[a * 4 + 3], v[3], o);
-      if (post) o *= post[idx[a]];
-      at(M, ld, idx[a], c) = o;
+      if (post) v[a] *= post[idx[a]];
+      at(M, ld, idx[a], c) = v[a];
     }
   }
 }
 
-__device__ void cb_right(double* M, int ld, int N, int L, int parity, const double* P,
-                         const double* pre, const double* post) {
+__device__ void cb_right(double* M, int ld, int N, int L, int parity, double h, const double* pre,
+                         const double* post) {
   const int nq = (L >> 1) * (L >> 1);
   for (int it = threadIdx.x; it < nq * N; it += kThreads) {
     const int r = it % N, q = it / N;
@@ -136,67 +168,79 @@ __device__ void cb_right(double* M, int ld, int N, int L, int parity, const doub
       v[a] = at(M, ld, r, idx[a]);
       if (pre) v[a] *= pre[idx[a]];
     }
+    plaq_apply(v, h);
 #pragma unroll
     for (int b = 0; b < 4; ++b) {
-      double o = v[0] * P[0 * 4 + b];
-      o = fma(v[1], P[1 * 4 + b], o);
-      o = fma(v[2], P[2 * 4 + b], o);
-      o = fma(v[3], P[3 * 4 + b], o);
-      if (post) o *= post[idx[b]];
-      at(M, ld, r, idx[b]) = o;
+      if (post) v[b] *= post[idx[b]];
+      at(M, ld, r, idx[b]) = v[b];
     }
   }
 }
 
 // --------------------------------------------------------------------------
-// Register-tiled block GEMM for N <= 64: each of the 16x16 threads owns a
-// T x T tile (rows ty+16a, cols tx+16b).  out(r,c) = sum_k A(r,k) B(k,c).
-// The caller-supplied loaders/stores make it serve in-place products
-// (SMEM or global: everyone reads before anyone writes).
+// Block GEMM for N <= 64: out(r,c) = sum_{k >= kbeg} A(r,k) B(k,c).  Output e = r + N c belongs
+// to thread e % 256, so a warp holds consecutive rows of one or two columns: A is read along
+// rows, B as a broadcast.  An FP64 warp instruction costs 64 cycles, an operand load a few, so
+// the mapping spends no FMA on padding (N = 36: 41 warp FMAs per k, 72 with a 48 x 48 register
+// tiling) and shares no operands across registers.  The caller-supplied loaders/stores make it
+// serve in-place products (SMEM or global: everyone reads before anyone writes).
 // --------------------------------------------------------------------------
 template <int T, class FA, class FB, class FS>
-__device__ __forceinline__ void tile_gemm(int N, int kbeg, FA A, FB B, FS store) {
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  double acc[T][T];
+__device__ __forceinline__ void flat_gemm(int N, int kbeg, FA A, FB B, FS store) {
+  const int NN = N * N, w0 = threadIdx.x & ~31;
+  double acc[T];
+  int r[T], c[T];
 #pragma unroll
-  for (int a = 0; a < T; ++a)
-#pragma unroll
-    for (int b = 0; b < T; ++b) acc[a][b] = 0.0;
+  for (int u = 0; u < T; ++u) {
+    const int e = min((int)threadIdx.x + u * kThreads, NN - 1);
+    acc[u] = 0.0;
+    r[u] = e % N;
+    c[u] = e / N;
+  }
+#pragma unroll(T == 1 ? 8 : T == 3 ? 4 : 2)
   for (int k = kbeg; k < N; ++k) {
-    double av[T], bv[T];
 #pragma unroll
-    for (int a = 0; a < T; ++a) {
-      const int r = ty + 16 * a;
-      av[a] = (r < N) ? A(r, k) : 0.0;
-    }
-#pragma unroll
-    for (int b = 0; b < T; ++b) {
-      const int c = tx + 16 * b;
-      bv[b] = (c < N) ? B(k, c) : 0.0;
-    }
-#pragma unroll
-    for (int a = 0; a < T; ++a)
-#pragma unroll
-      for (int b = 0; b < T; ++b) acc[a][b] = fma(av[a], bv[b], acc[a][b]);
+    for (int u = 0; u < T; ++u)
+      if (w0 + u * kThreads < NN)  // uniform in the warp
+        acc[u] = fma(A(r[u], k), B(k, c[u]), acc[u]);
   }
   __syncthreads();
 #pragma unroll
-  for (int a = 0; a < T; ++a)
-#pragma unroll
-    for (int b = 0; b < T; ++b) {
-      const int r = ty + 16 * a, c = tx + 16 * b;
-      if (r < N && c < N) store(r, c, acc[a][b]);
-    }
+  for (int u = 0; u < T; ++u)
+    if ((int)threadIdx.x + u * kThreads < NN) store(r[u], c[u], acc[u]);
   __syncthreads();
 }
 
-// dispatch on N to the smallest tile that covers it
+// The same for 50 < N <= 64: row tid % 64, columns tid / 64 + 4 u, so a thread keeps one row.
+template <class FA, class FB, class FS>
+__device__ __forceinline__ void row_gemm(int N, int kbeg, FA A, FB B, FS store) {
+  constexpr int T = 16;
+  const int r = threadIdx.x & 63, c0 = threadIdx.x >> 6;
+  double acc[T];
+#pragma unroll
+  for (int u = 0; u < T; ++u) acc[u] = 0.0;
+  if (r < N)
+    for (int k = kbeg; k < N; ++k) {
+      const double a = A(r, k);
+#pragma unroll
+      for (int u = 0; u < T; ++u)
+        if (c0 + 4 * u < N) acc[u] = fma(a, B(k, c0 + 4 * u), acc[u]);
+    }
+  __syncthreads();
+#pragma unroll
+  for (int u = 0; u < T; ++u)
+    if (r < N && c0 + 4 * u < N) store(r, c0 + 4 * u, acc[u]);
+  __syncthreads();
+}
+
+// outputs per thread: 1 up to N = 16, 3 up to 27, 6 up to 39, 10 up to 50, 16 up to 64
 template <class FA, class FB, class FS>
 __device__ __forceinline__ void block_gemm(int N, FA A, FB B, FS store, int kbeg = 0) {
-  if (N <= 16) tile_gemm<1>(N, kbeg, A, B, store);
-  else if (N <= 32) tile_gemm<2>(N, kbeg, A, B, store);
-  else if (N <= 48) tile_gemm<3>(N, kbeg, A, B, store);
-  else tile_gemm<4>(N, kbeg, A, B, store);
+  if (N <= 16) flat_gemm<1>(N, kbeg, A, B, store);
+  else if (N <= 27) flat_gemm<3>(N, kbeg, A, B, store);
+  else if (N <= 39) flat_gemm<6>(N, kbeg, A, B, store);
+  else if (N <= 50) flat_gemm<10>(N, kbeg, A, B, store);
+  else row_gemm(N, kbeg, A, B, store);
 }
 
 // --------------------------------------------------------------------------
@@ -207,9 +251,9 @@ __device__ __forceinline__ void block_gemm(int N, FA A, FB B, FS store, int kbeg
 __device__ void mult_B_left(const WalkerDev& w, double* M, int ld, const double* dpos) {
   const int N = w.N;
   if (w.cb) {
-    cb_left(M, ld, N, w.L, 1, w.cbP, nullptr, nullptr);  // sublattice B first
+    cb_left(M, ld, N, w.L, 1, w.cb_h, nullptr, nullptr);  // sublattice B first
     __syncthreads();
-    cb_left(M, ld, N, w.L, 0, w.cbP, nullptr, dpos);     // then A, scale rows
+    cb_left(M, ld, N, w.L, 0, w.cb_h, nullptr, dpos);     // then A, scale rows
     __syncthreads();
   } else {
     const double* K = w.expK;
@@ -222,9 +266,9 @@ __device__ void mult_B_left(const WalkerDev& w, double* M, int ld, const double*
 __device__ void mult_invB_right(const WalkerDev& w, double* M, int ld, const double* dneg) {
   const int N = w.N;
   if (w.cb) {
-    cb_right(M, ld, N, w.L, 1, w.cbI, nullptr, nullptr);  // B then A
+    cb_right(M, ld, N, w.L, 1, -w.cb_h, nullptr, nullptr);  // B then A
     __syncthreads();
-    cb_right(M, ld, N, w.L, 0, w.cbI, nullptr, dneg);
+    cb_right(M, ld, N, w.L, 0, -w.cb_h, nullptr, dneg);
     __syncthreads();
   } else {
     const double* K = w.invK;
@@ -237,9 +281,9 @@ __device__ void mult_invB_right(const WalkerDev& w, double* M, int ld, const dou
 __device__ void mult_B_right(const WalkerDev& w, double* M, int ld, const double* dpos) {
   const int N = w.N;
   if (w.cb) {
-    cb_right(M, ld, N, w.L, 0, w.cbP, dpos, nullptr);  // scale cols, A then B
+    cb_right(M, ld, N, w.L, 0, w.cb_h, dpos, nullptr);  // scale cols, A then B
     __syncthreads();
-    cb_right(M, ld, N, w.L, 1, w.cbP, nullptr, nullptr);
+    cb_right(M, ld, N, w.L, 1, w.cb_h, nullptr, nullptr);
     __syncthreads();
   } else {
     const double* K = w.expK;
@@ -252,9 +296,9 @@ __device__ void mult_B_right(const WalkerDev& w, double* M, int ld, const double
 __device__ void mult_invB_left(const WalkerDev& w, double* M, int ld, const double* dneg) {
   const int N = w.N;
   if (w.cb) {
-    cb_left(M, ld, N, w.L, 0, w.cbI, dneg, nullptr);  // scale rows, A then B
+    cb_left(M, ld, N, w.L, 0, -w.cb_h, dneg, nullptr);  // scale rows, A then B
     __syncthreads();
-    cb_left(M, ld, N, w.L, 1, w.cbI, nullptr, nullptr);
+    cb_left(M, ld, N, w.L, 1, -w.cb_h, nullptr, nullptr);
     __syncthreads();
   } else {
     const double* K = w.invK;
@@ -264,12 +308,13 @@ __device__ void mult_invB_left(const WalkerDev& w, double* M, int ld, const doub
   }
 }
 // M <- B(t)^T M = expK^T diag(e^{+sa s}) M   (mult_transB_from_left)
-__device__ void mult_transB_left(const WalkerDev& w, double* M, int ld, const double* dpos) {
+__device__ void mult_transB_left(const WalkerDev& w, double* M, int ld, const double* dpos,
+                                 const double* P = nullptr) {
   const int N = w.N;
   if (w.cb) {
-    cb_left(M, ld, N, w.L, 0, w.cbP, dpos, nullptr);  // scale rows, A then B
+    cb_left(M, ld, N, w.L, 0, w.cb_h, dpos, nullptr, P);  // scale rows, A then B
     __syncthreads();
-    cb_left(M, ld, N, w.L, 1, w.cbP, nullptr, nullptr);
+    cb_left(M, ld, N, w.L, 1, w.cb_h, nullptr, nullptr, P);
     __syncthreads();
   } else {
     const double* K = w.expK;  // (expK^T)(r,k) = expK(k,r)
@@ -280,30 +325,60 @@ __device__ void mult_transB_left(const WalkerDev& w, double* M, int ld, const do
 }
 
 // --------------------------------------------------------------------------
-// Fused equal-time measurement of one slice (measure_methods.cpp:22-255).
+// Fused equal-time measurement (measure_methods.cpp:22-255), split in two: measure_slice adds
+// one slice's sums into each thread's accumulators, measure_close reduces them over the CTA and
+// adds them to the walker's observables, once per launch.  The reduction of 8 FP64 values
+// costs a warp 40 adds of 64 cycles and thread 0 its divisions, more than a slice's sums at
+// small N.  Unordered pairs {i, j} are visited once (lanes over i, j = i + d mod N), with
+// X = G_ij G_ji summed over spins and the site's sums and differences of 1 - G_ii: 14 FP64
+// operations per pair against 13 per ordered pair for the sums written out.
 // gu/gd in shared memory (ld), sg the recorded sign of the slice.
 // --------------------------------------------------------------------------
+struct MeasureAcc {
+  // sign * sums: 0 trace, 1 double occupancy, 2 local spin, 3 kinetic, 4 n(k), 5 spin and
+  // 6 charge structure factor, 7 s-wave pairing; all times sg
+  double v[8];
+  double sg;      // the common factor, +1 or -1
+  double sign_sum;
+  int slices;
+};
+
+__device__ __forceinline__ void measure_open(MeasureAcc& m) {
+#pragma unroll
+  for (int k = 0; k < 8; ++k) m.v[k] = 0.0;
+  m.sg = 1.0;
+  m.sign_sum = 0.0;
+  m.slices = 0;
+}
+
+// scratch: 3N doubles
 __device__ void measure_slice(const WalkerDev& w, const double* gu, const double* gd, int ld, double sg,
-                              double* scratch /* 2N */, double* red) {
+                              double* scratch, MeasureAcc& m) {
   const int N = w.N, L = w.L, LL = L * L;
-  double* du = scratch;
-  double* dd = scratch + N;
+  double* ssum = scratch;       // (1 - gu_ii) + (1 - gd_ii)
+  double* sdif = scratch + N;   // (1 - gu_ii) - (1 - gd_ii)
+  double* ff = scratch + 2 * N;
   __shared__ signed char s_x[kMaxSmemN], s_y[kMaxSmemN], s_z[kMaxSmemN];
+  if (sg != m.sg) {
+#pragma unroll
+    for (int k = 0; k < 8; ++k) m.v[k] = -m.v[k];
+    m.sg = sg;
+  }
+  m.sign_sum += sg;
+  ++m.slices;
+  // one warp per 32 sites for the site sums
   for (int i = threadIdx.x; i < N; i += kThreads) {
-    du[i] = 1.0 - at(gu, ld, i, i);
-    dd[i] = 1.0 - at(gd, ld, i, i);
+    const double a = at(gu, ld, i, i), b = at(gd, ld, i, i);
+    const double du = 1.0 - a, dd = 1.0 - b, ab = a + b, n = du + dd, q = du - dd;
+    ssum[i] = n;
+    sdif[i] = q;
+    ff[i] = w.ff[i];
     s_x[i] = (signed char)(i % L);
     s_y[i] = (signed char)((i / L) % L);
     s_z[i] = (signed char)(i / LL);  // 0 on the square lattice
-  }
-  __syncthreads();
-  // v: 0 trace, 1 double occ, 2 local spin, 3 kinetic, 4 n(k), 5 common, 6 cross, 7 s-wave
-  double v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  for (int i = threadIdx.x; i < N; i += kThreads) {
-    const double a = at(gu, ld, i, i), b = at(gd, ld, i, i);
-    v[0] += a + b;
-    v[1] += du[i] * dd[i];
-    v[2] += a + b - 2 * a * b;
+    m.v[0] += ab;
+    m.v[1] = fma(du, dd, m.v[1]);
+    m.v[2] += fma(-2.0 * a, b, ab);
     // bonds to the +x, +y (, +z) neighbours (measure_methods.cpp:87-95)
     const int jx = site_nn(L, i, 0), jy = site_nn(L, i, 1);
     double kin = at(gu, ld, i, jx) + at(gd, ld, i, jx) + at(gu, ld, i, jy) + at(gd, ld, i, jy);
@@ -311,42 +386,143 @@ __device__ void measure_slice(const WalkerDev& w, const double* gu, const double
       const int jz = site_nn(L, i, 2);
       kin += at(gu, ld, i, jz) + at(gd, ld, i, jz);
     }
-    v[3] += kin;
+    m.v[3] += kin;
+    // the pair i = j (Fourier factor 1)
+    const double x = fma(du, a, dd * b);
+    m.v[4] += ab;
+    m.v[5] += fma(q, q, x);
+    m.v[6] += fma(n, n, x);
+    m.v[7] = fma(du, dd, m.v[7]);
   }
+  __syncthreads();
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  for (int j = wid; j < N; j += kThreads / 32)
-  for (int i = lane; i < N; i += 32) {
-    int dx = s_x[j] - s_x[i], dy = s_y[j] - s_y[i], dz = s_z[j] - s_z[i];
-    dx += (dx < 0) ? L : 0;
-    dy += (dy < 0) ? L : 0;
-    dz += (dz < 0) ? L : 0;
-    const double ff = w.ff[dx + dy * L + dz * LL];
-    const double gu_ij = at(gu, ld, i, j), gu_ji = at(gu, ld, j, i);
-    const double gd_ij = at(gd, ld, i, j), gd_ji = at(gd, ld, j, i);
-    const double dij = (i == j) ? 1.0 : 0.0;
-    const double guc_ij = dij - gu_ji, gdc_ij = dij - gd_ji;
-    v[4] += (gu_ji + gd_ji) * ff;
-    v[5] += ff * (du[i] * du[j] + guc_ij * gu_ij + dd[i] * dd[j] + gdc_ij * gd_ij);
-    v[6] += ff * (dd[i] * du[j] + du[i] * dd[j]);
-    v[7] += guc_ij * gdc_ij;
-  }
-  block_sum<8>(v, red);
-  if (threadIdx.x == 0) {
-    const double n = (double)N;
+  double p4 = 0.0, p5 = 0.0, p6 = 0.0;
+  for (int d = 1 + wid; 2 * d <= N; d += kThreads / 32)
+    for (int i = lane; i < ((2 * d == N) ? d : N); i += 32) {
+      const int j = (i + d < N) ? i + d : i + d - N;
+      // both displacements: on odd sides the momentum pi is not the lattice's and the table not even
+      const int dx = s_x[j] - s_x[i], dy = s_y[j] - s_y[i], dz = s_z[j] - s_z[i];
+      const double f_ij = ff[(dx + (dx < 0 ? L : 0)) + (dy + (dy < 0 ? L : 0)) * L + (dz + (dz < 0 ? L : 0)) * LL];
+      const double f_ji = ff[(-dx + (dx > 0 ? L : 0)) + (-dy + (dy > 0 ? L : 0)) * L + (-dz + (dz > 0 ? L : 0)) * LL];
+      const double f = f_ij + f_ji;
+      const double gu_ij = at(gu, ld, i, j), gu_ji = at(gu, ld, j, i);
+      const double gd_ij = at(gd, ld, i, j), gd_ji = at(gd, ld, j, i);
+      const double x = fma(gd_ij, gd_ji, gu_ij * gu_ji);
+      p4 = fma(f_ij, gu_ji + gd_ji, p4);
+      p4 = fma(f_ji, gu_ij + gd_ij, p4);
+      p5 = fma(f, fma(sdif[i], sdif[j], -x), p5);
+      p6 = fma(f, fma(ssum[i], ssum[j], -x), p6);
+      m.v[7] = fma(gu_ij, gd_ij, m.v[7]);
+      m.v[7] = fma(gu_ji, gd_ji, m.v[7]);
+    }
+  m.v[4] += p4;
+  m.v[5] += p5;
+  m.v[6] += p6;
+  __syncthreads();
+}
+
+__device__ void measure_close(const WalkerDev& w, MeasureAcc& m, double* red) {
+  block_sum<8>(m.v, red);
+  if (threadIdx.x == 0 && m.slices) {
+    const double n = (double)w.N, sn = m.sg / n, snn = sn / n;
     double* o = w.obs;
-    o[0] += sg * (2.0 - v[0] / n);
-    o[1] += sg * v[1] / n;
-    o[2] += sg * (2.0 * w.hop_t) * v[3] / n;
-    o[3] += sg * (1.0 - 0.5 * v[4] / n);
-    o[4] += sg * v[2] / n;
-    o[5] += sg * (v[5] - v[6]) / (n * n);
-    o[6] += sg * (v[5] + v[6]) / (n * n);
-    o[7] += sg * v[7] / n;
-    o[8] += sg;
-    for (int k = 0; k < kNumObs; ++k) w.obs_cnt[k] += 1;
+    o[0] += 2.0 * m.sign_sum - m.v[0] * sn;
+    o[1] += m.v[1] * sn;
+    o[2] += (2.0 * w.hop_t) * (m.v[3] * sn);
+    o[3] += m.sign_sum - 0.5 * (m.v[4] * sn);
+    o[4] += m.v[2] * sn;
+    o[5] += m.v[5] * snn;
+    o[6] += m.v[6] * snn;
+    o[7] += m.v[7] * sn;
+    o[8] += m.sign_sum;
+    for (int k = 0; k < kNumObs; ++k) w.obs_cnt[k] += m.slices;
   }
   __syncthreads();
 }
+
+// --------------------------------------------------------------------------
+// Metropolis decisions of one warp.  The lanes evaluate the ratios of a window of sites at once
+// (both spins of 16 sites when the spins differ, 32 sites otherwise); the lowest accepted site is
+// the next accept of the sequential visit, since every site before it saw the same diagonal.  An
+// FP64 instruction holds the warp 64 cycles for one lane or for 32, so a window costs what one
+// site costs, and each spin's factor 1 + (1 - G_ii) Delta and its division Delta / factor share
+// an instruction.  The uniform is compared through its bit pattern: u < min(1, |r|) is u < |r|
+// for u in [0, 1), and doubles of one sign order as integers (a NaN ratio accepts, as fmin does).
+// What bounds an accept at N = 16 (2700 cycles) is this chain: 5 dependent FP64 operations and the
+// division (9 more) at 64 cycles each, 2100 cycles with its shared-memory and shuffle latencies
+// beside the update's FMAs.  One thread visiting the sites in turn, with the Philox rounds and
+// the descriptor's loads in the chain, made a pass of 4 x 4, beta = 4 take 11.0 ms, this 8.1 ms
+// (with measure_slice, flat_gemm and the shared-memory chain); 256 walkers of 8 x 8 240 -> 208 ms.
+// --------------------------------------------------------------------------
+struct SiteScan {
+  static constexpr int kWin = 4;  // windows that cover N <= 64
+  int S, width, sp, dl;           // spins, sites per window, this lane's spin and site in the window
+  double c[2], e2[2];             // Delta of this lane's spin and exp(2 alpha s), by field s = +1, -1
+
+  __device__ __forceinline__ SiteScan(const WalkerDev& w, int lane) {
+    S = w.S;
+    width = (S == 2) ? 16 : 32;
+    sp = (S == 2) ? lane >> 4 : 0;
+    dl = lane & (width - 1);
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      c[k] = (w.model == 0 && sp == 1) ? w.cp[k] : w.cm[k];
+      e2[k] = w.ex2[k];
+    }
+  }
+  // the diagonal elements of the windows from site `from`
+  __device__ __forceinline__ void load_diag(double (&dg)[kWin], double* const* G, int ld, int from, int N) const {
+#pragma unroll
+    for (int b = 0; b < kWin; ++b) {
+      const int l = from + b * width + dl;
+      dg[b] = (l < N) ? at(G[sp], ld, l, l) : 0.0;
+    }
+  }
+  // The next accepted site from `from` on (N: none) on the diagonal dg, after the pending update
+  // of vec (u [2][N], w [2][N]; null: none); flips the field and leaves the update's factors in
+  // f[2].  The whole warp calls; sign and accepts are uniform in it.
+  __device__ __forceinline__ int next(const WalkerDev& w, const double (&dg)[kWin], const double* vec, int from, int N,
+                                      const double* uni, int8_t* field, double* f, double& sign,
+                                      long long& accepts) const {
+#pragma unroll
+    for (int b = 0; b < kWin; ++b) {
+      const int base = from + b * width;
+      if (base >= N) break;
+      const int l = base + dl;
+      const bool in = l < N;
+      double g = dg[b];
+      if (vec && in) g = fma(-vec[(2 + sp) * N + l], vec[sp * N + l], g);
+      const int s = in ? field[l] : 1;
+      const double ck = s > 0 ? c[0] : c[1];
+      const double qs = __dadd_rn(1.0, __dmul_rn(__dsub_rn(1.0, g), ck));
+      const double fq = __ddiv_rn(ck, qs);  // beside the acceptance, not after it
+      // reference operation order (flip_ratio)
+      const double r = (S == 2) ? __dmul_rn(qs, __shfl_xor_sync(0xffffffffu, qs, 16))
+                                : __dmul_rn(__dmul_rn(s > 0 ? e2[0] : e2[1], qs), qs);
+      const long long rb = __double_as_longlong(r), ab = rb & 0x7fffffffffffffffLL;
+      const bool acc = in && __double_as_longlong(in ? uni[l] : 0.0) < ab;
+      const unsigned mask = __ballot_sync(0xffffffffu, acc) & (S == 2 ? 0xffffu : 0xffffffffu);
+      const int first = mask ? __ffs(mask) - 1 : 32;
+      if (in && dl <= first && ab >= 0x7ff0000000000000LL) atomicOr(w.status, ST_NONFINITE_RATIO);
+      if (mask) {
+        if (dl == first) {
+          f[sp] = fq;
+          if (S == 1) f[1] = fq;
+          if (sp == 0) field[l] = (int8_t)(-s);
+        }
+        const long long rf = __shfl_sync(0xffffffffu, rb, first);
+        // r >= 0 (false for a NaN)
+        if (!((rf >= 0 && rf <= 0x7ff0000000000000LL) || rf == (long long)0x8000000000000000ULL)) sign = -sign;
+        ++accepts;
+        return base + first;
+      }
+    }
+    return N;
+  }
+};
+
+// shared memory of the segment kernel with the chain beside G: two CTAs still share an SM up to N = 50
+__host__ __device__ inline bool segment_chain_smem(int maxN) { return maxN <= 50; }
 
 // --------------------------------------------------------------------------
 // Segment kernel: the slices of one stabilization interval for one walker.
@@ -358,7 +534,8 @@ __device__ void measure_slice(const WalkerDev& w, const double* gu, const double
 // column by column, the scale-separated order svd_stack.cpp:51 asks for.
 // --------------------------------------------------------------------------
 template <int MODE>
-__global__ void __launch_bounds__(kThreads) segment_kernel(const WalkerDev* __restrict__ W, int j, int measure) {
+__global__ void __launch_bounds__(kThreads, 2) segment_kernel(const WalkerDev* __restrict__ W, int j, int measure,
+                                                           int maxN) {
   const WalkerDev& w = W[blockIdx.x];
   if (j >= w.nstack || w.path != 0) return;
   extern __shared__ double smem[];
@@ -369,11 +546,15 @@ __global__ void __launch_bounds__(kThreads) segment_kernel(const WalkerDev* __re
   double* vec = smem + (long long)S * N * ld;  // ucol[2][N], wrow[2][N]
   double* dtab = vec + 4 * N;                   // [2 spins][2 (pos,neg)][N]
   double* red = dtab + 4 * N;                   // 64
-  double* scratch = red + 64;                   // 2N
+  double* scratch = red + 64;                   // 3N
+  // the running chain lives beside G in shared memory where that leaves room for two CTAs an SM
+  const bool chain_smem = segment_chain_smem(maxN);
+  double* Cs = scratch + 3 * N;
+  const int ldc = chain_smem ? ld : N;
   __shared__ int s_next;
-  __shared__ double s_f[2];
+  __shared__ double s_f[2], s_sign;
   __shared__ int8_t s_field[kMaxSmemN];
-  __shared__ double diag_pre[2 * kMaxSmemN];
+  __shared__ double s_uni[kMaxSmemN];
 
   const int k = (MODE == MODE_FWD) ? j : (w.nstack - 1 - j);
   const int t_lo = k * p + 1, t_hi = min((k + 1) * p, Lt);
@@ -383,12 +564,12 @@ __global__ void __launch_bounds__(kThreads) segment_kernel(const WalkerDev* __re
   constexpr int nwarp = kThreads / 32;
   // chain <- U_top diag(D_top)  or  I
   for (int sp = 0; sp < S; ++sp) {
-    double* C = w.chain + (long long)sp * N * N;
+    double* C = chain_smem ? Cs + (long long)sp * N * ld : w.chain + (long long)sp * N * N;
     const double* lv = (j == 0) ? nullptr : stack_level(w, side, sp, j - 1);
     for (int c = wid; c < N; c += nwarp) {
       const double dc = lv ? lv[2LL * N * N + c] : 1.0;
       for (int r = lane; r < N; r += 32)
-        C[(long long)c * N + r] = lv ? lv[(long long)c * N + r] * dc : ((r == c) ? 1.0 : 0.0);
+        C[(long long)c * ldc + r] = lv ? lv[(long long)c * N + r] * dc : ((r == c) ? 1.0 : 0.0);
     }
   }
   if (MODE != MODE_INIT) {
@@ -400,22 +581,30 @@ __global__ void __launch_bounds__(kThreads) segment_kernel(const WalkerDev* __re
   }
   __syncthreads();
 
-  double sign = *w.sign;
+  double sign = *w.sign;  // warp 0 keeps it current
   long long acc_count = 0;
   const unsigned long long sweep = (w.rng == 1) ? *w.sweep_ctr : 0ULL;
   const int nsl = t_hi - t_lo + 1;
+  MeasureAcc meas;
+  measure_open(meas);
+  const SiteScan scan(w, lane);
   for (int q = 0; q < nsl; ++q) {
     const int t = (MODE == MODE_FWD) ? t_lo + q : t_hi - q;
     const int eff = t - 1;  // 1 <= t <= Lt
     const int8_t* frow = w.fields + (long long)eff * N;
-    for (int i = threadIdx.x; i < N; i += kThreads) s_field[i] = frow[i];
+    for (int i = threadIdx.x; i < N; i += kThreads) {
+      s_field[i] = frow[i];
+      if (MODE != MODE_INIT)
+        s_uni[i] = (w.rng == 0) ? w.uni[(MODE == MODE_FWD) ? (eff * N + i) : ((Lt - t) * N + i)]
+                                : philox_uniform(w.seed, (unsigned)w.widx, sweep, (unsigned)(eff * N + i));
+    }
     __syncthreads();
     // scale tables for this slice: dtab[sp][0][i] = e^{+sa s_i}, dtab[sp][1][i] = e^{-sa s_i}
     for (int e = threadIdx.x; e < S * N; e += kThreads) {
       const int sp = e / N, i = e % N;
       const int ss = spin_sign(w, sp) * (int)s_field[i];
-      dtab[(sp * 2 + 0) * N + i] = bdiag(w, ss);
-      dtab[(sp * 2 + 1) * N + i] = bdiag(w, -ss);
+      dtab[(sp * 2 + 0) * N + i] = bdiag(w, ss, 0, MODE != MODE_INIT);
+      dtab[(sp * 2 + 1) * N + i] = bdiag(w, -ss, 1, MODE != MODE_INIT);
     }
     __syncthreads();
 
@@ -427,76 +616,54 @@ __global__ void __launch_bounds__(kThreads) segment_kernel(const WalkerDev* __re
     }
 
     if (MODE != MODE_INIT) {
-      // Metropolis over sites i = 0..N-1 (dqmc_walker.cpp:173-197).
-      // Warp 0 decides; warps 1.. apply the rank-1 update of the last accepted
-      // site meanwhile.  Sites rejected in between leave G unchanged, so the
-      // decision thread scans ahead with the diagonal the pending update will
-      // produce, computed with the same fma the update uses (bit-identical).
-      auto decide_from = [&](int i0, bool pending) {
-        // returns the next accepted site (or N); thread 0 only
-        for (int i = i0; i < N; ++i) {
-          const int s = s_field[i];
-          const int si = s > 0 ? 0 : 1;
-          double gu, gd;
-          if (pending) {
-            gu = fma(-vec[(2 + 0) * N + i], vec[0 * N + i], diag_pre[i]);
-            gd = (S == 2) ? fma(-vec[(2 + 1) * N + i], vec[1 * N + i], diag_pre[N + i]) : gu;
-          } else {
-            gu = at(Gs[0], ld, i, i);
-            gd = at(Gs[1], ld, i, i);
-          }
-          const FlipRatio q = flip_ratio(w, si, gu, gd);  // reference operation order
-          const double r = q.r;
-          const int attempt = (MODE == MODE_FWD) ? (eff * N + i) : ((Lt - t) * N + i);
-          const double u = (w.rng == 0) ? w.uni[attempt]
-                                        : philox_uniform(w.seed, (unsigned)w.widx, sweep, (unsigned)(eff * N + i));
-          const double prob = fmin(1.0, fabs(r));
-          if (!isfinite(r)) atomicOr(w.status, ST_NONFINITE_RATIO);
-          if (u < prob) {
-            flip_factors(w, q, s_f);
-            s_field[i] = (int8_t)(-s);
-            sign = (r >= 0) ? sign : -sign;
-            ++acc_count;
-            return i;
-          }
-        }
-        return N;
-      };
-      if (threadIdx.x == 0) s_next = decide_from(0, false);
+      // Metropolis over sites i = 0..N-1 (dqmc_walker.cpp:173-197), two barriers per accept.
+      // After the first, warps 1 .. 2S form the update's vectors u = f G(:, i) and
+      // w = e_i - G(i, :)^T and warp 0 reads the diagonal as it stands; after the second,
+      // warp 0 scans the sites past i for the next accept while warps 1 .. 7 apply the rank-1
+      // update.  The scan uses the diagonal that the pending update will produce, computed with
+      // the same fma the update uses (bit-identical).
+      double dg[SiteScan::kWin];
+      if (wid == 0) {
+        scan.load_diag(dg, Gs, ld, 0, N);
+        const int nx = scan.next(w, dg, nullptr, 0, N, s_uni, s_field, s_f, sign, acc_count);
+        if (lane == 0) s_next = nx;
+      }
       __syncthreads();
-      while (s_next < N) {
+      while (true) {
         const int i = s_next;
-        // vectors of site i from the fully updated G, and the diagonal before its update
-        if (threadIdx.x < N) {
-          const int r = threadIdx.x;
-          for (int sp = 0; sp < S; ++sp) {
-            const double* g = Gs[sp];
-            vec[sp * N + r] = s_f[sp] * at(g, ld, r, i);                       // f u
-            vec[(2 + sp) * N + r] = ((r == i) ? 1.0 : 0.0) - at(g, ld, i, r);  // e_i - G(i,:)
-            diag_pre[sp * N + r] = at(g, ld, r, r);
-          }
+        if (i >= N) break;
+        if (wid == 0) {
+          scan.load_diag(dg, Gs, ld, i + 1, N);
+        } else if (wid <= 2 * S) {
+          const int sp = (wid - 1) % S, role = (wid - 1) / S;
+          const double* g = Gs[sp];
+          double* o = vec + (2 * role + sp) * N;
+          const double f = s_f[sp];
+          for (int r = lane; r < N; r += 32)
+            o[r] = role ? ((r == i) ? 1.0 : 0.0) - at(g, ld, i, r)  // e_i - G(i,:)
+                        : f * at(g, ld, r, i);                      // f u
         }
         __syncthreads();
-        if (threadIdx.x < 32) {
-          if (threadIdx.x == 0) s_next = decide_from(i + 1, true);
+        if (wid == 0) {
+          const int nx = scan.next(w, dg, vec, i + 1, N, s_uni, s_field, s_f, sign, acc_count);
+          if (lane == 0) s_next = nx;
         } else {
-          // warps 1..7: column c per warp, rows lane and lane+32 per lane
-          const int lane = threadIdx.x & 31, uw = (threadIdx.x >> 5) - 1;
-          const int r0 = lane, r1 = lane + 32;
-          for (int sp = 0; sp < S; ++sp) {
+          // warps 1..7: the S N columns in turn, rows lane and lane + 32 (N <= 16: two columns
+          // at a time, 16 lanes each)
+          const int per = (N <= 16) ? 2 : 1;
+          const int sub = (per == 2) ? lane >> 4 : 0, r0 = (per == 2) ? lane & 15 : lane, r1 = lane + 32;
+          for (int qc = (wid - 1) * per + sub; qc < S * N; qc += per * (nwarp - 1)) {
+            const int sp = (qc >= N) ? 1 : 0, c = qc - sp * N;
             double* g = Gs[sp];
-            const double* wv = vec + (2 + sp) * N;
-            const double u0 = (r0 < N) ? vec[sp * N + r0] : 0.0;
-            const double u1 = (r1 < N) ? vec[sp * N + r1] : 0.0;
-            for (int c = uw; c < N; c += kThreads / 32 - 1) {
-              const double wc = -wv[c];
-              if (r0 < N) at(g, ld, r0, c) = fma(wc, u0, at(g, ld, r0, c));
-              if (r1 < N) at(g, ld, r1, c) = fma(wc, u1, at(g, ld, r1, c));
-            }
+            const double* u = vec + sp * N;
+            const double wc = -vec[(2 + sp) * N + c];
+            if (r0 < N) at(g, ld, r0, c) = fma(wc, u[r0], at(g, ld, r0, c));
+            if (per == 1 && r1 < N) at(g, ld, r1, c) = fma(wc, u[r1], at(g, ld, r1, c));
           }
         }
         __syncthreads();
       }
+      if (threadIdx.x == 0) s_sign = sign;
       // write back the flipped fields of this slice
       int8_t* frw = w.fields + (long long)eff * N;
       for (int i = threadIdx.x; i < N; i += kThreads) frw[i] = s_field[i];
@@ -504,8 +671,8 @@ __global__ void __launch_bounds__(kThreads) segment_kernel(const WalkerDev* __re
       for (int e = threadIdx.x; e < S * N; e += kThreads) {
         const int sp = e / N, i = e % N;
         const int ss = spin_sign(w, sp) * (int)s_field[i];
-        dtab[(sp * 2 + 0) * N + i] = bdiag(w, ss);
-        dtab[(sp * 2 + 1) * N + i] = bdiag(w, -ss);
+        dtab[(sp * 2 + 0) * N + i] = bdiag(w, ss, 0, MODE != MODE_INIT);
+        dtab[(sp * 2 + 1) * N + i] = bdiag(w, -ss, 1, MODE != MODE_INIT);
       }
       __syncthreads();
 
@@ -514,16 +681,16 @@ __global__ void __launch_bounds__(kThreads) segment_kernel(const WalkerDev* __re
       // their stabilization, dqmc_walker.cpp:307-310 and :408-411)
       if (measure) {
         const bool here = (MODE == MODE_FWD) ? (t != t_hi) : (t != Lt);
-        if (here) measure_slice(w, Gs[0], Gs[1], ld, sign, scratch, red);
+        if (here) measure_slice(w, Gs[0], Gs[1], ld, s_sign, scratch, meas);
       }
       if (MODE == MODE_BWD && t == Lt && threadIdx.x == 0) *w.sign_Lt = sign;
     }
 
     // B-chain of the stabilization interval
     for (int sp = 0; sp < S; ++sp) {
-      double* C = w.chain + (long long)sp * N * N;
-      if (MODE == MODE_FWD) mult_B_left(w, C, N, dtab + (sp * 2 + 0) * N);
-      else mult_transB_left(w, C, N, dtab + (sp * 2 + 0) * N);
+      double* C = chain_smem ? Cs + (long long)sp * N * ld : w.chain + (long long)sp * N * N;
+      if (MODE == MODE_FWD) mult_B_left(w, C, ldc, dtab + (sp * 2 + 0) * N);
+      else mult_transB_left(w, C, ldc, dtab + (sp * 2 + 0) * N, MODE == MODE_INIT ? w.cbP : nullptr);
     }
 
     if (MODE == MODE_BWD) {  // wrap_from_beta_to_0(t): G <- B(t)^-1 G B(t)
@@ -535,12 +702,19 @@ __global__ void __launch_bounds__(kThreads) segment_kernel(const WalkerDev* __re
     __syncthreads();
   }
 
+  if (chain_smem)
+    for (int sp = 0; sp < S; ++sp) {
+      double* C = w.chain + (long long)sp * N * N;
+      for (int c = wid; c < N; c += nwarp)
+        for (int r = lane; r < N; r += 32) C[(long long)c * N + r] = at(Cs + (long long)sp * N * ld, ld, r, c);
+    }
   if (MODE != MODE_INIT) {
     for (int sp = 0; sp < S; ++sp) {
       double* Gg = w.G + (long long)sp * N * N;
       for (int c = wid; c < N; c += nwarp)
         for (int r = lane; r < N; r += 32) Gg[(long long)c * N + r] = at(Gs[sp], ld, r, c);
     }
+    if (measure) measure_close(w, meas, red);
     if (threadIdx.x == 0) {
       *w.sign = sign;
       *w.accepts += acc_count;
@@ -846,7 +1020,7 @@ __device__ bool lu_solve_smem(double* M, double* Y, int N, int ld, double* red) 
 //   left  empty (t = 0):  G = [same of the right stack]^T
 // Also the wrap error max|G_fresh - G| (matrix_compare_error, :34-47) and the trace.
 // --------------------------------------------------------------------------
-__global__ void __launch_bounds__(kThreads) greens_kernel(const WalkerDev* __restrict__ W, int mode, int j,
+__global__ void __launch_bounds__(kThreads, 2) greens_kernel(const WalkerDev* __restrict__ W, int mode, int j,
                                                           int check_error, int trace_slot) {
   const int wi = blockIdx.x >> 1, sp = blockIdx.x & 1;
   const WalkerDev& w = W[wi];
@@ -984,7 +1158,10 @@ __global__ void __launch_bounds__(kThreads) measure_kernel(const WalkerDev* __re
   }
   __syncthreads();
   const double sg = (mode == MODE_BWD) ? *w.sign_Lt : *w.sign;
-  measure_slice(w, gu, gd, ld, sg, scratch, red);
+  MeasureAcc meas;
+  measure_open(meas);
+  measure_slice(w, gu, gd, ld, sg, scratch, meas);
+  measure_close(w, meas, red);
 }
 
 // sign(det G_up det G_dn) (dqmc_walker.cpp:150-163) via in-SMEM LU.
@@ -1117,13 +1294,16 @@ double run_fp64_probe(cudaError_t* err) {
 // --------------------------------------------------------------------------
 // host-side launch helpers
 // --------------------------------------------------------------------------
-size_t segment_smem_bytes(int N, int S) { return sizeof(double) * ((size_t)S * N * (N + 1) + 8 * N + 64 + 2 * N); }
+size_t segment_smem_bytes(int N, int S) {
+  return sizeof(double) * ((size_t)S * N * (N + 1) * (segment_chain_smem(N) ? 2 : 1) + 8 * N + 64 + 3 * N);
+}
 size_t push_smem_bytes(int N) { return sizeof(double) * ((size_t)N * (N + 1) + 4 * N) + sizeof(int) * N; }
 size_t greens_smem_bytes(int N) { return sizeof(double) * (2 * (size_t)N * (N + 1) + 4 * N + 64); }
-size_t measure_smem_bytes(int N) { return sizeof(double) * (2 * (size_t)N * (N + 1) + 64 + 2 * N); }
+size_t measure_smem_bytes(int N) { return sizeof(double) * (2 * (size_t)N * (N + 1) + 64 + 3 * N); }
 
 cudaError_t configure_fp64_kernels(int maxN) {
-  const size_t s1 = segment_smem_bytes(maxN, 2), s2 = push_smem_bytes(maxN), s3 = greens_smem_bytes(maxN),
+  // the largest of both placements of the chain
+  const size_t s1 = std::max(segment_smem_bytes(maxN, 2), segment_smem_bytes(50, 2)), s2 = push_smem_bytes(maxN), s3 = greens_smem_bytes(maxN),
                s4 = measure_smem_bytes(maxN);
   cudaError_t e;
   if ((e = cudaFuncSetAttribute(segment_kernel<MODE_INIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s1))) return e;
@@ -1140,9 +1320,9 @@ cudaError_t configure_fp64_kernels(int maxN) {
 
 void launch_segment(int mode, const WalkerDev* W, int nw, int j, int measure, int maxN, cudaStream_t st) {
   const size_t sm = segment_smem_bytes(maxN, 2);
-  if (mode == MODE_INIT) segment_kernel<MODE_INIT><<<nw, kThreads, sm, st>>>(W, j, 0);
-  else if (mode == MODE_FWD) segment_kernel<MODE_FWD><<<nw, kThreads, sm, st>>>(W, j, measure);
-  else segment_kernel<MODE_BWD><<<nw, kThreads, sm, st>>>(W, j, measure);
+  if (mode == MODE_INIT) segment_kernel<MODE_INIT><<<nw, kThreads, sm, st>>>(W, j, 0, maxN);
+  else if (mode == MODE_FWD) segment_kernel<MODE_FWD><<<nw, kThreads, sm, st>>>(W, j, measure, maxN);
+  else segment_kernel<MODE_BWD><<<nw, kThreads, sm, st>>>(W, j, measure, maxN);
 }
 void launch_push(int mode, const WalkerDev* W, int nw, int j, int maxN, cudaStream_t st) {
   const size_t sm = push_smem_bytes(maxN);
