@@ -160,6 +160,86 @@ __device__ __forceinline__ void flip_factors(const WalkerDev& w, const FlipRatio
   f[1] = (w.model == 0) ? __ddiv_rn(q.cd, q.rd) : f[0];
 }
 
+// Metropolis decisions of one warp.  The lanes evaluate the ratios of a window of sites at once
+// (both spins of 16 sites when the spins differ, 32 sites otherwise); the lowest accepted site is
+// the next accept of the sequential visit, since every site before it saw the same diagonal.  An
+// FP64 instruction holds the warp 64 cycles for one lane or for 32, so a window costs what one
+// site costs, and each spin's factor 1 + (1 - G_ii) Delta and its division Delta / factor share
+// an instruction.  The uniform is compared through its bit pattern: u < min(1, |r|) is u < |r|
+// for u in [0, 1), and doubles of one sign order as integers (a NaN ratio accepts, as fmin does).
+// What bounds an accept at N = 16 (2700 cycles) is this chain: 5 dependent FP64 operations and the
+// division (9 more) at 64 cycles each, 2100 cycles with its shared-memory and shuffle latencies
+// beside the update's FMAs.  One thread visiting the sites in turn, with the Philox rounds and
+// the descriptor's loads in the chain, made a pass of 4 x 4, beta = 4 take 11.0 ms, this 8.1 ms
+// (with measure_slice, flat_gemm and the shared-memory chain); 256 walkers of 8 x 8 240 -> 208 ms.
+struct SiteScan {
+  int S, width, sp, dl;           // spins, sites per window, this lane's spin and site in the window
+  double c[2], e2[2];             // Delta of this lane's spin and exp(2 alpha s), by field s = +1, -1
+
+  __device__ __forceinline__ SiteScan(const WalkerDev& w, int lane) {
+    S = w.S;
+    width = (S == 2) ? 16 : 32;
+    sp = (S == 2) ? lane >> 4 : 0;
+    dl = lane & (width - 1);
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      c[k] = (w.model == 0 && sp == 1) ? w.cp[k] : w.cm[k];
+      e2[k] = w.ex2[k];
+    }
+  }
+  // the diagonal elements of NW windows from site `from` of this lane's spin's matrix
+  template <int NW>
+  __device__ __forceinline__ void load_diag(double (&dg)[NW], const double* G, int ld, int from, int N) const {
+#pragma unroll
+    for (int b = 0; b < NW; ++b) {
+      const int l = from + b * width + dl;
+      dg[b] = (l < N) ? G[l * (ld + 1)] : 0.0;
+    }
+  }
+  // The next accepted site from `from` on (N: none; NW windows reach N) on the diagonal dg, after
+  // the pending update of this lane's spin (u, wv by site; null: none); flips the field and leaves
+  // the update's factors in f[2].  The whole warp calls; sign and accepts are uniform in it.
+  template <int NW>
+  __device__ __forceinline__ int next(const WalkerDev& w, const double (&dg)[NW], const double* u, const double* wv,
+                                      int from, int N, const double* uni, int8_t* field, double* f, double& sign,
+                                      long long& accepts) const {
+#pragma unroll
+    for (int b = 0; b < NW; ++b) {
+      const int base = from + b * width;
+      if (base >= N) break;
+      const int l = base + dl;
+      const bool in = l < N;
+      double g = dg[b];
+      if (u && in) g = fma(-wv[l], u[l], g);
+      const int s = in ? field[l] : 1;
+      const double ck = s > 0 ? c[0] : c[1];
+      const double qs = __dadd_rn(1.0, __dmul_rn(__dsub_rn(1.0, g), ck));
+      const double fq = __ddiv_rn(ck, qs);  // beside the acceptance, not after it
+      // reference operation order (flip_ratio)
+      const double r = (S == 2) ? __dmul_rn(qs, __shfl_xor_sync(0xffffffffu, qs, 16))
+                                : __dmul_rn(__dmul_rn(s > 0 ? e2[0] : e2[1], qs), qs);
+      const long long rb = __double_as_longlong(r), ab = rb & 0x7fffffffffffffffLL;
+      const bool acc = in && __double_as_longlong(in ? uni[l] : 0.0) < ab;
+      const unsigned mask = __ballot_sync(0xffffffffu, acc) & (S == 2 ? 0xffffu : 0xffffffffu);
+      const int first = mask ? __ffs(mask) - 1 : 32;
+      if (in && dl <= first && ab >= 0x7ff0000000000000LL) atomicOr(w.status, ST_NONFINITE_RATIO);
+      if (mask) {
+        if (dl == first) {
+          f[sp] = fq;
+          if (S == 1) f[1] = fq;
+          if (sp == 0) field[l] = (int8_t)(-s);
+        }
+        const long long rf = __shfl_sync(0xffffffffu, rb, first);
+        // r >= 0 (false for a NaN)
+        if (!((rf >= 0 && rf <= 0x7ff0000000000000LL) || rf == (long long)0x8000000000000000ULL)) sign = -sign;
+        ++accepts;
+        return base + first;
+      }
+    }
+    return N;
+  }
+};
+
 // Site i of a walker's lattice is x + L y (+ L^2 z).  The displacement from site i to site j
 // as the site index of its vector, each component mod L (src/lattice/square.cpp:88-105,
 // src/lattice/cubic.cpp:112-132), and the neighbour of site i in direction +x, +y or +z.

@@ -441,86 +441,6 @@ __device__ void measure_close(const WalkerDev& w, MeasureAcc& m, double* red) {
 }
 
 // --------------------------------------------------------------------------
-// Metropolis decisions of one warp.  The lanes evaluate the ratios of a window of sites at once
-// (both spins of 16 sites when the spins differ, 32 sites otherwise); the lowest accepted site is
-// the next accept of the sequential visit, since every site before it saw the same diagonal.  An
-// FP64 instruction holds the warp 64 cycles for one lane or for 32, so a window costs what one
-// site costs, and each spin's factor 1 + (1 - G_ii) Delta and its division Delta / factor share
-// an instruction.  The uniform is compared through its bit pattern: u < min(1, |r|) is u < |r|
-// for u in [0, 1), and doubles of one sign order as integers (a NaN ratio accepts, as fmin does).
-// What bounds an accept at N = 16 (2700 cycles) is this chain: 5 dependent FP64 operations and the
-// division (9 more) at 64 cycles each, 2100 cycles with its shared-memory and shuffle latencies
-// beside the update's FMAs.  One thread visiting the sites in turn, with the Philox rounds and
-// the descriptor's loads in the chain, made a pass of 4 x 4, beta = 4 take 11.0 ms, this 8.1 ms
-// (with measure_slice, flat_gemm and the shared-memory chain); 256 walkers of 8 x 8 240 -> 208 ms.
-// --------------------------------------------------------------------------
-struct SiteScan {
-  static constexpr int kWin = 4;  // windows that cover N <= 64
-  int S, width, sp, dl;           // spins, sites per window, this lane's spin and site in the window
-  double c[2], e2[2];             // Delta of this lane's spin and exp(2 alpha s), by field s = +1, -1
-
-  __device__ __forceinline__ SiteScan(const WalkerDev& w, int lane) {
-    S = w.S;
-    width = (S == 2) ? 16 : 32;
-    sp = (S == 2) ? lane >> 4 : 0;
-    dl = lane & (width - 1);
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      c[k] = (w.model == 0 && sp == 1) ? w.cp[k] : w.cm[k];
-      e2[k] = w.ex2[k];
-    }
-  }
-  // the diagonal elements of the windows from site `from`
-  __device__ __forceinline__ void load_diag(double (&dg)[kWin], double* const* G, int ld, int from, int N) const {
-#pragma unroll
-    for (int b = 0; b < kWin; ++b) {
-      const int l = from + b * width + dl;
-      dg[b] = (l < N) ? at(G[sp], ld, l, l) : 0.0;
-    }
-  }
-  // The next accepted site from `from` on (N: none) on the diagonal dg, after the pending update
-  // of vec (u [2][N], w [2][N]; null: none); flips the field and leaves the update's factors in
-  // f[2].  The whole warp calls; sign and accepts are uniform in it.
-  __device__ __forceinline__ int next(const WalkerDev& w, const double (&dg)[kWin], const double* vec, int from, int N,
-                                      const double* uni, int8_t* field, double* f, double& sign,
-                                      long long& accepts) const {
-#pragma unroll
-    for (int b = 0; b < kWin; ++b) {
-      const int base = from + b * width;
-      if (base >= N) break;
-      const int l = base + dl;
-      const bool in = l < N;
-      double g = dg[b];
-      if (vec && in) g = fma(-vec[(2 + sp) * N + l], vec[sp * N + l], g);
-      const int s = in ? field[l] : 1;
-      const double ck = s > 0 ? c[0] : c[1];
-      const double qs = __dadd_rn(1.0, __dmul_rn(__dsub_rn(1.0, g), ck));
-      const double fq = __ddiv_rn(ck, qs);  // beside the acceptance, not after it
-      // reference operation order (flip_ratio)
-      const double r = (S == 2) ? __dmul_rn(qs, __shfl_xor_sync(0xffffffffu, qs, 16))
-                                : __dmul_rn(__dmul_rn(s > 0 ? e2[0] : e2[1], qs), qs);
-      const long long rb = __double_as_longlong(r), ab = rb & 0x7fffffffffffffffLL;
-      const bool acc = in && __double_as_longlong(in ? uni[l] : 0.0) < ab;
-      const unsigned mask = __ballot_sync(0xffffffffu, acc) & (S == 2 ? 0xffffu : 0xffffffffu);
-      const int first = mask ? __ffs(mask) - 1 : 32;
-      if (in && dl <= first && ab >= 0x7ff0000000000000LL) atomicOr(w.status, ST_NONFINITE_RATIO);
-      if (mask) {
-        if (dl == first) {
-          f[sp] = fq;
-          if (S == 1) f[1] = fq;
-          if (sp == 0) field[l] = (int8_t)(-s);
-        }
-        const long long rf = __shfl_sync(0xffffffffu, rb, first);
-        // r >= 0 (false for a NaN)
-        if (!((rf >= 0 && rf <= 0x7ff0000000000000LL) || rf == (long long)0x8000000000000000ULL)) sign = -sign;
-        ++accepts;
-        return base + first;
-      }
-    }
-    return N;
-  }
-};
-
 // shared memory of the segment kernel with the chain beside G: two CTAs still share an SM up to N = 50
 __host__ __device__ inline bool segment_chain_smem(int maxN) { return maxN <= 50; }
 
@@ -622,10 +542,12 @@ __global__ void __launch_bounds__(kThreads, 2) segment_kernel(const WalkerDev* _
       // warp 0 scans the sites past i for the next accept while warps 1 .. 7 apply the rank-1
       // update.  The scan uses the diagonal that the pending update will produce, computed with
       // the same fma the update uses (bit-identical).
-      double dg[SiteScan::kWin];
+      double dg[4];  // windows of 16 sites that cover N <= 64
+      const double* su = vec + scan.sp * N;
+      const double* sw = vec + (2 + scan.sp) * N;
       if (wid == 0) {
-        scan.load_diag(dg, Gs, ld, 0, N);
-        const int nx = scan.next(w, dg, nullptr, 0, N, s_uni, s_field, s_f, sign, acc_count);
+        scan.load_diag(dg, Gs[scan.sp], ld, 0, N);
+        const int nx = scan.next(w, dg, nullptr, nullptr, 0, N, s_uni, s_field, s_f, sign, acc_count);
         if (lane == 0) s_next = nx;
       }
       __syncthreads();
@@ -633,7 +555,7 @@ __global__ void __launch_bounds__(kThreads, 2) segment_kernel(const WalkerDev* _
         const int i = s_next;
         if (i >= N) break;
         if (wid == 0) {
-          scan.load_diag(dg, Gs, ld, i + 1, N);
+          scan.load_diag(dg, Gs[scan.sp], ld, i + 1, N);
         } else if (wid <= 2 * S) {
           const int sp = (wid - 1) % S, role = (wid - 1) / S;
           const double* g = Gs[sp];
@@ -645,7 +567,7 @@ __global__ void __launch_bounds__(kThreads, 2) segment_kernel(const WalkerDev* _
         }
         __syncthreads();
         if (wid == 0) {
-          const int nx = scan.next(w, dg, vec, i + 1, N, s_uni, s_field, s_f, sign, acc_count);
+          const int nx = scan.next(w, dg, su, sw, i + 1, N, s_uni, s_field, s_f, sign, acc_count);
           if (lane == 0) s_next = nx;
         } else {
           // warps 1..7: the S N columns in turn, rows lane and lane + 32 (N <= 16: two columns

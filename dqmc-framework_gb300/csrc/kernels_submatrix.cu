@@ -65,7 +65,7 @@ __device__ __forceinline__ void wsync() { asm volatile("bar.sync 1, %0;" ::"n"(k
 // per-spin scratch in HBM (WalkerDev::msub): the operands' slices as tensor-core
 // images (ozaki::tc_index, k stride 32) and the line exponents
 struct SubOff {
-  size_t sGm, sG, sR, sT, eGm, eG, eR, eT, mc, total;
+  size_t sGm, sG, sR, sT, eGm, eG, eR, eT, mc, pos, total;
 };
 __host__ __device__ inline size_t sub_sst(int N) { return (size_t)ozaki::tc_lines(N) * KB; }
 __host__ __device__ inline SubOff sub_offsets(int N) {
@@ -80,7 +80,8 @@ __host__ __device__ inline SubOff sub_offsets(int N) {
   o.eR = o.eG + al256((size_t)N * sizeof(int));
   o.eT = o.eR + al256((size_t)N * sizeof(int));
   o.mc = o.eT + al256((size_t)N * sizeof(int));  // accepts of the current block (split kernels, spin 0's)
-  o.total = o.mc + 256;
+  o.pos = o.mc + 256;                            // and their block positions [KB]
+  o.total = o.pos + al256(KB * sizeof(int));
   return o;
 }
 
@@ -93,16 +94,16 @@ __device__ __forceinline__ bool sub_slice_of(const WalkerDev& w, int mode, int j
   return true;
 }
 
-// Slices nlines lines x K (<= KB) of NOP operands (1 or 2) into their tensor-core images
+// Slices lines line0 .. line1 - 1 x K (<= KB) of NOP operands (1 or 2) into their tensor-core images
 // dst[o] (slice stride sst, nlb 8-line blocks per k chunk; k past K written as zeros) with one
 // exponent per line (ex[o][line]); get(o, line, k) is the FP64 element.  The worker threads
 // take part; 4 threads per line, 8 k each, both operands' loads in flight together.
 // etmp: [2][256] scratch.
 template <int NOP, class Get>
-__device__ void slice_lines(Get get, int nlines, int K, unsigned short* const* dst, long long sst, int nlb,
+__device__ void slice_lines(Get get, int line0, int line1, int K, unsigned short* const* dst, long long sst, int nlb,
                             int* const* ex, int* etmp) {
-  const int tid = threadIdx.x, ll = tid & 63, part = tid >> 6;
-  for (int l0 = 0; l0 < nlines; l0 += 64) {
+  const int tid = threadIdx.x, ll = tid & 63, part = tid >> 6, nlines = line1;
+  for (int l0 = line0; l0 < line1; l0 += 64) {
     const int line = l0 + ll;
     double v[NOP][8];
     int e[NOP];
@@ -325,113 +326,123 @@ __device__ __forceinline__ void sub_load_block(const SubState& st, const double*
 
 // The decisions of one block, flip by flip, and Gamma = sum_q a_q b_q^T; returns m, the
 // accepts, with their block positions in s_pos.  uni and fld are the block's uniforms and
-// fields (position l).  The sites are visited in order: warp 0 evaluates the ratios of all
-// sites still to visit at once, on the diagonal as it stands, and the lowest accepted one is
-// the next accept of the sequential visit, since every site before it saw the same diagonal.
-// Each accept then takes two phases: (1) the coefficients u~, w~, a, b of the accept; (2)
-// its rank-1 update of the block, warp 0 updating the diagonal of the sites still to visit
-// before it scans them for the next accept, while warps 1-7 update the rest of the block and
-// add a b^T to Gamma (the fma sequence of the closed sum over accepts, so Gamma is the same
-// to the bit).  sign and acc_count are thread 0's.  Worker threads only.
+// fields (position l).  The sites are visited in order by warp 0's scan (SiteScan).  Each accept
+// takes two barriers.  After the first, warps 1 .. 2S form u~ and w~ of the accept on the block
+// and warp 0 reads the diagonal as it stands; after the second
+//   warp 0       scans the sites past it for the next accept, on the diagonal that the pending
+//                update will produce (the update's own fma),
+//   warps 1 - 3  apply the rank-1 update to the block's sites still to visit and add the
+//                previous accept's a b^T to Gamma, column by column,
+//   warps 4 - 7  form the accept's coefficients, one chain of m FMAs per (spin, a or b); with one
+//                spin warps 5 and 6, which do not share warp 0's FP64 pipe,
+// so the coefficients and Gamma, which no decision needs, stay off the decisions' path.  An accept
+// costs max(scan, warps 1-3, chains) + 240 cycles of vectors and barriers.  Gamma receives its
+// terms in the order of the accepts.  sign and acc_count are warp 0's.  Worker threads only.
 __device__ __forceinline__ int sub_decide(const WalkerDev& w, int S, int kb, const double* uni, int8_t* fld,
                                           const SubState& st, int* s_pos, int* s_next, double* s_f, double& sign,
                                           long long& acc_count) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const SiteScan scan(w, lane);
   for (int e = tid; e < S * KK; e += kSubThreads) st.Gam[e] = 0.0;
-  int m = 0, cur = 0;
+  // column y of Gamma += a_q b_q[y], spin sp (lanes x)
+  auto gamma_column = [&](int sp, int q, int y) {
+    if (lane <= q)
+      st.Gam[sp * KK + y * KB + lane] =
+          fma(st.Ac[sp * KK + q * KB + lane], st.Bc[sp * KK + q * KB + y], st.Gam[sp * KK + y * KB + lane]);
+  };
+  const int cw = warp - ((S == 2) ? 4 : 5);  // coefficient chain: a of spin cw, then b
+  double dg[2];
+  if (warp == 0) {
+    scan.load_diag(dg, st.Gb + scan.sp * KK, KB, 0, kb);
+    const int nx = scan.next(w, dg, nullptr, nullptr, 0, kb, uni, fld, s_f, sign, acc_count);
+    if (lane == 0) *s_next = nx;
+  }
+  wsync();
+  int m = 0;
   while (true) {
-    if (warp == 0) {
-      const int l = cur + lane;
-      FlipRatio q{};
-      double fq[2] = {0.0, 0.0};
-      int s = 0;
-      bool acc = false;
-      if (l < kb) {
-        if (m > 0)  // the previous accept's update of this site's diagonal element
-          for (int sp = 0; sp < S; ++sp) {
-            double* gb = st.Gb + sp * KK;
-            gb[l * KB + l] = fma(-st.Ut[sp * KK + (m - 1) * KB + l], st.Wt[sp * KK + (m - 1) * KB + l], gb[l * KB + l]);
-          }
-        s = fld[l];
-        const int si = s > 0 ? 0 : 1;
-        const double gu = st.Gb[l * KB + l];
-        const double gd = (S == 2) ? st.Gb[KK + l * KB + l] : gu;
-        q = flip_ratio(w, si, gu, gd);  // reference operation order
-        acc = uni[l] < fmin(1.0, fabs(q.r));
-        flip_factors(w, q, fq);         // every lane: off the accepted lane's critical path
-      }
-      const unsigned amask = __ballot_sync(0xffffffffu, acc);
-      const int first = amask ? __ffs(amask) - 1 : 32;
-      if (l < kb && lane <= first && !isfinite(q.r)) atomicOr(w.status, ST_NONFINITE_RATIO);
-      if (lane == first) {
-        s_f[0] = fq[0];
-        s_f[1] = fq[1];
-        fld[l] = (int8_t)(-s);
-      }
-      const double rf = __shfl_sync(0xffffffffu, q.r, first & 31);
-      if (lane == 0) {
-        if (amask) {
-          sign = (rf >= 0) ? sign : -sign;
-          ++acc_count;
-        }
-        *s_next = amask ? cur + first : kb;
-      }
-    } else if (m > 0) {
-      // the previous accept (position cur - 1): rank-1 update off the diagonal, Gamma term
-      const int lp = cur - 1, q1 = m - 1;
-      for (int e = tid - 32; e < S * KK; e += kSubThreads - 32) {
-        const int sp = e / KK, c = (e % KK) / KB, r = e % KB;
-        if (r > lp && c > lp && r < kb && c < kb && r != c)
-          st.Gb[e] = fma(-st.Ut[sp * KK + q1 * KB + r], st.Wt[sp * KK + q1 * KB + c], st.Gb[e]);
-        const int y = c, x = r;
-        if (x <= q1 && y <= q1)
-          st.Gam[e] = fma(st.Ac[sp * KK + q1 * KB + x], st.Bc[sp * KK + q1 * KB + y], st.Gam[e]);
-      }
-    }
-    wsync();
     const int l = *s_next;
     if (l >= kb) break;
-    // u~, w~ of accept m on the block, and its coefficients a_m, b_m
-    for (int e = tid; e < S * 4 * KB; e += kSubThreads) {
-      const int sp = e / (4 * KB), role = (e / KB) & 3, x = e % KB;
-      const double f = s_f[sp];
+    if (warp == 0) {
+      scan.load_diag(dg, st.Gb + scan.sp * KK, KB, l + 1, kb);
+      if (lane == 0) s_pos[m] = l;
+    } else if (warp <= 2 * S) {
+      const int sp = (warp - 1) % S;
       const double* gb = st.Gb + sp * KK;
-      double* ut = st.Ut + sp * KK;
-      double* wt = st.Wt + sp * KK;
+      if (warp <= S)
+        st.Ut[sp * KK + m * KB + lane] = s_f[sp] * gb[l * KB + lane];  // f G(x, l)
+      else
+        st.Wt[sp * KK + m * KB + lane] = ((lane == l) ? 1.0 : 0.0) - gb[lane * KB + l];  // delta - G(l, x)
+    }
+    const double f_acc = (cw >= 0) ? s_f[cw % S] : 0.0;  // before the scan replaces it
+    wsync();
+    if (warp == 0) {
+      const int nx = scan.next(w, dg, st.Ut + scan.sp * KK + m * KB, st.Wt + scan.sp * KK + m * KB, l + 1, kb, uni, fld,
+                               s_f, sign, acc_count);
+      if (lane == 0) *s_next = nx;
+    } else if (warp < 4) {
+      const int nc = kb - 1 - l;  // columns still to visit, then Gamma's
+      for (int q = warp - 1; q < S * (nc + m); q += 3) {
+        if (q < S * nc) {
+          const int sp = q >= nc ? 1 : 0, c = l + 1 + q - sp * nc;
+          if (lane > l && lane < kb)
+            st.Gb[sp * KK + c * KB + lane] = fma(-st.Ut[sp * KK + m * KB + lane], st.Wt[sp * KK + m * KB + c],
+                                                 st.Gb[sp * KK + c * KB + lane]);
+        } else {
+          const int g = q - S * nc, sp = g >= m ? 1 : 0;
+          gamma_column(sp, m - 1, g - sp * m);
+        }
+      }
+    } else if (cw >= 0 && cw < 2 * S) {
+      // a_m and b_m at compact index x = lane
+      const int sp = cw % S, x = lane;
+      const double* ut = st.Ut + sp * KK;
+      const double* wt = st.Wt + sp * KK;
       double* ac = st.Ac + sp * KK;
       double* bc = st.Bc + sp * KK;
-      if (role == 0) {
-        ut[m * KB + x] = f * gb[l * KB + x];  // f G(x, l)
-      } else if (role == 1) {
-        wt[m * KB + x] = ((x == l) ? 1.0 : 0.0) - gb[x * KB + l];  // delta - G(l, x)
-      } else if (role == 2) {
-        double a = (x == m) ? 1.0 : 0.0;
-        for (int p = x; p < m; ++p) a = fma(-wt[p * KB + l], ac[p * KB + x], a);
-        ac[m * KB + x] = (x <= m) ? f * a : 0.0;
+      double v = (x == m) ? 1.0 : 0.0;
+      if (cw < S) {
+        for (int p = 0; p < m; ++p)
+          if (p >= x) v = fma(-wt[p * KB + l], ac[p * KB + x], v);
+        ac[m * KB + x] = (x <= m) ? f_acc * v : 0.0;
       } else {
-        double b = (x == m) ? 1.0 : 0.0;
-        for (int p = x; p < m; ++p) b = fma(ut[p * KB + l], bc[p * KB + x], b);
-        bc[m * KB + x] = (x <= m) ? b : 0.0;
+        for (int p = 0; p < m; ++p)
+          if (p >= x) v = fma(ut[p * KB + l], bc[p * KB + x], v);
+        bc[m * KB + x] = (x <= m) ? v : 0.0;
       }
     }
-    if (tid == 0) s_pos[m] = l;
     wsync();
     ++m;
-    cur = l + 1;
+  }
+  if (m > 0) {  // the last accept's term
+    for (int q = warp; q < S * m; q += kSubThreads / 32) {
+      const int sp = q >= m ? 1 : 0;
+      gamma_column(sp, m - 1, q - sp * m);
+    }
+    wsync();
   }
   return m;
 }
 
-// Spin sp of a block with m accepts at sites i0 + s_pos[q]: the slices of Gamma, G0(:, I_A) and
-// R_A = E_A^T - G0(I_A, :) (taken before G changes), then T^T = R_A^T Gamma^T on the tensor
-// cores: warp w and w + 4 share TMEM lanes 32 (w & 3).. (columns c) and take x in [0, 16) and
+// The slices of Gamma of a block with m accepts, and their exponents eGm [KB] (worker threads)
+__device__ __forceinline__ void sub_slice_gamma(const WalkerDev& w, int sp, int N, int m, const double* gam, int* eGm,
+                                                int* etmp) {
+  const SubOff so = sub_offsets(N);
+  unsigned short* dGm[1] = {reinterpret_cast<unsigned short*>(w.msub + (size_t)sp * so.total + so.sGm)};
+  int* xGm[1] = {eGm};
+  slice_lines<1>([&](int, int line, int k) { return gam[k * KB + line]; }, 0, m, m, dGm, (long long)sub_sst(1), TM / 8,
+                 xGm, etmp);
+}
+
+// Spin sp of a block with m accepts at sites i0 + s_pos[q], Gamma's slices made: the row blocks
+// rb0 .. rb0 + nrb - 1 (128 lines) of the slices of G0(:, I_A) and R_A = E_A^T - G0(I_A, :) (taken
+// before G changes), then of T^T = R_A^T Gamma^T on the tensor cores: warp w and w + 4 share TMEM lanes 32 (w & 3).. (columns c) and take x in [0, 16) and
 // [16, 32); the column exponent max over x goes through etmp, and the epilogue slices T straight
 // into the B image of the flush (line c, k = x).  Line exponents: eGm [KB] of Gamma, eG [N] of
 // G0(:, I_A), eR [N] of R_A, eT [N] of T (shared or global memory); etmp: [2][256] scratch.
 // Called by all kSubCTA threads; the workers slice.
-__device__ __forceinline__ void sub_prepare(const SubTC& tcs, unsigned& gt, unsigned& nA, const WalkerDev& w, int sp, int N, int m,
-                            int i0, const int* s_pos, const double* gam, const double* Gs, int* eGm, int* eG, int* eR,
-                            int* eT, int* etmp) {
+__device__ __forceinline__ void sub_prepare(const SubTC& tcs, unsigned& gt, unsigned& nA, const WalkerDev& w, int sp,
+                                            int N, int m, int i0, const int* s_pos, const double* Gs, const int* eGm,
+                                            int* eG, int* eR, int* eT, int* etmp, int rb0, int nrb) {
   const SubOff so = sub_offsets(N);
   unsigned char* ms = w.msub + (size_t)sp * so.total;
   unsigned short* sGm = reinterpret_cast<unsigned short*>(ms + so.sGm);
@@ -442,9 +453,6 @@ __device__ __forceinline__ void sub_prepare(const SubTC& tcs, unsigned& gt, unsi
   const int nlbN = ozaki::tc_lines(N) / 8, nk = (m + 15) / 16;
   const long long sstN = (long long)sub_sst(N), sstG = (long long)sub_sst(1);
   if (tid < kSubThreads) {
-    unsigned short* dGm[1] = {sGm};
-    int* xGm[1] = {eGm};
-    slice_lines<1>([&](int, int line, int k) { return gam[k * KB + line]; }, m, m, dGm, sstG, TM / 8, xGm, etmp);
     // G0(:, I_A) (lines = rows) and R_A (lines = columns) in one pass
     unsigned short* dGR[2] = {sG, sR};
     int* xGR[2] = {eG, eR};
@@ -453,14 +461,15 @@ __device__ __forceinline__ void sub_prepare(const SubTC& tcs, unsigned& gt, unsi
           const int i = i0 + s_pos[k];
           return o == 0 ? Gs[(long long)i * N + line] : ((line == i) ? 1.0 : 0.0) - Gs[(long long)line * N + i];
         },
-        N, m, dGR, sstN, nlbN, xGR, etmp);
+        rb0 * TM, min(N, (rb0 + nrb) * TM), m, dGR, sstN, nlbN, xGR, etmp);
     asm volatile("fence.proxy.async.global;" ::: "memory");  // generic writes -> bulk-copy reads
   }
   __syncthreads();
-  sub_gemm(tcs, gt, nA, sR, sstN, nlbN, (N + TM - 1) / TM, sGm, sstG, TM / 8, 1, nk, [&](int, int, int) {},
+  sub_gemm(tcs, gt, nA, sR + (long long)rb0 * (TM / 8) * 128, sstN, nlbN, nrb, sGm, sstG, TM / 8, 1, nk,
+           [&](int, int, int) {},
            [&](int rb, int, unsigned tacc, bool ok, int tl, bool) {
              const int wq = (tid >> 5) & 3, xh = tid >> 7;
-             const int c = rb * TM + wq * 32 + (tid & 31);
+             const int c = (rb0 + rb) * TM + wq * 32 + (tid & 31);
              const int ec = (c < N) ? eR[c] : 0;
              double tv[16];
              int e = -1100;
@@ -644,7 +653,8 @@ __global__ void __launch_bounds__(kSubCTA, 1) metropolis_sub_kernel(const Walker
     const int m = s_m;
     if (m == 0) continue;
     for (int sp = 0; sp < S; ++sp) {
-      sub_prepare(tcs, gt, nA, w, sp, N, m, i0, s_pos, st.Gam + sp * KK, G[sp], s_eGm, s_eG, s_eR, s_eT, etmp);
+      if (worker) sub_slice_gamma(w, sp, N, m, st.Gam + sp * KK, s_eGm, etmp);
+      sub_prepare(tcs, gt, nA, w, sp, N, m, i0, s_pos, G[sp], s_eGm, s_eG, s_eR, s_eT, etmp, 0, (N + TM - 1) / TM);
       sub_flush(tcs, gt, nA, w, sp, N, m, G[sp], s_eG, s_eT, stage, 0, 1);
     }
   }
@@ -664,39 +674,41 @@ __global__ void __launch_bounds__(kSubCTA, 1) metropolis_sub_kernel(const Walker
   }
 }
 
-// ---- the same updates split per 32-site block into two kernels ----------------
+// ---- the same updates split per 32-site block into three kernels ---------------
 // For walkers too few to fill the GPU (one CTA per walker leaves most SMs idle at
 // 32 walkers of N = 576), each block runs as a decision kernel (one CTA per walker:
-// the decisions, Gamma, the slices of Gamma, G0(:, I_A) and R_A, T^T on the tensor
-// cores) followed by a flush kernel whose CTAs share the walker's column tiles of G.
-// The arithmetic is the fused kernel's (the same device functions).  The autotuner
-// times both.
+// the decisions, Gamma and its slices), a preparation kernel (a CTA per walker, spin and
+// 128-line block: the slices of G0(:, I_A) and R_A, T^T on the tensor cores) and a flush
+// kernel whose CTAs share a walker's spins and column tiles of G.  Only the decisions are
+// serial in a walker; with the preparation in the decision kernel they took 203 us of a 313 us
+// block at N = 576 (2 spins), 133 of 183 us at N = 256.  The arithmetic is the fused kernel's
+// (the same device functions).  The autotuner times both.
 
-// dynamic shared memory of the decision kernel: the operand buffers, the block's uniforms,
-// the FP64 block state, the exponent scratch [2][256] and the block's fields; of the flush
-// kernel: the operand buffers, the G staging and the line exponents eG, eT [N]
+// dynamic shared memory of the decision kernel: the block's uniforms, the FP64 block state, the
+// exponent scratch [2][256] and the block's fields; of the preparation kernel: the operand
+// buffers, the exponent scratch and eR of one row block; of the flush kernel: the operand
+// buffers, the G staging and the line exponents eG, eT [N]
 size_t submatrix_block_smem_bytes(int S) {
-  return (size_t)A_BYTES + (size_t)NBB * B_BYTES + sizeof(double) * (KB + 6ull * S * KK) +
-         2 * kSubThreads * sizeof(int) + KB;
+  return sizeof(double) * (KB + 6ull * S * KK) + 2 * kSubThreads * sizeof(int) + KB;
 }
+constexpr size_t kPrepSmem = (size_t)A_BYTES + (size_t)NBB * B_BYTES + 2 * kSubThreads * sizeof(int);
 size_t submatrix_flush_smem_bytes(int N) {
   return (size_t)A_BYTES + (size_t)NBB * B_BYTES + kStageBytes + 2 * sizeof(int) * (size_t)((N + 1) & ~1);
 }
 
-__global__ void __launch_bounds__(kSubCTA) metropolis_sub_block_kernel(const WalkerDev* __restrict__ W, int mode,
-                                                                       int j, int q, int blk) {
+__global__ void __launch_bounds__(kSubThreads) metropolis_sub_block_kernel(const WalkerDev* __restrict__ W, int mode,
+                                                                           int j, int q, int blk) {
   const WalkerDev& w = W[blockIdx.x];
   if (w.path != 2) return;
   int t;
   if (!sub_slice_of(w, mode, j, q, t)) return;
   const int N = w.N, S = w.S, Lt = w.Lt, tid = threadIdx.x;
-  const bool worker = tid < kSubThreads;
   const int i0 = blk * KB;
   if (i0 >= N) return;
   const int kb = min(KB, N - i0);
   const long long NN = (long long)N * N;
   extern __shared__ __align__(1024) unsigned char smem[];
-  double* uni = reinterpret_cast<double*>(smem + A_BYTES + NBB * B_BYTES);  // [KB] uniforms of the block
+  double* uni = reinterpret_cast<double*>(smem);  // [KB] uniforms of the block
   SubState st;
   st.Gam = uni + KB;
   st.Gb = st.Gam + S * KK;
@@ -706,74 +718,105 @@ __global__ void __launch_bounds__(kSubCTA) metropolis_sub_block_kernel(const Wal
   st.Wt = st.Ut + S * KK;
   int* etmp = reinterpret_cast<int*>(st.Wt + S * KK);                   // [2][256]
   int8_t* s_field = reinterpret_cast<int8_t*>(etmp + 2 * kSubThreads);  // [KB]
-  __shared__ int s_next, s_pos[KB], s_m;
+  __shared__ int s_next, s_pos[KB];
   __shared__ double s_f[2];
-  __shared__ __align__(8) unsigned long long bar_ldA, bar_ldB[NBB], bar_mma[2], bar_bfree[NBB], bar_accfree[2];
-  __shared__ unsigned s_tmem;
-  __shared__ int s_tcfail;
 
   const SubOff so = sub_offsets(N);
   const double* G[2] = {w.G, (S == 2) ? w.G + NN : w.G};
   const int eff = t - 1;
   const unsigned long long sweep = (w.rng == 1) ? *w.sweep_ctr : 0ULL;
-  if (worker) {
-    for (int l = tid; l < kb; l += kSubThreads) {
-      const int i = i0 + l;
-      s_field[l] = w.fields[(long long)eff * N + i];
-      const int attempt = (mode == MODE_FWD) ? (eff * N + i) : ((Lt - t) * N + i);
-      uni[l] = (w.rng == 0) ? w.uni[attempt] : philox_uniform(w.seed, (unsigned)w.widx, sweep, (unsigned)(eff * N + i));
-    }
-    sub_load_block(st, G, S, N, i0, kb);
-    double sign = (tid == 0) ? *w.sign : 0.0;
-    long long acc_count = 0;
-    wsync();
-    const int m = sub_decide(w, S, kb, uni, s_field, st, s_pos, &s_next, s_f, sign, acc_count);
-    int8_t* frw = w.fields + (long long)eff * N + i0;
-    for (int l = tid; l < kb; l += kSubThreads) frw[l] = s_field[l];
-    if (tid == 0) {
-      *w.sign = sign;
-      *w.accepts += acc_count;
-      if (mode == MODE_BWD && t == Lt && i0 + KB >= N) *w.sign_Lt = sign;
-      *reinterpret_cast<int*>(w.msub + so.mc) = m;
-      s_m = m;
-      s_tcfail = 0;
-      if (m > 0) sub_tc_init(&bar_ldA, bar_ldB, bar_mma, bar_bfree, bar_accfree);
-    }
+  for (int l = tid; l < kb; l += kSubThreads) {
+    const int i = i0 + l;
+    s_field[l] = w.fields[(long long)eff * N + i];
+    const int attempt = (mode == MODE_FWD) ? (eff * N + i) : ((Lt - t) * N + i);
+    uni[l] = (w.rng == 0) ? w.uni[attempt] : philox_uniform(w.seed, (unsigned)w.widx, sweep, (unsigned)(eff * N + i));
   }
-  __syncthreads();
-  const int m = s_m;
-  if (m == 0) return;
+  sub_load_block(st, G, S, N, i0, kb);
+  double sign = (tid < 32) ? *w.sign : 0.0;
+  long long acc_count = 0;
+  wsync();
+  const int m = sub_decide(w, S, kb, uni, s_field, st, s_pos, &s_next, s_f, sign, acc_count);
+  int8_t* frw = w.fields + (long long)eff * N + i0;
+  for (int l = tid; l < kb; l += kSubThreads) frw[l] = s_field[l];
+  if (tid == 0) {
+    *w.sign = sign;
+    *w.accepts += acc_count;
+    if (mode == MODE_BWD && t == Lt && i0 + KB >= N) *w.sign_Lt = sign;
+    *reinterpret_cast<int*>(w.msub + so.mc) = m;
+  }
+  if (tid < m) reinterpret_cast<int*>(w.msub + so.pos)[tid] = s_pos[tid];
+  if (m > 0)
+    for (int sp = 0; sp < S; ++sp)
+      sub_slice_gamma(w, sp, N, m, st.Gam + sp * KK,
+                      reinterpret_cast<int*>(w.msub + (size_t)sp * so.total + so.eGm), etmp);
+}
 
-  if (tid < 32) tc::alloc(&s_tmem, TMEM_COLS);
+// The mbarriers and the TMEM of a kernel that runs sub_gemm (every thread calls)
+struct SubTCShared {
+  unsigned long long ldA, ldB[NBB], mma[2], bfree[NBB], accfree[2];
+  unsigned tmem;
+  int fail;
+};
+__device__ __forceinline__ SubTC sub_tc_open(SubTCShared& b, unsigned char* smem) {
+  if (threadIdx.x == 0) {
+    b.fail = 0;
+    sub_tc_init(&b.ldA, b.ldB, b.mma, b.bfree, b.accfree);
+  }
+  if (threadIdx.x < 32) tc::alloc(&b.tmem, TMEM_COLS);
   tc::fence_before();
   __syncthreads();
   tc::fence_after();
-  const SubTC tcs{smem, smem + A_BYTES, &bar_ldA, bar_ldB, bar_mma, bar_bfree, bar_accfree, s_tmem, &s_tcfail};
-  unsigned gt = 0, nA = 0;
-  for (int sp = 0; sp < S; ++sp) {
-    unsigned char* ms = w.msub + (size_t)sp * so.total;
-    sub_prepare(tcs, gt, nA, w, sp, N, m, i0, s_pos, st.Gam + sp * KK, G[sp], reinterpret_cast<int*>(ms + so.eGm),
-                reinterpret_cast<int*>(ms + so.eG), reinterpret_cast<int*>(ms + so.eR),
-                reinterpret_cast<int*>(ms + so.eT), etmp);
-  }
+  return SubTC{smem, smem + A_BYTES, &b.ldA, b.ldB, b.mma, b.bfree, b.accfree, b.tmem, &b.fail};
+}
+// Every committed MMA has completed (each tile's commit was waited on)
+__device__ __forceinline__ void sub_tc_close(SubTCShared& b, const WalkerDev& w) {
   tc::fence_before();
   __syncthreads();
-  if (tid < 32) tc::dealloc(s_tmem, TMEM_COLS);
-  if (tid == 0 && s_tcfail) {
-    atomicOr(w.status, ST_TIMEOUT);
-    *reinterpret_cast<int*>(w.msub + so.mc) = 0;  // no flush from a product that gave up
-  }
+  if (threadIdx.x < 32) tc::dealloc(b.tmem, TMEM_COLS);
+  if (threadIdx.x == 0 && b.fail) atomicOr(w.status, ST_TIMEOUT);
 }
 
-// The flush of block blk: G -= G0(:, I_A) T for both spins, the column tiles of G spread over
-// the gridDim.x CTAs of a walker (CTA p takes tiles p, p + gridDim.x, ...).
-__global__ void __launch_bounds__(kSubCTA) metropolis_sub_flush_kernel(const WalkerDev* __restrict__ W, int mode,
-                                                                       int j, int q, int blk) {
-  const WalkerDev& w = W[blockIdx.y];
-  if (w.path != 2) return;
+// The preparation of block blk: row block blockIdx.x of spin blockIdx.y of walker blockIdx.z
+__global__ void __launch_bounds__(kSubCTA) metropolis_sub_prep_kernel(const WalkerDev* __restrict__ W, int mode, int j,
+                                                                      int q, int blk) {
+  const WalkerDev& w = W[blockIdx.z];
+  const int sp = blockIdx.y, rb = blockIdx.x, tid = threadIdx.x;
+  if (w.path != 2 || sp >= w.S) return;
   int t;
   if (!sub_slice_of(w, mode, j, q, t)) return;
-  const int N = w.N, S = w.S, tid = threadIdx.x;
+  const int N = w.N;
+  if (blk * KB >= N || rb * TM >= N) return;
+  const SubOff so = sub_offsets(N);
+  const int m = *reinterpret_cast<const int*>(w.msub + so.mc);
+  if (m == 0) return;
+  extern __shared__ __align__(1024) unsigned char smem[];
+  int* etmp = reinterpret_cast<int*>(smem + A_BYTES + NBB * B_BYTES);  // [2][256]
+  __shared__ int s_pos[KB], s_eGm[KB];
+  __shared__ __align__(8) SubTCShared bar;
+  unsigned char* ms = w.msub + (size_t)sp * so.total;
+  if (tid < m) {
+    s_pos[tid] = reinterpret_cast<const int*>(w.msub + so.pos)[tid];
+    s_eGm[tid] = reinterpret_cast<const int*>(ms + so.eGm)[tid];
+  }
+  const SubTC tcs = sub_tc_open(bar, smem);
+  unsigned gt = 0, nA = 0;
+  sub_prepare(tcs, gt, nA, w, sp, N, m, blk * KB, s_pos, w.G + (long long)sp * N * N, s_eGm,
+              reinterpret_cast<int*>(ms + so.eG), reinterpret_cast<int*>(ms + so.eR), reinterpret_cast<int*>(ms + so.eT),
+              etmp, rb, 1);
+  sub_tc_close(bar, w);
+  if (tid == 0 && bar.fail) *reinterpret_cast<int*>(w.msub + so.mc) = 0;  // no flush from a product that gave up
+}
+
+// The flush of block blk: G -= G0(:, I_A) T for spin blockIdx.y of walker blockIdx.z, the column
+// tiles of G spread over gridDim.x CTAs (CTA p takes tiles p, p + gridDim.x, ...).
+__global__ void __launch_bounds__(kSubCTA) metropolis_sub_flush_kernel(const WalkerDev* __restrict__ W, int mode,
+                                                                       int j, int q, int blk) {
+  const WalkerDev& w = W[blockIdx.z];
+  const int sp = blockIdx.y;
+  if (w.path != 2 || sp >= w.S) return;
+  int t;
+  if (!sub_slice_of(w, mode, j, q, t)) return;
+  const int N = w.N, tid = threadIdx.x;
   if (blk * KB >= N) return;
   const int nct = (N + TN - 1) / TN;
   if ((int)blockIdx.x >= nct) return;
@@ -781,40 +824,20 @@ __global__ void __launch_bounds__(kSubCTA) metropolis_sub_flush_kernel(const Wal
   const int m = *reinterpret_cast<const int*>(w.msub + so.mc);
   if (m == 0) return;
   const int Nu = (N + 1) & ~1;
-  const long long NN = (long long)N * N;
   extern __shared__ __align__(1024) unsigned char smem[];
   double* stage = reinterpret_cast<double*>(smem + A_BYTES + NBB * B_BYTES);
   int* s_eG = reinterpret_cast<int*>(reinterpret_cast<unsigned char*>(stage) + kStageBytes);
   int* s_eT = s_eG + Nu;
-  __shared__ __align__(8) unsigned long long bar_ldA, bar_ldB[NBB], bar_mma[2], bar_bfree[NBB], bar_accfree[2];
-  __shared__ unsigned s_tmem;
-  __shared__ int s_tcfail;
-  if (tid == 0) {
-    s_tcfail = 0;
-    sub_tc_init(&bar_ldA, bar_ldB, bar_mma, bar_bfree, bar_accfree);
+  __shared__ __align__(8) SubTCShared bar;
+  const unsigned char* ms = w.msub + (size_t)sp * so.total;
+  for (int i = tid; i < N; i += kSubCTA) {
+    s_eG[i] = reinterpret_cast<const int*>(ms + so.eG)[i];
+    s_eT[i] = reinterpret_cast<const int*>(ms + so.eT)[i];
   }
-  if (tid < 32) tc::alloc(&s_tmem, TMEM_COLS);
-  tc::fence_before();
-  __syncthreads();
-  tc::fence_after();
-  const SubTC tcs{smem, smem + A_BYTES, &bar_ldA, bar_ldB, bar_mma, bar_bfree, bar_accfree, s_tmem, &s_tcfail};
+  const SubTC tcs = sub_tc_open(bar, smem);
   unsigned gt = 0, nA = 0;
-  for (int sp = 0; sp < S; ++sp) {
-    const unsigned char* ms = w.msub + (size_t)sp * so.total;
-    const int* eG = reinterpret_cast<const int*>(ms + so.eG);
-    const int* eT = reinterpret_cast<const int*>(ms + so.eT);
-    if (tid < kSubThreads)
-      for (int i = tid; i < N; i += kSubThreads) {
-        s_eG[i] = eG[i];
-        s_eT[i] = eT[i];
-      }
-    __syncthreads();
-    sub_flush(tcs, gt, nA, w, sp, N, m, w.G + sp * NN, s_eG, s_eT, stage, (int)blockIdx.x, (int)gridDim.x);
-  }
-  tc::fence_before();
-  __syncthreads();
-  if (tid < 32) tc::dealloc(s_tmem, TMEM_COLS);
-  if (tid == 0 && s_tcfail) atomicOr(w.status, ST_TIMEOUT);
+  sub_flush(tcs, gt, nA, w, sp, N, m, w.G + (long long)sp * N * N, s_eG, s_eT, stage, (int)blockIdx.x, (int)gridDim.x);
+  sub_tc_close(bar, w);
 }
 
 static size_t g_sub_smem_limit = 0;  // dynamic shared memory the kernel may use
@@ -834,6 +857,8 @@ cudaError_t configure_submatrix_kernel() {
     e = cudaFuncSetAttribute(metropolis_sub_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)submatrix_block_smem_bytes(2));
   if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(metropolis_sub_prep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPrepSmem);
+  if (e == cudaSuccess)
     e = cudaFuncSetAttribute(metropolis_sub_flush_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)submatrix_flush_smem_bytes(kMaxN));
   return e;
@@ -843,19 +868,19 @@ void launch_metropolis_sub(const WalkerDev* W, int nw, int mode, int j, int q, i
   metropolis_sub_kernel<<<nw, kSubCTA, submatrix_smem_bytes(maxN, S_max), st>>>(W, mode, j, q);
 }
 
-// CTAs per walker of the split flush: two column tiles of 32 each (at least one CTA)
-int submatrix_flush_ctas(int maxN) { return std::max(1, ((maxN + TN - 1) / TN + 1) / 2); }
-
 // One slice of Metropolis by the split kernels: for each 32-site block the decisions (one CTA
-// per walker) then the flush (submatrix_flush_ctas CTAs per walker); walkers whose N ends
-// earlier skip the blocks past it.
+// per walker), the preparation (a CTA per walker, spin and 128 lines) and the flush; walkers whose
+// N ends earlier skip the blocks past it.  A flush CTA takes two column tiles (its operand ring
+// then overlaps the second tile's copies), or one where that still leaves SMs idle.
 void launch_metropolis_sub_split(const WalkerDev* W, int nw, int mode, int j, int q, int maxN, int S_max,
                                  cudaStream_t st) {
-  const int nb = (maxN + KB - 1) / KB, P = submatrix_flush_ctas(maxN);
+  const int nb = (maxN + KB - 1) / KB, nct = (maxN + TN - 1) / TN, nrb = (maxN + TM - 1) / TM;
+  const int P = (nw * S_max * nct <= 152) ? nct : (nct + 1) / 2;
   const size_t sm1 = submatrix_block_smem_bytes(S_max), sm2 = submatrix_flush_smem_bytes(maxN);
   for (int blk = 0; blk < nb; ++blk) {
-    metropolis_sub_block_kernel<<<nw, kSubCTA, sm1, st>>>(W, mode, j, q, blk);
-    metropolis_sub_flush_kernel<<<dim3(P, nw), kSubCTA, sm2, st>>>(W, mode, j, q, blk);
+    metropolis_sub_block_kernel<<<nw, kSubThreads, sm1, st>>>(W, mode, j, q, blk);
+    metropolis_sub_prep_kernel<<<dim3(nrb, S_max, nw), kSubCTA, kPrepSmem, st>>>(W, mode, j, q, blk);
+    metropolis_sub_flush_kernel<<<dim3(P, S_max, nw), kSubCTA, sm2, st>>>(W, mode, j, q, blk);
   }
 }
 
