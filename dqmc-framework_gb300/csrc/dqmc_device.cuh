@@ -187,30 +187,19 @@ struct SiteScan {
       e2[k] = w.ex2[k];
     }
   }
-  // the diagonal elements of NW windows from site `from` of this lane's spin's matrix
-  template <int NW>
-  __device__ __forceinline__ void load_diag(double (&dg)[NW], const double* G, int ld, int from, int N) const {
-#pragma unroll
-    for (int b = 0; b < NW; ++b) {
-      const int l = from + b * width + dl;
-      dg[b] = (l < N) ? G[l * (ld + 1)] : 0.0;
-    }
-  }
-  // The next accepted site from `from` on (N: none; NW windows reach N) on the diagonal dg, after
-  // the pending update of this lane's spin (u, wv by site; null: none); flips the field and leaves
+  // The next accepted site from `from` on (N: none; NW windows reach N); diag(b, l) is the current
+  // diagonal element of this lane's spin at site l < N of window b.  Flips the field and leaves
   // the update's factors in f[2].  The whole warp calls; sign and accepts are uniform in it.
-  template <int NW>
-  __device__ __forceinline__ int next(const WalkerDev& w, const double (&dg)[NW], const double* u, const double* wv,
-                                      int from, int N, const double* uni, int8_t* field, double* f, double& sign,
-                                      long long& accepts) const {
+  template <int NW, class Diag>
+  __device__ __forceinline__ int next(const WalkerDev& w, Diag diag, int from, int N, const double* uni,
+                                      int8_t* field, double* f, double& sign, long long& accepts) const {
 #pragma unroll
     for (int b = 0; b < NW; ++b) {
       const int base = from + b * width;
       if (base >= N) break;
       const int l = base + dl;
       const bool in = l < N;
-      double g = dg[b];
-      if (u && in) g = fma(-wv[l], u[l], g);
+      const double g = in ? diag(b, l) : 0.0;
       const int s = in ? field[l] : 1;
       const double ck = s > 0 ? c[0] : c[1];
       const double qs = __dadd_rn(1.0, __dmul_rn(__dsub_rn(1.0, g), ck));

@@ -546,8 +546,8 @@ __global__ void __launch_bounds__(kThreads, 2) segment_kernel(const WalkerDev* _
       const double* su = vec + scan.sp * N;
       const double* sw = vec + (2 + scan.sp) * N;
       if (wid == 0) {
-        scan.load_diag(dg, Gs[scan.sp], ld, 0, N);
-        const int nx = scan.next(w, dg, nullptr, nullptr, 0, N, s_uni, s_field, s_f, sign, acc_count);
+        const int nx = scan.next<4>(w, [&](int, int l) { return at(Gs[scan.sp], ld, l, l); }, 0, N, s_uni, s_field, s_f,
+                                    sign, acc_count);
         if (lane == 0) s_next = nx;
       }
       __syncthreads();
@@ -555,7 +555,11 @@ __global__ void __launch_bounds__(kThreads, 2) segment_kernel(const WalkerDev* _
         const int i = s_next;
         if (i >= N) break;
         if (wid == 0) {
-          scan.load_diag(dg, Gs[scan.sp], ld, i + 1, N);
+#pragma unroll
+          for (int b = 0; b < 4; ++b) {
+            const int l = i + 1 + b * scan.width + scan.dl;
+            dg[b] = (l < N) ? at(Gs[scan.sp], ld, l, l) : 0.0;
+          }
         } else if (wid <= 2 * S) {
           const int sp = (wid - 1) % S, role = (wid - 1) / S;
           const double* g = Gs[sp];
@@ -567,7 +571,8 @@ __global__ void __launch_bounds__(kThreads, 2) segment_kernel(const WalkerDev* _
         }
         __syncthreads();
         if (wid == 0) {
-          const int nx = scan.next(w, dg, su, sw, i + 1, N, s_uni, s_field, s_f, sign, acc_count);
+          const int nx = scan.next<4>(w, [&](int b, int l) { return fma(-sw[l], su[l], dg[b]); }, i + 1, N, s_uni,
+                                      s_field, s_f, sign, acc_count);
           if (lane == 0) s_next = nx;
         } else {
           // warps 1..7: the S N columns in turn, rows lane and lane + 32 (N <= 16: two columns

@@ -304,15 +304,18 @@ __device__ __forceinline__ void cp_async_wait(bool one_pending) {
 // The flush's G staging: two tiles of 16 elements per thread, [tile & 1][u][thread]
 constexpr int kStageBytes = 2 * 16 * kSubThreads * 8;
 
-// FP64 state of one block's decisions in shared memory, each [S][KK]: the diagonal block
-// G(I, I) ((r, c) at c * KB + r), the coefficients a_q, b_q ([q][x] at compact index x), u~_q,
+// The diagonal block's columns are GL doubles apart: rows and columns are both read by lanes
+constexpr int GL = KB + 1, GBS = KB * GL;
+
+// FP64 state of one block's decisions in shared memory: the diagonal block G(I, I) [S][GBS]
+// ((r, c) at c * GL + r) and, each [S][KK], the coefficients a_q, b_q ([q][x] at compact index x), u~_q,
 // w~_q ([q][l] at block position l) and Gamma ((x, y) at y * KB + x)
 struct SubState {
   double *Gb, *Ac, *Bc, *Ut, *Wt, *Gam;
 };
 // bytes of Gb .. Wt (the part the fused kernel's flush overlays with its G staging)
 __host__ __device__ inline size_t sub_state_bytes(int S) {
-  const size_t b = 5ull * S * KK * sizeof(double);
+  const size_t b = (size_t)S * (GBS + 4 * KK) * sizeof(double);
   return b > (size_t)kStageBytes ? b : (size_t)kStageBytes;
 }
 
@@ -320,117 +323,146 @@ __host__ __device__ inline size_t sub_state_bytes(int S) {
 __device__ __forceinline__ void sub_load_block(const SubState& st, const double* const* G, int S, int N, int i0, int kb) {
   for (int e = threadIdx.x; e < S * KK; e += kSubThreads) {
     const int sp = e / KK, c = (e % KK) / KB, r = e % KB;
-    st.Gb[e] = (r < kb && c < kb) ? G[sp][(long long)(i0 + c) * N + i0 + r] : 0.0;
+    st.Gb[sp * GBS + c * GL + r] = (r < kb && c < kb) ? G[sp][(long long)(i0 + c) * N + i0 + r] : 0.0;
   }
+}
+
+// What the decisions of one block leave for the next accept, double-buffered by the accept's
+// parity: the accepted position and its factors, and the diagonal of G on the block
+struct SubAccept {
+  int next[2];
+  double f[2][2];
+  double diag[2][2][KB];
+};
+
+// r + sum_{p < n} (+-a[p KB]) b[p KB] in order of p, four terms' loads ahead of their FMAs.  The
+// coefficients are zero above their diagonal (x > q), so a chain needs no test of p against x.
+template <bool NEG>
+__device__ __forceinline__ double sub_chain(const double* a, const double* b, int n, double r) {
+  int p = 0;
+  for (; p + 4 <= n; p += 4) {
+    double u[4], v[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      u[k] = a[(p + k) * KB];
+      v[k] = b[(p + k) * KB];
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) r = fma(NEG ? -u[k] : u[k], v[k], r);
+  }
+  for (; p < n; ++p) r = fma(NEG ? -a[p * KB] : a[p * KB], b[p * KB], r);
+  return r;
 }
 
 // The decisions of one block, flip by flip, and Gamma = sum_q a_q b_q^T; returns m, the
 // accepts, with their block positions in s_pos.  uni and fld are the block's uniforms and
-// fields (position l).  The sites are visited in order by warp 0's scan (SiteScan).  Each accept
-// takes two barriers.  After the first, warps 1 .. 2S form u~ and w~ of the accept on the block
-// and warp 0 reads the diagonal as it stands; after the second
-//   warp 0       scans the sites past it for the next accept, on the diagonal that the pending
-//                update will produce (the update's own fma),
-//   warps 1 - 3  apply the rank-1 update to the block's sites still to visit and add the
-//                previous accept's a b^T to Gamma, column by column,
+// fields (position l).  The sites are visited in order by warp 0's scan (SiteScan).  The decisions
+// need only the sites past the last accept l, so its update leaves row l and column l as they
+// stand: every warp takes u = f G(:, l) and -w = G(l, :) from them without a hand-over, and an
+// accept costs one barrier, after which
+//   warp 0       scans the sites past l for the next accept, on their diagonal after the update,
+//   warps 1 - 3  apply the update to the block's rows and columns past l; warps 1 .. S also
+//                record u and w and write the updated diagonal for the next accept,
 //   warps 4 - 7  form the accept's coefficients, one chain of m FMAs per (spin, a or b); with one
-//                spin warps 5 and 6, which do not share warp 0's FP64 pipe,
-// so the coefficients and Gamma, which no decision needs, stay off the decisions' path.  An accept
-// costs max(scan, warps 1-3, chains) + 240 cycles of vectors and barriers.  Gamma receives its
-// terms in the order of the accepts.  sign and acc_count are warp 0's.  Worker threads only.
+//                spin warps 5 and 6, which do not share warp 0's FP64 pipe.
+// Gamma, which no decision needs, is summed at the end in the order of the accepts.  The scan's
+// chain bounds an accept (SiteScan), with two spins the SM's FP64 pipes as well (about 100 warp
+// operations an accept at 19 cycles each).  One slice of all walkers, N = 256: 6 walkers of two
+// spins (split form) 1.34 ms with the ratios of both spins and two divisions in one lane and the
+// coefficients on the path, 0.98 with two barriers an accept, 0.78 so; 128 walkers of one spin
+// (fused) 1.36, 1.10 and 1.05 ms.
+// sign and acc_count are warp 0's.  Worker threads only.
 __device__ __forceinline__ int sub_decide(const WalkerDev& w, int S, int kb, const double* uni, int8_t* fld,
-                                          const SubState& st, int* s_pos, int* s_next, double* s_f, double& sign,
+                                          const SubState& st, int* s_pos, SubAccept& sa, double& sign,
                                           long long& acc_count) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const SiteScan scan(w, lane);
-  for (int e = tid; e < S * KK; e += kSubThreads) st.Gam[e] = 0.0;
-  // column y of Gamma += a_q b_q[y], spin sp (lanes x)
-  auto gamma_column = [&](int sp, int q, int y) {
-    if (lane <= q)
-      st.Gam[sp * KK + y * KB + lane] =
-          fma(st.Ac[sp * KK + q * KB + lane], st.Bc[sp * KK + q * KB + y], st.Gam[sp * KK + y * KB + lane]);
-  };
   const int cw = warp - ((S == 2) ? 4 : 5);  // coefficient chain: a of spin cw, then b
-  double dg[2];
   if (warp == 0) {
-    scan.load_diag(dg, st.Gb + scan.sp * KK, KB, 0, kb);
-    const int nx = scan.next(w, dg, nullptr, nullptr, 0, kb, uni, fld, s_f, sign, acc_count);
-    if (lane == 0) *s_next = nx;
+    const int nx = scan.next<2>(w, [&](int, int l) { return st.Gb[scan.sp * GBS + l * (GL + 1)]; }, 0, kb, uni, fld,
+                                sa.f[0], sign, acc_count);
+    if (lane == 0) sa.next[0] = nx;
+  } else if (warp <= S) {
+    sa.diag[0][warp - 1][lane] = st.Gb[(warp - 1) * GBS + lane * (GL + 1)];
   }
   wsync();
   int m = 0;
-  while (true) {
-    const int l = *s_next;
+  for (;; ++m) {
+    const int par = m & 1, l = sa.next[par];
     if (l >= kb) break;
     if (warp == 0) {
-      scan.load_diag(dg, st.Gb + scan.sp * KK, KB, l + 1, kb);
-      if (lane == 0) s_pos[m] = l;
-    } else if (warp <= 2 * S) {
-      const int sp = (warp - 1) % S;
-      const double* gb = st.Gb + sp * KK;
-      if (warp <= S)
-        st.Ut[sp * KK + m * KB + lane] = s_f[sp] * gb[l * KB + lane];  // f G(x, l)
-      else
-        st.Wt[sp * KK + m * KB + lane] = ((lane == l) ? 1.0 : 0.0) - gb[lane * KB + l];  // delta - G(l, x)
-    }
-    const double f_acc = (cw >= 0) ? s_f[cw % S] : 0.0;  // before the scan replaces it
-    wsync();
-    if (warp == 0) {
-      const int nx = scan.next(w, dg, st.Ut + scan.sp * KK + m * KB, st.Wt + scan.sp * KK + m * KB, l + 1, kb, uni, fld,
-                               s_f, sign, acc_count);
-      if (lane == 0) *s_next = nx;
+      const double* gb = st.Gb + scan.sp * GBS;
+      const double* d = sa.diag[par][scan.sp];
+      const double f = sa.f[par][scan.sp];
+      const int nx = scan.next<2>(
+          w, [&](int, int x) { return fma(gb[x * GL + l], f * gb[l * GL + x], d[x]); }, l + 1, kb, uni, fld,
+          sa.f[par ^ 1], sign, acc_count);
+      if (lane == 0) {
+        sa.next[par ^ 1] = nx;
+        s_pos[m] = l;
+      }
     } else if (warp < 4) {
-      const int nc = kb - 1 - l;  // columns still to visit, then Gamma's
-      for (int q = warp - 1; q < S * (nc + m); q += 3) {
-        if (q < S * nc) {
-          const int sp = q >= nc ? 1 : 0, c = l + 1 + q - sp * nc;
-          if (lane > l && lane < kb)
-            st.Gb[sp * KK + c * KB + lane] = fma(-st.Ut[sp * KK + m * KB + lane], st.Wt[sp * KK + m * KB + c],
-                                                 st.Gb[sp * KK + c * KB + lane]);
-        } else {
-          const int g = q - S * nc, sp = g >= m ? 1 : 0;
-          gamma_column(sp, m - 1, g - sp * m);
+      double u[2] = {0.0, 0.0};
+#pragma unroll
+      for (int sp = 0; sp < 2; ++sp)
+        if (sp < S && lane > l) u[sp] = sa.f[par][sp] * st.Gb[sp * GBS + l * GL + lane];
+      if (warp <= S) {
+        const int sp = warp - 1;
+        const double us = sp ? u[1] : u[0], gr = (lane > l) ? st.Gb[sp * GBS + lane * GL + l] : 0.0;
+        st.Ut[sp * KK + m * KB + lane] = us;
+        st.Wt[sp * KK + m * KB + lane] = -gr;
+        sa.diag[par ^ 1][sp][lane] = fma(gr, us, sa.diag[par][sp][lane]);
+      }
+      const int nc = kb - 1 - l, nq = S * nc;  // columns past l
+      for (int q0 = warp - 1; q0 < nq; q0 += 12) {  // four columns' loads before their stores
+        double g[4], gl[4];
+        int at[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const int q = min(q0 + 3 * k, nq - 1), sp = q >= nc ? 1 : 0, c = l + 1 + q - sp * nc;
+          at[k] = sp * GBS + c * GL;
+          g[k] = st.Gb[at[k] + lane];
+          gl[k] = st.Gb[at[k] + l];
         }
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          if (q0 + 3 * k < nq && lane > l) st.Gb[at[k] + lane] = fma(gl[k], at[k] >= GBS ? u[1] : u[0], g[k]);
       }
     } else if (cw >= 0 && cw < 2 * S) {
       // a_m and b_m at compact index x = lane
       const int sp = cw % S, x = lane;
-      const double* ut = st.Ut + sp * KK;
-      const double* wt = st.Wt + sp * KK;
-      double* ac = st.Ac + sp * KK;
-      double* bc = st.Bc + sp * KK;
-      double v = (x == m) ? 1.0 : 0.0;
+      const double r0 = (x == m) ? 1.0 : 0.0;
       if (cw < S) {
-        for (int p = 0; p < m; ++p)
-          if (p >= x) v = fma(-wt[p * KB + l], ac[p * KB + x], v);
-        ac[m * KB + x] = (x <= m) ? f_acc * v : 0.0;
+        const double r = sub_chain<true>(st.Wt + sp * KK + l, st.Ac + sp * KK + x, m, r0);
+        st.Ac[sp * KK + m * KB + x] = (x <= m) ? sa.f[par][sp] * r : 0.0;
       } else {
-        for (int p = 0; p < m; ++p)
-          if (p >= x) v = fma(ut[p * KB + l], bc[p * KB + x], v);
-        bc[m * KB + x] = (x <= m) ? v : 0.0;
+        const double r = sub_chain<false>(st.Ut + sp * KK + l, st.Bc + sp * KK + x, m, r0);
+        st.Bc[sp * KK + m * KB + x] = (x <= m) ? r : 0.0;
       }
     }
     wsync();
-    ++m;
   }
-  if (m > 0) {  // the last accept's term
-    for (int q = warp; q < S * m; q += kSubThreads / 32) {
-      const int sp = q >= m ? 1 : 0;
-      gamma_column(sp, m - 1, q - sp * m);
-    }
-    wsync();
+  // Gamma, a column y per warp at a time, short and long columns in turn (lanes x)
+  for (int k = warp; k < S * m; k += kSubThreads / 32) {
+    const int sp = k % S, yy = k / S, y = (yy & 1) ? m - 1 - (yy >> 1) : (yy >> 1);
+    st.Gam[sp * KK + y * KB + lane] =
+        sub_chain<false>(st.Ac + sp * KK + y * KB + lane, st.Bc + sp * KK + y * KB + y, m - y, 0.0);
   }
+  wsync();
   return m;
 }
 
-// The slices of Gamma of a block with m accepts, and their exponents eGm [KB] (worker threads)
-__device__ __forceinline__ void sub_slice_gamma(const WalkerDev& w, int sp, int N, int m, const double* gam, int* eGm,
-                                                int* etmp) {
+// The slices of Gamma of a block with m accepts, both spins together, and their exponents eGm [KB]
+// per spin (worker threads)
+__device__ __forceinline__ void sub_slice_gamma(const WalkerDev& w, int S, int N, int m, const double* gam,
+                                                int* const* eGm, int* etmp) {
   const SubOff so = sub_offsets(N);
-  unsigned short* dGm[1] = {reinterpret_cast<unsigned short*>(w.msub + (size_t)sp * so.total + so.sGm)};
-  int* xGm[1] = {eGm};
-  slice_lines<1>([&](int, int line, int k) { return gam[k * KB + line]; }, 0, m, m, dGm, (long long)sub_sst(1), TM / 8,
-                 xGm, etmp);
+  unsigned short* dGm[2];
+  for (int sp = 0; sp < 2; ++sp)
+    dGm[sp] = reinterpret_cast<unsigned short*>(w.msub + (size_t)(sp < S ? sp : 0) * so.total + so.sGm);
+  auto get = [&](int sp, int line, int k) { return gam[sp * KK + k * KB + line]; };
+  if (S == 2) slice_lines<2>(get, 0, m, m, dGm, (long long)sub_sst(1), TM / 8, eGm, etmp);
+  else slice_lines<1>(get, 0, m, m, dGm, (long long)sub_sst(1), TM / 8, eGm, etmp);
 }
 
 // Spin sp of a block with m accepts at sites i0 + s_pos[q], Gamma's slices made: the row blocks
@@ -577,12 +609,12 @@ size_t submatrix_scratch_bytes(int N) { return sub_offsets(N).total; }
 
 // dynamic shared memory of the fused kernel: tensor-core operand buffers first (1024-byte
 // aligned base), then the slice's uniforms [N], Gamma [S][KK], the block state (overlaid by the
-// flush's G staging), the line exponents eG, eT, eR [N] and eGm [KB], the exponent scratch
+// flush's G staging), the line exponents eG, eT, eR [N], the exponent scratch
 // [2][256] and the fields [N]
 size_t submatrix_smem_bytes(int N, int S) {
   const size_t Nu = (size_t)((N + 1) & ~1);
   return (size_t)A_BYTES + (size_t)NBB * B_BYTES + sizeof(double) * (Nu + (size_t)S * KK) + sub_state_bytes(S) +
-         sizeof(int) * (3 * Nu + KB + 2 * kSubThreads) + (size_t)N;
+         sizeof(int) * (3 * Nu + 2 * kSubThreads) + (size_t)N;
 }
 
 // One slice for one walker per CTA: kSubCTA threads, the eight worker warps and the producer.
@@ -601,7 +633,7 @@ __global__ void __launch_bounds__(kSubCTA, 1) metropolis_sub_kernel(const Walker
   SubState st;
   st.Gam = uni + Nu;
   st.Gb = st.Gam + S * KK;
-  st.Ac = st.Gb + S * KK;
+  st.Ac = st.Gb + S * GBS;
   st.Bc = st.Ac + S * KK;
   st.Ut = st.Bc + S * KK;
   st.Wt = st.Ut + S * KK;
@@ -609,11 +641,10 @@ __global__ void __launch_bounds__(kSubCTA, 1) metropolis_sub_kernel(const Walker
   int* s_eG = reinterpret_cast<int*>(reinterpret_cast<unsigned char*>(st.Gb) + sub_state_bytes(S));
   int* s_eT = s_eG + Nu;
   int* s_eR = s_eT + Nu;
-  int* s_eGm = s_eR + Nu;
-  int* etmp = s_eGm + KB;                                               // [2][256]
+  int* etmp = s_eR + Nu;                                                // [2][256]
   int8_t* s_field = reinterpret_cast<int8_t*>(etmp + 2 * kSubThreads);  // [N]
-  __shared__ int s_next, s_pos[KB], s_m;
-  __shared__ double s_f[2];
+  __shared__ int s_pos[KB], s_m, s_eGm[2][KB];
+  __shared__ SubAccept s_acc;
   __shared__ __align__(8) unsigned long long bar_ldA, bar_ldB[NBB], bar_mma[2], bar_bfree[NBB], bar_accfree[2];
   __shared__ unsigned s_tmem;
   __shared__ int s_tcfail;
@@ -646,15 +677,18 @@ __global__ void __launch_bounds__(kSubCTA, 1) metropolis_sub_kernel(const Walker
     if (worker) {
       sub_load_block(st, G, S, N, i0, kb);
       wsync();
-      const int mm = sub_decide(w, S, kb, uni + i0, s_field + i0, st, s_pos, &s_next, s_f, sign, acc_count);
+      const int mm = sub_decide(w, S, kb, uni + i0, s_field + i0, st, s_pos, s_acc, sign, acc_count);
       if (tid == 0) s_m = mm;
     }
     __syncthreads();
     const int m = s_m;
     if (m == 0) continue;
+    if (worker) {
+      int* xGm[2] = {s_eGm[0], s_eGm[1]};
+      sub_slice_gamma(w, S, N, m, st.Gam, xGm, etmp);
+    }
     for (int sp = 0; sp < S; ++sp) {
-      if (worker) sub_slice_gamma(w, sp, N, m, st.Gam + sp * KK, s_eGm, etmp);
-      sub_prepare(tcs, gt, nA, w, sp, N, m, i0, s_pos, G[sp], s_eGm, s_eG, s_eR, s_eT, etmp, 0, (N + TM - 1) / TM);
+      sub_prepare(tcs, gt, nA, w, sp, N, m, i0, s_pos, G[sp], s_eGm[sp], s_eG, s_eR, s_eT, etmp, 0, (N + TM - 1) / TM);
       sub_flush(tcs, gt, nA, w, sp, N, m, G[sp], s_eG, s_eT, stage, 0, 1);
     }
   }
@@ -689,7 +723,7 @@ __global__ void __launch_bounds__(kSubCTA, 1) metropolis_sub_kernel(const Walker
 // buffers, the exponent scratch and eR of one row block; of the flush kernel: the operand
 // buffers, the G staging and the line exponents eG, eT [N]
 size_t submatrix_block_smem_bytes(int S) {
-  return sizeof(double) * (KB + 6ull * S * KK) + 2 * kSubThreads * sizeof(int) + KB;
+  return sizeof(double) * (KB + (size_t)S * (GBS + 5 * KK)) + 2 * kSubThreads * sizeof(int) + KB;
 }
 constexpr size_t kPrepSmem = (size_t)A_BYTES + (size_t)NBB * B_BYTES + 2 * kSubThreads * sizeof(int);
 size_t submatrix_flush_smem_bytes(int N) {
@@ -712,14 +746,14 @@ __global__ void __launch_bounds__(kSubThreads) metropolis_sub_block_kernel(const
   SubState st;
   st.Gam = uni + KB;
   st.Gb = st.Gam + S * KK;
-  st.Ac = st.Gb + S * KK;
+  st.Ac = st.Gb + S * GBS;
   st.Bc = st.Ac + S * KK;
   st.Ut = st.Bc + S * KK;
   st.Wt = st.Ut + S * KK;
   int* etmp = reinterpret_cast<int*>(st.Wt + S * KK);                   // [2][256]
   int8_t* s_field = reinterpret_cast<int8_t*>(etmp + 2 * kSubThreads);  // [KB]
-  __shared__ int s_next, s_pos[KB];
-  __shared__ double s_f[2];
+  __shared__ int s_pos[KB];
+  __shared__ SubAccept s_acc;
 
   const SubOff so = sub_offsets(N);
   const double* G[2] = {w.G, (S == 2) ? w.G + NN : w.G};
@@ -735,7 +769,7 @@ __global__ void __launch_bounds__(kSubThreads) metropolis_sub_block_kernel(const
   double sign = (tid < 32) ? *w.sign : 0.0;
   long long acc_count = 0;
   wsync();
-  const int m = sub_decide(w, S, kb, uni, s_field, st, s_pos, &s_next, s_f, sign, acc_count);
+  const int m = sub_decide(w, S, kb, uni, s_field, st, s_pos, s_acc, sign, acc_count);
   int8_t* frw = w.fields + (long long)eff * N + i0;
   for (int l = tid; l < kb; l += kSubThreads) frw[l] = s_field[l];
   if (tid == 0) {
@@ -745,10 +779,10 @@ __global__ void __launch_bounds__(kSubThreads) metropolis_sub_block_kernel(const
     *reinterpret_cast<int*>(w.msub + so.mc) = m;
   }
   if (tid < m) reinterpret_cast<int*>(w.msub + so.pos)[tid] = s_pos[tid];
-  if (m > 0)
-    for (int sp = 0; sp < S; ++sp)
-      sub_slice_gamma(w, sp, N, m, st.Gam + sp * KK,
-                      reinterpret_cast<int*>(w.msub + (size_t)sp * so.total + so.eGm), etmp);
+  if (m > 0) {
+    int* xGm[2] = {reinterpret_cast<int*>(w.msub + so.eGm), reinterpret_cast<int*>(w.msub + so.total + so.eGm)};
+    sub_slice_gamma(w, S, N, m, st.Gam, xGm, etmp);
+  }
 }
 
 // The mbarriers and the TMEM of a kernel that runs sub_gemm (every thread calls)
