@@ -13,6 +13,7 @@
 // Reference behaviour is the same as kernels_fp64.cu (src/dqmc_walker.cpp,
 // src/model/*.cpp, src/svd_stack.cpp, include/utils/numerical_stable.hpp,
 // src/measure/measure_methods.cpp); only the data placement differs.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -493,10 +494,25 @@ __global__ void __launch_bounds__(kMetroThreads) metropolis_general_kernel(const
 // Equal-time measurement on global G (general N); mode/j/q select the slot as
 // in the SMEM kernels.  after_stab = 1 measures the slot closing the step
 // with the fresh G (forward) or slot Lt-1 with the final G(0) (backward).
+//
+// A cluster of P CTAs per walker shares the pairs of 32-site tiles (I <= J); rank 0 adds the
+// parts, read from the other CTAs' shared memory, in rank order.  Unordered site pairs {i, j} are
+// visited once, 13 FP64 operations (9 with one spin matrix), with X = G_ij G_ji summed over spins
+// and the sites' sums n and differences m of 1 - G_ii:
+//   n(k)          ff_ij G_ji + ff_ji G_ij, spins summed (ff is not even on odd sides)
+//   SDW, CDW      (ff_ij + ff_ji) (m_i m_j - X), (n_i n_j - X)
+//   s-wave        Gu_ij Gd_ij + Gu_ji Gd_ji
+// The tile above the diagonal is read along its columns, the one below through shared memory.
+// FP64 throughput of one SM and the strided reads of G(j, i) bounded the one-CTA form: 264 us a
+// slice for 6 walkers of two spins at N = 256, 222 us for 128 walkers of one.
 // --------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) measure_general_kernel(const WalkerDev* __restrict__ W, int mode, int j, int q,
-                                                              int after_stab) {
-  const WalkerDev& w = W[blockIdx.x];
+template <int P>
+__global__ void __launch_bounds__(256) __cluster_dims__(P, 1, 1)
+    measure_general_kernel(const WalkerDev* __restrict__ W, int mode, int j, int q, int after_stab) {
+  namespace cg = cooperative_groups;
+  const WalkerDev& w = W[blockIdx.y];
+  const int rank = blockIdx.x;
+  // the whole cluster leaves or stays
   if (!is_general(w)) return;
   double sg;
   if (after_stab) {
@@ -510,109 +526,148 @@ __global__ void __launch_bounds__(256) measure_general_kernel(const WalkerDev* _
     if (!here) return;
     sg = *w.sign;
   }
-  const int N = w.N, L = w.L;
+  const int N = w.N, L = w.L, LL = L * L;
   const long long NN = (long long)N * N;
-  const double* gu = w.G;
-  const double* gd = (w.S == 2) ? w.G + NN : w.G;
-  extern __shared__ double sh[];
-  double* du = sh;
-  double* dd = sh + N;
-  __shared__ double red[8 * 8];
-  for (int i = threadIdx.x; i < N; i += blockDim.x) {
-    du[i] = 1.0 - gu[(long long)i * N + i];
-    dd[i] = 1.0 - gd[(long long)i * N + i];
-  }
-  __syncthreads();
-  // The pair sums run with the separable parts factored out (per column jj the lane
-  // sums c_u = sum_i ff(jj - i) du_i and c_d) and the i = jj terms corrected in the
-  // site loop, so a pair costs 8 FP64 operations (5 with one spin matrix) instead of 14:
-  //   v4 = sum ff (Gu_ji + Gd_ji),  v5 = sum ff (du_i du_j + dd_i dd_j + guc Gu_ij + gdc Gd_ij),
-  //   v6 = sum ff (dd_i du_j + du_i dd_j),  v7 = sum guc gdc,  guc = delta_ij - Gu_ji.
   const bool one = (w.S == 1);
-  const double ff0 = w.ff[0];
+  const double* gu = w.G;
+  const double* gd = one ? w.G : w.G + NN;
+  extern __shared__ double sh[];
+  double* sn = sh;           // n_i = (1 - gu_ii) + (1 - gd_ii)
+  double* sm = sh + N;       // m_i = (1 - gu_ii) - (1 - gd_ii)
+  double* ff = sh + 2 * N;
+  int* sxyz = reinterpret_cast<int*>(ff + N);  // x | y << 10 | z << 20
+  __shared__ double s_t[2][32][33];            // the tiles below the diagonal, [spin][i][j]
+  __shared__ double red[8 * 8], part[8];
   double v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  for (int i = threadIdx.x; i < N; i += blockDim.x) {
-    const double a = 1.0 - du[i], b = 1.0 - dd[i];
-    v[0] += a + b;
-    v[1] += du[i] * dd[i];
-    v[2] += a + b - 2 * a * b;
-    // bonds to the +x, +y (, +z) neighbours (measure_methods.cpp:87-95)
-    const int jx = site_nn(L, i, 0), jy = site_nn(L, i, 1);
-    double kin = gu[(long long)jx * N + i] + gd[(long long)jx * N + i] + gu[(long long)jy * N + i] + gd[(long long)jy * N + i];
-    if (w.dim == 3) {
-      const int jz = site_nn(L, i, 2);
-      kin += gu[(long long)jz * N + i] + gd[(long long)jz * N + i];
-    }
-    v[3] += kin;
-    // i = jj: the pair loop's off-diagonal forms give -ff0 (Gu_ii^2 + Gd_ii^2) and Gu_ii Gd_ii
-    v[5] += ff0 * (a + b);
-    v[7] += du[i] * dd[i] - a * b;
-  }
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  double p4 = 0.0, p5 = 0.0;  // pair parts of v4 and v5 (one spin matrix: doubled below)
-  const int dim = w.dim;
-  for (int jj = wid; jj < N; jj += blockDim.x >> 5) {
-    const int xj = jj % L, yj = jj / L;
-    double cu = 0.0, cd = 0.0;
-    for (int i = lane; i < N; i += 32) {
-      int r;
-      if (dim == 2) {
-        int dx = xj - i % L, dy = yj - i / L;
-        dx += (dx < 0) ? L : 0;
-        dy += (dy < 0) ? L : 0;
-        r = dx + dy * L;
-      } else {
-        r = site_disp(L, 3, i, jj);
+  for (int i = threadIdx.x; i < N; i += 256) {
+    const double a = gu[(long long)i * N + i], b = gd[(long long)i * N + i];
+    const double du = 1.0 - a, dd = 1.0 - b, n = du + dd, mm = du - dd;
+    sn[i] = n;
+    sm[i] = mm;
+    ff[i] = w.ff[i];
+    sxyz[i] = (i % L) | ((i / L) % L) << 10 | (i / LL) << 20;  // z = 0 on the square lattice
+    if (rank == 0) {
+      const double ab = a + b, x = fma(du, a, dd * b);
+      v[0] += ab;
+      v[1] = fma(du, dd, v[1]);
+      v[2] += fma(-2.0 * a, b, ab);
+      // bonds to the +x, +y (, +z) neighbours (measure_methods.cpp:87-95)
+      for (int d = 0; d < w.dim; ++d) {
+        const long long c = (long long)site_nn(L, i, d) * N + i;
+        v[3] += gu[c] + gd[c];
       }
-      const double ff = w.ff[r];
-      const double gu_ij = gu[(long long)jj * N + i], gu_ji = gu[(long long)i * N + jj];
-      cu = fma(ff, du[i], cu);
-      if (one) {
-        p4 = fma(ff, gu_ji, p4);
-        p5 = fma(-ff, gu_ji * gu_ij, p5);
-        v[7] = fma(gu_ji, gu_ji, v[7]);
-      } else {
-        const double gd_ij = gd[(long long)jj * N + i], gd_ji = gd[(long long)i * N + jj];
-        cd = fma(ff, dd[i], cd);
-        p4 = fma(ff, gu_ji + gd_ji, p4);
-        p5 = fma(-ff, fma(gd_ji, gd_ij, gu_ji * gu_ij), p5);
-        v[7] = fma(gu_ji, gd_ji, v[7]);
-      }
+      // the pair i = j (Fourier factor 1)
+      v[4] += ab;
+      v[5] += fma(mm, mm, x);
+      v[6] += fma(n, n, x);
+      v[7] = fma(du, dd, v[7]);
     }
-    if (one) {
-      v[5] = fma(2.0 * du[jj], cu, v[5]);
-      v[6] = fma(2.0 * du[jj], cu, v[6]);
-    } else {
-      v[5] += du[jj] * cu + dd[jj] * cd;
-      v[6] += du[jj] * cd + dd[jj] * cu;
-    }
-  }
-  v[4] += one ? 2.0 * p4 : p4;
-  v[5] += one ? 2.0 * p5 : p5;
-  for (int k = 0; k < 8; ++k) {
-    const double s = warp_sum_g(v[k]);
-    if (lane == 0) red[k * 8 + wid] = s;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    double tot[8];
-    for (int k = 0; k < 8; ++k) {
-      tot[k] = 0;
-      for (int q2 = 0; q2 < (int)(blockDim.x >> 5); ++q2) tot[k] += red[k * 8 + q2];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int nt = (N + 31) / 32;
+  double p4 = 0.0, p5 = 0.0, p6 = 0.0, p7 = 0.0;
+  int k = 0;  // tile pairs, dealt to the CTAs in turn
+  for (int tj = 0; tj < nt; ++tj)
+    for (int ti = 0; ti <= tj; ++ti, ++k) {
+      if (k % P != rank) continue;
+      const int i0 = ti * 32, j0 = tj * 32, i = i0 + lane;
+      __syncthreads();  // the previous tile's readers are done
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {  // column i of the tile below: G(j, i), lanes along j
+        const int c = wid + 8 * u;
+        const bool in = j0 + lane < N && i0 + c < N;
+        s_t[0][c][lane] = in ? gu[(long long)(i0 + c) * N + j0 + lane] : 0.0;
+        if (!one) s_t[1][c][lane] = in ? gd[(long long)(i0 + c) * N + j0 + lane] : 0.0;
+      }
+      double gij[2][4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int jj = j0 + wid + 8 * u;
+        const bool in = i < N && jj < N;
+        gij[0][u] = in ? gu[(long long)jj * N + i] : 0.0;
+        gij[1][u] = (in && !one) ? gd[(long long)jj * N + i] : 0.0;
+      }
+      __syncthreads();
+      const int ci = (i < N) ? sxyz[i] : 0, xi = ci & 1023, yi = (ci >> 10) & 1023, zi = ci >> 20;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int cj = wid + 8 * u, jj = j0 + cj;
+        if (jj >= N) continue;  // uniform in the warp
+        if (i >= N || i >= jj) continue;
+        const int c = sxyz[jj], dx = (c & 1023) - xi, dy = ((c >> 10) & 1023) - yi, dz = (c >> 20) - zi;
+        const double f_ij = ff[(dx + (dx < 0 ? L : 0)) + (dy + (dy < 0 ? L : 0)) * L + (dz + (dz < 0 ? L : 0)) * LL];
+        const double f_ji = ff[(-dx + (dx > 0 ? L : 0)) + (-dy + (dy > 0 ? L : 0)) * L + (-dz + (dz > 0 ? L : 0)) * LL];
+        const double f = f_ij + f_ji, a = gij[0][u], at = s_t[0][lane][cj];
+        if (one) {  // m = 0; the spins' factor 2 of n(k) and X follows the loop
+          const double x = a * at;
+          p4 = fma(f_ij, at, p4);
+          p4 = fma(f_ji, a, p4);
+          p5 = fma(f, x, p5);
+          p6 = fma(f, fma(0.5 * sn[i], sn[jj], -x), p6);
+          p7 = fma(a, a, p7);
+          p7 = fma(at, at, p7);
+        } else {
+          const double b = gij[1][u], bt = s_t[1][lane][cj];
+          const double x = fma(b, bt, a * at);
+          p4 = fma(f_ij, at + bt, p4);
+          p4 = fma(f_ji, a + b, p4);
+          p5 = fma(f, fma(sm[i], sm[jj], -x), p5);
+          p6 = fma(f, fma(sn[i], sn[jj], -x), p6);
+          p7 = fma(a, b, p7);
+          p7 = fma(at, bt, p7);
+        }
+      }
+    }
+  v[4] += one ? 2.0 * p4 : p4;
+  v[5] += one ? -2.0 * p5 : p5;
+  v[6] += one ? 2.0 * p6 : p6;
+  v[7] += p7;
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {
+    const double s = warp_sum_g(v[e]);
+    if (lane == 0) red[e * 8 + wid] = s;
+  }
+  __syncthreads();
+  if (threadIdx.x < 8) {
+    double s = 0.0;
+    for (int e = 0; e < 8; ++e) s += red[threadIdx.x * 8 + e];
+    part[threadIdx.x] = s;
+  }
+  cg::cluster_group cl = cg::this_cluster();
+  if (P > 1) cl.sync();
+  else __syncthreads();
+  if (rank == 0 && threadIdx.x < kNumObs) {
+    // thread k adds observable k
+    const int o = threadIdx.x;
+    const int src[kNumObs] = {0, 1, 3, 4, 2, 5, 6, 7, 0};
+    double tot = 0.0;
+    for (int p = 0; p < P; ++p) {
+      const double* rp = (P > 1) ? cl.map_shared_rank(part, p) : part;
+      tot += rp[src[o]];
     }
     const double n = (double)N;
-    double* o = w.obs;
-    o[0] += sg * (2.0 - tot[0] / n);
-    o[1] += sg * tot[1] / n;
-    o[2] += sg * (2.0 * w.hop_t) * tot[3] / n;
-    o[3] += sg * (1.0 - 0.5 * tot[4] / n);
-    o[4] += sg * tot[2] / n;
-    o[5] += sg * (tot[5] - tot[6]) / (n * n);
-    o[6] += sg * (tot[5] + tot[6]) / (n * n);
-    o[7] += sg * tot[7] / n;
-    o[8] += sg;
-    for (int k = 0; k < kNumObs; ++k) w.obs_cnt[k] += 1;
+    double add = sg * tot / n;
+    if (o == 0) add = sg * (2.0 - tot / n);
+    if (o == 2) add = sg * (2.0 * w.hop_t) * tot / n;
+    if (o == 3) add = sg * (1.0 - 0.5 * tot / n);
+    if (o == 5 || o == 6) add = sg * tot / (n * n);
+    if (o == 8) add = sg;
+    w.obs[o] += add;
+    w.obs_cnt[o] += 1;
   }
+  if (P > 1) cl.sync();  // the parts stay until rank 0 has read them
+}
+
+// CTAs per walker: the tile pairs of the largest walker, at most a portable cluster of 8
+static void launch_measure_general(const WalkerDev* W, int nw, int maxN, int mode, int j, int q, int after_stab,
+                                   cudaStream_t st) {
+  const int nt = (maxN + 31) / 32, pairs = nt * (nt + 1) / 2;
+  const size_t sm = (size_t)maxN * (3 * sizeof(double) + sizeof(int));
+  if (pairs >= 8) measure_general_kernel<8><<<dim3(8, nw), 256, sm, st>>>(W, mode, j, q, after_stab);
+  else if (pairs >= 4) measure_general_kernel<4><<<dim3(4, nw), 256, sm, st>>>(W, mode, j, q, after_stab);
+  else if (pairs >= 2) measure_general_kernel<2><<<dim3(2, nw), 256, sm, st>>>(W, mode, j, q, after_stab);
+  else measure_general_kernel<1><<<dim3(1, nw), 256, sm, st>>>(W, mode, j, q, after_stab);
 }
 
 // --------------------------------------------------------------------------
@@ -1314,7 +1369,7 @@ void general_slice_metro(int mode, const WalkerDev* W, int nw, int j, int q, int
   else if (mixed && tc_flush == 3) launch_metropolis_sub_split(W, nw, mode, j, q, maxN, smax, st);
   else if (kd > 0) launch_metropolis_delayed(mixed, W, nw, mode, j, q, maxN, smax, kd, tc_flush, st);
   else metropolis_general_kernel<<<nw, kMetroThreads, met_sm, st>>>(W, mode, j, q);
-  if (measure) measure_general_kernel<<<nw, 256, sizeof(double) * 2 * maxN, st>>>(W, mode, j, q, 0);
+  if (measure) launch_measure_general(W, nw, maxN, mode, j, q, 0, st);
 }
 
 void general_slice_post(int mode, const WalkerDev* W, int nw, int j, int q, int maxN, bool any_dense, bool any_cb,
@@ -1435,7 +1490,7 @@ void general_greens(int mode, const WalkerDev* W, int nw, int j, int trace_slot,
 }
 
 void general_measure_after(int mode, const WalkerDev* W, int nw, int j, int maxN, cudaStream_t st) {
-  measure_general_kernel<<<nw, 256, sizeof(double) * 2 * maxN, st>>>(W, mode, j, 0, 1);
+  launch_measure_general(W, nw, maxN, mode, j, 0, 1, st);
 }
 
 void general_sign(const WalkerDev* W, int nw, int maxN, cudaStream_t st) {
