@@ -220,6 +220,22 @@ std::vector<double> fourier_table(int L, int kidx, int dim) {
   return f;
 }
 
+// The ring exponentials whose Kronecker product, one factor per direction, is exp(-dtau K) ([0][L],
+// entries by distance) or exp(+dtau K) ([1][L]) of the square or cubic lattice: K is a sum over
+// directions, so exp(-dtau K)(r, 0) = e(x) e(y) (e(z)) with exp(-dtau mu) shared out among the
+// factors.  They are read off the dense pair, so that the factored and the dense products use the
+// same exponentials to rounding (the pair's own error, that of the diagonalisation, sets the
+// wrap error of a sweep).
+std::vector<double> ring_exponentials(int L, int dim, const std::pair<std::vector<double>, std::vector<double>>& k) {
+  std::vector<double> e(2 * (size_t)L);
+  for (int inv = 0; inv < 2; ++inv) {
+    const std::vector<double>& m = inv ? k.second : k.first;  // column 0: sites 0 .. L - 1 lie along x
+    const double e0 = (dim == 2) ? std::sqrt(m[0]) : std::cbrt(m[0]), rest = (dim == 2) ? e0 : e0 * e0;
+    for (int d = 0; d < L; ++d) e[(size_t)inv * L + d] = m[d] / rest;
+  }
+  return e;
+}
+
 size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 // exp(-dtau K) and exp(+dtau K) of a lattice, kept for the life of the process: the Jacobi
@@ -473,12 +489,16 @@ int dqmc_batch_create(const dqmc_walker_desc* descs, int n, const dqmc_batch_opt
     if (!ff_off.count(fk)) ff_off[fk] = take(sizeof(double) * N);
     off[w].ff = ff_off[fk];
   }
-  std::vector<size_t> dense_off(dense.size()), dense_sl(dense.size()), dense_sle(dense.size());
+  std::vector<size_t> dense_off(dense.size()), dense_sl(dense.size()), dense_sle(dense.size()), dense_kin(dense.size());
+  std::vector<std::vector<double>> rings(dense.size());
+  for (auto& kv : dense_ids)
+    rings[kv.second] = ring_exponentials(std::get<0>(kv.first), std::get<1>(kv.first), dense[kv.second]);
   std::vector<int> dense_n(dense.size());
   for (auto& kv : dense_ids) dense_n[kv.second] = lattice_sites(std::get<0>(kv.first), std::get<1>(kv.first));
   for (size_t i = 0; i < dense.size(); ++i) {
     const size_t nn = dense[i].first.size();
     dense_off[i] = take(sizeof(double) * 2 * nn);
+    dense_kin[i] = take(sizeof(double) * rings[i].size());
     if (o.precision == DQMC_MIXED) {  // 4 sliced copies: expK (A, B roles), invK (A, B roles)
       const int N = dense_n[i], ldk = (N + 15) / 16 * 16;
       dense_sl[i] = take(sizeof(unsigned short) * 4 * ozaki::kMaxSlices * ozaki::tc_slice_elems(N, ldk));
@@ -544,6 +564,8 @@ int dqmc_batch_create(const dqmc_walker_desc* descs, int n, const dqmc_batch_opt
     cudaMemcpyAsync(base + dense_off[i], dense[i].first.data(), sizeof(double) * nn, cudaMemcpyHostToDevice, b->stream);
     cudaMemcpyAsync(base + dense_off[i] + sizeof(double) * nn, dense[i].second.data(), sizeof(double) * nn,
                     cudaMemcpyHostToDevice, b->stream);
+    cudaMemcpyAsync(base + dense_kin[i], rings[i].data(), sizeof(double) * rings[i].size(), cudaMemcpyHostToDevice,
+                    b->stream);
     if (o.precision == DQMC_MIXED) {
       const int N = dense_n[i], ldk = (N + 15) / 16 * 16;
       const auto c = ozaki::cfg_for_k(N);
@@ -607,8 +629,9 @@ int dqmc_batch_create(const dqmc_walker_desc* descs, int n, const dqmc_batch_opt
     h.cb_h = std::tanh(dtau * d.hopping_t);
     for (int inv = 0; inv < 2; ++inv) {
       const double f = inv ? h.cbI[0] : h.cbP[0];  // exp(+-dtau mu / 2) cosh^2
-      h.cb_e[inv][0] = h.e_pa * (f * f);
-      h.cb_e[inv][1] = h.e_ma * (f * f);
+      const double c = d.checkerboard ? f * f : 1.0;
+      h.kin_e[inv][0] = h.e_pa * c;
+      h.kin_e[inv][1] = h.e_ma * c;
     }
     h.G = reinterpret_cast<double*>(base + off[w].G);
     h.chain = reinterpret_cast<double*>(base + off[w].chain);
@@ -642,6 +665,7 @@ int dqmc_batch_create(const dqmc_walker_desc* descs, int n, const dqmc_batch_opt
     if (off[w].dense_id >= 0) {
       h.expK = reinterpret_cast<const double*>(base + dense_off[off[w].dense_id]);
       h.invK = h.expK + (size_t)N * N;
+      h.kin = reinterpret_cast<const double*>(base + dense_kin[off[w].dense_id]);
     }
     h.ff = reinterpret_cast<const double*>(base + off[w].ff);
     dqmc_batch::Scal* sc = b->d_scal + w;

@@ -42,9 +42,13 @@ struct WalkerDev {
   // ratio constants indexed by [s>0 ? 0 : 1]: exp(-2 alpha s) - 1, exp(+2 alpha s) - 1, exp(2 alpha s)
   double cm[2], cp[2], ex2[2];
   double cbP[16], cbI[16];   // checkerboard plaquettes exp(+dtau t h) e^{0.5 dtau mu}, inverse
-  // the plaquette as f c^2 [[1, h], [h, 1]] (x) [[1, h], [h, 1]]: h (its inverse has -h), and
-  // exp(+alpha), exp(-alpha) times (f c^2)^2 of the two passes of a product ([1]: of the inverse)
-  double cb_h, cb_e[2][2];
+  // Factored exp(-+dtau K), index [0] and its inverse [1].  Checkerboard: the plaquette is
+  // f c^2 [[1, h], [h, 1]] (x) [[1, h], [h, 1]] (its inverse has -h).  Otherwise the Kronecker
+  // product of one ring exponential per direction: kin [2][L], by the distance |x - x'| on the ring
+  // of L sites.  kin_e: exp(+alpha), exp(-alpha), for checkerboard walkers times the (f c^2)^2 of a
+  // product's two passes.
+  double cb_h, kin_e[2][2];
+  const double* kin;
   double* G;                 // [2][N*N]
   double* chain;             // [S][N*N] (general walkers: [2][S][N*N], ping-pong)
   double* work;              // general walkers: GEMM temporary [S][N*N]
@@ -228,6 +232,47 @@ struct SiteScan {
     return N;
   }
 };
+
+// The sites of plaquette q of a checkerboard layer (corner (x, y), x and y of the layer's parity)
+__device__ __forceinline__ void plaq_sites(int L, int q, int parity, int (&idx)[4]) {
+  const int half = L >> 1;
+  const int x = 2 * (q % half) + parity, y = 2 * (q / half) + parity;
+  const int x1 = (x + 1) % L, y1 = (y + 1) % L;
+  idx[0] = x + L * y;
+  idx[1] = x1 + L * y;
+  idx[2] = x + L * y1;
+  idx[3] = x1 + L * y1;
+}
+
+// The plaquette matrix is f c^2 [[1, h], [h, 1]] (x) [[1, h], [h, 1]] with c = cosh, h = tanh of
+// +-dtau t: applied as two butterflies of 8 FMAs on the plaquette's 4 values instead of a 4 x 4
+// product of 4 multiplies and 12 FMAs (an FP64 warp instruction holds its pipe for 64 cycles,
+// and the passes are half of a checkerboard slice's FP64 work).  The factors f c^2 of a product's
+// two passes are folded into the diagonal scale of the product (bdiag).
+__device__ __forceinline__ void plaq_apply(double (&v)[4], double h) {
+  const double a0 = fma(h, v[1], v[0]), a1 = fma(h, v[0], v[1]);
+  const double a2 = fma(h, v[3], v[2]), a3 = fma(h, v[2], v[3]);
+  v[0] = fma(h, a2, a0);
+  v[1] = fma(h, a3, a1);
+  v[2] = fma(h, a0, a2);
+  v[3] = fma(h, a1, a3);
+}
+
+// The plain 4 x 4 product: the set-up keeps it, because the sign it takes from an LU of the
+// initial G is rounding noise once G has eigenvalues below its rounding (8 x 8 at beta = 8), and
+// a given seed has to keep its sign.
+__device__ __forceinline__ void plaq_product(double (&v)[4], const double* P) {
+  double o[4];
+#pragma unroll
+  for (int a = 0; a < 4; ++a) {
+    o[a] = P[a * 4 + 0] * v[0];
+    o[a] = fma(P[a * 4 + 1], v[1], o[a]);
+    o[a] = fma(P[a * 4 + 2], v[2], o[a]);
+    o[a] = fma(P[a * 4 + 3], v[3], o[a]);
+  }
+#pragma unroll
+  for (int a = 0; a < 4; ++a) v[a] = o[a];
+}
 
 // Site i of a walker's lattice is x + L y (+ L^2 z).  The displacement from site i to site j
 // as the site index of its vector, each component mod L (src/lattice/square.cpp:88-105,

@@ -79,7 +79,7 @@ __device__ __forceinline__ int spin_sign(const WalkerDev& w, int spin) {
 // exp(+/- alpha) for the product sgn * s, with the checkerboard products' constant factor folded
 // in when fold (inv: of the products with exp(+dtau K))
 __device__ __forceinline__ double bdiag(const WalkerDev& w, int sgn_times_s, int inv, bool fold) {
-  if (fold && w.cb) return w.cb_e[inv][sgn_times_s > 0 ? 0 : 1];
+  if (fold) return w.kin_e[inv][sgn_times_s > 0 ? 0 : 1];
   return sgn_times_s > 0 ? w.e_pa : w.e_ma;
 }
 
@@ -91,88 +91,28 @@ __device__ __forceinline__ double bdiag(const WalkerDev& w, int sgn_times_s, int
 //   left pass : rows r_a  <- sum_b P[a][b] rows r_b     (optionally pre/post-scaled)
 //   right pass: cols c_b  <- sum_a cols c_a P[a][b]
 // --------------------------------------------------------------------------
-__device__ __forceinline__ void plaq_sites(int L, int q, int parity, int (&idx)[4]) {
-  const int half = L >> 1;
-  const int x = 2 * (q % half) + parity, y = 2 * (q / half) + parity;
-  const int x1 = (x + 1) % L, y1 = (y + 1) % L;
-  idx[0] = x + L * y;
-  idx[1] = x1 + L * y;
-  idx[2] = x + L * y1;
-  idx[3] = x1 + L * y1;
-}
-
-// The plaquette matrix is f c^2 [[1, h], [h, 1]] (x) [[1, h], [h, 1]] with c = cosh, h = tanh of
-// +-dtau t: applied as two butterflies of 8 FMAs on the plaquette's 4 values instead of a 4 x 4
-// product of 4 multiplies and 12 FMAs (an FP64 warp instruction holds its pipe for 64 cycles,
-// and the passes are half of a checkerboard slice's FP64 work).  The factors f c^2 of a product's
-// two passes are folded into the diagonal scale of the product (bdiag).
-__device__ __forceinline__ void plaq_apply(double (&v)[4], double h) {
-  const double a0 = fma(h, v[1], v[0]), a1 = fma(h, v[0], v[1]);
-  const double a2 = fma(h, v[3], v[2]), a3 = fma(h, v[2], v[3]);
-  v[0] = fma(h, a2, a0);
-  v[1] = fma(h, a3, a1);
-  v[2] = fma(h, a0, a2);
-  v[3] = fma(h, a1, a3);
-}
-
-// The plain 4 x 4 product: the set-up keeps it, because the sign it takes from an LU of the
-// initial G is rounding noise once G has eigenvalues below its rounding (8 x 8 at beta = 8), and
-// a given seed has to keep its sign.
-__device__ __forceinline__ void plaq_product(double (&v)[4], const double* P) {
-  double o[4];
-#pragma unroll
-  for (int a = 0; a < 4; ++a) {
-    o[a] = P[a * 4 + 0] * v[0];
-    o[a] = fma(P[a * 4 + 1], v[1], o[a]);
-    o[a] = fma(P[a * 4 + 2], v[2], o[a]);
-    o[a] = fma(P[a * 4 + 3], v[3], o[a]);
-  }
-#pragma unroll
-  for (int a = 0; a < 4; ++a) v[a] = o[a];
-}
-
-// pre: scale inputs by pre[row] (null = none); post likewise on outputs; P: plain product
-__device__ void cb_left(double* M, int ld, int N, int L, int parity, double h, const double* pre,
-                        const double* post, const double* P = nullptr) {
+// One layer's pass: rows (left) or, RIGHT, columns of every plaquette; PRE scales the inputs by d
+// at their site, POST the outputs
+template <bool RIGHT, bool PRE, bool POST, bool PLAIN>
+__device__ __forceinline__ void cb_pass(double* M, int ld, int N, int L, int parity, double h, const double* d,
+                                        const double* P) {
   const int nq = (L >> 1) * (L >> 1);
   for (int it = threadIdx.x; it < nq * N; it += kThreads) {
-    const int q = it % nq, c = it / nq;
+    const int q = RIGHT ? it / N : it % nq, x = RIGHT ? it % N : it / nq;
     int idx[4];
     plaq_sites(L, q, parity, idx);
     double v[4];
 #pragma unroll
     for (int a = 0; a < 4; ++a) {
-      v[a] = at(M, ld, idx[a], c);
-      if (pre) v[a] *= pre[idx[a]];
+      v[a] = RIGHT ? at(M, ld, x, idx[a]) : at(M, ld, idx[a], x);
+      if (PRE) v[a] *= d[idx[a]];
     }
-    if (P) plaq_product(v, P);
+    if (PLAIN) plaq_product(v, P);
     else plaq_apply(v, h);
 #pragma unroll
     for (int a = 0; a < 4; ++a) {
-      if (post) v[a] *= post[idx[a]];
-      at(M, ld, idx[a], c) = v[a];
-    }
-  }
-}
-
-__device__ void cb_right(double* M, int ld, int N, int L, int parity, double h, const double* pre,
-                         const double* post) {
-  const int nq = (L >> 1) * (L >> 1);
-  for (int it = threadIdx.x; it < nq * N; it += kThreads) {
-    const int r = it % N, q = it / N;
-    int idx[4];
-    plaq_sites(L, q, parity, idx);
-    double v[4];
-#pragma unroll
-    for (int a = 0; a < 4; ++a) {
-      v[a] = at(M, ld, r, idx[a]);
-      if (pre) v[a] *= pre[idx[a]];
-    }
-    plaq_apply(v, h);
-#pragma unroll
-    for (int b = 0; b < 4; ++b) {
-      if (post) v[b] *= post[idx[b]];
-      at(M, ld, r, idx[b]) = v[b];
+      if (POST) v[a] *= d[idx[a]];
+      (RIGHT ? at(M, ld, x, idx[a]) : at(M, ld, idx[a], x)) = v[a];
     }
   }
 }
@@ -244,83 +184,87 @@ __device__ __forceinline__ void block_gemm(int N, FA A, FB B, FS store, int kbeg
 }
 
 // --------------------------------------------------------------------------
-// B-matrix products on a matrix M (ld) for slice t (uses field row t-1).
-// sd[i] holds the row/col scale of the current slice and spin.
+// B-matrix products for one slice on the nm matrices M, M + ms, ... (leading dimension ld; the
+// spins of a walker), in place.  exp(-+dtau K) is applied in its factors: the two plaquette layers
+// of a checkerboard walker, else one ring exponential per lattice direction (2 L or 3 L FMAs an
+// element instead of N, two or three passes over the matrix).  Each pass writes every element
+// from the L elements of its line, M -> tmp and back (tmp: nm matrices, leading dimension ldt).
+//   RIGHT 0: M <- post A pre M (rows),  1: M <- M pre A post (columns),  A = exp(-dtau K) or, INV,
+//   its inverse; sc: the diagonal, applied first (PRE) or last, of matrix m at sc + m * scs.
+//   PLAIN: the plain plaquette product (plaq_product), sc without the constant factor.
 // --------------------------------------------------------------------------
-// M <- B(t) M = diag(e^{+sa s}) expK M   (mult_B_from_left)
-__device__ void mult_B_left(const WalkerDev& w, double* M, int ld, const double* dpos) {
-  const int N = w.N;
+// k / d as (k mul) >> 20 with mul = small_div_mul(d): exact for k d < 2^20 (here k < 2 N^2, d <= N <= 64)
+__device__ __forceinline__ unsigned small_div_mul(int d) { return ((1u << 20) + d - 1) / d; }
+__device__ __forceinline__ int small_div(int k, unsigned mul) { return (int)(((unsigned)k * mul) >> 20); }
+template <bool RIGHT, bool INV, bool PRE, bool PLAIN = false>
+__device__ __noinline__ void kin_product(const WalkerDev& w, double* M, int ms, int ld, int nm,
+                                         double* tmp, int tms, int ldt, const double* sc, int scs,
+                                         const double* ring) {
+  const int N = w.N, L = w.L, NN = N * N;
   if (w.cb) {
-    cb_left(M, ld, N, w.L, 1, w.cb_h, nullptr, nullptr);  // sublattice B first
-    __syncthreads();
-    cb_left(M, ld, N, w.L, 0, w.cb_h, nullptr, dpos);     // then A, scale rows
-    __syncthreads();
-  } else {
-    const double* K = w.expK;
-    block_gemm(N, [&](int r, int k) { return __ldg(K + (long long)k * N + r); },
-               [&](int k, int c) { return at(M, ld, k, c); },
-               [&](int r, int c, double v) { at(M, ld, r, c) = v * dpos[r]; });
+    // B M and M B^-1: layer B (parity 1) then A; B^T M, M B and B^-1 M: A then B
+    for (int m = 0; m < nm; ++m) {
+      double* X = M + (long long)m * ms;
+      const double* d = sc + m * scs;
+      const double h = INV ? -w.cb_h : w.cb_h;
+      const int p0 = PRE ? 0 : 1;
+      cb_pass<RIGHT, PRE, false, PLAIN>(X, ld, N, L, p0, h, d, w.cbP);
+      __syncthreads();
+      cb_pass<RIGHT, false, !PRE, PLAIN>(X, ld, N, L, p0 ^ 1, h, d, w.cbP);
+      __syncthreads();
+    }
+    return;
   }
-}
-// M <- M B(t)^-1 = M expK^-1 diag(e^{-sa s})   (mult_invB_from_right)
-__device__ void mult_invB_right(const WalkerDev& w, double* M, int ld, const double* dneg) {
-  const int N = w.N;
-  if (w.cb) {
-    cb_right(M, ld, N, w.L, 1, -w.cb_h, nullptr, nullptr);  // B then A
+  const double* e = ring + (INV ? L : 0);
+  const unsigned dN = small_div_mul(N), dL = small_div_mul(L);
+  // element k: matrix m, row r, column c
+  auto split = [&](int k, int& m, int& r, int& c) {
+    m = (k >= NN) ? 1 : 0;
+    c = small_div(k - m * NN, dN);
+    r = k - m * NN - c * N;
+  };
+  if (PRE) {
+    for (int k = threadIdx.x; k < nm * NN; k += kThreads) {
+      int m, r, c;
+      split(k, m, r, c);
+      M[(long long)m * ms + c * ld + r] *= sc[m * scs + (RIGHT ? c : r)];
+    }
     __syncthreads();
-    cb_right(M, ld, N, w.L, 0, -w.cb_h, nullptr, dneg);
-    __syncthreads();
-  } else {
-    const double* K = w.invK;
-    block_gemm(N, [&](int r, int k) { return at(M, ld, r, k); },
-               [&](int k, int c) { return __ldg(K + (long long)c * N + k); },
-               [&](int r, int c, double v) { at(M, ld, r, c) = v * dneg[c]; });
   }
-}
-// M <- M B(t) = M diag(e^{+sa s}) expK   (mult_B_from_right)
-__device__ void mult_B_right(const WalkerDev& w, double* M, int ld, const double* dpos) {
-  const int N = w.N;
-  if (w.cb) {
-    cb_right(M, ld, N, w.L, 0, w.cb_h, dpos, nullptr);  // scale cols, A then B
+  const double* in = M;
+  double* out = tmp;
+  int ims = ms, ild = ld, oms = tms, old = ldt;
+  for (int d = 0, st = 1; d < w.dim; ++d, st *= L) {
+    const bool last = d == w.dim - 1;
+    const int step = RIGHT ? st * ild : st;
+    for (int k = threadIdx.x; k < nm * NN; k += kThreads) {
+      int m, r, c;
+      split(k, m, r, c);
+      const int site = RIGHT ? c : r;
+      int x = site;
+      for (int a = 0; a < d; ++a) x = small_div(x, dL);
+      x -= L * small_div(x, dL);
+      const double* p = in + (long long)m * ims + c * ild + r - x * step;
+      double acc = 0.0;
+      for (int y = 0; y < L; ++y) acc = fma(e[abs(x - y)], p[y * step], acc);
+      if (last && !PRE) acc *= sc[m * scs + site];
+      out[(long long)m * oms + c * old + r] = acc;
+    }
     __syncthreads();
-    cb_right(M, ld, N, w.L, 1, w.cb_h, nullptr, nullptr);
-    __syncthreads();
-  } else {
-    const double* K = w.expK;
-    block_gemm(N, [&](int r, int k) { return at(M, ld, r, k) * dpos[k]; },
-               [&](int k, int c) { return __ldg(K + (long long)c * N + k); },
-               [&](int r, int c, double v) { at(M, ld, r, c) = v; });
+    in = out;
+    out = (in == tmp) ? M : tmp;
+    ims = (in == tmp) ? tms : ms;
+    ild = (in == tmp) ? ldt : ld;
+    oms = (in == tmp) ? ms : tms;
+    old = (in == tmp) ? ld : ldt;
   }
-}
-// M <- B(t)^-1 M = expK^-1 diag(e^{-sa s}) M   (mult_invB_from_left)
-__device__ void mult_invB_left(const WalkerDev& w, double* M, int ld, const double* dneg) {
-  const int N = w.N;
-  if (w.cb) {
-    cb_left(M, ld, N, w.L, 0, -w.cb_h, dneg, nullptr);  // scale rows, A then B
+  if (in == tmp) {  // three directions: back to M
+    for (int k = threadIdx.x; k < nm * NN; k += kThreads) {
+      int m, r, c;
+      split(k, m, r, c);
+      M[(long long)m * ms + c * ld + r] = tmp[(long long)m * tms + c * ldt + r];
+    }
     __syncthreads();
-    cb_left(M, ld, N, w.L, 1, -w.cb_h, nullptr, nullptr);
-    __syncthreads();
-  } else {
-    const double* K = w.invK;
-    block_gemm(N, [&](int r, int k) { return __ldg(K + (long long)k * N + r); },
-               [&](int k, int c) { return at(M, ld, k, c) * dneg[k]; },
-               [&](int r, int c, double v) { at(M, ld, r, c) = v; });
-  }
-}
-// M <- B(t)^T M = expK^T diag(e^{+sa s}) M   (mult_transB_from_left)
-__device__ void mult_transB_left(const WalkerDev& w, double* M, int ld, const double* dpos,
-                                 const double* P = nullptr) {
-  const int N = w.N;
-  if (w.cb) {
-    cb_left(M, ld, N, w.L, 0, w.cb_h, dpos, nullptr, P);  // scale rows, A then B
-    __syncthreads();
-    cb_left(M, ld, N, w.L, 1, w.cb_h, nullptr, nullptr, P);
-    __syncthreads();
-  } else {
-    const double* K = w.expK;  // (expK^T)(r,k) = expK(k,r)
-    block_gemm(N, [&](int r, int k) { return __ldg(K + (long long)r * N + k); },
-               [&](int k, int c) { return at(M, ld, k, c) * dpos[k]; },
-               [&](int r, int c, double v) { at(M, ld, r, c) = v; });
   }
 }
 
@@ -443,6 +387,8 @@ __device__ void measure_close(const WalkerDev& w, MeasureAcc& m, double* red) {
 // --------------------------------------------------------------------------
 // shared memory of the segment kernel with the chain beside G: two CTAs still share an SM up to N = 50
 __host__ __device__ inline bool segment_chain_smem(int maxN) { return maxN <= 50; }
+// and the products take both spins' matrices in one pass up to N = 36 (64 KB of shared memory)
+__host__ __device__ inline bool segment_joint_spins(int maxN) { return maxN <= 36; }
 
 // --------------------------------------------------------------------------
 // Segment kernel: the slices of one stabilization interval for one walker.
@@ -471,6 +417,10 @@ __global__ void __launch_bounds__(kThreads, 2) segment_kernel(const WalkerDev* _
   const bool chain_smem = segment_chain_smem(maxN);
   double* Cs = scratch + 3 * N;
   const int ldc = chain_smem ? ld : N;
+  // the products' second buffer, for both spins at once where small walkers need the parallelism
+  double* tmp = Cs + (chain_smem ? (long long)S * N * ld : 0);
+  const int nm = (segment_joint_spins(maxN)) ? S : 1;
+  __shared__ double ring[2 * 8];
   __shared__ int s_next;
   __shared__ double s_f[2], s_sign;
   __shared__ int8_t s_field[kMaxSmemN];
@@ -482,6 +432,7 @@ __global__ void __launch_bounds__(kThreads, 2) segment_kernel(const WalkerDev* _
 
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   constexpr int nwarp = kThreads / 32;
+  if (!w.cb && threadIdx.x < 2 * w.L) ring[threadIdx.x] = w.kin[threadIdx.x];
   // chain <- U_top diag(D_top)  or  I
   for (int sp = 0; sp < S; ++sp) {
     double* C = chain_smem ? Cs + (long long)sp * N * ld : w.chain + (long long)sp * N * N;
@@ -523,15 +474,16 @@ __global__ void __launch_bounds__(kThreads, 2) segment_kernel(const WalkerDev* _
     for (int e = threadIdx.x; e < S * N; e += kThreads) {
       const int sp = e / N, i = e % N;
       const int ss = spin_sign(w, sp) * (int)s_field[i];
-      dtab[(sp * 2 + 0) * N + i] = bdiag(w, ss, 0, MODE != MODE_INIT);
-      dtab[(sp * 2 + 1) * N + i] = bdiag(w, -ss, 1, MODE != MODE_INIT);
+      dtab[(sp * 2 + 0) * N + i] = bdiag(w, ss, 0, MODE != MODE_INIT || !w.cb);
+      dtab[(sp * 2 + 1) * N + i] = bdiag(w, -ss, 1, MODE != MODE_INIT || !w.cb);
     }
     __syncthreads();
 
     if (MODE == MODE_FWD) {  // wrap_from_0_to_beta(t-1): G <- B(t) G B(t)^-1
-      for (int sp = 0; sp < S; ++sp) {
-        mult_B_left(w, Gs[sp], ld, dtab + (sp * 2 + 0) * N);
-        mult_invB_right(w, Gs[sp], ld, dtab + (sp * 2 + 1) * N);
+      for (int sp = 0; sp < S; sp += nm) {
+        kin_product<false, false, false>(w, Gs[sp], N * ld, ld, nm, tmp, N * ld, ld, dtab + sp * 2 * N, 2 * N, ring);
+        kin_product<true, true, false>(w, Gs[sp], N * ld, ld, nm, tmp, N * ld, ld, dtab + (sp * 2 + 1) * N, 2 * N,
+                    ring);
       }
     }
 
@@ -598,8 +550,8 @@ __global__ void __launch_bounds__(kThreads, 2) segment_kernel(const WalkerDev* _
       for (int e = threadIdx.x; e < S * N; e += kThreads) {
         const int sp = e / N, i = e % N;
         const int ss = spin_sign(w, sp) * (int)s_field[i];
-        dtab[(sp * 2 + 0) * N + i] = bdiag(w, ss, 0, MODE != MODE_INIT);
-        dtab[(sp * 2 + 1) * N + i] = bdiag(w, -ss, 1, MODE != MODE_INIT);
+        dtab[(sp * 2 + 0) * N + i] = bdiag(w, ss, 0, MODE != MODE_INIT || !w.cb);
+        dtab[(sp * 2 + 1) * N + i] = bdiag(w, -ss, 1, MODE != MODE_INIT || !w.cb);
       }
       __syncthreads();
 
@@ -614,16 +566,21 @@ __global__ void __launch_bounds__(kThreads, 2) segment_kernel(const WalkerDev* _
     }
 
     // B-chain of the stabilization interval
-    for (int sp = 0; sp < S; ++sp) {
+    for (int sp = 0; sp < S; sp += nm) {
       double* C = chain_smem ? Cs + (long long)sp * N * ld : w.chain + (long long)sp * N * N;
-      if (MODE == MODE_FWD) mult_B_left(w, C, ldc, dtab + (sp * 2 + 0) * N);
-      else mult_transB_left(w, C, ldc, dtab + (sp * 2 + 0) * N, MODE == MODE_INIT ? w.cbP : nullptr);
+      if (MODE == MODE_FWD) {
+        kin_product<false, false, false>(w, C, N * ldc, ldc, nm, tmp, N * ld, ld, dtab + sp * 2 * N, 2 * N, ring);
+      } else {
+        // B^T: the plaquette layers in the order of the inverse's left product
+        kin_product<false, false, true, MODE == MODE_INIT>(w, C, N * ldc, ldc, nm, tmp, N * ld, ld, dtab + sp * 2 * N, 2 * N, ring);
+      }
     }
 
     if (MODE == MODE_BWD) {  // wrap_from_beta_to_0(t): G <- B(t)^-1 G B(t)
-      for (int sp = 0; sp < S; ++sp) {
-        mult_B_right(w, Gs[sp], ld, dtab + (sp * 2 + 0) * N);
-        mult_invB_left(w, Gs[sp], ld, dtab + (sp * 2 + 1) * N);
+      for (int sp = 0; sp < S; sp += nm) {
+        kin_product<true, false, true>(w, Gs[sp], N * ld, ld, nm, tmp, N * ld, ld, dtab + sp * 2 * N, 2 * N, ring);
+        kin_product<false, true, true>(w, Gs[sp], N * ld, ld, nm, tmp, N * ld, ld, dtab + (sp * 2 + 1) * N, 2 * N,
+                    ring);
       }
     }
     __syncthreads();
@@ -1222,7 +1179,8 @@ double run_fp64_probe(cudaError_t* err) {
 // host-side launch helpers
 // --------------------------------------------------------------------------
 size_t segment_smem_bytes(int N, int S) {
-  return sizeof(double) * ((size_t)S * N * (N + 1) * (segment_chain_smem(N) ? 2 : 1) + 8 * N + 64 + 3 * N);
+  const size_t mats = S * (segment_chain_smem(N) ? 2 : 1) + (segment_joint_spins(N) ? S : 1);
+  return sizeof(double) * (mats * N * (N + 1) + 8 * N + 64 + 3 * N);
 }
 size_t push_smem_bytes(int N) { return sizeof(double) * ((size_t)N * (N + 1) + 4 * N) + sizeof(int) * N; }
 size_t greens_smem_bytes(int N) { return sizeof(double) * (2 * (size_t)N * (N + 1) + 4 * N + 64); }

@@ -3,9 +3,9 @@
 //
 // G, the B-chain and the stacks stay in HBM/L2; a half-sweep runs slice by
 // slice as a short sequence of batched launches:
-//   wrap (two batched GEMMs with the diagonal exp(+/-alpha s) fused, or
-//   checkerboard passes) -> Metropolis (one CTA per walker, rank-1 updates,
-//   look-ahead decisions) -> measurement -> B-chain step (GEMM, ping-pong).
+//   wrap (two products in the factors of exp(-dtau K), the diagonal
+//   exp(+/-alpha s) fused) -> Metropolis (one CTA per walker, rank-1 updates,
+//   look-ahead decisions) -> measurement -> B-chain step (one product).
 // Stabilization: column-pivoted QR with one thread per column (row-major copy,
 // coalesced across threads), Green's assembly by batched GEMMs and an LU solve
 // with one thread per column of [M | Y].
@@ -44,13 +44,6 @@ __device__ __forceinline__ bool slice_of(const WalkerDev& w, int mode, int j, in
   return true;
 }
 
-// exp(sgn * spin_factor * alpha * s(t-1, i))
-__device__ __forceinline__ double bscale(const WalkerDev& w, int t, int spin, int sgn, int i) {
-  const int sf = (w.model == 0 && spin == 1) ? -1 : 1;
-  const int s = w.fields[(long long)(t - 1) * w.N + i];
-  return (sgn * sf * s > 0) ? w.e_pa : w.e_ma;
-}
-
 __device__ __forceinline__ double* chain_buf(const WalkerDev& w, int spin, int which) {
   return w.chain + ((long long)which * w.S + spin) * w.N * w.N;
 }
@@ -64,18 +57,10 @@ __device__ __forceinline__ double* chain_buf(const WalkerDev& w, int spin, int w
 // walker, spin and slice from the descriptors.
 // --------------------------------------------------------------------------
 enum GemmOp {
-  OP_WL_FWD = 0,   // work = diag(e^{+}) expK G          (mult_B_from_left)
-  OP_WR_FWD = 1,   // G    = work expK^-1 diag(e^{-})    (mult_invB_from_right)
-  OP_WR_BWD = 2,   // work = G diag(e^{+}) expK          (mult_B_from_right)
-  OP_WL_BWD = 3,   // G    = expK^-1 diag(e^{-}) work    (mult_invB_from_left)
-  OP_CH_FWD = 4,   // chain' = diag(e^{+}) expK chain    (B-chain, forward)
-  OP_CH_BWD = 5,   // chain' = expK^T diag(e^{+}) chain  (B-chain, backward / init)
   OP_GA = 6,       // M  = Dlmax^-1 (U_L^T U_R) Drmax^-1
   OP_GB = 7,       // M += Dlmin (F_L F_R^T) Drmin
   OP_GG = 8,       // G  = (U_R Drmax^-1) X, wrap error, trace
   // dynamic half-sweep (sweep_for_dynamic_greens, src/dqmc_walker.cpp:424-524)
-  OP_DT0 = 9,      // G(t,0) = diag(e+) expK G(t-1,0)          (mult_B_from_left)
-  OP_D0T = 10,     // G(0,t) = G(0,t-1) expK^-1 diag(e-)       (mult_invB_from_right)
   OP_DT0_OUT = 11, // G(t,0) = (U_R Drmax^-1) X1, X1 = M^-1 Dlmin F_L; wrap error
   OP_D0T_OUT = 12, // G(0,t) = -(F_R^T Drmin) X, X = M^-1 Dlmax^-1 U_L^T; wrap error
 };
@@ -91,31 +76,21 @@ __global__ void __launch_bounds__(256) gemm_op_kernel(const WalkerDev* __restric
   const int N = w.N;
   const int r0 = blockIdx.y * kTile, c0 = blockIdx.x * kTile;
   if (r0 >= N || c0 >= N) return;
-  int t = 0, nsl = 0, t_hi = 0;
-  constexpr bool dyn_prop = OP == OP_DT0 || OP == OP_D0T;
   constexpr bool dyn_out = OP == OP_DT0_OUT || OP == OP_D0T_OUT;
-  const bool slice_op = OP <= OP_CH_BWD || dyn_prop;
-  if ((dyn_prop || dyn_out) && !w.gt0) return;
-  if (slice_op && w.cb) return;  // checkerboard walkers take cb_general_kernel (expK is null for them)
-  if (slice_op && w.path == 2) return;  // mixed walkers take the tensor-core products
-  if (slice_op && !slice_of(w, mode, j, q, t, nsl, t_hi)) return;
-  if (!slice_op && j >= w.nstack) return;
-  if (!slice_op && w.ozstab) return;  // stabilized by kernels_stab_oz.cu
+  if (dyn_out && !w.gt0) return;
+  if (j >= w.nstack || w.ozstab) return;  // ozstab: stabilized by kernels_stab_oz.cu
 
   const long long NN = (long long)N * N;
   double* G = w.G + sp * NN;
-  double* work = w.work + sp * NN;
   const double* A = nullptr;
   const double* B = nullptr;
   double* C = nullptr;
   // stack tops for the Green's assembly (lengths after this step's push)
   int nl = 0, nr = 0;
-  if (!slice_op) {
-    if (mode == MODE_FWD) { nl = j + 1; nr = w.nstack - 1 - j; }
-    else if (mode == MODE_BWD) { nl = w.nstack - 1 - j; nr = j + 1; }
-    else { nl = 0; nr = w.nstack; }
-  }
-  if (!slice_op && !(nl > 0 && nr > 0)) return;  // boundary steps: prep/out kernels
+  if (mode == MODE_FWD) { nl = j + 1; nr = w.nstack - 1 - j; }
+  else if (mode == MODE_BWD) { nl = w.nstack - 1 - j; nr = j + 1; }
+  else { nl = 0; nr = w.nstack; }
+  if (!(nl > 0 && nr > 0)) return;  // boundary steps: prep/out kernels
   const double* UL = nl ? stack_level(w, 0, sp, nl - 1) : nullptr;
   const double* UR = nr ? stack_level(w, 1, sp, nr - 1) : nullptr;
   const double* DL = UL ? UL + 2 * NN : nullptr;
@@ -125,17 +100,9 @@ __global__ void __launch_bounds__(256) gemm_op_kernel(const WalkerDev* __restric
   const int t_end = min((j + 1) * w.pace, w.Lt);  // forward step j ends at this slice
   auto dbuf = [&](double* base, int par) { return base + ((long long)(par & 1) * w.S + sp) * NN; };
   switch (OP) {
-    case OP_WL_FWD: A = w.expK; B = G; C = work; break;
-    case OP_WR_FWD: A = work; B = w.invK; C = G; break;
-    case OP_WR_BWD: A = G; B = w.expK; C = work; break;
-    case OP_WL_BWD: A = w.invK; B = work; C = G; break;
-    case OP_CH_FWD:
-    case OP_CH_BWD: A = w.expK; B = chain_buf(w, sp, q & 1); C = chain_buf(w, sp, (q + 1) & 1); break;
     case OP_GA: A = UL; B = UR; C = scr; break;
     case OP_GB: A = UL + NN; B = UR + NN; C = scr; break;      // F_L, F_R
     case OP_GG: A = UR; B = scr + NN; C = G; break;           // U_R, X (row-major)
-    case OP_DT0: A = w.expK; B = dbuf(w.gt0, t - 1); C = dbuf(w.gt0, t); break;
-    case OP_D0T: A = dbuf(w.g0t, t - 1); B = w.invK; C = dbuf(w.g0t, t); break;
     case OP_DT0_OUT: A = UR; B = w.dynx + sp * NN; C = dbuf(w.gt0, t_end); break;   // X1 row-major
     case OP_D0T_OUT: A = UR + NN; B = scr + NN; C = dbuf(w.g0t, t_end); break;      // F_R, X row-major
   }
@@ -167,17 +134,9 @@ __global__ void __launch_bounds__(256) gemm_op_kernel(const WalkerDev* __restric
       double v = 0.0;
       if (r < N && k < N) {
         switch (OP) {
-          case OP_WL_FWD: v = A[(long long)k * N + r] * bscale(w, t, sp, +1, r); break;
-          case OP_WR_FWD: v = A[(long long)k * N + r]; break;
-          case OP_WR_BWD: v = A[(long long)k * N + r] * bscale(w, t, sp, +1, k); break;
-          case OP_WL_BWD: v = A[(long long)k * N + r]; break;
-          case OP_CH_FWD: v = A[(long long)k * N + r] * bscale(w, t, sp, +1, r); break;
-          case OP_CH_BWD: v = A[(long long)r * N + k] * bscale(w, t, sp, +1, k); break;  // expK^T
           case OP_GA: v = A[(long long)r * N + k]; break;  // U_L^T (r,k) = U_L(k,r)
           case OP_GB: v = A[(long long)k * N + r]; break;
           case OP_GG: v = A[(long long)k * N + r] * s_inv[k]; break;  // U_R(r,k) / drmax_k
-          case OP_DT0: v = A[(long long)k * N + r] * bscale(w, t, sp, +1, r); break;
-          case OP_D0T: v = A[(long long)k * N + r]; break;
           case OP_DT0_OUT: v = A[(long long)k * N + r] * s_inv[k]; break;
           case OP_D0T_OUT: v = A[(long long)r * N + k] * s_inv[k]; break;  // F_R^T(r,k) drmin_k
         }
@@ -192,17 +151,9 @@ __global__ void __launch_bounds__(256) gemm_op_kernel(const WalkerDev* __restric
       double v = 0.0;
       if (k < N && c < N) {
         switch (OP) {
-          case OP_WL_FWD: v = B[(long long)c * N + k]; break;
-          case OP_WR_FWD: v = B[(long long)c * N + k]; break;
-          case OP_WR_BWD: v = B[(long long)c * N + k]; break;
-          case OP_WL_BWD: v = B[(long long)c * N + k] * bscale(w, t, sp, -1, k); break;
-          case OP_CH_FWD: v = B[(long long)c * N + k]; break;
-          case OP_CH_BWD: v = B[(long long)c * N + k]; break;
           case OP_GA: v = B[(long long)c * N + k]; break;
           case OP_GB: v = B[(long long)k * N + c]; break;  // F_R^T(k,c) = F_R(c,k)
           case OP_GG: v = B[(long long)k * N + c]; break;                     // X row-major
-          case OP_DT0: v = B[(long long)c * N + k]; break;
-          case OP_D0T: v = B[(long long)c * N + k]; break;
           case OP_DT0_OUT: v = B[(long long)k * N + c]; break;  // X1 row-major
           case OP_D0T_OUT: v = B[(long long)k * N + c]; break;  // X row-major
         }
@@ -240,8 +191,6 @@ __global__ void __launch_bounds__(256) gemm_op_kernel(const WalkerDev* __restric
       double v = acc[a][b];
       const long long o = (long long)c * N + r;
       switch (OP) {
-        case OP_WR_FWD: v *= bscale(w, t, sp, -1, c); break;
-        case OP_D0T: v *= bscale(w, t, sp, -1, c); break;
         case OP_D0T_OUT: v = -v; break;
         case OP_GA: v /= fmax(DL[r], 1.0) * fmax(DR[c], 1.0); break;
         case OP_GB: v *= fmin(DL[r], 1.0) * fmin(DR[c], 1.0); break;
@@ -282,96 +231,125 @@ __global__ void __launch_bounds__(256) gemm_op_kernel(const WalkerDev* __restric
 }
 
 // --------------------------------------------------------------------------
-// Checkerboard on global matrices (general N): one CTA per (walker, spin).
-//   kind 0: wrap fwd  G <- P_A P_B G (scale rows e^+) ; G <- G P_B^-1 P_A^-1 (scale cols e^-)
-//   kind 1: wrap bwd  G <- G diag(e^+) P_A P_B ; G <- P_B^-1 P_A^-1 diag(e^-) G
-//   kind 2: chain fwd C <- diag(e^+) P_A P_B C
-//   kind 3: chain bwd C <- P_B P_A diag(e^+) C
-//   kind 4: time-displaced steps of the dynamic half-sweep (mult_B_from_left and
-//           mult_invB_from_right, src/dqmc_walker.cpp:455-466):
-//           G(t,0) <- diag(e^+) P_A P_B G(t-1,0),  G(0,t) <- G(0,t-1) P_B^-1 P_A^-1 diag(e^-)
+// One slice's products with B on global matrices, in the factors of exp(-+dtau K): the two
+// plaquette layers of a checkerboard walker (any path), else one ring exponential per lattice
+// direction (FP64 walkers; the mixed path's dense walkers take the tensor-core products).
+//   KIN_WL_FWD  G <- diag(e+) K G         KIN_WR_FWD  G <- G K^-1 diag(e-)
+//   KIN_WR_BWD  G <- G diag(e+) K         KIN_WL_BWD  G <- K^-1 diag(e-) G
+//   KIN_CH_FWD  chain' = diag(e+) K chain KIN_CH_BWD  chain' = K^T diag(e+) chain
+//   KIN_DT0     G(t,0) = diag(e+) K G(t-1,0)   KIN_D0T  G(0,t) = G(0,t-1) K^-1 diag(e-)
+// (mult_B_from_left and its relatives, src/model/repulsive_hubbard.cpp:158-243, with the
+// checkerboard's layer order, src/checkerboard/square.cpp:130-226.)  A left product mixes a
+// column's sites, a right product a row's, so a CTA takes about 2048 elements of whole columns or
+// rows into shared memory, does every pass there and writes them back once: 2 L (3 L) FMAs an
+// element instead of N, and one read and one write of the matrix.  As a batched 64 x 64-tile GEMM a
+// product of 16 walkers of 16 x 16 took 0.80 ms; a pass of them (48 products) went from 163 to 135
+// ms, of 32 walkers of 9 x 9 from 52 to 38 ms.
 // --------------------------------------------------------------------------
-__device__ void cbg_pass(double* M, int N, int L, int parity, const double* P, bool left, const double* pre,
-                         const double* post) {
-  const int nq = (L >> 1) * (L >> 1), half = L >> 1;
-  for (int it = threadIdx.x; it < nq * N; it += blockDim.x) {
-    int q, x2;
-    if (left) { q = it % nq; x2 = it / nq; } else { x2 = it % N; q = it / N; }
-    const int x = 2 * (q % half) + parity, y = 2 * (q / half) + parity;
-    const int x1 = (x + 1) % L, y1 = (y + 1) % L;
-    const int idx[4] = {x + L * y, x1 + L * y, x + L * y1, x1 + L * y1};
-    double v[4];
-    for (int a = 0; a < 4; ++a) {
-      v[a] = left ? M[(long long)x2 * N + idx[a]] : M[(long long)idx[a] * N + x2];
-      if (pre) v[a] *= pre[idx[a]];
-    }
-    for (int a = 0; a < 4; ++a) {
-      double o = 0.0;
-      for (int b = 0; b < 4; ++b) o = left ? fma(P[a * 4 + b], v[b], o) : fma(v[b], P[b * 4 + a], o);
-      if (post) o *= post[idx[a]];
-      if (left) M[(long long)x2 * N + idx[a]] = o; else M[(long long)idx[a] * N + x2] = o;
-    }
-  }
-}
+enum KinOp { KIN_WL_FWD, KIN_WR_FWD, KIN_WR_BWD, KIN_WL_BWD, KIN_CH_FWD, KIN_CH_BWD, KIN_DT0, KIN_D0T };
+constexpr int kKinElems = 2048, kKinPer = kKinElems / 256;
+// columns (rows) a CTA takes
+__host__ __device__ inline int kin_lines(int N) { return kKinElems / N; }
 
-__global__ void __launch_bounds__(256) cb_general_kernel(const WalkerDev* __restrict__ W, int mode, int j, int q,
-                                                         int kind) {
-  const int wi = blockIdx.x >> 1, sp = blockIdx.x & 1;
-  const WalkerDev& w = W[wi];
-  if (!is_general(w) || !w.cb || sp >= w.S) return;
+__global__ void __launch_bounds__(256) kin_op_kernel(const WalkerDev* __restrict__ W, int op, int mode, int j, int q) {
+  const WalkerDev& w = W[blockIdx.z];
+  const int sp = blockIdx.y;
+  if (!is_general(w) || sp >= w.S || (w.path == 2 && !w.cb)) return;
+  const int N = w.N, L = w.L, V = kin_lines(N), v0 = blockIdx.x * V, nv = min(V, N - v0);
+  if (nv <= 0) return;
   int t, nsl, t_hi;
   if (!slice_of(w, mode, j, q, t, nsl, t_hi)) return;
-  extern __shared__ double sh[];
-  const int N = w.N, L = w.L;
-  double* dpos = sh;
-  double* dneg = sh + N;
-  for (int i = threadIdx.x; i < N; i += blockDim.x) {
-    dpos[i] = bscale(w, t, sp, +1, i);
-    dneg[i] = bscale(w, t, sp, -1, i);
+  if ((op == KIN_DT0 || op == KIN_D0T) && !w.gt0) return;
+  const long long NN = (long long)N * N;
+  const bool right = op == KIN_WR_FWD || op == KIN_WR_BWD || op == KIN_D0T;
+  const bool inv = op == KIN_WR_FWD || op == KIN_WL_BWD || op == KIN_D0T;
+  const bool pre = op == KIN_WR_BWD || op == KIN_WL_BWD || op == KIN_CH_BWD;  // else the diagonal comes last
+  const double* src = w.G + sp * NN;
+  double* dst = w.G + sp * NN;
+  if (op == KIN_CH_FWD || op == KIN_CH_BWD) {  // ping-pong, checkerboard walkers in place
+    src = chain_buf(w, sp, w.cb ? 0 : q & 1);
+    dst = chain_buf(w, sp, w.cb ? 0 : (q + 1) & 1);
+  } else if (op == KIN_DT0 || op == KIN_D0T) {
+    double* base = op == KIN_DT0 ? w.gt0 : w.g0t;
+    src = base + ((long long)((t - 1) & 1) * w.S + sp) * NN;
+    dst = base + ((long long)(t & 1) * w.S + sp) * NN;
+  }
+  __shared__ double m[kKinElems], sc[kMaxN], e[32];
+  const int tid = threadIdx.x;
+  const bool plain = mode == MODE_INIT && w.cb;  // the set-up keeps the plain plaquette product (plaq_product)
+  for (int i = tid; i < N; i += 256) {
+    const int sf = (w.model == 0 && sp == 1) ? -1 : 1, s = w.fields[(long long)(t - 1) * N + i];
+    const int up = ((inv ? -1 : 1) * sf * s > 0) ? 0 : 1;
+    sc[i] = plain ? (up ? w.e_ma : w.e_pa) : w.kin_e[inv][up];
+  }
+  if (!w.cb && tid < L) e[tid] = w.kin[(inv ? L : 0) + tid];
+  // element k of the tile: site and line, left k = line N + site (contiguous in the matrix),
+  // right k = site nv + line
+  const int nel = N * nv, ss = right ? nv : 1;
+  int site[kKinPer];
+#pragma unroll
+  for (int u = 0; u < kKinPer; ++u) {
+    const int k = tid + 256 * u;
+    site[u] = right ? k / nv : k % N;
+  }
+  auto gofs = [&](int k, int s) { return right ? (long long)s * N + v0 + (k - s * nv) : (long long)v0 * N + k; };
+  __syncthreads();
+#pragma unroll
+  for (int u = 0; u < kKinPer; ++u) {
+    const int k = tid + 256 * u;
+    if (k < nel) {
+      const double x = src[gofs(k, site[u])];
+      m[k] = pre ? x * sc[site[u]] : x;
+    }
   }
   __syncthreads();
-  double* G = w.G + (long long)sp * N * N;
-  double* C = chain_buf(w, sp, 0);
-  switch (kind) {
-    case 0:
-      cbg_pass(G, N, L, 1, w.cbP, true, nullptr, nullptr); __syncthreads();
-      cbg_pass(G, N, L, 0, w.cbP, true, nullptr, dpos); __syncthreads();
-      cbg_pass(G, N, L, 1, w.cbI, false, nullptr, nullptr); __syncthreads();
-      cbg_pass(G, N, L, 0, w.cbI, false, nullptr, dneg); __syncthreads();
-      break;
-    case 1:
-      cbg_pass(G, N, L, 0, w.cbP, false, dpos, nullptr); __syncthreads();
-      cbg_pass(G, N, L, 1, w.cbP, false, nullptr, nullptr); __syncthreads();
-      cbg_pass(G, N, L, 0, w.cbI, true, dneg, nullptr); __syncthreads();
-      cbg_pass(G, N, L, 1, w.cbI, true, nullptr, nullptr); __syncthreads();
-      break;
-    case 2:
-      cbg_pass(C, N, L, 1, w.cbP, true, nullptr, nullptr); __syncthreads();
-      cbg_pass(C, N, L, 0, w.cbP, true, nullptr, dpos); __syncthreads();
-      break;
-    case 3:
-      cbg_pass(C, N, L, 0, w.cbP, true, dpos, nullptr); __syncthreads();
-      cbg_pass(C, N, L, 1, w.cbP, true, nullptr, nullptr); __syncthreads();
-      break;
-    case 4: {
-      if (!w.gt0) return;
-      // ping-pong slots [parity][S][N*N]: read slice t - 1's, write slice t's, then in place
-      const long long NN = (long long)N * N;
-      const double* a0 = w.gt0 + ((long long)((t - 1) & 1) * w.S + sp) * NN;
-      double* a1 = w.gt0 + ((long long)(t & 1) * w.S + sp) * NN;
-      const double* b0 = w.g0t + ((long long)((t - 1) & 1) * w.S + sp) * NN;
-      double* b1 = w.g0t + ((long long)(t & 1) * w.S + sp) * NN;
-      for (long long e = threadIdx.x; e < NN; e += blockDim.x) {
-        a1[e] = a0[e];
-        b1[e] = b0[e];
+  if (w.cb) {
+    const int nq = (L >> 1) * (L >> 1), first = pre ? 0 : 1;  // layer A (parity 0) or B first
+    const double h = inv ? -w.cb_h : w.cb_h;
+    const int sv = right ? 1 : N;
+    for (int p = 0; p < 2; ++p) {
+      for (int it = tid; it < nq * nv; it += 256) {
+        const int pq = right ? it / nv : it % nq, v = right ? it % nv : it / nq;
+        int idx[4];
+        plaq_sites(L, pq, first ^ p, idx);
+        double x[4];
+#pragma unroll
+        for (int a = 0; a < 4; ++a) x[a] = m[idx[a] * ss + v * sv];
+        if (plain) plaq_product(x, w.cbP);
+        else plaq_apply(x, h);
+#pragma unroll
+        for (int a = 0; a < 4; ++a) m[idx[a] * ss + v * sv] = x[a];
       }
       __syncthreads();
-      cbg_pass(a1, N, L, 1, w.cbP, true, nullptr, nullptr); __syncthreads();
-      cbg_pass(a1, N, L, 0, w.cbP, true, nullptr, dpos); __syncthreads();
-      cbg_pass(b1, N, L, 1, w.cbI, false, nullptr, nullptr); __syncthreads();
-      cbg_pass(b1, N, L, 0, w.cbI, false, nullptr, dneg); __syncthreads();
-      break;
     }
+  } else {
+    for (int d = 0, st = 1; d < w.dim; ++d, st *= L) {
+      double acc[kKinPer];
+      int x[kKinPer], base[kKinPer];
+      const int step = st * ss;
+#pragma unroll
+      for (int u = 0; u < kKinPer; ++u) {
+        const int k = tid + 256 * u;
+        x[u] = (k < nel) ? (site[u] / st) % L : 0;
+        base[u] = (k < nel) ? k - x[u] * step : 0;
+        acc[u] = 0.0;
+      }
+      for (int y = 0; y < L; ++y)
+#pragma unroll
+        for (int u = 0; u < kKinPer; ++u)
+          if ((tid & ~31) + 256 * u < nel)  // uniform in the warp
+            acc[u] = fma(e[abs(x[u] - y)], m[base[u] + y * step], acc[u]);
+      __syncthreads();
+#pragma unroll
+      for (int u = 0; u < kKinPer; ++u)
+        if (tid + 256 * u < nel) m[tid + 256 * u] = acc[u];
+      __syncthreads();
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < kKinPer; ++u) {
+    const int k = tid + 256 * u;
+    if (k < nel) dst[gofs(k, site[u])] = pre ? m[k] : m[k] * sc[site[u]];
   }
 }
 
@@ -1347,18 +1325,20 @@ void launch_metropolis_sub_split(const WalkerDev* W, int nw, int mode, int j, in
 // host): the dense products before the updates (forward wrap), the Metropolis
 // updates with the fused measurement, and the products after them (B-chain
 // step and backward wrap).
+static void launch_kin(const WalkerDev* W, int nw, int maxN, int op, int mode, int j, int q, cudaStream_t st) {
+  const int V = kin_lines(maxN);
+  kin_op_kernel<<<dim3((maxN + V - 1) / V, 2, nw), 256, 0, st>>>(W, op, mode, j, q);
+}
+
 void general_slice_pre(int mode, const WalkerDev* W, int nw, int j, int q, int maxN, bool any_dense, bool any_cb,
                        bool mixed, cudaStream_t st) {
   if (mode != MODE_FWD) return;
   // in a mixed batch the dense products go through the tensor cores (kernels_ozaki.cu)
-  const bool fp64_dense = any_dense && !mixed;
-  const dim3 g = gemm_grid(maxN, nw);
-  if (fp64_dense) {
-    gemm_op_kernel<OP_WL_FWD><<<g, 256, 0, st>>>(W, mode, j, q, -1);
-    gemm_op_kernel<OP_WR_FWD><<<g, 256, 0, st>>>(W, mode, j, q, -1);
+  if (any_cb || (any_dense && !mixed)) {
+    launch_kin(W, nw, maxN, KIN_WL_FWD, mode, j, q, st);
+    launch_kin(W, nw, maxN, KIN_WR_FWD, mode, j, q, st);
   }
   if (any_dense && mixed) mixed_wrap_fwd(W, nw, maxN, j, q, st);
-  if (any_cb) cb_general_kernel<<<2 * nw, 256, sizeof(double) * 2 * maxN, st>>>(W, mode, j, q, 0);
 }
 
 void general_slice_metro(int mode, const WalkerDev* W, int nw, int j, int q, int maxN, int measure, bool mixed,
@@ -1374,23 +1354,15 @@ void general_slice_metro(int mode, const WalkerDev* W, int nw, int j, int q, int
 
 void general_slice_post(int mode, const WalkerDev* W, int nw, int j, int q, int maxN, bool any_dense, bool any_cb,
                         bool mixed, cudaStream_t st) {
-  const bool fp64_dense = any_dense && !mixed;
-  const bool mixed_dense = any_dense && mixed;
-  const dim3 g = gemm_grid(maxN, nw);
-  const size_t cb_sm = sizeof(double) * 2 * maxN;
-  if (fp64_dense) {
-    if (mode == MODE_FWD) gemm_op_kernel<OP_CH_FWD><<<g, 256, 0, st>>>(W, mode, j, q, -1);
-    else gemm_op_kernel<OP_CH_BWD><<<g, 256, 0, st>>>(W, mode, j, q, -1);
-  }
+  const bool kin = any_cb || (any_dense && !mixed), mixed_dense = any_dense && mixed;
+  if (kin) launch_kin(W, nw, maxN, mode == MODE_FWD ? KIN_CH_FWD : KIN_CH_BWD, mode, j, q, st);
   if (mixed_dense) mixed_chain(W, nw, maxN, mode, j, q, st);
-  if (any_cb) cb_general_kernel<<<2 * nw, 256, cb_sm, st>>>(W, mode, j, q, mode == MODE_FWD ? 2 : 3);
   if (mode == MODE_BWD) {
-    if (fp64_dense) {
-      gemm_op_kernel<OP_WR_BWD><<<g, 256, 0, st>>>(W, mode, j, q, -1);
-      gemm_op_kernel<OP_WL_BWD><<<g, 256, 0, st>>>(W, mode, j, q, -1);
+    if (kin) {
+      launch_kin(W, nw, maxN, KIN_WR_BWD, mode, j, q, st);
+      launch_kin(W, nw, maxN, KIN_WL_BWD, mode, j, q, st);
     }
     if (mixed_dense) mixed_wrap_bwd(W, nw, maxN, j, q, st);
-    if (any_cb) cb_general_kernel<<<2 * nw, 256, cb_sm, st>>>(W, mode, j, q, 1);
   }
 }
 
@@ -1400,41 +1372,22 @@ void general_slice_post(int mode, const WalkerDev* W, int nw, int j, int q, int 
 // checkerboard walkers through the plaquette passes.
 void general_dynamic_wrap(const WalkerDev* W, int nw, int j, int q, int maxN, bool mixed, bool any_dense,
                           bool any_cb, cudaStream_t st) {
-  const dim3 g = gemm_grid(maxN, nw);
-  if (any_dense) {
-    if (mixed) {
-      mixed_wrap_fwd(W, nw, maxN, j, q, st);
-    } else {
-      gemm_op_kernel<OP_WL_FWD><<<g, 256, 0, st>>>(W, MODE_FWD, j, q, -1);
-      gemm_op_kernel<OP_WR_FWD><<<g, 256, 0, st>>>(W, MODE_FWD, j, q, -1);
-    }
-  }
-  if (any_cb) cb_general_kernel<<<2 * nw, 256, sizeof(double) * 2 * maxN, st>>>(W, MODE_FWD, j, q, 0);
+  general_slice_pre(MODE_FWD, W, nw, j, q, maxN, any_dense, any_cb, mixed, st);
 }
 
 void general_dynamic_prop(const WalkerDev* W, int nw, int j, int q, int maxN, bool mixed, bool any_dense,
                           bool any_cb, cudaStream_t st) {
-  const dim3 g = gemm_grid(maxN, nw);
-  if (any_dense) {
-    if (mixed) {
-      mixed_dynamic_prop(W, nw, maxN, j, q, st);
-    } else {
-      gemm_op_kernel<OP_DT0><<<g, 256, 0, st>>>(W, MODE_FWD, j, q, -1);
-      gemm_op_kernel<OP_D0T><<<g, 256, 0, st>>>(W, MODE_FWD, j, q, -1);
-    }
+  if (any_cb || (any_dense && !mixed)) {
+    launch_kin(W, nw, maxN, KIN_DT0, MODE_FWD, j, q, st);
+    launch_kin(W, nw, maxN, KIN_D0T, MODE_FWD, j, q, st);
   }
-  if (any_cb) cb_general_kernel<<<2 * nw, 256, sizeof(double) * 2 * maxN, st>>>(W, MODE_FWD, j, q, 4);
+  if (any_dense && mixed) mixed_dynamic_prop(W, nw, maxN, j, q, st);
   dyn_measure_kernel<<<nw, 256, sizeof(double) * 32, st>>>(W, j, q, 0);
 }
 
 void general_dynamic_chain(const WalkerDev* W, int nw, int j, int q, int maxN, bool mixed, bool any_dense,
                            bool any_cb, cudaStream_t st) {
-  const dim3 g = gemm_grid(maxN, nw);
-  if (any_dense) {
-    if (mixed) mixed_chain(W, nw, maxN, MODE_FWD, j, q, st);
-    else gemm_op_kernel<OP_CH_FWD><<<g, 256, 0, st>>>(W, MODE_FWD, j, q, -1);
-  }
-  if (any_cb) cb_general_kernel<<<2 * nw, 256, sizeof(double) * 2 * maxN, st>>>(W, MODE_FWD, j, q, 2);
+  general_slice_post(MODE_FWD, W, nw, j, q, maxN, any_dense, any_cb, mixed, st);
 }
 
 // stabilization of the dynamic pieces after general_greens of forward step j (walkers
