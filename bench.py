@@ -390,7 +390,7 @@ def metropolis_work(d, accepts: float, tc_flush: int, kd: int):
       submatrix (tc_flush 2, or 3 split per block): per 32-site block with m accepts, Gamma's m x m products and the
         rank-1 updates of the block in FP64, T = Gamma R_A (N x m x m) and the flush
         G -= G0(:, I_A) T (N x N x m) as 6 x 7-bit slice products (21 pairs);
-      delayed (tc_flush 0 / 1): the corrected diagonal and the u, w vectors per accept in FP64
+      delayed (tc_flush 0 / 1; FP64 walkers take submatrix updates with an FP64 flush of the same 2 N^2 per accept): the corrected diagonal and the u, w vectors per accept in FP64
         (about 4 N k), the flush G -= U V^T (N x N x k) in FP64 or as 21 slice pairs."""
     N, Lt = d.L ** 2, d.Lt
     S = 1 if d.model == 1 else 2

@@ -40,19 +40,20 @@ double run_fp64_probe(cudaError_t* err);
 void launch_bump(unsigned long long* ctr, cudaStream_t st);
 void launch_bin_close(const WalkerDev* W, int nw, double* bins, int nbins, int bin, cudaStream_t st);
 // general (N > 64) walkers, kernels_general.cu
-cudaError_t configure_general_kernels();
 void general_slice_pre(int mode, const WalkerDev* W, int nw, int j, int q, int maxN, bool any_dense, bool any_cb,
                        bool mixed, cudaStream_t st);
 void general_slice_metro(int mode, const WalkerDev* W, int nw, int j, int q, int maxN, int measure, bool mixed,
                          int kd, int smax, int tc_flush, cudaStream_t st);
 void general_slice_post(int mode, const WalkerDev* W, int nw, int j, int q, int maxN, bool any_dense, bool any_cb,
                         bool mixed, cudaStream_t st);
-void launch_metropolis_delayed(bool mixed, const WalkerDev* W, int nw, int mode, int j, int q, int maxN, int S_max,
-                               int KD, int tc_flush, cudaStream_t st);
+void launch_metropolis_delayed(const WalkerDev* W, int nw, int mode, int j, int q, int maxN, int S_max, int KD,
+                               int tc_flush, cudaStream_t st);
 size_t delayed_smem_bytes_host(int N, int S, int KD);
 cudaError_t configure_delayed_kernels();
 cudaError_t configure_submatrix_kernel();
 size_t submatrix_scratch_bytes(int N);
+size_t submatrix64_scratch_bytes(int N, int S);
+void launch_metropolis_sub64(const WalkerDev* W, int nw, int mode, int j, int q, int maxN, int S_max, cudaStream_t st);
 void launch_metropolis_sub(const WalkerDev* W, int nw, int mode, int j, int q, int maxN, int S_max, cudaStream_t st);
 void launch_metropolis_sub_split(const WalkerDev* W, int nw, int mode, int j, int q, int maxN, int S_max,
                                  cudaStream_t st);
@@ -270,8 +271,8 @@ struct dqmc_batch {
   bool any_ozstab = false;  // walkers stabilized by the tensor-core blocked QR
   int maxN_oz = 0;
   bool mixed = false;
-  int kd = 0, smax = 1;  // delayed-update block size of the general walkers (0: rank-1 kernel)
-  // Metropolis of HBM walkers: 0 delayed with FP64 flush, 1 delayed with tensor-core
+  int kd = 0, smax = 1;  // flips a block update takes: delayed updates' k, 32 for submatrix updates
+  // Metropolis of HBM walkers: 0 FP64 flush (FP64 walkers: submatrix updates; mixed: delayed), 1 delayed with tensor-core
   // flush, 2 submatrix updates with tensor-core flush (mixed walkers, one CTA per walker),
   // 3 the same split per 32-site block into a decision and a multi-CTA flush kernel
   int tc_flush = 1;
@@ -438,8 +439,8 @@ int dqmc_batch_create(const dqmc_walker_desc* descs, int n, const dqmc_batch_opt
   b->mixed = (o.precision == DQMC_MIXED);
   for (auto& d : b->desc)
     if (d.model == DQMC_REPULSIVE_HUBBARD) b->smax = 2;
-  if (b->any_general) b->kd = delayed_pick_kd(b->maxN_general, b->smax);
-  if (b->mixed) b->tc_flush = 2;  // submatrix updates until the tuner has timed the candidates
+  if (b->any_general) b->kd = (o.precision == DQMC_MIXED) ? delayed_pick_kd(b->maxN_general, b->smax) : 32;
+  b->tc_flush = b->mixed ? 2 : 0;  // submatrix updates until the tuner has timed the candidates
 
   // ---- arena layout ----
   struct Off { size_t G, chain, work, scr, sl, sle, stack, fields, ff, trace, msub, zsl; int dense_id; };
@@ -470,7 +471,9 @@ int dqmc_batch_create(const dqmc_walker_desc* descs, int n, const dqmc_batch_opt
     off[w].stack = take(sizeof(double) * 2 * S * ns * lvl);
     off[w].fields = take((size_t)d.Lt * N);
     off[w].trace = b->trace_cap ? take(sizeof(double) * (size_t)b->trace_cap * 2 * N * N) : 0;
-    off[w].msub = (o.precision == DQMC_MIXED) ? take((size_t)S * submatrix_scratch_bytes(N)) : 0;
+    off[w].msub = (o.precision == DQMC_MIXED) ? take((size_t)S * submatrix_scratch_bytes(N))
+                  : general                     ? take(submatrix64_scratch_bytes(N, S))
+                                                : 0;
     off[w].zsl = uses_ozstab(N, o.precision)
                      ? take(sizeof(unsigned short) * (size_t)S * 2 * 9 * ozaki::tc_lines(N) * (size_t)((N + 31) / 32 * 32))
                      : 0;
@@ -516,7 +519,6 @@ int dqmc_batch_create(const dqmc_walker_desc* descs, int n, const dqmc_batch_opt
   }
   e = cudaStreamCreateWithFlags(&b->own, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = configure_fp64_kernels(kMaxSmemN);
-  if (e == cudaSuccess) e = configure_general_kernels();
   if (e == cudaSuccess) e = configure_ozaki_kernels();
   if (e == cudaSuccess) e = configure_delayed_kernels();
   if (e == cudaSuccess) e = configure_submatrix_kernel();
@@ -639,7 +641,7 @@ int dqmc_batch_create(const dqmc_walker_desc* descs, int n, const dqmc_batch_opt
     h.path = (o.precision == DQMC_MIXED) ? 2 : (gen ? 1 : 0);
     h.work = gen ? reinterpret_cast<double*>(base + off[w].work) : nullptr;
     h.scr = gen ? reinterpret_cast<double*>(base + off[w].scr) : nullptr;
-    h.msub = (o.precision == DQMC_MIXED) ? reinterpret_cast<unsigned char*>(base + off[w].msub) : nullptr;
+    h.msub = gen ? reinterpret_cast<unsigned char*>(base + off[w].msub) : nullptr;
     h.ozstab = uses_ozstab(N, o.precision) ? 1 : 0;
     h.zld = (N + 31) / 32 * 32;
     h.zsl = h.ozstab ? reinterpret_cast<unsigned short*>(base + off[w].zsl) : nullptr;
@@ -794,10 +796,11 @@ static int launch_check(const char* what) {
 // Autotuner of the Metropolis of HBM walkers: times one slice of every walker
 // for each candidate (block size k, update kind) on the batch's own state,
 // restoring G, the fields and the walker scalars after each trial, and keeps
-// the fastest.  Candidates: delayed updates with k in {32, 16, 8} that fit
-// shared memory; on the mixed path, submatrix updates (k = 32) fused in one
-// kernel per walker and split per block (decision and multi-CTA flush kernels),
-// and each delayed k with the tensor-core flush and with the FP64 flush.
+// the fastest.  Candidates on the mixed path: submatrix updates (k = 32) fused in
+// one kernel per walker and split per block (decision and multi-CTA flush
+// kernels), and delayed updates with k in {32, 16, 8} that fit shared memory,
+// each with the tensor-core flush and with the FP64 flush.  FP64 walkers have
+// one form, submatrix updates with the FP64 flush (k = 32).
 static int autotune_delayed(dqmc_batch* b) {
   std::vector<std::pair<int, int>> cand;
   const int kmax = b->kd;
@@ -806,7 +809,7 @@ static int autotune_delayed(dqmc_batch* b) {
     cand.push_back({32, 3});
   }
   for (int kd : {32, 16, 8}) {
-    if (kd > kmax) continue;
+    if (kd > kmax || (!b->mixed && kd != 32)) continue;
     if (b->mixed && kd >= 16) cand.push_back({kd, 1});
     cand.push_back({kd, 0});
   }
@@ -841,9 +844,10 @@ static int autotune_delayed(dqmc_batch* b) {
         launch_metropolis_sub(b->dW, b->nw, MODE_FWD, 0, 0, b->maxN_general, b->smax, b->stream);
       else if (c.second == 3)
         launch_metropolis_sub_split(b->dW, b->nw, MODE_FWD, 0, 0, b->maxN_general, b->smax, b->stream);
+      else if (b->mixed)
+        launch_metropolis_delayed(b->dW, b->nw, MODE_FWD, 0, 0, b->maxN_general, b->smax, c.first, c.second, b->stream);
       else
-        launch_metropolis_delayed(b->mixed, b->dW, b->nw, MODE_FWD, 0, 0, b->maxN_general, b->smax, c.first,
-                                  c.second, b->stream);
+        launch_metropolis_sub64(b->dW, b->nw, MODE_FWD, 0, 0, b->maxN_general, b->smax, b->stream);
       cudaEventRecord(e1, b->stream);
       CUDA_TRY(cudaEventSynchronize(e1));
       float ms = 0;

@@ -1,5 +1,5 @@
-// kernels_delayed.cu — Metropolis with delayed rank-k updates for walkers
-// whose G lives in HBM/L2 (the HBM FP64 path and the mixed path).
+// kernels_delayed.cu — Metropolis with delayed rank-k updates for the mixed
+// path's walkers (candidates of the autotuner beside the submatrix kernels).
 //
 // The reference applies each accepted flip at once as a rank-1 update
 // (update_greens_function, src/model/repulsive_hubbard.cpp:127-155):
@@ -9,8 +9,8 @@
 //     u = f (G0(:,i) - U V(i,:)^T),  w = e_i - (G0(i,:) - U(i,:) V^T)^T,
 // the corrected diagonal is kept up to date per accept (one FMA per site),
 // and every k accepts (and at the end of the slice) G0 <- G0 - U V^T is
-// applied as one dense product: register-light FP64 on the plain path, the
-// exact-slice BF16 tensor-core product on the mixed path.  The decisions are
+// applied as one dense product: register-light FP64, or the exact-slice BF16
+// tensor-core product.  The decisions are
 // the reference's (same ratio, same uniform per site); only the order in which
 // the flips reach G changes, so G agrees with sequential rank-1 updates to
 // rounding.
@@ -165,11 +165,10 @@ __device__ void flush_ozaki(double* G0, int N, const double* U, const double* V,
 // --------------------------------------------------------------------------
 // One slice of Metropolis for general walkers.  One CTA per walker.
 // --------------------------------------------------------------------------
-template <bool MIXED>
 __global__ void __launch_bounds__(kDelThreads) metropolis_delayed_kernel(const WalkerDev* __restrict__ W, int mode,
                                                                         int j, int q, int KD, int tc_flush) {
   const WalkerDev& w = W[blockIdx.x];
-  if (w.path == 0 || (MIXED != (w.path == 2))) return;
+  if (w.path != 2) return;
   int t;
   if (!d_slice_of(w, mode, j, q, t)) return;
   const int N = w.N, S = w.S, Lt = w.Lt, ldu = KD + 1;
@@ -198,7 +197,7 @@ __global__ void __launch_bounds__(kDelThreads) metropolis_delayed_kernel(const W
   int M = 0;  // pending columns of U, V
   auto flush = [&]() {
     if (M == 0) return;
-    if (MIXED && tc_flush && KD >= 16) {
+    if (tc_flush && KD >= 16) {
       // zero the stale columns m >= M so the K = KD product sees only the pending block
       for (int sp = 0; sp < S; ++sp)
         for (int e = threadIdx.x; e < N * (KD - M); e += kDelThreads) {
@@ -301,16 +300,13 @@ static cudaError_t allow_max_smem(K kernel) {
 
 cudaError_t configure_delayed_kernels() {
   cudaError_t e;
-  if ((e = allow_max_smem(metropolis_delayed_kernel<false>))) return e;
-  if ((e = allow_max_smem(metropolis_delayed_kernel<true>))) return e;
+  if ((e = allow_max_smem(metropolis_delayed_kernel))) return e;
   return cudaSuccess;
 }
 
-void launch_metropolis_delayed(bool mixed, const WalkerDev* W, int nw, int mode, int j, int q, int maxN, int S_max,
-                               int KD, int tc_flush, cudaStream_t st) {
-  const size_t sm = delayed_smem_bytes(maxN, S_max, KD);
-  if (mixed) metropolis_delayed_kernel<true><<<nw, kDelThreads, sm, st>>>(W, mode, j, q, KD, tc_flush);
-  else metropolis_delayed_kernel<false><<<nw, kDelThreads, sm, st>>>(W, mode, j, q, KD, 0);
+void launch_metropolis_delayed(const WalkerDev* W, int nw, int mode, int j, int q, int maxN, int S_max, int KD,
+                               int tc_flush, cudaStream_t st) {
+  metropolis_delayed_kernel<<<nw, kDelThreads, delayed_smem_bytes(maxN, S_max, KD), st>>>(W, mode, j, q, KD, tc_flush);
 }
 
 }  // namespace dqmc

@@ -4,8 +4,8 @@
 // G, the B-chain and the stacks stay in HBM/L2; a half-sweep runs slice by
 // slice as a short sequence of batched launches:
 //   wrap (two products in the factors of exp(-dtau K), the diagonal
-//   exp(+/-alpha s) fused) -> Metropolis (one CTA per walker, rank-1 updates,
-//   look-ahead decisions) -> measurement -> B-chain step (one product).
+//   exp(+/-alpha s) fused) -> Metropolis (submatrix updates, kernels_submatrix.cu)
+//   -> measurement -> B-chain step (one product).
 // Stabilization: column-pivoted QR with one thread per column (row-major copy,
 // coalesced across threads), Green's assembly by batched GEMMs and an LU solve
 // with one thread per column of [M | Y].
@@ -368,103 +368,6 @@ __global__ void __launch_bounds__(256) chain_init_general_kernel(const WalkerDev
        e += (long long)gridDim.x * blockDim.x) {
     const int r = (int)(e % N), c = (int)(e / N);
     C[e] = lv ? lv[e] * lv[2LL * N * N + c] : ((r == c) ? 1.0 : 0.0);
-  }
-}
-
-// --------------------------------------------------------------------------
-// Metropolis on global G (general N), one CTA of 512 threads per walker.
-// Warp 0 decides with look-ahead (as in the SMEM kernel), warps 1..15 apply
-// the rank-1 update of the previous accepted site.
-// --------------------------------------------------------------------------
-constexpr int kMetroThreads = 512;
-
-__global__ void __launch_bounds__(kMetroThreads) metropolis_general_kernel(const WalkerDev* __restrict__ W, int mode,
-                                                                          int j, int q) {
-  const WalkerDev& w = W[blockIdx.x];
-  if (!is_general(w)) return;
-  int t, nsl, t_hi;
-  if (!slice_of(w, mode, j, q, t, nsl, t_hi)) return;
-  extern __shared__ double sh[];
-  const int N = w.N, S = w.S, Lt = w.Lt;
-  double* vec = sh;             // [4][N]: f u (2 spins), e_i - G(i,:) (2 spins)
-  double* diag_pre = sh + 4 * N;  // [2][N]
-  int8_t* s_field = (int8_t*)(sh + 6 * N);
-  __shared__ int s_next;
-  __shared__ double s_f[2];
-  const long long NN = (long long)N * N;
-  double* Gs[2] = {w.G, (S == 2) ? w.G + NN : w.G};
-  const int eff = t - 1;
-  for (int i = threadIdx.x; i < N; i += blockDim.x) s_field[i] = w.fields[(long long)eff * N + i];
-  double sign = *w.sign;
-  long long acc_count = 0;
-  const unsigned long long sweep = (w.rng == 1) ? *w.sweep_ctr : 0ULL;
-  __syncthreads();
-
-  auto decide_from = [&](int i0, bool pending) {
-    for (int i = i0; i < N; ++i) {
-      const int s = s_field[i];
-      const int si = s > 0 ? 0 : 1;
-      double gu, gd;
-      if (pending) {
-        gu = fma(-vec[2 * N + i], vec[i], diag_pre[i]);
-        gd = (S == 2) ? fma(-vec[3 * N + i], vec[N + i], diag_pre[N + i]) : gu;
-      } else {
-        gu = Gs[0][(long long)i * N + i];
-        gd = Gs[1][(long long)i * N + i];
-      }
-      const FlipRatio q = flip_ratio(w, si, gu, gd);  // reference operation order
-      const double r = q.r;
-      const int attempt = (mode == MODE_FWD) ? (eff * N + i) : ((Lt - t) * N + i);
-      const double u = (w.rng == 0) ? w.uni[attempt]
-                                    : philox_uniform(w.seed, (unsigned)w.widx, sweep, (unsigned)(eff * N + i));
-      const double prob = fmin(1.0, fabs(r));
-      if (!isfinite(r)) atomicOr(w.status, ST_NONFINITE_RATIO);
-      if (u < prob) {
-        flip_factors(w, q, s_f);
-        s_field[i] = (int8_t)(-s);
-        sign = (r >= 0) ? sign : -sign;
-        ++acc_count;
-        return i;
-      }
-    }
-    return N;
-  };
-  if (threadIdx.x == 0) s_next = decide_from(0, false);
-  __syncthreads();
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
-  while (s_next < N) {
-    const int i = s_next;
-    for (int r = threadIdx.x; r < N; r += blockDim.x) {
-      for (int sp = 0; sp < S; ++sp) {
-        const double* g = Gs[sp];
-        vec[sp * N + r] = s_f[sp] * g[(long long)i * N + r];
-        vec[(2 + sp) * N + r] = ((r == i) ? 1.0 : 0.0) - g[(long long)r * N + i];
-        diag_pre[sp * N + r] = g[(long long)r * N + r];
-      }
-    }
-    __syncthreads();
-    if (wid == 0) {
-      if (lane == 0) s_next = decide_from(i + 1, true);
-    } else {
-      for (int sp = 0; sp < S; ++sp) {
-        double* g = Gs[sp];
-        const double* wv = vec + (2 + sp) * N;
-        const double* uv = vec + sp * N;
-        for (int c = wid - 1; c < N; c += nwarp - 1) {
-          const double wc = -wv[c];
-          double* gc = g + (long long)c * N;
-          for (int r = lane; r < N; r += 32) gc[r] = fma(wc, uv[r], gc[r]);
-        }
-      }
-    }
-    __syncthreads();
-  }
-  int8_t* frw = w.fields + (long long)eff * N;
-  for (int i = threadIdx.x; i < N; i += blockDim.x) frw[i] = s_field[i];
-  if (threadIdx.x == 0) {
-    *w.sign = sign;
-    *w.accepts += acc_count;
-    if (mode == MODE_BWD && t == Lt) *w.sign_Lt = sign;
   }
 }
 
@@ -1315,8 +1218,9 @@ void mixed_wrap_bwd(const WalkerDev* W, int nw, int maxN, int j, int q, cudaStre
 void mixed_chain(const WalkerDev* W, int nw, int maxN, int mode, int j, int q, cudaStream_t st);
 void mixed_dynamic_prop(const WalkerDev* W, int nw, int maxN, int j, int q, cudaStream_t st);
 
-void launch_metropolis_delayed(bool mixed, const WalkerDev* W, int nw, int mode, int j, int q, int maxN, int S_max,
-                               int KD, int tc_flush, cudaStream_t st);
+void launch_metropolis_delayed(const WalkerDev* W, int nw, int mode, int j, int q, int maxN, int S_max, int KD,
+                               int tc_flush, cudaStream_t st);
+void launch_metropolis_sub64(const WalkerDev* W, int nw, int mode, int j, int q, int maxN, int S_max, cudaStream_t st);
 void launch_metropolis_sub(const WalkerDev* W, int nw, int mode, int j, int q, int maxN, int S_max, cudaStream_t st);
 void launch_metropolis_sub_split(const WalkerDev* W, int nw, int mode, int j, int q, int maxN, int S_max,
                                  cudaStream_t st);
@@ -1344,11 +1248,10 @@ void general_slice_pre(int mode, const WalkerDev* W, int nw, int j, int q, int m
 void general_slice_metro(int mode, const WalkerDev* W, int nw, int j, int q, int maxN, int measure, bool mixed,
                          int kd, int smax, int tc_flush, cudaStream_t st) {
   if (mode == MODE_INIT) return;
-  const size_t met_sm = sizeof(double) * 6 * maxN + maxN + 16;
-  if (mixed && tc_flush == 2) launch_metropolis_sub(W, nw, mode, j, q, maxN, smax, st);
-  else if (mixed && tc_flush == 3) launch_metropolis_sub_split(W, nw, mode, j, q, maxN, smax, st);
-  else if (kd > 0) launch_metropolis_delayed(mixed, W, nw, mode, j, q, maxN, smax, kd, tc_flush, st);
-  else metropolis_general_kernel<<<nw, kMetroThreads, met_sm, st>>>(W, mode, j, q);
+  if (!mixed) launch_metropolis_sub64(W, nw, mode, j, q, maxN, smax, st);
+  else if (tc_flush == 2) launch_metropolis_sub(W, nw, mode, j, q, maxN, smax, st);
+  else if (tc_flush == 3) launch_metropolis_sub_split(W, nw, mode, j, q, maxN, smax, st);
+  else launch_metropolis_delayed(W, nw, mode, j, q, maxN, smax, kd, tc_flush, st);
   if (measure) launch_measure_general(W, nw, maxN, mode, j, q, 0, st);
 }
 
@@ -1410,13 +1313,6 @@ void general_dynamic_begin(const WalkerDev* W, int nw, cudaStream_t st) {
 }
 void general_dynamic_end(const WalkerDev* W, int nw, int maxN, cudaStream_t st) {
   dyn_measure_kernel<<<nw, 256, sizeof(double) * (32 + 2 * maxN), st>>>(W, 0, 0, 2);
-}
-
-cudaError_t configure_general_kernels() {
-  cudaError_t e;
-  const int met = (int)(sizeof(double) * 6 * kMaxN + kMaxN + 16);
-  if ((e = cudaFuncSetAttribute(metropolis_general_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, met))) return e;
-  return cudaSuccess;
 }
 
 void general_chain_init(int mode, const WalkerDev* W, int nw, int j, cudaStream_t st) {

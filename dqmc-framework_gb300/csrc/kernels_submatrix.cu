@@ -607,6 +607,21 @@ __device__ __forceinline__ void sub_flush(const SubTC& tcs, unsigned& gt, unsign
 
 size_t submatrix_scratch_bytes(int N) { return sub_offsets(N).total; }
 
+// ---- FP64 walkers: the scratch of a block's update (WalkerDev::msub), per spin Gamma [KK],
+// U = G0(:, I_A) and T = Gamma R_A, both [KB][N], after the accept count and positions [1 + KB]
+size_t submatrix64_scratch_bytes(int N, int S) { return 256 + (size_t)S * sizeof(double) * (KK + 2ull * KB * N); }
+
+namespace {
+struct Sub64 {
+  double *gam, *U, *T;
+};
+__device__ __forceinline__ int* sub64_counts(const WalkerDev& w) { return reinterpret_cast<int*>(w.msub); }
+__device__ __forceinline__ Sub64 sub64_spin(const WalkerDev& w, int sp) {
+  double* b = reinterpret_cast<double*>(w.msub + 256) + (size_t)sp * (KK + 2ull * KB * w.N);
+  return Sub64{b, b + KK, b + KK + (size_t)KB * w.N};
+}
+}  // namespace
+
 // dynamic shared memory of the fused kernel: tensor-core operand buffers first (1024-byte
 // aligned base), then the slice's uniforms [N], Gamma [S][KK], the block state (overlaid by the
 // flush's G staging), the line exponents eG, eT, eR [N], the exponent scratch
@@ -730,10 +745,11 @@ size_t submatrix_flush_smem_bytes(int N) {
   return (size_t)A_BYTES + (size_t)NBB * B_BYTES + kStageBytes + 2 * sizeof(int) * (size_t)((N + 1) & ~1);
 }
 
+template <bool F64>
 __global__ void __launch_bounds__(kSubThreads) metropolis_sub_block_kernel(const WalkerDev* __restrict__ W, int mode,
                                                                            int j, int q, int blk) {
   const WalkerDev& w = W[blockIdx.x];
-  if (w.path != 2) return;
+  if (w.path != (F64 ? 1 : 2)) return;
   int t;
   if (!sub_slice_of(w, mode, j, q, t)) return;
   const int N = w.N, S = w.S, Lt = w.Lt, tid = threadIdx.x;
@@ -756,6 +772,8 @@ __global__ void __launch_bounds__(kSubThreads) metropolis_sub_block_kernel(const
   __shared__ SubAccept s_acc;
 
   const SubOff so = sub_offsets(N);
+  int* mc = F64 ? sub64_counts(w) : reinterpret_cast<int*>(w.msub + so.mc);
+  int* gpos = F64 ? sub64_counts(w) + 1 : reinterpret_cast<int*>(w.msub + so.pos);
   const double* G[2] = {w.G, (S == 2) ? w.G + NN : w.G};
   const int eff = t - 1;
   const unsigned long long sweep = (w.rng == 1) ? *w.sweep_ctr : 0ULL;
@@ -776,10 +794,13 @@ __global__ void __launch_bounds__(kSubThreads) metropolis_sub_block_kernel(const
     *w.sign = sign;
     *w.accepts += acc_count;
     if (mode == MODE_BWD && t == Lt && i0 + KB >= N) *w.sign_Lt = sign;
-    *reinterpret_cast<int*>(w.msub + so.mc) = m;
+    *mc = m;
   }
-  if (tid < m) reinterpret_cast<int*>(w.msub + so.pos)[tid] = s_pos[tid];
-  if (m > 0) {
+  if (tid < m) gpos[tid] = s_pos[tid];
+  if (F64) {
+    for (int e = tid; e < S * KK; e += kSubThreads)
+      if ((e % KB) < m && (e % KK) / KB < m) sub64_spin(w, e / KK).gam[e % KK] = st.Gam[e];
+  } else if (m > 0) {
     int* xGm[2] = {reinterpret_cast<int*>(w.msub + so.eGm), reinterpret_cast<int*>(w.msub + so.total + so.eGm)};
     sub_slice_gamma(w, S, N, m, st.Gam, xGm, etmp);
   }
@@ -874,6 +895,86 @@ __global__ void __launch_bounds__(kSubCTA) metropolis_sub_flush_kernel(const Wal
   sub_tc_close(bar, w);
 }
 
+// ---- FP64 walkers (HBM path): the same block updates in FP64 ---------------------
+// The decision kernel above, then U and T of the block (a CTA per walker, spin and 32 lines) and
+// G -= U T over 32 x 64 tiles of G.  The update's N^2 FMAs per accept run on every SM that the
+// tiles reach (16 walkers of 16 x 16: 36 + 14 + 47 us a block, bound by the decisions' chain and the
+// flush's FP64 rate).  One CTA per walker with k delayed flips in shared memory kept that batch on
+// 16 SMs for 3.6 ms a slice; a pass went from 135 to 92 ms, of 32 walkers of 9 x 9 from 38 to 26.
+
+// T(x, c) = sum_y Gamma(x, y) R(y, c), R = E_A^T - G0(I_A, :), for the 32 lines c of this CTA, and U
+__global__ void __launch_bounds__(256) metropolis_sub64_prep_kernel(const WalkerDev* __restrict__ W, int mode, int j,
+                                                                    int q, int blk) {
+  const WalkerDev& w = W[blockIdx.z];
+  const int sp = blockIdx.y, c0 = blockIdx.x * 32, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (w.path != 1 || sp >= w.S) return;
+  int t;
+  if (!sub_slice_of(w, mode, j, q, t)) return;
+  const int N = w.N;
+  if (blk * KB >= N || c0 >= N) return;
+  const int m = sub64_counts(w)[0];
+  if (m == 0) return;
+  const Sub64 z = sub64_spin(w, sp);
+  const double* G = w.G + (long long)sp * N * N;
+  __shared__ double R[KB][33], Gm[KB][33];  // R[y][line], Gm[y][x]
+  __shared__ int s_i[KB];
+  if (tid < m) s_i[tid] = blk * KB + sub64_counts(w)[1 + tid];
+  for (int e = tid; e < m * KB; e += 256)
+    if (e % KB < m) Gm[e / KB][e % KB] = z.gam[e];
+  __syncthreads();
+  for (int e = tid; e < 32 * 32; e += 256) {  // R along the stored column: lanes over y
+    const int y = e & 31, c = c0 + (e >> 5);
+    if (y < m && c < N) R[y][e >> 5] = ((c == s_i[y]) ? 1.0 : 0.0) - G[(long long)c * N + s_i[y]];
+  }
+  const int c = c0 + lane;
+  if (c < N)
+    for (int y = warp; y < m; y += 8) z.U[(long long)y * N + c] = G[(long long)s_i[y] * N + c];
+  __syncthreads();
+  if (c < N)
+    for (int x = warp; x < m; x += 8) {
+      double v = 0.0;
+#pragma unroll 4
+      for (int y = 0; y < m; ++y) v = fma(Gm[y][x], R[y][lane], v);
+      z.T[(long long)x * N + c] = v;
+    }
+}
+
+// G -= U T on the tile of rows 32 blockIdx.y.., columns 64 blockIdx.x..: a lane per row, 8 columns
+// per warp; the accepts are subtracted in turn, as the flips came
+__global__ void __launch_bounds__(256) metropolis_sub64_flush_kernel(const WalkerDev* __restrict__ W, int mode, int j,
+                                                                     int q, int blk) {
+  const WalkerDev& w = W[blockIdx.z >> 1];
+  const int sp = blockIdx.z & 1, r0 = blockIdx.y * 32, c0 = blockIdx.x * 64, tid = threadIdx.x, lane = tid & 31,
+            warp = tid >> 5;
+  if (w.path != 1 || sp >= w.S) return;
+  int t;
+  if (!sub_slice_of(w, mode, j, q, t)) return;
+  const int N = w.N;
+  if (blk * KB >= N || r0 >= N || c0 >= N) return;
+  const int m = sub64_counts(w)[0];
+  if (m == 0) return;
+  const Sub64 z = sub64_spin(w, sp);
+  __shared__ double Us[KB][32], Ts[KB][64];
+  for (int e = tid; e < m * 32; e += 256) Us[e >> 5][e & 31] = (r0 + (e & 31) < N) ? z.U[(long long)(e >> 5) * N + r0 + (e & 31)] : 0.0;
+  for (int e = tid; e < m * 64; e += 256) Ts[e >> 6][e & 63] = (c0 + (e & 63) < N) ? z.T[(long long)(e >> 6) * N + c0 + (e & 63)] : 0.0;
+  const int r = r0 + lane, cw = c0 + warp * 8;
+  double* g = w.G + (long long)sp * N * N + (long long)cw * N + r;
+  double v[8];
+#pragma unroll
+  for (int k = 0; k < 8; ++k) v[k] = (r < N && cw + k < N) ? g[(long long)k * N] : 0.0;
+  __syncthreads();
+  if (cw >= N) return;
+  for (int y = 0; y < m; ++y) {
+    const double u = -Us[y][lane];
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+      if (cw + k < N) v[k] = fma(u, Ts[y][warp * 8 + k], v[k]);  // uniform in the warp
+  }
+#pragma unroll
+  for (int k = 0; k < 8; ++k)
+    if (r < N && cw + k < N) g[(long long)k * N] = v[k];
+}
+
 static size_t g_sub_smem_limit = 0;  // dynamic shared memory the kernel may use
 
 cudaError_t configure_submatrix_kernel() {
@@ -888,7 +989,10 @@ cudaError_t configure_submatrix_kernel() {
                              (int)g_sub_smem_limit);
   }
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(metropolis_sub_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    e = cudaFuncSetAttribute(metropolis_sub_block_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)submatrix_block_smem_bytes(2));
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(metropolis_sub_block_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)submatrix_block_smem_bytes(2));
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(metropolis_sub_prep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPrepSmem);
@@ -912,9 +1016,20 @@ void launch_metropolis_sub_split(const WalkerDev* W, int nw, int mode, int j, in
   const int P = (nw * S_max * nct <= 152) ? nct : (nct + 1) / 2;
   const size_t sm1 = submatrix_block_smem_bytes(S_max), sm2 = submatrix_flush_smem_bytes(maxN);
   for (int blk = 0; blk < nb; ++blk) {
-    metropolis_sub_block_kernel<<<nw, kSubThreads, sm1, st>>>(W, mode, j, q, blk);
+    metropolis_sub_block_kernel<false><<<nw, kSubThreads, sm1, st>>>(W, mode, j, q, blk);
     metropolis_sub_prep_kernel<<<dim3(nrb, S_max, nw), kSubCTA, kPrepSmem, st>>>(W, mode, j, q, blk);
     metropolis_sub_flush_kernel<<<dim3(P, S_max, nw), kSubCTA, sm2, st>>>(W, mode, j, q, blk);
+  }
+}
+
+// One slice of Metropolis of the FP64 HBM walkers
+void launch_metropolis_sub64(const WalkerDev* W, int nw, int mode, int j, int q, int maxN, int S_max, cudaStream_t st) {
+  const int nb = (maxN + KB - 1) / KB, n32 = (maxN + 31) / 32, n64 = (maxN + 63) / 64;
+  const size_t sm = submatrix_block_smem_bytes(S_max);
+  for (int blk = 0; blk < nb; ++blk) {
+    metropolis_sub_block_kernel<true><<<nw, kSubThreads, sm, st>>>(W, mode, j, q, blk);
+    metropolis_sub64_prep_kernel<<<dim3(n32, S_max, nw), 256, 0, st>>>(W, mode, j, q, blk);
+    metropolis_sub64_flush_kernel<<<dim3(n64, n32, 2 * nw), 256, 0, st>>>(W, mode, j, q, blk);
   }
 }
 

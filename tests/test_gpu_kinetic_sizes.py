@@ -1,6 +1,6 @@
 """The factored exp(-+dtau K) products of HBM walkers (kin_op_kernel: whole columns or rows of about
 2048 elements a CTA) against the shared-memory kernels' on the same chains: every side from 2 to 8,
-both kinds of factors, two and three directions; the last tile of columns or rows is ragged at
+both kinds of factors, two and three directions (and the FP64 submatrix updates); the last tile of columns or rows is ragged at
 most sides.  Identical decisions and G within 1e-10, the bar of the FP64 paths."""
 import numpy as np
 import pytest
