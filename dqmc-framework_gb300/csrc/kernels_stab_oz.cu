@@ -600,9 +600,42 @@ __global__ void __launch_bounds__(256) zpush_prep_kernel(const WalkerDev* __rest
 
 // --------------------------------------------------------------------------
 // Householder panel p of X (rows j0:N, columns j0:j0+pb) in shared memory:
-// reflectors into X below the diagonal, R on and above, T_p (dlarft) into the
-// scratch; for the push also D = |diag R| into the stack level and 1/D.
+// reflectors into X below the diagonal, R on and above, tau on the diagonal of the panel's T
+// slot; for the push also D = |diag R| into the stack level and 1/D.
+//
+// Column c takes two barriers.  After the first, warps 1-7 form the dot products of the column
+// with the remaining ones from the unscaled column x, while warp 0 reduces its norm and computes
+// tau and the scale of the reflector v = x scale (a square root and one division, the two
+// quotients on two lanes); after the second, warps 1-7 apply the reflector, A -= x (scale w), and
+// warp 0 does so for column c + 1 and accumulates its norm.  The columns' scales are applied when
+// the panel is written back.  The dot products of a warp's columns share their shuffle steps
+// (zsum4, zsum8): an FP64 add costs a warp 64 cycles whatever its lanes hold.  What bounds it: the
+// FP64 rate of one SM (2 m pb^2 operations) for long panels, warp 0's chain for short ones.
+// Average of the 8 panels at N = 256 (12 CTAs): 134 us; 185 with a norm pass, a scaling pass, serial
+// quotients and a shuffle reduction per column.  A pass of 6 walkers of 16 x 16 went from 59.8 to
+// 55.6 ms (with ztfac_kernel), of 128 walkers from 794 to 771.
 // --------------------------------------------------------------------------
+// Sums of 4 (8) values over the warp, value k left in lanes 8 k .. 8 k + 7 (4 k .. 4 k + 3)
+__device__ __forceinline__ double zsum4(double a0, double a1, double a2, double a3, int lane) {
+  const bool h = lane & 16, q = lane & 8;
+  double x = (h ? a2 : a0) + __shfl_xor_sync(0xffffffffu, h ? a0 : a2, 16);
+  double y = (h ? a3 : a1) + __shfl_xor_sync(0xffffffffu, h ? a1 : a3, 16);
+  double v = (q ? y : x) + __shfl_xor_sync(0xffffffffu, q ? x : y, 8);
+  for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+__device__ __forceinline__ double zsum8(const double (&a)[8], int lane) {
+  const bool h = lane & 16, q = lane & 8, e = lane & 4;
+  double x[4], y[2];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) x[k] = (h ? a[k + 4] : a[k]) + __shfl_xor_sync(0xffffffffu, h ? a[k] : a[k + 4], 16);
+#pragma unroll
+  for (int k = 0; k < 2; ++k) y[k] = (q ? x[k + 2] : x[k]) + __shfl_xor_sync(0xffffffffu, q ? x[k] : x[k + 2], 8);
+  double v = (e ? y[1] : y[0]) + __shfl_xor_sync(0xffffffffu, e ? y[0] : y[1], 4);
+  for (int o = 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
 __global__ void __launch_bounds__(256) zqr_panel_kernel(const WalkerDev* __restrict__ W, int mode, int j, int p,
                                                         int push) {
   const int wi = blockIdx.x >> 1, sp = blockIdx.x & 1;
@@ -612,60 +645,108 @@ __global__ void __launch_bounds__(256) zqr_panel_kernel(const WalkerDev* __restr
   if (j0 >= N) return;
   const int m = N - j0, pb = min(TB, m);
   const ZScr z = zscr(w, sp);
-  extern __shared__ double psm[];
-  double* P = psm;                // [TB][m], P[c * m + r]
-  double* T = P + TB * m;         // [TB][TB], T[c * TB + r] (tau on the diagonal)
-  __shared__ double s_red[8];
-  __shared__ double s_tau, s_scal;
+  extern __shared__ double P[];  // [TB][m], P[c * m + r]
+  __shared__ double s_tau[TB], s_scal[TB], s_dot[TB];
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  for (int c = 0; c < pb; ++c)
-    for (int r = tid; r < m; r += 256) P[c * m + r] = z.X[(long long)(j0 + c) * N + j0 + r];
+  for (int c = wid; c < pb; c += 8)
+    for (int r = lane; r < m; r += 32) P[c * m + r] = z.X[(long long)(j0 + c) * N + j0 + r];
   __syncthreads();
+  double xn2 = 0.0;  // warp 0: this lane's part of the squared norm of column c below the diagonal
+  if (wid == 0)
+    for (int r = 1 + lane; r < m; r += 32) xn2 = fma(P[r], P[r], xn2);
   for (int c = 0; c < pb; ++c) {
-    double s = 0.0;
-    for (int r = c + 1 + tid; r < m; r += 256) s = fma(P[c * m + r], P[c * m + r], s);
-    s = zwarp_sum(s);
-    if (lane == 0) s_red[wid] = s;
-    __syncthreads();
-    if (tid == 0) {
-      double xn2 = 0.0;
-      for (int q = 0; q < 8; ++q) xn2 += s_red[q];
-      const double alpha = P[c * m + c];
-      double tau = 0.0, beta = alpha, scal = 1.0;
-      if (xn2 != 0.0) {
-        const double nrm = sqrt(alpha * alpha + xn2);
-        beta = alpha >= 0 ? -nrm : nrm;
-        tau = (beta - alpha) / beta;
-        scal = 1.0 / (alpha - beta);
+    const double* x = P + c * m;
+    const int nr = pb - 1 - c;  // columns after c
+    if (wid == 0) {
+      const double n2 = zwarp_sum(xn2), alpha = x[c];
+      const double nrm = sqrt(fma(alpha, alpha, n2));
+      const bool any = __double_as_longlong(n2) != 0;  // n2 >= 0; bit tests keep off the FP64 pipe
+      const double beta = __double_as_longlong(alpha) < 0 ? nrm : -nrm;
+      // lane 0: tau = (beta - alpha) / beta, lane 1: scale = 1 / (alpha - beta)
+      const double d = beta - alpha, quo = __ddiv_rn(lane == 1 ? 1.0 : d, lane == 1 ? -d : beta);
+      if (lane == 0) s_tau[c] = any ? quo : 0.0;
+      if (lane == 1) s_scal[c] = any ? quo : 1.0;
+      __syncwarp();
+      if (lane == 0) P[c * m + c] = any ? beta : alpha;
+    } else {
+      // columns c + 1 + (wid - 1) + 7 k, at most 5
+      double acc[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) acc[k] = 0.0;
+      const int c0 = c + wid, nc = (c0 < pb) ? (pb - c0 + 6) / 7 : 0;
+      if (nc > 0) {
+        for (int r = c + 1 + lane; r < m; r += 32) {
+          const double xr = x[r];
+#pragma unroll
+          for (int k = 0; k < 5; ++k)
+            if (k < nc) acc[k] = fma(xr, P[(c0 + 7 * k) * m + r], acc[k]);
+        }
+        __syncwarp();
+        if (nc <= 4) {
+          const double v = zsum4(acc[0], acc[1], acc[2], acc[3], lane);
+          if ((lane & 7) == 0 && (lane >> 3) < nc) s_dot[c0 + 7 * (lane >> 3)] = v;
+        } else {
+          const double v = zsum8(acc, lane);
+          if ((lane & 3) == 0 && (lane >> 2) < nc) s_dot[c0 + 7 * (lane >> 2)] = v;
+        }
       }
-      s_tau = tau;
-      s_scal = scal;
-      P[c * m + c] = beta;
-      T[c * TB + c] = tau;
     }
     __syncthreads();
-    const double scal = s_scal, tau = s_tau;
-    for (int r = c + 1 + tid; r < m; r += 256) P[c * m + r] *= scal;
-    __syncthreads();
-    if (tau != 0.0)
-      for (int cc = c + 1 + wid; cc < pb; cc += 8) {
-        double d = 0.0;
-        for (int r = c + 1 + lane; r < m; r += 32) d = fma(P[c * m + r], P[cc * m + r], d);
-        d = zwarp_sum(d) + P[cc * m + c];
-        const double wv = tau * d;
-        if (lane == 0) P[cc * m + c] -= wv;
-        for (int r = c + 1 + lane; r < m; r += 32) P[cc * m + r] = fma(-wv, P[c * m + r], P[cc * m + r]);
+    const double tau = s_tau[c], scal = s_scal[c];
+    if (nr > 0) {
+      if (wid == 0) {
+        // column c + 1, and its norm below row c + 1
+        double* a = P + (c + 1) * m;
+        const double wv = tau * fma(scal, s_dot[c + 1], a[c]), ws = -(wv * scal);
+        __syncwarp();
+        if (lane == 0) a[c] -= wv;
+        xn2 = 0.0;
+        for (int r = c + 1 + lane; r < m; r += 32) {
+          const double v = fma(ws, x[r], a[r]);
+          a[r] = v;
+          if (r > c + 1) xn2 = fma(v, v, xn2);
+        }
+        __syncwarp();
+      } else {
+        // columns c + 2 + (wid - 1) + 7 k: lane k forms column k's factor
+        const int c0 = c + 1 + wid, nc = (c0 < pb) ? (pb - c0 + 6) / 7 : 0;
+        double ws = 0.0;
+        if (lane < nc) {
+          double* a = P + (c0 + 7 * lane) * m;
+          const double wv = tau * fma(scal, s_dot[c0 + 7 * lane], a[c]);
+          a[c] -= wv;
+          ws = -(wv * scal);
+        }
+        double f[5];
+#pragma unroll
+        for (int k = 0; k < 5; ++k) f[k] = __shfl_sync(0xffffffffu, ws, k);
+        if (nc > 0)
+          for (int r = c + 1 + lane; r < m; r += 32) {
+            const double xr = x[r];
+            double v[5];
+#pragma unroll
+            for (int k = 0; k < 5; ++k) v[k] = (k < nc) ? P[(c0 + 7 * k) * m + r] : 0.0;
+#pragma unroll
+            for (int k = 0; k < 5; ++k)
+              if (k < nc) P[(c0 + 7 * k) * m + r] = fma(f[k], xr, v[k]);
+          }
       }
+    }
     __syncthreads();
   }
-  for (int c = 0; c < pb; ++c)
-    for (int r = tid; r < m; r += 256) z.X[(long long)(j0 + c) * N + j0 + r] = P[c * m + r];
+  for (int c = wid; c < pb; c += 8) {
+    const double scal = s_scal[c];
+    for (int r = lane; r < m; r += 32) {
+      const double v = P[c * m + r];
+      z.X[(long long)(j0 + c) * N + j0 + r] = (r > c) ? v * scal : v;
+    }
+  }
   // the Gram matrix V^T V, the T factor and Vt = V T follow on the tensor cores (Z_GRAM,
   // ztfac_kernel, Z_VT); the panel leaves tau on the diagonal of its T slot
   double* Tg = z.Tb + (long long)p * TB * TB;
   for (int e = tid; e < TB * TB; e += 256) {
     const int r = e % TB, c = e / TB;
-    Tg[e] = (r == c && c < pb) ? T[c * TB + c] : 0.0;
+    Tg[e] = (r == c && c < pb) ? s_tau[c] : 0.0;
   }
   if (push && tid < pb) {
     const int side = (mode == MODE_FWD) ? 0 : 1;
@@ -677,34 +758,46 @@ __global__ void __launch_bounds__(256) zqr_panel_kernel(const WalkerDev* __restr
   }
 }
 
-// The T factor of panel p (LAPACK dlarft, forward, columnwise): T(c, c) = tau_c and
-// T(0:c, c) = -tau_c T(0:c, 0:c) Zg(0:c, c), Zg = V^T V from the Z_GRAM product (in Wb).
-// One warp per (walker, spin).
-__global__ void __launch_bounds__(32) ztfac_kernel(const WalkerDev* __restrict__ W, int mode, int j, int p) {
+// The T factor of panel p: T^-1 = diag(1 / tau) + the strict upper part of Zg = V^T V (the Z_GRAM
+// product, in Wb), so row i of T is tau_i (e_i - sum_{k > i} Zg(i, k) T(k, :)), rows from the last
+// up: when row k is known every warp adds its term to its own rows above (rows i = warp mod 8, lane
+// per column), two barriers apart at most 4 FMAs.  One warp adding the columns' terms one after the
+// other (LAPACK's dlarft) took 36 us, this 20.
+__global__ void __launch_bounds__(256) ztfac_kernel(const WalkerDev* __restrict__ W, int mode, int j, int p) {
   const int wi = blockIdx.x >> 1, sp = blockIdx.x & 1;
   const WalkerDev& w = W[wi];
   if (!w.ozstab || sp >= w.S || j >= w.nstack) return;
   const int N = w.N, j0 = p * TB;
   if (j0 >= N) return;
-  const int pb = min(TB, N - j0), tid = threadIdx.x;
+  const int pb = min(TB, N - j0), tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const ZScr z = zscr(w, sp);
-  __shared__ double T[TB * TB], Zg[TB * TB];
+  __shared__ double Zg[TB][TB + 1], Tr[TB][TB];  // Zg[k][i] = Zg(i, k); Tr[k][j] = T(k, j)
+  __shared__ double tau[TB];
   double* Tg = z.Tb + (long long)p * TB * TB;
-  for (int e = tid; e < TB * TB; e += 32) {
-    T[e] = Tg[e];  // tau on the diagonal, zeros elsewhere
-    const int i = e % TB, c = e / TB;
-    Zg[e] = (i < pb && c < pb) ? z.Wb[(long long)c * TB + i] : 0.0;
+  for (int e = tid; e < TB * TB; e += 256) {
+    const int i = e % TB, k = e / TB;
+    Zg[k][i] = (i < k && k < pb) ? z.Wb[(long long)k * TB + i] : 0.0;
+    if (i == k) tau[k] = (k < pb) ? Tg[e] : 0.0;
   }
-  __syncwarp();
-  for (int c = 1; c < pb; ++c) {
-    double s = 0.0;
-    if (tid < c)
-      for (int k = tid; k < c; ++k) s = fma(T[k * TB + tid], Zg[c * TB + k], s);
-    __syncwarp();
-    if (tid < c) T[c * TB + tid] = -T[c * TB + c] * s;
-    __syncwarp();
+  double acc[4] = {0.0, 0.0, 0.0, 0.0};  // rows wid + 8 u
+  __syncthreads();
+  for (int k = pb - 1; k >= 0; --k) {
+    if (wid == (k & 7)) {
+      const int u = k >> 3;
+      const double a = (u == 0) ? acc[0] : (u == 1) ? acc[1] : (u == 2) ? acc[2] : acc[3];
+      Tr[k][lane] = tau[k] * (((lane == k) ? 1.0 : 0.0) - a);
+    }
+    __syncthreads();
+    const double t = Tr[k][lane];
+#pragma unroll
+    for (int u = 3; u >= 0; --u)
+      if (wid + 8 * u < k) acc[u] = fma(Zg[k][wid + 8 * u], t, acc[u]);  // uniform in the warp
   }
-  for (int e = tid; e < TB * TB; e += 32) Tg[e] = T[e];
+  __syncthreads();
+  for (int e = tid; e < TB * TB; e += 256) {
+    const int i = e % TB, k = e / TB;  // T(i, k)
+    Tg[e] = (i <= k && k < pb) ? Tr[i][k] : 0.0;
+  }
 }
 
 // Vt = V_p T_p^T (m x pb, ld N) for forming Q: Vt(r, c) = sum_{c <= q <= r} V(r, q) T(c, q).
@@ -923,7 +1016,7 @@ __global__ void __launch_bounds__(256) zdyn_boundary_kernel(const WalkerDev* __r
 #define ZGEMM56 zgemm_tc_kernel<8, 7, 32, 2, 2>
 #define ZGEMM54 zgemm_tc_kernel<9, 6, 32, 4, 1>
 static size_t ztc_smem(int S, int NT, int NS) { return (size_t)NS * oztc::stage_bytes(S, 128, NT); }
-static size_t zpanel_smem(int maxN) { return sizeof(double) * ((size_t)TB * maxN + TB * TB); }
+static size_t zpanel_smem(int maxN) { return sizeof(double) * (size_t)TB * maxN; }
 
 cudaError_t configure_stab_oz_kernels(int maxN) {
   cudaError_t e;
@@ -952,7 +1045,7 @@ static void zgemm(const WalkerDev* W, int nw, int maxN, int op, int mode, int j,
 static void zpanel(const WalkerDev* W, int nw, int maxN, int mode, int j, int p, int push, cudaStream_t st) {
   zqr_panel_kernel<<<2 * nw, 256, zpanel_smem(maxN), st>>>(W, mode, j, p, push);
   zgemm(W, nw, maxN, Z_GRAM, mode, j, p, TB, TB, -1, st);
-  ztfac_kernel<<<2 * nw, 32, 0, st>>>(W, mode, j, p);
+  ztfac_kernel<<<2 * nw, 256, 0, st>>>(W, mode, j, p);
   zgemm(W, nw, maxN, Z_VT, mode, j, p, maxN, TB, -1, st);
 }
 
