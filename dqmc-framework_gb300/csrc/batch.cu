@@ -70,9 +70,10 @@ void general_dynamic_stab(const WalkerDev* W, int nw, int j, int maxN, cudaStrea
 void general_dynamic_stab_measure(const WalkerDev* W, int nw, int j, cudaStream_t st);
 void general_dynamic_begin(const WalkerDev* W, int nw, cudaStream_t st);
 void general_dynamic_end(const WalkerDev* W, int nw, int maxN, cudaStream_t st);
-void oz_push(int mode, const WalkerDev* W, int nw, int j, int maxN, cudaStream_t st);
-void oz_greens(int mode, const WalkerDev* W, int nw, int j, int trace_slot, int maxN, cudaStream_t st,
+void oz_push(int mode, const WalkerDev* W, int nw, int j, StabSizes zs, cudaStream_t st);
+void oz_greens(int mode, const WalkerDev* W, int nw, int j, int trace_slot, StabSizes zs, cudaStream_t st,
                bool dyn = false);
+size_t stab_scratch_elems(int N);
 cudaError_t configure_stab_oz_kernels(int maxN);
 void general_greens(int mode, const WalkerDev* W, int nw, int j, int trace_slot, int maxN, cudaStream_t st);
 void general_measure_after(int mode, const WalkerDev* W, int nw, int j, int maxN, cudaStream_t st);
@@ -93,10 +94,15 @@ using namespace dqmc;
 
 namespace {
 
-// walkers of the tensor-core path with 128 <= N <= 768 are stabilized by the
-// blocked QR of kernels_stab_oz.cu (its FP64 panel of 32 columns fits shared memory)
+// HBM walkers with 32 < N <= 768 are stabilized by the blocked QR of kernels_stab_oz.cu (its
+// FP64 panel of 32 columns fits shared memory up to 768 rows; one panel or less gains nothing
+// from blocks): 1 with tensor-core products (mixed walkers of N >= 128), 2 with FP64 products.
+// The others keep the column-pivoted QR and the LU with one thread per column.
 constexpr int kMaxOzN = 768;
-bool uses_ozstab(int N, int precision) { return precision == DQMC_MIXED && N >= 128 && N <= kMaxOzN; }
+int stab_kind(int N, int precision, bool general) {
+  if (!general || N <= 32 || N > kMaxOzN) return 0;
+  return (precision == DQMC_MIXED && N >= 128) ? 1 : 2;
+}
 
 thread_local std::string g_err;
 
@@ -268,8 +274,9 @@ struct dqmc_batch {
   // walkers split by kernel family: N <= 64 (SMEM-resident) and N > 64 (general)
   int maxN_small = 0, maxN_general = 0, maxPace_general = 0;
   bool any_small = false, any_general = false, any_general_dense = false, any_general_cb = false;
-  bool any_ozstab = false;  // walkers stabilized by the tensor-core blocked QR
-  int maxN_oz = 0;
+  bool any_ozstab = false;  // walkers stabilized by the blocked QR
+  bool any_qrp = false;     // HBM walkers stabilized by the column-pivoted QR and LU
+  StabSizes stab{};
   bool mixed = false;
   int kd = 0, smax = 1;  // flips a block update takes: delayed updates' k, 32 for submatrix updates
   // Metropolis of HBM walkers: 0 FP64 flush (FP64 walkers: submatrix updates; mixed: delayed), 1 delayed with tensor-core
@@ -422,9 +429,12 @@ int dqmc_batch_create(const dqmc_walker_desc* descs, int n, const dqmc_batch_opt
       b->maxN_general = std::max(b->maxN_general, N);
       b->maxPace_general = std::max(b->maxPace_general, d.pace);
       if (d.checkerboard) b->any_general_cb = true; else b->any_general_dense = true;
-      if (uses_ozstab(N, o.precision)) {
+      if (const int kind = stab_kind(N, o.precision, true)) {
         b->any_ozstab = true;
-        b->maxN_oz = std::max(b->maxN_oz, N);
+        int& n = (kind == 1) ? b->stab.tc : b->stab.f64;
+        n = std::max(n, N);
+      } else {
+        b->any_qrp = true;
       }
     } else {
       b->any_small = true;
@@ -443,7 +453,7 @@ int dqmc_batch_create(const dqmc_walker_desc* descs, int n, const dqmc_batch_opt
   b->tc_flush = b->mixed ? 2 : 0;  // submatrix updates until the tuner has timed the candidates
 
   // ---- arena layout ----
-  struct Off { size_t G, chain, work, scr, sl, sle, stack, fields, ff, trace, msub, zsl; int dense_id; };
+  struct Off { size_t G, chain, work, scr, sl, sle, stack, fields, ff, trace, msub, zsl, zwk; int dense_id; };
   std::vector<Off> off(n);
   std::map<std::tuple<int, int, double, double, double>, int> dense_ids;  // (L, dim, t, mu, dtau) -> id
   std::vector<std::pair<std::vector<double>, std::vector<double>>> dense;
@@ -474,7 +484,11 @@ int dqmc_batch_create(const dqmc_walker_desc* descs, int n, const dqmc_batch_opt
     off[w].msub = (o.precision == DQMC_MIXED) ? take((size_t)S * submatrix_scratch_bytes(N))
                   : general                     ? take(submatrix64_scratch_bytes(N, S))
                                                 : 0;
-    off[w].zsl = uses_ozstab(N, o.precision)
+    // the blocked QR's scratch is the product temporary where that has room (N >= 110)
+    off[w].zwk = off[w].work;
+    if (stab_kind(N, o.precision, general) && stab_scratch_elems(N) > (size_t)N * N)
+      off[w].zwk = take(sizeof(double) * S * stab_scratch_elems(N));
+    off[w].zsl = stab_kind(N, o.precision, general) == 1
                      ? take(sizeof(unsigned short) * (size_t)S * 2 * 9 * ozaki::tc_lines(N) * (size_t)((N + 31) / 32 * 32))
                      : 0;
     off[w].dense_id = -1;
@@ -642,9 +656,11 @@ int dqmc_batch_create(const dqmc_walker_desc* descs, int n, const dqmc_batch_opt
     h.work = gen ? reinterpret_cast<double*>(base + off[w].work) : nullptr;
     h.scr = gen ? reinterpret_cast<double*>(base + off[w].scr) : nullptr;
     h.msub = gen ? reinterpret_cast<unsigned char*>(base + off[w].msub) : nullptr;
-    h.ozstab = uses_ozstab(N, o.precision) ? 1 : 0;
+    h.ozstab = stab_kind(N, o.precision, gen);
+    h.zwk = gen ? reinterpret_cast<double*>(base + off[w].zwk) : nullptr;
+    h.zwk_stride = (off[w].zwk == off[w].work) ? (long long)N * N : (long long)stab_scratch_elems(N);
     h.zld = (N + 31) / 32 * 32;
-    h.zsl = h.ozstab ? reinterpret_cast<unsigned short*>(base + off[w].zsl) : nullptr;
+    h.zsl = h.ozstab == 1 ? reinterpret_cast<unsigned short*>(base + off[w].zsl) : nullptr;
     if (o.precision == DQMC_MIXED) {
       h.ldk = (N + 15) / 16 * 16;
       h.slice_bits = ozaki::cfg_for_k(N).bits;
@@ -941,8 +957,8 @@ int dqmc_init_greens(dqmc_batch* b) {
       for (int q = 0; q < b->maxPace_general; ++q)
         general_slice_post(MODE_INIT, b->dW, b->nw, j, q, b->maxN_general, b->any_general_dense, b->any_general_cb,
                            b->mixed, b->stream);  // the transposed B-chain of the initial right stack
-      general_push(MODE_INIT, b->dW, b->nw, j, b->maxN_general, b->stream);
-      if (b->any_ozstab) oz_push(MODE_INIT, b->dW, b->nw, j, b->maxN_oz, b->stream);
+      if (b->any_qrp) general_push(MODE_INIT, b->dW, b->nw, j, b->maxN_general, b->stream);
+      if (b->any_ozstab) oz_push(MODE_INIT, b->dW, b->nw, j, b->stab, b->stream);
     }
   }
   if (b->any_small) {
@@ -950,8 +966,8 @@ int dqmc_init_greens(dqmc_batch* b) {
     launch_sign(b->dW, b->nw, b->maxN_small, b->stream);
   }
   if (b->any_general) {
-    general_greens(MODE_INIT, b->dW, b->nw, 0, -1, b->maxN_general, b->stream);
-    if (b->any_ozstab) oz_greens(MODE_INIT, b->dW, b->nw, 0, -1, b->maxN_oz, b->stream);
+    if (b->any_qrp) general_greens(MODE_INIT, b->dW, b->nw, 0, -1, b->maxN_general, b->stream);
+    if (b->any_ozstab) oz_greens(MODE_INIT, b->dW, b->nw, 0, -1, b->stab, b->stream);
     general_sign(b->dW, b->nw, b->maxN_general, b->stream);
   }
   if (int r = launch_check("init kernels")) return r;
@@ -988,12 +1004,12 @@ static void issue_general_level(dqmc_batch* b, int mode, int measure, int j, int
     });
   }
   b->timed(DQMC_KCLASS_PUSH, [&] {
-    general_push(mode, W, nw, j, b->maxN_general, st);
-    if (b->any_ozstab) oz_push(mode, W, nw, j, b->maxN_oz, st);
+    if (b->any_qrp) general_push(mode, W, nw, j, b->maxN_general, st);
+    if (b->any_ozstab) oz_push(mode, W, nw, j, b->stab, st);
   });
   b->timed(DQMC_KCLASS_GREENS, [&] {
-    general_greens(mode, W, nw, j, slot, b->maxN_general, st);
-    if (b->any_ozstab) oz_greens(mode, W, nw, j, slot, b->maxN_oz, st);
+    if (b->any_qrp) general_greens(mode, W, nw, j, slot, b->maxN_general, st);
+    if (b->any_ozstab) oz_greens(mode, W, nw, j, slot, b->stab, st);
   });
   if (measure) b->timed(DQMC_KCLASS_MEASURE, [&] { general_measure_after(mode, W, nw, j, b->maxN_general, st); });
 }
@@ -1252,6 +1268,7 @@ struct DynShape {
 static void issue_dynamic_level(dqmc_batch* b, const DynShape& ds, int j, const WalkerDev* W, int nw,
                                 cudaStream_t st) {
   const int maxN = ds.maxN;
+  const bool qrp = b->any_qrp || b->any_small;  // shared-memory walkers run this half-sweep as HBM walkers
   b->timed(DQMC_KCLASS_SEGMENT, [&] { general_chain_init(MODE_FWD, W, nw, j, st); });
   for (int q = 0; q < ds.maxPace; ++q) {
     b->timed(DQMC_KCLASS_PRODUCT,
@@ -1262,15 +1279,17 @@ static void issue_dynamic_level(dqmc_batch* b, const DynShape& ds, int j, const 
              [&] { general_dynamic_chain(W, nw, j, q, maxN, b->mixed, ds.any_dense, ds.any_cb, st); });
   }
   b->timed(DQMC_KCLASS_PUSH, [&] {
-    general_push(MODE_FWD, W, nw, j, maxN, st);
-    if (b->any_ozstab) oz_push(MODE_FWD, W, nw, j, b->maxN_oz, st);
+    if (qrp) general_push(MODE_FWD, W, nw, j, maxN, st);
+    if (b->any_ozstab) oz_push(MODE_FWD, W, nw, j, b->stab, st);
   });
-  b->timed(DQMC_KCLASS_GREENS, [&] { general_greens(MODE_FWD, W, nw, j, -1, maxN, st); });
+  b->timed(DQMC_KCLASS_GREENS, [&] {
+    if (qrp) general_greens(MODE_FWD, W, nw, j, -1, maxN, st);
+  });
   // the tensor-core walkers' equal-time assembly and their G(t,0), G(0,t) come from one
   // oz_greens (one factorization of M), timed in this class
   b->timed(DQMC_KCLASS_DYN_STAB, [&] {
-    general_dynamic_stab(W, nw, j, maxN, st);
-    if (b->any_ozstab) oz_greens(MODE_FWD, W, nw, j, -1, b->maxN_oz, st, true);
+    if (qrp) general_dynamic_stab(W, nw, j, maxN, st);
+    if (b->any_ozstab) oz_greens(MODE_FWD, W, nw, j, -1, b->stab, st, true);
     general_dynamic_stab_measure(W, nw, j, st);
   });
 }
@@ -1313,8 +1332,8 @@ int dqmc_sweep_dynamic(dqmc_batch* b, const int* taus, int ntau) {
     for (auto& h : b->hw) h.dyn_ntau = ntau;
     if (int r = dqmc_clear_dynamic(b)) return r;
   }
-  // walkers of the tensor-core path with 128 <= N <= 768 stabilize with the blocked QR
-  // (oz_push, oz_greens with the second right-hand side), the others with the FP64 kernels;
+  // HBM walkers with 32 < N <= 768 stabilize with the blocked QR (oz_push, oz_greens with the
+  // second right-hand side), the others with the column-pivoted QR and LU kernels;
   // shared-memory walkers run this half-sweep on the HBM path's kernels with their own
   // buffers (the stacks, G and the fields are laid out alike on both paths)
   std::vector<WalkerDev> hv = b->hw;

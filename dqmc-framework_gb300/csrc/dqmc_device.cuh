@@ -104,11 +104,20 @@ struct WalkerDev {
   const unsigned long long* sweep_ctr;  // Philox counter word: the batch's half-sweep index (device)
   double* trace;             // [trace_cap][2][N*N] or null
   int trace_cap;
-  int ozstab;                // 1: stabilization by the tensor-core blocked QR (kernels_stab_oz.cu)
+  int ozstab;                // stabilization by the blocked QR (kernels_stab_oz.cu): 1 with tensor-core
+                             // products, 2 with FP64 products, 0 not
+  double* zwk;               // its scratch per spin, zwk_stride doubles apart
+  long long zwk_stride;
   int widx;                  // index of the walker in its batch (Philox counter word)
   // iteration limit of the wraps' and B-chain products' waits for their operands to land
   // (oz_prod_tc_kernel); kDefaultWaitLimit unless a test lowers it (dqmc_set_wait_limit)
   int wait_limit;
+};
+
+// The largest N of a batch's walkers stabilized with tensor-core and with FP64 products (0: none)
+struct StabSizes {
+  int tc, f64;
+  __host__ __device__ int max() const { return tc > f64 ? tc : f64; }
 };
 
 constexpr int kDefaultWaitLimit = 1 << 24;

@@ -1,6 +1,8 @@
-// kernels_stab_oz.cu — stabilization of tensor-core-path walkers (N >= 128):
-// the UDT push and the Green's assembly as blocked Householder factorizations
-// whose matrix products run on the BF16 tensor cores at FP64 accuracy.
+// kernels_stab_oz.cu — stabilization of HBM walkers (32 < N <= 768): the UDT
+// push and the Green's assembly as blocked Householder factorizations whose
+// matrix products run on the BF16 tensor cores at FP64 accuracy (mixed walkers
+// with N >= 128, WalkerDev::ozstab 1) or in FP64 (FP64 walkers, and mixed ones
+// below 128 sites, where a product does not fill the tensor core's tiles; 2).
 //
 // Reference: SvdStack::push (src/svd_stack.cpp:34-87) factors the B-chain with
 // MKL dgesvd and compute_equaltime_greens (include/utils/numerical_stable.hpp:
@@ -59,9 +61,9 @@ __device__ __forceinline__ void zstack_tops(const WalkerDev& w, int mode, int j,
 }
 
 // per-spin scratch: scr = X (matrix being factored) | Y (right-hand sides);
-// work = Wb [TB N] | W2 [TB N] | T factors [ceil(N/TB) TB TB] | invd | four
+// zwk = Wb [TB N] | W2 [TB N] | T factors [ceil(N/TB) TB TB] | invd | four
 // diagonal scale vectors | perm | line exponents of the two operands of the
-// current product: 2 TB N + TB (N + TB) + 6.5 N <= N^2 for N >= 110
+// current product (stab_scratch_elems; the product temporary `work` where it has room)
 struct ZScr {
   double *X, *Y, *Wb, *W2, *Tb, *invd, *dlmaxi, *drmaxi, *dlmin, *drmin;
   int *perm, *expA, *expB;
@@ -73,7 +75,7 @@ __device__ __forceinline__ ZScr zscr(const WalkerDev& w, int sp) {
   ZScr z;
   z.X = w.scr + sp * 2 * NN;
   z.Y = z.X + NN;
-  double* wk = w.work + sp * NN;
+  double* wk = w.zwk + sp * w.zwk_stride;
   z.Wb = wk;
   z.W2 = wk + TN;
   z.Tb = wk + 2 * TN;
@@ -337,7 +339,7 @@ template <int S, int B>
 __global__ void __launch_bounds__(256) zslice_kernel(const WalkerDev* __restrict__ W, int op, int mode, int j, int p) {
   const int wi = blockIdx.z >> 1, sp = blockIdx.z & 1;
   const WalkerDev& w = W[wi];
-  if (!w.ozstab || sp >= w.S) return;
+  if (w.ozstab != 1 || sp >= w.S) return;
   ZJob jb;
   if (!zjob(w, op, mode, j, p, sp, jb)) return;
   if ((jb.K <= 256) != (B == 7)) return;
@@ -430,7 +432,7 @@ __global__ void __launch_bounds__(256, MINB) zgemm_tc_kernel(const WalkerDev* __
   static_assert(MINB == 1 || S * NT <= 256, "two CTAs per SM need at most 256 TMEM columns each");
   const int wi = blockIdx.z >> 1, sp = blockIdx.z & 1;
   const WalkerDev& w = W[wi];
-  if (!w.ozstab || sp >= w.S) return;
+  if (w.ozstab != 1 || sp >= w.S) return;
   ZJob jb;
   if (!zjob(w, op, mode, j, p, sp, jb)) return;
   if ((jb.K <= 256) != (B == 7)) return;
@@ -550,6 +552,75 @@ __global__ void __launch_bounds__(256, MINB) zgemm_tc_kernel(const WalkerDev* __
   tc::fence_before();
   __syncthreads();
   if (warp == 0) tc::dealloc(taddr, TCOLS);
+}
+
+// --------------------------------------------------------------------------
+// The same product in FP64 (ozstab 2): a 16 x 16 output tile per CTA, an element per thread, K in
+// steps of 32 through shared memory, operands read through zel.  FP64 issue bounds it (one warp
+// operation per 19 cycles and SM), so the tile is small: a product of 32 rows and K = 256 still
+// reaches 32 SMs per matrix.
+// --------------------------------------------------------------------------
+__global__ void __launch_bounds__(256) zgemm_f64_kernel(const WalkerDev* __restrict__ W, int op, int mode, int j, int p,
+                                                        int trace_slot) {
+  const int wi = blockIdx.z >> 1, sp = blockIdx.z & 1;
+  const WalkerDev& w = W[wi];
+  if (w.ozstab != 2 || sp >= w.S) return;
+  ZJob jb;
+  if (!zjob(w, op, mode, j, p, sp, jb)) return;
+  const int r0 = blockIdx.y * 16, c0 = blockIdx.x * 16;
+  if (r0 >= jb.M || c0 >= jb.N) return;
+  __shared__ double As[32][17], Bs[32][17];
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int rl = tid & 15, cl = tid >> 4, r = r0 + rl, col = c0 + cl;
+  const bool a_fast = jb.a.tr == 0, b_fast = jb.b.tr == 1;  // lines contiguous in memory
+  double acc4[4] = {0.0, 0.0, 0.0, 0.0};  // k mod 4: independent FMA chains, and shorter sums
+  // the upper (kind 2, not transposed) operand A is zero left of the diagonal
+  const int k_first = (jb.a.kind == 2 && !jb.a.tr) ? r0 / 32 * 32 : 0;
+  for (int k0 = k_first; k0 < jb.K; k0 += 32) {
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int e = tid + 256 * u;
+      const int la = a_fast ? e & 15 : e >> 5, ka = a_fast ? e >> 4 : e & 31;
+      As[ka][la] = (r0 + la < jb.M && k0 + ka < jb.K) ? zel(jb.a, r0 + la, k0 + ka, false) : 0.0;
+      const int lb = b_fast ? e & 15 : e >> 5, kb = b_fast ? e >> 4 : e & 31;
+      Bs[kb][lb] = (c0 + lb < jb.N && k0 + kb < jb.K) ? zel(jb.b, c0 + lb, k0 + kb, true) : 0.0;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 32; ++k) acc4[k & 3] = fma(As[k][rl], Bs[k][cl], acc4[k & 3]);
+    __syncthreads();
+  }
+  const double acc = (acc4[0] + acc4[1]) + (acc4[2] + acc4[3]);
+  const long long NN = (long long)w.N * w.N;
+  const bool check = (jb.out == 2) || (jb.out && !(mode == MODE_INIT || (mode == MODE_BWD && j == w.nstack - 1)));
+  double err = 0.0;
+  if (r < jb.M && col < jb.N) {
+    double val = acc;
+    if (jb.rs) val *= jb.rs[r];
+    if (jb.cs) val *= jb.cs[col];
+    if (jb.neg) val = -val;
+    const long long o = (long long)col * jb.ldc + r;
+    if (!jb.out) {
+      jb.c[o] = jb.beta ? jb.c[o] + val : val;
+    } else {
+      if (check) err = fabs(val - jb.c[o]);
+      if (!isfinite(val)) atomicOr(w.status, ST_NONFINITE_G);
+      jb.c[o] = val;
+      if (jb.out == 1) {
+        double* tr = (w.trace && trace_slot >= 0 && trace_slot < w.trace_cap)
+                         ? w.trace + ((long long)trace_slot * 2 + sp) * NN : nullptr;
+        if (tr) tr[o] = val;
+        if (w.S == 1) {
+          jb.c[NN + o] = val;
+          if (tr) tr[NN + o] = val;
+        }
+      }
+    }
+  }
+  if (check) {
+    for (int o = 16; o > 0; o >>= 1) err = fmax(err, __shfl_xor_sync(0xffffffffu, err, o));
+    if (lane == 0) atomicMax(w.wrap_bits, (unsigned long long)__double_as_longlong(err));
+  }
 }
 
 // --------------------------------------------------------------------------
@@ -1030,8 +1101,20 @@ cudaError_t configure_stab_oz_kernels(int maxN) {
   return cudaSuccess;
 }
 
-static void zgemm(const WalkerDev* W, int nw, int maxN, int op, int mode, int j, int p, int rows_max, int cols_max,
+// doubles of scratch a spin's stabilization takes in zwk
+size_t stab_scratch_elems(int N) {
+  return 2ull * TB * N + (size_t)TB * TB * ((N + TB - 1) / TB) + 5ull * N + (3ull * N + 1) / 2;
+}
+
+// rows / cols: 0 the whole matrix (maxN), TB a panel's width
+static void zgemm(const WalkerDev* W, int nw, StabSizes zs, int op, int mode, int j, int p, int rows, int cols,
                   int trace_slot, cudaStream_t st) {
+  if (zs.f64) {
+    const int rm = rows ? rows : zs.f64, cm = cols ? cols : zs.f64;
+    zgemm_f64_kernel<<<dim3((cm + 15) / 16, (rm + 15) / 16, 2 * nw), 256, 0, st>>>(W, op, mode, j, p, trace_slot);
+  }
+  if (!zs.tc) return;
+  const int maxN = zs.tc, rows_max = rows ? rows : maxN, cols_max = cols ? cols : maxN;
   const dim3 gs((std::max(rows_max, cols_max) + 31) / 32, 2, 2 * nw);
   zslice_kernel<8, 7><<<gs, 256, 0, st>>>(W, op, mode, j, p);
   if (maxN > 256) zslice_kernel<9, 6><<<gs, 256, 0, st>>>(W, op, mode, j, p);
@@ -1042,62 +1125,62 @@ static void zgemm(const WalkerDev* W, int nw, int maxN, int op, int mode, int j,
 
 // Householder panel p: the FP64 column factorization, then its Gram matrix, T factor and
 // Vt = V T (the block reflector in the form the trailing products apply)
-static void zpanel(const WalkerDev* W, int nw, int maxN, int mode, int j, int p, int push, cudaStream_t st) {
-  zqr_panel_kernel<<<2 * nw, 256, zpanel_smem(maxN), st>>>(W, mode, j, p, push);
-  zgemm(W, nw, maxN, Z_GRAM, mode, j, p, TB, TB, -1, st);
+static void zpanel(const WalkerDev* W, int nw, StabSizes zs, int mode, int j, int p, int push, cudaStream_t st) {
+  zqr_panel_kernel<<<2 * nw, 256, zpanel_smem(zs.max()), st>>>(W, mode, j, p, push);
+  zgemm(W, nw, zs, Z_GRAM, mode, j, p, TB, TB, -1, st);
   ztfac_kernel<<<2 * nw, 256, 0, st>>>(W, mode, j, p);
-  zgemm(W, nw, maxN, Z_VT, mode, j, p, maxN, TB, -1, st);
+  zgemm(W, nw, zs, Z_VT, mode, j, p, 0, TB, -1, st);
 }
 
-void oz_push(int mode, const WalkerDev* W, int nw, int j, int maxN, cudaStream_t st) {
-  const int np = (maxN + TB - 1) / TB;
+void oz_push(int mode, const WalkerDev* W, int nw, int j, StabSizes zs, cudaStream_t st) {
+  const int maxN = zs.max(), np = (maxN + TB - 1) / TB;
   zpush_prep_kernel<<<2 * nw, 256, sizeof(long long) * maxN, st>>>(W, mode, j);
   for (int p = 0; p < np; ++p) {
-    zpanel(W, nw, maxN, mode, j, p, 1, st);
-    zgemm(W, nw, maxN, Z_QR_W, mode, j, p, TB, maxN, -1, st);
-    zgemm(W, nw, maxN, Z_QR_UPD, mode, j, p, maxN, maxN, -1, st);
+    zpanel(W, nw, zs, mode, j, p, 1, st);
+    zgemm(W, nw, zs, Z_QR_W, mode, j, p, TB, 0, -1, st);
+    zgemm(W, nw, zs, Z_QR_UPD, mode, j, p, 0, 0, -1, st);
   }
   zpush_fin_kernel<<<dim3(64, 2 * nw), 256, 0, st>>>(W, mode, j);
-  zgemm(W, nw, maxN, Z_F, mode, j, 0, maxN, maxN, -1, st);
+  zgemm(W, nw, zs, Z_F, mode, j, 0, 0, 0, -1, st);
   for (int p = np - 1; p >= 0; --p) {
     zvt_kernel<<<dim3((maxN + 31) / 32, 2 * nw), 256, 0, st>>>(W, mode, j, p);
-    zgemm(W, nw, maxN, Z_Q_W, mode, j, p, TB, maxN, -1, st);
-    zgemm(W, nw, maxN, Z_Q_UPD, mode, j, p, maxN, maxN, -1, st);
+    zgemm(W, nw, zs, Z_Q_W, mode, j, p, TB, 0, -1, st);
+    zgemm(W, nw, zs, Z_Q_UPD, mode, j, p, 0, 0, -1, st);
   }
 }
 
 // The Green's assembly; with dyn (forward steps of the dynamic half-sweep) the same
 // factorization of M also solves the second right-hand side and G(t,0), G(0,t) follow.
-void oz_greens(int mode, const WalkerDev* W, int nw, int j, int trace_slot, int maxN, cudaStream_t st, bool dyn) {
-  const int np = (maxN + TB - 1) / TB;
+void oz_greens(int mode, const WalkerDev* W, int nw, int j, int trace_slot, StabSizes zs, cudaStream_t st, bool dyn) {
+  const int maxN = zs.max(), np = (maxN + TB - 1) / TB;
   zgreens_prep_kernel<<<dim3(64, 2 * nw), 256, 0, st>>>(W, mode, j);
   if (dyn) zdyn_prep_kernel<<<dim3(64, 2 * nw), 256, 0, st>>>(W, j);
-  zgemm(W, nw, maxN, Z_GA, mode, j, 0, maxN, maxN, -1, st);
-  zgemm(W, nw, maxN, Z_GB, mode, j, 0, maxN, maxN, -1, st);
+  zgemm(W, nw, zs, Z_GA, mode, j, 0, 0, 0, -1, st);
+  zgemm(W, nw, zs, Z_GB, mode, j, 0, 0, 0, -1, st);
   for (int p = 0; p < np; ++p) {
-    zpanel(W, nw, maxN, mode, j, p, 0, st);
-    zgemm(W, nw, maxN, Z_QR_W, mode, j, p, TB, maxN, -1, st);
-    zgemm(W, nw, maxN, Z_QR_UPD, mode, j, p, maxN, maxN, -1, st);
-    zgemm(W, nw, maxN, Z_AQ_W, mode, j, p, TB, maxN, -1, st);
-    zgemm(W, nw, maxN, Z_AQ_UPD, mode, j, p, maxN, maxN, -1, st);
+    zpanel(W, nw, zs, mode, j, p, 0, st);
+    zgemm(W, nw, zs, Z_QR_W, mode, j, p, TB, 0, -1, st);
+    zgemm(W, nw, zs, Z_QR_UPD, mode, j, p, 0, 0, -1, st);
+    zgemm(W, nw, zs, Z_AQ_W, mode, j, p, TB, 0, -1, st);
+    zgemm(W, nw, zs, Z_AQ_UPD, mode, j, p, 0, 0, -1, st);
     if (dyn) {
-      zgemm(W, nw, maxN, Z_AQ2_W, mode, j, p, TB, maxN, -1, st);
-      zgemm(W, nw, maxN, Z_AQ2_UPD, mode, j, p, maxN, maxN, -1, st);
+      zgemm(W, nw, zs, Z_AQ2_W, mode, j, p, TB, 0, -1, st);
+      zgemm(W, nw, zs, Z_AQ2_UPD, mode, j, p, 0, 0, -1, st);
     }
   }
   for (int p = np - 1; p >= 0; --p) {
-    zgemm(W, nw, maxN, Z_TR_UPD, mode, j, p, TB, maxN, -1, st);
+    zgemm(W, nw, zs, Z_TR_UPD, mode, j, p, TB, 0, -1, st);
     ztrsm_diag_kernel<<<dim3((maxN + 127) / 128, 2 * nw), 128, 0, st>>>(W, mode, j, p, 0);
     if (dyn) {
-      zgemm(W, nw, maxN, Z_TR2_UPD, mode, j, p, TB, maxN, -1, st);
+      zgemm(W, nw, zs, Z_TR2_UPD, mode, j, p, TB, 0, -1, st);
       ztrsm_diag_kernel<<<dim3((maxN + 127) / 128, 2 * nw), 128, 0, st>>>(W, mode, j, p, 1);
     }
   }
-  zgemm(W, nw, maxN, Z_GG, mode, j, 0, maxN, maxN, trace_slot, st);
+  zgemm(W, nw, zs, Z_GG, mode, j, 0, 0, 0, trace_slot, st);
   zgreens_out_kernel<<<dim3(64, 2 * nw), 256, 0, st>>>(W, mode, j, trace_slot);
   if (dyn) {
-    zgemm(W, nw, maxN, Z_DT0_OUT, mode, j, 0, maxN, maxN, -1, st);
-    zgemm(W, nw, maxN, Z_D0T_OUT, mode, j, 0, maxN, maxN, -1, st);
+    zgemm(W, nw, zs, Z_DT0_OUT, mode, j, 0, 0, 0, -1, st);
+    zgemm(W, nw, zs, Z_D0T_OUT, mode, j, 0, 0, 0, -1, st);
     zdyn_boundary_kernel<<<dim3(64, 2 * nw), 256, 0, st>>>(W, j);
   }
 }

@@ -158,8 +158,8 @@ int dqmc_sweep_beta_to_0(dqmc_batch* b, int measure);
  * included (they run this half-sweep on the HBM path's kernels).  On the
  * DQMC_MIXED path the G(t,0), G(0,t) steps run on the tensor cores and walkers
  * with 128 <= N <= 768 stabilize with the blocked Householder QR (one
- * factorization of M for both right-hand sides); the others with the FP64
- * kernels.  A new tau list (at most 256 entries) restarts the accumulators. */
+ * factorization of M for both right-hand sides) on tensor-core products; other
+ * HBM walkers in FP64.  A new tau list (at most 256 entries) restarts the accumulators. */
 int dqmc_sweep_dynamic(dqmc_batch* b, const int* taus, int ntau);
 /* Sums of sign * G(k,tau) and their counts, in the order of the last tau list. */
 int dqmc_get_dynamic(dqmc_batch* b, int walker, double* sums, int64_t* counts);
