@@ -903,53 +903,82 @@ __global__ void __launch_bounds__(256) greens_out_general_kernel(const WalkerDev
   }
 }
 
-// sign(det G_up det G_dn) for general walkers: LU of a copy in scr (col-major)
-__global__ void __launch_bounds__(1024) sign_general_kernel(const WalkerDev* __restrict__ W) {
-  const WalkerDev& w = W[blockIdx.x];
+// sign(det G_up det G_dn) for general walkers: LU with partial pivoting of a copy in scr (col-major),
+// a CTA per spin in a cluster of two.  Per column one barrier: warp 0 updates the next column in
+// shared memory and finds its pivot and multipliers while the other warps update the rest, lanes
+// along the rows; the row exchange happens in the update.  The order of the FMAs on an element is
+// that of the plain right-looking LU.  48 walkers of 12 x 12: 6.1 ms with both spins in one CTA, a
+// serial pivot search and a thread per column; a warm start of them went from 23.9 to 18.1 ms.
+__global__ void __launch_bounds__(512) __cluster_dims__(2, 1, 1) sign_general_kernel(const WalkerDev* __restrict__ W) {
+  namespace cg = cooperative_groups;
+  const WalkerDev& w = W[blockIdx.y];
+  const int sp = blockIdx.x;  // the cluster's rank
   if (!is_general(w)) return;
-  const int N = w.N;
-  const long long NN = (long long)N * N;
-  __shared__ int s_p, s_neg;
-  extern __shared__ double sh[];
-  double* l = sh;
-  if (threadIdx.x == 0) s_neg = 0;
-  for (int sp = 0; sp < 2; ++sp) {
-    double* M = w.scr;  // spin 0 scratch reused sequentially
-    const double* Gg = w.G + sp * NN;
-    for (long long e = threadIdx.x; e < NN; e += blockDim.x) M[e] = Gg[e];
-    __syncthreads();
-    for (int k = 0; k < N; ++k) {
-      if (threadIdx.x == 0) {
-        int p = k;
-        double m = fabs(M[(long long)k * N + k]);
-        for (int r = k + 1; r < N; ++r) {
-          const double a = fabs(M[(long long)k * N + r]);
-          if (a > m) { m = a; p = r; }
-        }
-        s_p = p;
-        if (p != k) ++s_neg;
-        if (M[(long long)k * N + p] < 0) ++s_neg;
-      }
-      __syncthreads();
-      const int p = s_p;
-      if (p != k)
-        for (int c = threadIdx.x; c < N; c += blockDim.x) {
-          double* mc = M + (long long)c * N;
-          const double a = mc[k]; mc[k] = mc[p]; mc[p] = a;
-        }
-      __syncthreads();
-      const double inv = 1.0 / M[(long long)k * N + k];
-      for (int r = k + 1 + threadIdx.x; r < N; r += blockDim.x) l[r] = M[(long long)k * N + r] * inv;
-      __syncthreads();
-      for (int c = k + 1 + threadIdx.x; c < N; c += blockDim.x) {
-        double* mc = M + (long long)c * N;
-        const double mk = mc[k];
-        for (int r = k + 1; r < N; ++r) mc[r] = fma(-l[r], mk, mc[r]);
-      }
-      __syncthreads();
-    }
+  if (w.S == 1) {  // equal spins: the determinants' signs multiply to +1
+    if (sp == 0 && threadIdx.x == 0) *w.sign = 1.0;
+    return;
   }
-  if (threadIdx.x == 0) *w.sign = (s_neg % 2 == 0) ? 1.0 : -1.0;
+  const int N = w.N, lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
+  const long long NN = (long long)N * N;
+  extern __shared__ double sh[];
+  double* l = sh;             // [2][N] multipliers of columns k, k + 1
+  double* col = sh + 2 * N;   // [N] the pivot column
+  __shared__ int s_p[2], s_neg;
+  double* M = w.scr + sp * 2 * NN;
+  const double* Gg = w.G + sp * NN;
+  for (long long e = threadIdx.x; e < NN; e += blockDim.x) M[e] = Gg[e];
+  int neg = 0;
+  // warp 0: pivot of column k (the first largest |a| of rows k.., kept in col) and its multipliers
+  auto factor = [&](int k, int buf) {
+    long long key = -1;
+    int p = k;
+    for (int r = k + lane; r < N; r += 32) {
+      long long a = __double_as_longlong(col[r]) & 0x7fffffffffffffffLL;
+      if (a > 0x7ff0000000000000LL) a = (r == k) ? a : -1;  // a NaN is the largest only on the diagonal
+      if (a > key) { key = a; p = r; }
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+      const long long ok = __shfl_xor_sync(0xffffffffu, key, o);
+      const int op = __shfl_xor_sync(0xffffffffu, p, o);
+      if (ok > key || (ok == key && op < p)) { key = ok; p = op; }
+    }
+    const double piv = col[p], below = col[k], inv = 1.0 / piv;
+    neg += (p != k ? 1 : 0) + (piv < 0 ? 1 : 0);
+    for (int r = k + 1 + lane; r < N; r += 32) l[buf * N + r] = ((r == p) ? below : col[r]) * inv;
+    if (lane == 0) s_p[buf] = p;
+    __syncwarp();
+  };
+  __syncthreads();
+  if (wid == 0) {
+    for (int r = lane; r < N; r += 32) col[r] = M[r];
+    __syncwarp();
+    factor(0, 0);
+  }
+  __syncthreads();
+  for (int k = 0; k + 1 < N; ++k) {
+    const int buf = k & 1, p = s_p[buf];
+    const double* lk = l + buf * N;
+    if (wid == 0) {  // column k + 1 first: the next pivot is found while the others update
+      const double* mc = M + (long long)(k + 1) * N;
+      const double mk = mc[p], old = mc[k];
+      for (int r = k + 1 + lane; r < N; r += 32) col[r] = fma(-lk[r], mk, (r == p) ? old : mc[r]);
+      __syncwarp();
+      factor(k + 1, buf ^ 1);
+    } else {
+      for (int c = k + 1 + wid; c < N; c += nwarp - 1) {
+        double* mc = M + (long long)c * N;
+        const double mk = mc[p], old = mc[k];
+        __syncwarp();  // row p is read before its lane writes it
+        for (int r = k + 1 + lane; r < N; r += 32) mc[r] = fma(-lk[r], mk, (r == p) ? old : mc[r]);
+      }
+    }
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) s_neg = neg;
+  cg::cluster_group cl = cg::this_cluster();
+  cl.sync();
+  if (sp == 0 && threadIdx.x == 0) *w.sign = ((s_neg + *cl.map_shared_rank(&s_neg, 1)) % 2 == 0) ? 1.0 : -1.0;
+  cl.sync();
 }
 
 // --------------------------------------------------------------------------
@@ -1343,7 +1372,7 @@ void general_measure_after(int mode, const WalkerDev* W, int nw, int j, int maxN
 }
 
 void general_sign(const WalkerDev* W, int nw, int maxN, cudaStream_t st) {
-  sign_general_kernel<<<nw, 1024, sizeof(double) * maxN, st>>>(W);
+  sign_general_kernel<<<dim3(2, nw), 512, 3 * sizeof(double) * maxN, st>>>(W);
 }
 
 }  // namespace dqmc
