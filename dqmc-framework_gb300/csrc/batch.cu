@@ -84,7 +84,7 @@ void mixed_wrap_fwd(const WalkerDev* W, int nw, int maxN, int j, int q, cudaStre
 void mixed_wrap_bwd(const WalkerDev* W, int nw, int maxN, int j, int q, cudaStream_t st);
 void mixed_chain(const WalkerDev* W, int nw, int maxN, int mode, int j, int q, cudaStream_t st);
 void oz_slice_const(const double* X, unsigned short* out, int* exps, int N, int ldk, int role, int bits, int slices,
-                    int layout, cudaStream_t st);
+                    cudaStream_t st);
 void oz_set_shape(int shape);
 void oz_selftest(const double* A, const double* B, double* C, unsigned short* sa, int* ea, unsigned short* sb, int* eb,
                  int N, cudaStream_t st);
@@ -591,10 +591,10 @@ int dqmc_batch_create(const dqmc_walker_desc* descs, int n, const dqmc_batch_opt
       auto* se = reinterpret_cast<int*>(base + dense_sle[i]);
       const double* ek = reinterpret_cast<const double*>(base + dense_off[i]);
       const double* ik = ek + nn;
-      oz_slice_const(ek, sl + 0 * one, se + 0 * N, N, ldk, 0, cfg.first, cfg.second, 1, b->stream);  // expK as A
-      oz_slice_const(ek, sl + 1 * one, se + 1 * N, N, ldk, 1, cfg.first, cfg.second, 1, b->stream);  // expK as B
-      oz_slice_const(ik, sl + 2 * one, se + 2 * N, N, ldk, 0, cfg.first, cfg.second, 1, b->stream);  // invK as A
-      oz_slice_const(ik, sl + 3 * one, se + 3 * N, N, ldk, 1, cfg.first, cfg.second, 1, b->stream);  // invK as B
+      oz_slice_const(ek, sl + 0 * one, se + 0 * N, N, ldk, 0, cfg.first, cfg.second, b->stream);  // expK as A
+      oz_slice_const(ek, sl + 1 * one, se + 1 * N, N, ldk, 1, cfg.first, cfg.second, b->stream);  // expK as B
+      oz_slice_const(ik, sl + 2 * one, se + 2 * N, N, ldk, 0, cfg.first, cfg.second, b->stream);  // invK as A
+      oz_slice_const(ik, sl + 3 * one, se + 3 * N, N, ldk, 1, cfg.first, cfg.second, b->stream);  // invK as B
     }
   }
   std::vector<std::vector<double>> fftabs;
@@ -1607,7 +1607,7 @@ int dqmc_product_check(int n, const double* a, const double* b, double* c) {
   // every piece 256-byte aligned (the product kernel copies slices in 16-byte chunks)
   const size_t o_b = align256(nn * sizeof(double)), o_c = o_b + align256(nn * sizeof(double));
   const size_t o_sa = o_c + align256(nn * sizeof(double));
-  const size_t sl_bytes = align256(ozaki::kMaxSlices * (size_t)n * ldk * sizeof(unsigned short));
+  const size_t sl_bytes = align256(ozaki::kMaxSlices * ozaki::tc_slice_elems(n, (int)ldk) * sizeof(unsigned short));
   const size_t o_sb = o_sa + sl_bytes, o_ea = o_sb + sl_bytes, o_eb = o_ea + align256(n * sizeof(int));
   const size_t bytes = o_eb + align256(n * sizeof(int));
   char* buf = nullptr;

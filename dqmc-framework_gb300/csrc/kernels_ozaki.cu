@@ -2,9 +2,8 @@
 // (49-bit) matrix products on the BF16 tensor cores (see ozaki.cuh).
 //
 // Slicing is integer work on the FP64 bit patterns; the product runs the
-// S(S+1)/2 slice pairs on the BF16 tensor cores (tcgen05, TMEM accumulators;
-// the stand-alone product of the test hook uses mma.sync) with FP32
-// accumulation, exact by construction, one accumulator per weight group, and
+// S(S+1)/2 slice pairs on the BF16 tensor cores (tcgen05, TMEM accumulators)
+// with FP32 accumulation, exact by construction, one accumulator per weight group, and
 // recombines the groups in the epilogue.  Used for the wraps and the B-chain (the reference's
 // mult_B_from_left/right, mult_invB_*, mult_transB_from_left,
 // src/model/repulsive_hubbard.cpp:158-243, src/model/model_base.cpp:7-35).
@@ -27,8 +26,7 @@ using ozaki::kMaxSlices;
 // Slicing.  role 0 (left operand, A): lines are rows r, k runs over columns.
 // role 1 (right operand, B): lines are columns c, k runs over rows.  X is
 // column-major N x N (ld N).  pre (may be null) scales element k of every line
-// before slicing.  layout 0 writes out[s][line][k] (row-major, ld ldk); layout
-// 1 writes the tensor-core image (ozaki::tc_index, slice stride
+// before slicing.  out: the tensor-core image (ozaki::tc_index, slice stride
 // ozaki::tc_slice_elems).  One CTA of 256 threads per 32 lines.
 // --------------------------------------------------------------------------
 struct SliceJob {
@@ -42,8 +40,7 @@ __device__ __forceinline__ double xelem(const double* X, int N, int role, int li
   return role == 0 ? X[(long long)k * N + line] : X[(long long)line * N + k];
 }
 
-__device__ void slice_lines(const SliceJob& job, int N, int ldk, int role, int bits, int slices, int line0,
-                            int layout) {
+__device__ void slice_lines(const SliceJob& job, int N, int ldk, int role, int bits, int slices, int line0) {
   __shared__ int s_e[8][32];
   __shared__ double s_t[32][33];
   const int tid = threadIdx.x;
@@ -84,18 +81,7 @@ __device__ void slice_lines(const SliceJob& job, int N, int ldk, int role, int b
     }
     __syncthreads();
     const int Q = bits * slices;
-    if (layout == 0) {
-      for (int e2 = tid; e2 < 32 * 32; e2 += blockDim.x) {
-        const int kk = e2 & 31, ll = e2 >> 5;
-        const int line = line0 + ll, k = k0 + kk;
-        if (line < N && k < ldk) {
-          bool neg;
-          const unsigned long long q = ozaki::fixedq(s_t[ll][kk], s_e[0][ll], Q, neg);
-          for (int s = 0; s < slices; ++s)
-            job.out[((long long)s * N + line) * ldk + k] = ozaki::slice_bf16q(q, s, bits, Q, neg);
-        }
-      }
-    } else {
+    {
       // one line and 4 consecutive k per thread: one 8-byte store per slice
       const int kq = tid & 7, ll = tid >> 3;
       const int line = line0 + ll, k = k0 + kq * 4;
@@ -120,129 +106,12 @@ __device__ void slice_lines(const SliceJob& job, int N, int ldk, int role, int b
   }
 }
 
-// --------------------------------------------------------------------------
-// Product kernel: C(r,c) = sum_k A(r,k) B(k,c) from slices, 64x64 tile per
-// CTA, 8 warps (2 x 4), warp tile 32 x 16, K staged 16 at a time (cp.async,
-// double buffered).  The epilogue functor receives (r, c, value).
-// --------------------------------------------------------------------------
 struct ProdJob {
-  const unsigned short* A;  // S slices: [S][N][ldk] (test hook) or tensor-core images (sweep)
+  const unsigned short* A;  // S slices, tensor-core images
   const unsigned short* B;
   const int* ea;
   const int* eb;
 };
-
-constexpr int kOzRow = 24;  // padded SMEM row (bf16): 48 bytes, conflict-free fragment loads
-
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem, bool valid) {
-  const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-  const int n = valid ? 16 : 0;
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(sa), "l"(gmem), "r"(n));
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::); }
-
-__device__ __forceinline__ void mma_bf16(float (&c)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3,
-                                         unsigned b0, unsigned b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-      "{%0,%1,%2,%3};\n"
-      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-
-template <int S, class Epi>
-__device__ void ozaki_product_tile(const ProdJob& job, int N, int ldk, int bits, int r0, int c0, unsigned short* sm,
-                                   Epi epi) {
-  // sm: [2 stages][2 operands][S][64][kOzRow]
-  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  const int wm = wid >> 2, wn = wid & 3;  // warp tile origin (wm*32, wn*16)
-  const int g = lane >> 2, t4 = lane & 3;
-  float acc[S][2][2][4];  // weight groups m = i + j <= S - 1
-#pragma unroll
-  for (int m = 0; m < S; ++m)
-#pragma unroll
-    for (int a = 0; a < 2; ++a)
-#pragma unroll
-      for (int b = 0; b < 2; ++b)
-#pragma unroll
-        for (int v = 0; v < 4; ++v) acc[m][a][b][v] = 0.f;
-
-  const int stage_elems = 2 * S * 64 * kOzRow;
-  auto load_stage = [&](int st, int k0) {
-    unsigned short* base = sm + st * stage_elems;
-    // 2 operands x S slices x 64 lines x 2 chunks of 16 bytes
-    for (int e = tid; e < 2 * S * 64 * 2; e += blockDim.x) {
-      const int ch = e & 1, line = (e >> 1) & 63, s = (e >> 7) % S, op = (e >> 7) / S;
-      const int gl = (op == 0 ? r0 : c0) + line;
-      const unsigned short* src = (op == 0 ? job.A : job.B) + ((long long)s * N + min(gl, N - 1)) * ldk + k0 + ch * 8;
-      unsigned short* dst = base + ((op * S + s) * 64 + line) * kOzRow + ch * 8;
-      cp_async16(dst, src, gl < N);
-    }
-    cp_async_commit();
-  };
-
-  const int nk = ldk / 16;
-  load_stage(0, 0);
-  for (int kb = 0; kb < nk; ++kb) {
-    cp_async_wait_all();
-    __syncthreads();
-    if (kb + 1 < nk) load_stage((kb + 1) & 1, (kb + 1) * 16);
-    const unsigned short* As = sm + (kb & 1) * stage_elems;
-    const unsigned short* Bs = As + S * 64 * kOzRow;
-#pragma unroll
-    for (int i = 0; i < S; ++i) {
-      unsigned a[2][4];
-#pragma unroll
-      for (int mt = 0; mt < 2; ++mt) {
-        const unsigned short* p = As + (i * 64 + wm * 32 + mt * 16 + g) * kOzRow + 2 * t4;
-        a[mt][0] = *(const unsigned*)(p);
-        a[mt][1] = *(const unsigned*)(p + 8 * kOzRow);
-        a[mt][2] = *(const unsigned*)(p + 8);
-        a[mt][3] = *(const unsigned*)(p + 8 * kOzRow + 8);
-      }
-#pragma unroll
-      for (int jj = 0; jj < S - i; ++jj) {
-        unsigned b[2][2];
-#pragma unroll
-        for (int nt = 0; nt < 2; ++nt) {
-          const unsigned short* p = Bs + (jj * 64 + wn * 16 + nt * 8 + g) * kOzRow + 2 * t4;
-          b[nt][0] = *(const unsigned*)(p);
-          b[nt][1] = *(const unsigned*)(p + 8);
-        }
-#pragma unroll
-        for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-          for (int nt = 0; nt < 2; ++nt)
-            mma_bf16(acc[i + jj][mt][nt], a[mt][0], a[mt][1], a[mt][2], a[mt][3], b[nt][0], b[nt][1]);
-      }
-    }
-    __syncthreads();
-  }
-  // epilogue: C = 2^{ea_r + eb_c} sum_m 2^{-bits (m+2)} S_m
-#pragma unroll
-  for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-    for (int nt = 0; nt < 2; ++nt)
-#pragma unroll
-      for (int v = 0; v < 4; ++v) {
-        const int r = r0 + wm * 32 + mt * 16 + g + ((v >> 1) << 3);
-        const int c = c0 + wn * 16 + nt * 8 + 2 * t4 + (v & 1);
-        if (r >= N || c >= N) continue;
-        // integer Horner in two halves (groups 0-3 and 4..S-1), each exact in 64 bits
-        long long hi = 0, lo = 0;
-#pragma unroll
-        for (int m = 0; m < 4; ++m) hi = (hi << bits) + (long long)__float2int_rn(acc[m][mt][nt][v]);
-#pragma unroll
-        for (int m = 4; m < S; ++m) lo = (lo << bits) + (long long)__float2int_rn(acc[m][mt][nt][v]);
-        const int e = job.ea[r] + job.eb[c];
-        epi(r, c, ozaki::ldexp_i64(hi, e - 5 * bits) + ozaki::ldexp_i64(lo, e - bits * (S + 1)));
-      }
-}
-
-}  // namespace dqmc
-
-namespace dqmc {
 
 namespace {
 __device__ __forceinline__ bool oz_slice_of(const WalkerDev& w, int mode, int j, int q, int& t) {
@@ -311,7 +180,7 @@ __global__ void __launch_bounds__(256) oz_slice_kernel(const WalkerDev* __restri
   __syncthreads();
   SliceJob job{X, w.sl + (long long)sp * w.slices * ozaki::tc_slice_elems(N, w.ldk), w.sle + (long long)sp * N,
                sgn ? s_pre : nullptr};
-  slice_lines(job, N, w.ldk, role, w.slice_bits, w.slices, blockIdx.x * 32, 1);
+  slice_lines(job, N, w.ldk, role, w.slice_bits, w.slices, blockIdx.x * 32);
 }
 
 // Product of op OP on the 5th-generation tensor cores: a 128 x NT output
@@ -333,51 +202,22 @@ __host__ __device__ constexpr int oz_tc_stage_bytes(int S, int SH) {
   return oztc::stage_bytes(S, 128, oz_tc_nt(S, SH));
 }
 
-template <int OP, int S, int SH>
-__global__ void __launch_bounds__(256, oz_tc_minb(S, SH)) oz_prod_tc_kernel(const WalkerDev* __restrict__ W, int mode,
-                                                                            int j, int q) {
-  constexpr int MT = 128, NT = oz_tc_nt(S, SH), NS = oz_tc_stages(S, SH);
-  constexpr int CW = (oz_tc_minb(S, SH) > 1) ? 8 : 16;  // TMEM columns per load in the epilogue
+// One 128 x NT tile (rows r0.., columns c0..) of a product of N x N operands: epi(rl, r, cl, col,
+// value) per element inside the matrix.  Returns whether a wait ran out (epi was then not called);
+// all 256 threads call.
+template <int S, int NT, int NS, int MINB, class Epi>
+__device__ __forceinline__ bool oz_tc_tile(const ProdJob& job, int N, int ldk, int r0, int c0, int wait_limit,
+                                           unsigned char* tsm, Epi epi) {
+  constexpr int MT = 128;
+  constexpr int CW = (MINB > 1) ? 8 : 16;  // TMEM columns per load in the epilogue
   constexpr unsigned TCOLS = (S * NT <= 256) ? 256u : 512u;
-  const int wi = blockIdx.z >> 1, sp = blockIdx.z & 1;
-  const WalkerDev& w = W[wi];
-  if (w.path != 2 || w.cb || sp >= w.S || w.slices != S) return;
-  int t;
-  if (!oz_slice_of(w, mode, j, q, t)) return;
-  const int N = w.N, ldk = w.ldk;
-  const int r0 = blockIdx.y * MT, c0 = blockIdx.x * NT;
-  if (r0 >= N || c0 >= N) return;
-  const long long NN = (long long)N * N;
-  const long long sstride = (long long)ozaki::tc_slice_elems(N, ldk);
-  const unsigned short* ws = w.sl + (long long)sp * w.slices * sstride;
-  const int* we = w.sle + (long long)sp * N;
-  ProdJob job{};
-  double* out = nullptr;
-  switch (OP) {
-    case OZ_WL_FWD: job = ProdJob{w.kA, ws, w.kAe, we}; out = w.work + sp * NN; break;
-    case OZ_WR_FWD: job = ProdJob{ws, w.iB, we, w.iBe}; out = w.G + sp * NN; break;
-    case OZ_CH_FWD: job = ProdJob{w.kA, ws, w.kAe, we}; out = oz_chain(w, sp, (q + 1) & 1); break;
-    case OZ_CH_BWD: job = ProdJob{w.kB, ws, w.kBe, we}; out = oz_chain(w, sp, (q + 1) & 1); break;
-    case OZ_WR_BWD: job = ProdJob{ws, w.kB, we, w.kBe}; out = w.work + sp * NN; break;
-    case OZ_WL_BWD: job = ProdJob{w.iA, ws, w.iAe, we}; out = w.G + sp * NN; break;
-    case OZ_DT0: job = ProdJob{w.kA, ws, w.kAe, we}; out = w.gt0 ? oz_dyn(w.gt0, w, sp, t) : nullptr; break;
-    case OZ_D0T: job = ProdJob{ws, w.iB, we, w.iBe}; out = w.g0t ? oz_dyn(w.g0t, w, sp, t) : nullptr; break;
-  }
-  if (!out) return;
-  extern __shared__ __align__(1024) unsigned char tsm[];
   __shared__ int eA[MT], eB[NT];
-  __shared__ double s_scale[MT];  // exp(+-alpha s) of the output rows (or columns)
   __shared__ __align__(8) unsigned long long full[NS], done[NS];
   __shared__ unsigned tbase;
   __shared__ int s_fail, s_last;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tid < MT) eA[tid] = (r0 + tid < N) ? job.ea[r0 + tid] : -1100;
   if (tid < NT) eB[tid] = (c0 + tid < N) ? job.eb[c0 + tid] : -1100;
-  if (OP == OZ_WL_FWD || OP == OZ_CH_FWD || OP == OZ_DT0) {
-    if (tid < MT) s_scale[tid] = (r0 + tid < N) ? oz_bscale(w, t, sp, +1, r0 + tid) : 0.0;
-  } else if (OP == OZ_WR_FWD || OP == OZ_D0T) {
-    if (tid < NT) s_scale[tid] = (c0 + tid < N) ? oz_bscale(w, t, sp, -1, c0 + tid) : 0.0;
-  }
   if (tid == 0) {
     s_fail = 0;
     s_last = -1;
@@ -394,11 +234,12 @@ __global__ void __launch_bounds__(256, oz_tc_minb(S, SH)) oz_prod_tc_kernel(cons
   const unsigned taddr = tbase;
   if (tid == 0) {
     // chunk c of the tile: (c * nlb + line0 / 8) 8-line blocks of 128 elements into each slice
+    const long long sstride = (long long)ozaki::tc_slice_elems(N, ldk);
     const long long cstep = (long long)(ozaki::tc_lines(N) / 8) * 128;
     bool ok;
     s_last = oztc::mainloop<S, MT, NT, NS>(tsm, full, done, taddr, job.A + (long long)(r0 / 8) * 128,
                                             job.B + (long long)(c0 / 8) * 128, sstride, cstep, ldk / 16, ok,
-                                            w.wait_limit);
+                                            wait_limit);
     s_fail = ok ? 0 : 1;
   }
   __syncthreads();
@@ -425,43 +266,150 @@ __global__ void __launch_bounds__(256, oz_tc_minb(S, SH)) oz_prod_tc_kernel(cons
           for (int m = 0; m < 4; ++m) hi = (hi << SB) + (long long)__float2int_rn(__uint_as_float(v[m][u]));
 #pragma unroll
           for (int m = 4; m < S; ++m) lo = (lo << SB) + (long long)__float2int_rn(__uint_as_float(v[m][u]));
-          const int e = eA[rl] + eB[cl];
-          double val = ozaki::combine_hilo<S, (S <= 7 ? 7 : 6)>(hi, lo, e);
-          if (OP == OZ_WL_FWD || OP == OZ_CH_FWD || OP == OZ_DT0) val *= s_scale[rl];
-          if (OP == OZ_WR_FWD || OP == OZ_D0T) val *= s_scale[cl];
-          out[(long long)col * N + r] = val;
+          epi(rl, r, cl, col, ozaki::combine_hilo<S, (S <= 7 ? 7 : 6)>(hi, lo, eA[rl] + eB[cl]));
         }
       }
     }
-  } else if (tid == 0) {
-    atomicOr(w.status, ST_TIMEOUT);
   }
   tc::fence_before();
   __syncthreads();
   if (warp == 0) tc::dealloc(taddr, TCOLS);
+  return failed != 0;
+}
+
+template <int OP, int S, int SH>
+__global__ void __launch_bounds__(256, oz_tc_minb(S, SH)) oz_prod_tc_kernel(const WalkerDev* __restrict__ W, int mode,
+                                                                            int j, int q) {
+  constexpr int MT = 128, NT = oz_tc_nt(S, SH), NS = oz_tc_stages(S, SH);
+  const int wi = blockIdx.z >> 1, sp = blockIdx.z & 1;
+  const WalkerDev& w = W[wi];
+  if (w.path != 2 || w.cb || sp >= w.S || w.slices != S) return;
+  int t;
+  if (!oz_slice_of(w, mode, j, q, t)) return;
+  const int N = w.N, ldk = w.ldk;
+  const int r0 = blockIdx.y * MT, c0 = blockIdx.x * NT;
+  if (r0 >= N || c0 >= N) return;
+  const long long NN = (long long)N * N;
+  const long long sstride = (long long)ozaki::tc_slice_elems(N, ldk);
+  const unsigned short* ws = w.sl + (long long)sp * w.slices * sstride;
+  const int* we = w.sle + (long long)sp * N;
+  ProdJob job{};
+  double* out = nullptr;
+  switch (OP) {
+    case OZ_WL_FWD: job = ProdJob{w.kA, ws, w.kAe, we}; out = w.work + sp * NN; break;
+    case OZ_WR_FWD: job = ProdJob{ws, w.iB, we, w.iBe}; out = w.G + sp * NN; break;
+    case OZ_CH_FWD: job = ProdJob{w.kA, ws, w.kAe, we}; out = oz_chain(w, sp, (q + 1) & 1); break;
+    case OZ_CH_BWD: job = ProdJob{w.kB, ws, w.kBe, we}; out = oz_chain(w, sp, (q + 1) & 1); break;
+    case OZ_WR_BWD: job = ProdJob{ws, w.kB, we, w.kBe}; out = w.work + sp * NN; break;
+    case OZ_WL_BWD: job = ProdJob{w.iA, ws, w.iAe, we}; out = w.G + sp * NN; break;
+    case OZ_DT0: job = ProdJob{w.kA, ws, w.kAe, we}; out = w.gt0 ? oz_dyn(w.gt0, w, sp, t) : nullptr; break;
+    case OZ_D0T: job = ProdJob{ws, w.iB, we, w.iBe}; out = w.g0t ? oz_dyn(w.g0t, w, sp, t) : nullptr; break;
+  }
+  if (!out) return;
+  extern __shared__ __align__(1024) unsigned char tsm[];
+  __shared__ double s_scale[MT];  // exp(+-alpha s) of the output rows (or columns); read after the tile's barriers
+  const int tid = threadIdx.x;
+  constexpr bool row_scale = OP == OZ_WL_FWD || OP == OZ_CH_FWD || OP == OZ_DT0;
+  constexpr bool col_scale = OP == OZ_WR_FWD || OP == OZ_D0T;
+  if (row_scale) {
+    if (tid < MT) s_scale[tid] = (r0 + tid < N) ? oz_bscale(w, t, sp, +1, r0 + tid) : 0.0;
+  } else if (col_scale) {
+    if (tid < NT) s_scale[tid] = (c0 + tid < N) ? oz_bscale(w, t, sp, -1, c0 + tid) : 0.0;
+  }
+  const bool failed = oz_tc_tile<S, NT, NS, oz_tc_minb(S, SH)>(
+      job, N, ldk, r0, c0, w.wait_limit, tsm, [&](int rl, int r, int cl, int col, double val) {
+        if (row_scale) val *= s_scale[rl];
+        if (col_scale) val *= s_scale[cl];
+        out[(long long)col * N + r] = val;
+      });
+  if (failed && tid == 0) atomicOr(w.status, ST_TIMEOUT);
 }
 
 // constant operands (exp(-dtau K), exp(+dtau K)), sliced once per batch
 __global__ void __launch_bounds__(256) oz_const_slice_kernel(const double* X, unsigned short* out, int* exps, int N,
-                                                             int ldk, int role, int bits, int slices, int layout) {
+                                                             int ldk, int role, int bits, int slices) {
   SliceJob job{X, out, exps, nullptr};
-  slice_lines(job, N, ldk, role, bits, slices, blockIdx.x * 32, layout);
+  slice_lines(job, N, ldk, role, bits, slices, blockIdx.x * 32);
 }
 
-// stand-alone product C = A B (test hook): A, B column-major N x N on the device
-__global__ void __launch_bounds__(256) oz_selftest_prod_kernel(const unsigned short* As, const int* ea,
-                                                               const unsigned short* Bs, const int* eb, double* C,
-                                                               int N, int ldk, int bits, int S) {
-  extern __shared__ unsigned short ozsm[];
-  ProdJob job{As, Bs, ea, eb};
-  const int r0 = blockIdx.y * 64, c0 = blockIdx.x * 64;
-  auto epi = [&](int r, int c, double v) { C[(long long)c * N + r] = v; };
-  if (S == 7) ozaki_product_tile<7>(job, N, ldk, bits, r0, c0, ozsm, epi);
-  else ozaki_product_tile<8>(job, N, ldk, bits, r0, c0, ozsm, epi);
+// ---- stand-alone product C = A B: A, B column-major N x N on the device -----------
+// One product is a matter of latency: both operands are sliced by one launch (8 lines a CTA, 8
+// consecutive k a thread, so that every element is read once from its own sector and each slice is
+// a 16-byte store), and the tiles run the sweep's tensor-core loop.  N = 256: 27 us a product, bound
+// by the two launches and the 16 chunks of a tile one after the other; 74 us as two slicing launches
+// of 32 lines a CTA and a 64 x 64-tile mma.sync product.
+__global__ void __launch_bounds__(256) oz_slice_pair_kernel(const double* A, const double* B, unsigned short* sa,
+                                                            int* ea, unsigned short* sb, int* eb, int N, int ldk,
+                                                            int bits, int slices) {
+  const bool isB = blockIdx.y == 1;
+  const double* X = isB ? B : A;
+  unsigned short* out = isB ? sb : sa;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  // A's lines are rows (8 consecutive elements of a column), B's are columns
+  const int ll = isB ? warp : lane & 7, kg = isB ? lane : warp * 4 + (lane >> 3), line = blockIdx.x * 8 + ll;
+  __shared__ int s_e[8];
+  if (tid < 8) s_e[tid] = -1100;
+  __syncthreads();
+  double x[8];
+  auto load = [&](int k0) {
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const int k = k0 + kg * 8 + u;
+      x[u] = (line < N && k < N) ? (isB ? X[(long long)line * N + k] : X[(long long)k * N + line]) : 0.0;
+    }
+  };
+  int e = -1100;
+  for (int k0 = 0; k0 < ldk; k0 += 256) {
+    load(k0);
+#pragma unroll
+    for (int u = 0; u < 8; ++u) e = max(e, ozaki::exp_bound(x[u]));
+  }
+  atomicMax(&s_e[ll], e);
+  __syncthreads();
+  e = s_e[ll];
+  if (tid < 8 && blockIdx.x * 8 + tid < N) (isB ? eb : ea)[blockIdx.x * 8 + tid] = s_e[tid];
+  if (line >= N) return;
+  const int Q = bits * slices;
+  const long long sstride = (long long)ozaki::tc_slice_elems(N, ldk);
+  for (int k0 = 0; k0 < ldk; k0 += 256) {
+    const int k = k0 + kg * 8;
+    if (k >= ldk) break;
+    if (ldk > 256) load(k0);
+    unsigned long long q[8];
+    bool ng[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) q[u] = ozaki::fixedq(x[u], e, Q, ng[u]);
+    unsigned short* o = out + ozaki::tc_index(line, k, ozaki::tc_lines(N) / 8);
+    for (int s2 = 0; s2 < slices; ++s2) {
+      unsigned v[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        v[u] = (unsigned)ozaki::slice_bf16q(q[2 * u], s2, bits, Q, ng[2 * u]) |
+               ((unsigned)ozaki::slice_bf16q(q[2 * u + 1], s2, bits, Q, ng[2 * u + 1]) << 16);
+      *reinterpret_cast<uint4*>(o + s2 * sstride) = make_uint4(v[0], v[1], v[2], v[3]);
+    }
+  }
+}
+
+// 128 x 32 tiles, the deepest ring that fits (one CTA per SM: a product has few tiles)
+__host__ __device__ constexpr int oz_one_stages(int S) { return S <= 7 ? 6 : 5; }
+template <int S>
+__global__ void __launch_bounds__(256, 1) oz_one_prod_kernel(ProdJob job, double* C, int N, int ldk) {
+  extern __shared__ __align__(1024) unsigned char tsm[];
+  // a wait that runs out leaves the tile unwritten: no status word here, the caller's C shows NaN
+  const int r0 = blockIdx.y * 128, c0 = blockIdx.x * 32;
+  const bool failed = oz_tc_tile<S, 32, oz_one_stages(S), 1>(
+      job, N, ldk, r0, c0, kDefaultWaitLimit, tsm,
+      [&](int, int r, int, int col, double val) { C[(long long)col * N + r] = val; });
+  if (failed)
+    for (int e = threadIdx.x; e < 128 * 32; e += 256) {
+      const int r = r0 + (e & 127), col = c0 + (e >> 7);
+      if (r < N && col < N) C[(long long)col * N + r] = __longlong_as_double(0x7ff8000000000000LL);
+    }
 }
 
 static size_t oz_tc_smem(int S, int SH) { return (size_t)oz_tc_stages(S, SH) * oz_tc_stage_bytes(S, SH); }
-size_t oz_prod_smem(int S) { return sizeof(unsigned short) * 2 * 2 * S * 64 * kOzRow; }
+static size_t oz_one_smem(int S) { return (size_t)oz_one_stages(S) * oztc::stage_bytes(S, 128, 32); }
 
 cudaError_t configure_ozaki_kernels() {
   cudaError_t e;
@@ -478,8 +426,10 @@ cudaError_t configure_ozaki_kernels() {
   OZCFG(OZ_WL_FWD); OZCFG(OZ_WR_FWD); OZCFG(OZ_CH_FWD); OZCFG(OZ_CH_BWD);
   OZCFG(OZ_WR_BWD); OZCFG(OZ_WL_BWD); OZCFG(OZ_DT0); OZCFG(OZ_D0T);
 #undef OZCFG
-  if ((e = cudaFuncSetAttribute(oz_selftest_prod_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)oz_prod_smem(8))))
+  if ((e = cudaFuncSetAttribute(oz_one_prod_kernel<7>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)oz_one_smem(7))) ||
+      (e = cudaFuncSetAttribute(oz_one_prod_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)oz_one_smem(8))))
     return e;
   return cudaSuccess;
 }
@@ -525,19 +475,19 @@ void mixed_wrap_bwd(const WalkerDev* W, int nw, int maxN, int j, int q, cudaStre
 }
 
 void oz_slice_const(const double* X, unsigned short* out, int* exps, int N, int ldk, int role, int bits, int slices,
-                    int layout, cudaStream_t st) {
-  oz_const_slice_kernel<<<(N + 31) / 32, 256, 0, st>>>(X, out, exps, N, ldk, role, bits, slices, layout);
+                    cudaStream_t st) {
+  oz_const_slice_kernel<<<(N + 31) / 32, 256, 0, st>>>(X, out, exps, N, ldk, role, bits, slices);
 }
 
 void oz_selftest(const double* A, const double* B, double* C, unsigned short* sa, int* ea, unsigned short* sb, int* eb,
                  int N, cudaStream_t st) {
   const ozaki::SliceCfg cfg = ozaki::cfg_for_k(N);
   const int ldk = (N + 15) / 16 * 16;
-  oz_slice_const(A, sa, ea, N, ldk, 0, cfg.bits, cfg.slices, 0, st);
-  oz_slice_const(B, sb, eb, N, ldk, 1, cfg.bits, cfg.slices, 0, st);
-  const int t = (N + 63) / 64;
-  oz_selftest_prod_kernel<<<dim3(t, t), 256, oz_prod_smem(cfg.slices), st>>>(sa, ea, sb, eb, C, N, ldk, cfg.bits,
-                                                                             cfg.slices);
+  oz_slice_pair_kernel<<<dim3((N + 7) / 8, 2), 256, 0, st>>>(A, B, sa, ea, sb, eb, N, ldk, cfg.bits, cfg.slices);
+  const dim3 g((N + 31) / 32, (N + 127) / 128);
+  const ProdJob job{sa, sb, ea, eb};
+  if (cfg.slices == 7) oz_one_prod_kernel<7><<<g, 256, oz_one_smem(7), st>>>(job, C, N, ldk);
+  else oz_one_prod_kernel<8><<<g, 256, oz_one_smem(8), st>>>(job, C, N, ldk);
 }
 
 }  // namespace dqmc

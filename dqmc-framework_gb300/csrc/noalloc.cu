@@ -12,7 +12,7 @@
 // The array is shared by all calls on a device and keeps the last call's
 // contents.  Nothing in it has to start at zero: every call rewrites all the
 // slices and exponents it reads (the slicing kernel also writes the zero
-// padding of each row).  Calls that overlap on the GPU (concurrent streams,
+// padding of each line; the lines past n only reach outputs past n).  Calls that overlap on the GPU (concurrent streams,
 // or several host threads) race on it; the caller serialises them.
 #include <cuda_runtime.h>
 
@@ -33,9 +33,10 @@ namespace {
 
 constexpr int kNoAllocMaxN = 256;                        // 7-bit x 7 slices, ldk = N
 constexpr size_t kSliceElems = 7ull * kNoAllocMaxN * kNoAllocMaxN;
-// the slicing kernel writes cfg_for_k(n).slices slices of n x ldk(n) elements per
-// operand; both grow with n, so the largest n bounds every call
-static_assert((size_t)dqmc::ozaki::cfg_for_k(kNoAllocMaxN).slices * kNoAllocMaxN * ((kNoAllocMaxN + 15) / 16 * 16) <=
+// the slicing kernel writes cfg_for_k(n).slices tensor-core images of n lines, padded to a multiple
+// of 128, times ldk(n) per operand; both grow with n, so the largest n bounds every call
+static_assert((size_t)dqmc::ozaki::cfg_for_k(kNoAllocMaxN).slices * ((kNoAllocMaxN + 127) / 128 * 128) *
+                      ((kNoAllocMaxN + 15) / 16 * 16) <=
                   kSliceElems,
               "no-alloc scratch too small for the slice configuration of its largest n");
 constexpr size_t kScratchBytes = 2 * kSliceElems * sizeof(unsigned short)  // A and B slices
