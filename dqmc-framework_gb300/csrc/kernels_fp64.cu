@@ -72,6 +72,10 @@ __device__ double block_max(double v, double* red) {
   return m;
 }
 
+// k / d as (k mul) >> 20 with mul = small_div_mul(d): exact for k d < 2^20 (N <= 64: k < 2 N^2, d <= N)
+__device__ __forceinline__ unsigned small_div_mul(int d) { return ((1u << 20) + d - 1) / d; }
+__device__ __forceinline__ int small_div(int k, unsigned mul) { return (int)(((unsigned)k * mul) >> 20); }
+
 // spin factor of the B matrices: repulsive couples spin down with -1, attractive +1
 __device__ __forceinline__ int spin_sign(const WalkerDev& w, int spin) {
   return (w.model == 0 && spin == 1) ? -1 : 1;
@@ -193,9 +197,6 @@ __device__ __forceinline__ void block_gemm(int N, FA A, FB B, FS store, int kbeg
 //   its inverse; sc: the diagonal, applied first (PRE) or last, of matrix m at sc + m * scs.
 //   PLAIN: the plain plaquette product (plaq_product), sc without the constant factor.
 // --------------------------------------------------------------------------
-// k / d as (k mul) >> 20 with mul = small_div_mul(d): exact for k d < 2^20 (here k < 2 N^2, d <= N <= 64)
-__device__ __forceinline__ unsigned small_div_mul(int d) { return ((1u << 20) + d - 1) / d; }
-__device__ __forceinline__ int small_div(int k, unsigned mul) { return (int)(((unsigned)k * mul) >> 20); }
 template <bool RIGHT, bool INV, bool PRE, bool PLAIN = false>
 __device__ __noinline__ void kin_product(const WalkerDev& w, double* M, int ms, int ld, int nm,
                                          double* tmp, int tms, int ldt, const double* sc, int scs,
@@ -649,6 +650,37 @@ __device__ __forceinline__ double block64_sum(double v, double* s_d) {
   return t;
 }
 
+// x . y over r0 <= r < n in two alternating chains from a0, and y += f x, four rows' loads ahead of
+// their FMAs: a thread walks its own column, so a load that waits for the previous store is latency
+__device__ __forceinline__ double push_dot(const double* x, const double* y, int r, int n, double a0) {
+  double a1 = 0.0;
+  for (; r + 3 < n; r += 4) {
+    const double x0 = x[r], x1 = x[r + 1], x2 = x[r + 2], x3 = x[r + 3];
+    const double y0 = y[r], y1 = y[r + 1], y2 = y[r + 2], y3 = y[r + 3];
+    a0 = fma(x0, y0, a0);
+    a1 = fma(x1, y1, a1);
+    a0 = fma(x2, y2, a0);
+    a1 = fma(x3, y3, a1);
+  }
+  for (; r + 1 < n; r += 2) {
+    a0 = fma(x[r], y[r], a0);
+    a1 = fma(x[r + 1], y[r + 1], a1);
+  }
+  if (r < n) a0 = fma(x[r], y[r], a0);
+  return a0 + a1;
+}
+__device__ __forceinline__ void push_axpy(const double* x, double* y, int r, int n, double f) {
+  for (; r + 3 < n; r += 4) {
+    const double x0 = x[r], x1 = x[r + 1], x2 = x[r + 2], x3 = x[r + 3];
+    const double y0 = y[r], y1 = y[r + 1], y2 = y[r + 2], y3 = y[r + 3];
+    y[r] = fma(f, x0, y0);
+    y[r + 1] = fma(f, x1, y1);
+    y[r + 2] = fma(f, x2, y2);
+    y[r + 3] = fma(f, x3, y3);
+  }
+  for (; r < n; ++r) y[r] = fma(f, x[r], y[r]);
+}
+
 template <int MODE>
 __global__ void __launch_bounds__(kPushThreads) push_kernel(const WalkerDev* __restrict__ W, int j) {
   const int wi = blockIdx.x >> 1, sp = blockIdx.x & 1;
@@ -708,17 +740,16 @@ __global__ void __launch_bounds__(kPushThreads) push_kernel(const WalkerDev* __r
     // ---- Householder reflector of X[k:,k]: row r > k held by thread r
     const double xr = (own && tj > k) ? at(X, ld, tj, k) : 0.0;
     const double xnorm2 = block64_sum(xr * xr, s_d);
-    if (tj == 0) {
+    if (tj < 2) {  // lane 0: tau = (beta - alpha) / beta, lane 1: scale = 1 / (alpha - beta)
       const double alpha = at(X, ld, k, k);
-      double t = 0.0, beta = alpha, scal = 1.0;
+      double q = (tj == 0) ? 0.0 : 1.0, beta = alpha;
       if (xnorm2 != 0.0) {
         const double nrm = sqrt(alpha * alpha + xnorm2);
         beta = alpha >= 0 ? -nrm : nrm;
-        t = (beta - alpha) / beta;
-        scal = 1.0 / (alpha - beta);
+        q = (tj == 0 ? beta - alpha : 1.0) / (tj == 0 ? beta : alpha - beta);
       }
-      s_tau = t; s_scal = scal; s_beta = beta;
-      tau[k] = t;
+      if (tj == 0) { s_tau = q; s_beta = beta; tau[k] = q; }
+      else s_scal = q;
     }
     __syncthreads();
     if (own && tj > k) at(X, ld, tj, k) *= s_scal;
@@ -727,16 +758,11 @@ __global__ void __launch_bounds__(kPushThreads) push_kernel(const WalkerDev* __r
     // ---- trailing update of column tj > k, then its norm downdate
     const double tk = s_tau;
     if (own && tj > k && tk != 0.0) {
-      double a0 = at(X, ld, k, tj), a1 = 0.0;
-      int r = k + 1;
-      for (; r + 1 < N; r += 2) {
-        a0 = fma(at(X, ld, r, k), at(X, ld, r, tj), a0);
-        a1 = fma(at(X, ld, r + 1, k), at(X, ld, r + 1, tj), a1);
-      }
-      if (r < N) a0 = fma(at(X, ld, r, k), at(X, ld, r, tj), a0);
-      const double wv = (a0 + a1) * tk;
-      at(X, ld, k, tj) -= wv;
-      for (r = k + 1; r < N; ++r) at(X, ld, r, tj) = fma(-wv, at(X, ld, r, k), at(X, ld, r, tj));
+      const double* xk = X + k * ld;
+      double* xj = X + tj * ld;
+      const double wv = push_dot(xk, xj, k + 1, N, xj[k]) * tk;
+      xj[k] -= wv;
+      push_axpy(xk, xj, k + 1, N, -wv);
     }
     if (own && tj > k) {
       const double v1 = vn1[tj];
@@ -788,6 +814,16 @@ __global__ void __launch_bounds__(kPushThreads) push_kernel(const WalkerDev* __r
     for (int i = 0; i < N; ++i) {
       double a0 = 0.0, a1 = 0.0;
       int k = i;
+      for (; k + 3 < N; k += 4) {  // four terms' loads ahead of their FMAs
+        const double f0 = __ldg(fp + perm[k]), f1 = __ldg(fp + perm[k + 1]);
+        const double f2 = __ldg(fp + perm[k + 2]), f3 = __ldg(fp + perm[k + 3]);
+        const double x0 = at(X, ld, i, k), x1 = at(X, ld, i, k + 1);
+        const double x2 = at(X, ld, i, k + 2), x3 = at(X, ld, i, k + 3);
+        a0 = fma(x0, f0, a0);
+        a1 = fma(x1, f1, a1);
+        a0 = fma(x2, f2, a0);
+        a1 = fma(x3, f3, a1);
+      }
       for (; k + 1 < N; k += 2) {
         a0 = fma(at(X, ld, i, k), __ldg(fp + perm[k]), a0);
         a1 = fma(at(X, ld, i, k + 1), __ldg(fp + perm[k + 1]), a1);
@@ -803,16 +839,11 @@ __global__ void __launch_bounds__(kPushThreads) push_kernel(const WalkerDev* __r
     const double ti = tau[i];
     if (i < N - 1 && own && tj > i) {
       // apply H_i to column tj (rows i..N-1), v = [1; X(i+1:,i)]
-      double a0 = at(X, ld, i, tj), a1 = 0.0;
-      int r = i + 1;
-      for (; r + 1 < N; r += 2) {
-        a0 = fma(at(X, ld, r, i), at(X, ld, r, tj), a0);
-        a1 = fma(at(X, ld, r + 1, i), at(X, ld, r + 1, tj), a1);
-      }
-      if (r < N) a0 = fma(at(X, ld, r, i), at(X, ld, r, tj), a0);
-      const double wv = (a0 + a1) * ti;
-      at(X, ld, i, tj) -= wv;
-      for (r = i + 1; r < N; ++r) at(X, ld, r, tj) = fma(-wv, at(X, ld, r, i), at(X, ld, r, tj));
+      const double* xi = X + i * ld;
+      double* xj = X + tj * ld;
+      const double wv = push_dot(xi, xj, i + 1, N, xj[i]) * ti;
+      xj[i] -= wv;
+      push_axpy(xi, xj, i + 1, N, -wv);
     }
     __syncthreads();
     if (own) {  // column i of Q: thread tj handles row tj
@@ -830,70 +861,74 @@ __global__ void __launch_bounds__(kPushThreads) push_kernel(const WalkerDev* __r
 // --------------------------------------------------------------------------
 // In-SMEM LU with partial pivoting of M, applied on the fly to the right-hand
 // sides Y (forward substitution fused), then back substitution: Y <- M^-1 Y.
-// Returns false if a zero pivot was met.
+// Returns false if a zero pivot was met.  Warp 0 finds a pivot by the bits of
+// its magnitude and forms its reciprocal once, for the multipliers and for the
+// back substitution: a division in every warp was a fifth of the kernel's FP64
+// operations at N = 64.
 // --------------------------------------------------------------------------
-__device__ bool lu_solve_smem(double* M, double* Y, int N, int ld, double* red) {
+__device__ bool lu_solve_smem(double* M, double* Y, int N, int ld) {
   __shared__ int s_p;
   __shared__ int s_bad;
+  __shared__ double s_inv[kMaxSmemN];  // 1 / pivot
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   if (threadIdx.x == 0) s_bad = 0;
   for (int k = 0; k < N; ++k) {
     if (wid == 0) {
-      double best = -1.0;
+      long long best = -1;
       int bi = k;
       for (int r = k + lane; r < N; r += 32) {
-        const double a = fabs(at(M, ld, r, k));
-        if (a > best) { best = a; bi = r; }
+        const long long a = __double_as_longlong(at(M, ld, r, k)) & 0x7fffffffffffffffLL;
+        if (a > best && a <= 0x7ff0000000000000LL) { best = a; bi = r; }  // a NaN is never the largest
       }
       for (int o = 16; o > 0; o >>= 1) {
-        const double ob = __shfl_xor_sync(0xffffffffu, best, o);
+        const long long ob = __shfl_xor_sync(0xffffffffu, best, o);
         const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
         if (ob > best || (ob == best && oi < bi)) { best = ob; bi = oi; }
       }
-      if (lane == 0) { s_p = bi; if (best == 0.0) s_bad = 1; }
+      const double inv = 1.0 / at(M, ld, bi, k);
+      if (lane == 0) { s_p = bi; s_inv[k] = inv; if (best == 0) s_bad = 1; }
     }
     __syncthreads();
     const int pr = s_p;
-    if (pr != k) {
-      for (int c = threadIdx.x; c < 2 * N; c += kThreads) {
+    if (wid == 1) {  // column k: the exchange and the multipliers
+      const double piv = at(M, ld, pr, k), top = at(M, ld, k, k), inv = (piv != 0.0) ? s_inv[k] : 0.0;
+      __syncwarp();
+      if (lane == 0) at(M, ld, k, k) = piv;
+      for (int r = k + 1 + lane; r < N; r += 32) at(M, ld, r, k) = ((r == pr) ? top : at(M, ld, r, k)) * inv;
+    } else if (pr != k) {
+      for (int c = (wid == 0) ? lane : threadIdx.x - 32; c < 2 * N; c += kThreads - 32) {
+        if (c == k) continue;
         double* m = (c < N) ? M : Y;
         const int cc = (c < N) ? c : c - N;
         const double tmp = at(m, ld, k, cc);
         at(m, ld, k, cc) = at(m, ld, pr, cc);
         at(m, ld, pr, cc) = tmp;
       }
-      __syncthreads();
     }
-    const double piv = at(M, ld, k, k);
-    const double inv = (piv != 0.0) ? 1.0 / piv : 0.0;
-    for (int r = k + 1 + threadIdx.x; r < N; r += kThreads) at(M, ld, r, k) *= inv;
     __syncthreads();
     const int nr = N - k - 1;
+    const unsigned dn = small_div_mul(max(nr, 1));
     // trailing update of M (cols k+1..N-1) and of Y (all cols)
     for (int e = threadIdx.x; e < nr * (nr + N); e += kThreads) {
-      const int r = k + 1 + e % nr, cc = e / nr;
+      const int cc = small_div(e, dn), r = k + 1 + e - cc * nr;
       const double l = at(M, ld, r, k);
-      if (cc < nr) {
-        const int c = k + 1 + cc;
-        at(M, ld, r, c) = fma(-l, at(M, ld, k, c), at(M, ld, r, c));
-      } else {
-        const int c = cc - nr;
-        at(Y, ld, r, c) = fma(-l, at(Y, ld, k, c), at(Y, ld, r, c));
-      }
+      double* m = (cc < nr) ? M : Y;
+      const int c = (cc < nr) ? k + 1 + cc : cc - nr;
+      at(m, ld, r, c) = fma(-l, at(m, ld, k, c), at(m, ld, r, c));
     }
     __syncthreads();
   }
   for (int k = N - 1; k >= 0; --k) {
-    const double inv = 1.0 / at(M, ld, k, k);
+    const double inv = s_inv[k];
     for (int c = threadIdx.x; c < N; c += kThreads) at(Y, ld, k, c) *= inv;
     __syncthreads();
+    const unsigned dk = small_div_mul(max(k, 1));
     for (int e = threadIdx.x; e < k * N; e += kThreads) {
-      const int r = e % k, c = e / k;
+      const int c = small_div(e, dk), r = e - c * k;
       at(Y, ld, r, c) = fma(-at(M, ld, r, k), at(Y, ld, k, c), at(Y, ld, r, c));
     }
     __syncthreads();
   }
-  (void)red;
   return s_bad == 0;
 }
 
@@ -974,7 +1009,7 @@ __global__ void __launch_bounds__(kThreads, 2) greens_kernel(const WalkerDev* __
     }
   }
   __syncthreads();
-  const bool ok = lu_solve_smem(Ms, Ys, N, ld, red);
+  const bool ok = lu_solve_smem(Ms, Ys, N, ld);
   if (!ok && threadIdx.x == 0) atomicOr(w.status, ST_SINGULAR);
 
   double* G = w.G + (long long)sp * N * N;
