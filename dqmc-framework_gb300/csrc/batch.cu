@@ -484,12 +484,12 @@ int dqmc_batch_create(const dqmc_walker_desc* descs, int n, const dqmc_batch_opt
     off[w].msub = (o.precision == DQMC_MIXED) ? take((size_t)S * submatrix_scratch_bytes(N))
                   : general                     ? take(submatrix64_scratch_bytes(N, S))
                                                 : 0;
-    // the blocked QR's scratch is the product temporary where that has room (N >= 110)
+    // the blocked QR's scratch is the product temporary where that has room
     off[w].zwk = off[w].work;
     if (stab_kind(N, o.precision, general) && stab_scratch_elems(N) > (size_t)N * N)
       off[w].zwk = take(sizeof(double) * S * stab_scratch_elems(N));
     off[w].zsl = stab_kind(N, o.precision, general) == 1
-                     ? take(sizeof(unsigned short) * (size_t)S * 2 * 9 * ozaki::tc_lines(N) * (size_t)((N + 31) / 32 * 32))
+                     ? take(sizeof(unsigned short) * (size_t)S * 4 * 9 * ozaki::tc_lines(N) * (size_t)((N + 31) / 32 * 32))
                      : 0;
     off[w].dense_id = -1;
     if (!d.checkerboard) {
