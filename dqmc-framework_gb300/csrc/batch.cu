@@ -433,6 +433,7 @@ int dqmc_batch_create(const dqmc_walker_desc* descs, int n, const dqmc_batch_opt
         b->any_ozstab = true;
         int& n = (kind == 1) ? b->stab.tc : b->stab.f64;
         n = std::max(n, N);
+        if (kind == 1) b->stab.tc_min = b->stab.tc_min ? std::min(b->stab.tc_min, N) : N;
       } else {
         b->any_qrp = true;
       }

@@ -114,9 +114,10 @@ struct WalkerDev {
   int wait_limit;
 };
 
-// The largest N of a batch's walkers stabilized with tensor-core and with FP64 products (0: none)
+// The largest N of a batch's walkers stabilized with tensor-core and with FP64 products (0: none),
+// and the smallest of the former
 struct StabSizes {
-  int tc, f64;
+  int tc, f64, tc_min;
   __host__ __device__ int max() const { return tc > f64 ? tc : f64; }
 };
 

@@ -1074,9 +1074,16 @@ __global__ void __launch_bounds__(256) dyn_boundary_kernel(const WalkerDev* __re
 // G(k,tau) += sign / N sum_ij FF(r_j - r_i) (G_up(t,0)(j,i) + G_dn(t,0)(j,i)) / 2 at the listed tau
 // (measure_greens_functions, src/measure/measure_methods.cpp:278-308).  phase 0: slices inside
 // the interval (after propagation); 1: the interval's last slice (after stabilization);
-// 2: tau = 0 from G(beta,beta) after the sweep.
-__global__ void __launch_bounds__(256) dyn_measure_kernel(const WalkerDev* __restrict__ W, int j, int q, int phase) {
-  const WalkerDev& w = W[blockIdx.x];
+// 2: tau = 0 from G(beta,beta) after the sweep.  A cluster of kDynCtas CTAs per walker shares the
+// columns, displacements and sites; rank 0 adds the parts in rank order.  One CTA per walker took
+// 1.0 ms a listed tau for 8 walkers of 24 x 24.
+constexpr int kDynCtas = 8;
+__global__ void __launch_bounds__(256) __cluster_dims__(kDynCtas, 1, 1)
+    dyn_measure_kernel(const WalkerDev* __restrict__ W, int j, int q, int phase) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cl = cg::this_cluster();
+  const WalkerDev& w = W[blockIdx.y];
+  const int rank = blockIdx.x;
   if (!w.gt0 || j >= w.nstack) return;
   int t;
   if (phase == 2) {
@@ -1099,7 +1106,7 @@ __global__ void __launch_bounds__(256) dyn_measure_kernel(const WalkerDev* __res
   const double sg = *w.sign;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   extern __shared__ double dsh[];  // [L] cos(-r kx1), phase 2 also [N] e_i and [N] B_i
-  __shared__ double red[8][4];
+  __shared__ double red[8][4], part[4];
   // FourierFactor(r, 1) of the reference's k-star 1 = (2 pi / L, 0) on the site (r, 0)
   const double kx1 = (double)((L + 1) / 2 + 1) / L * 2 * M_PI - M_PI;
   for (int r = threadIdx.x; r < L; r += blockDim.x) dsh[r] = cos(-r * kx1);
@@ -1116,10 +1123,10 @@ __global__ void __launch_bounds__(256) dyn_measure_kernel(const WalkerDev* __res
     // cubic lattice: G(k,tau) only; the stiffness is a square-lattice observable
     // (dqmc_initializer.cpp:233-237, measure_methods.cpp:350)
     if (w.dim == 3)
-      for (int jj = wid; jj < N; jj += 8)
+      for (int jj = rank * 8 + wid; jj < N; jj += 8 * kDynCtas)
         for (int i = lane; i < N; i += 32)
           v += w.ff[site_disp(L, 3, i, jj)] * (gk[0][(long long)i * N + jj] + gk[1][(long long)i * N + jj]);
-    for (int jj = wid; jj < N && w.dim == 2; jj += 8) {
+    for (int jj = rank * 8 + wid; jj < N && w.dim == 2; jj += 8 * kDynCtas) {
       const int xj = jj % L, yj = jj / L;
       const int jpx = (xj + 1) % L + L * yj;
       for (int i = lane; i < N; i += 32) {
@@ -1142,7 +1149,7 @@ __global__ void __launch_bounds__(256) dyn_measure_kernel(const WalkerDev* __res
       }
     }
     // per-displacement sums S(r) = sum_i G(i + r, i) (both spins): G(k,tau) = sum_r cos(k r) S(r)
-    for (int r = wid; r < N; r += 8) {
+    for (int r = rank * 8 + wid; r < N; r += 8 * kDynCtas) {
       const int rx = r % L, ry = r / L;
       double sr = 0.0;
       for (int i = lane; i < N; i += 32) {
@@ -1152,7 +1159,7 @@ __global__ void __launch_bounds__(256) dyn_measure_kernel(const WalkerDev* __res
       sr = warp_sum_g(sr);
       if (lane == 0) w.dyn_r[(long long)slot * N + r] += sg * 0.5 * sr / N;
     }
-    for (int i = threadIdx.x; i < N; i += blockDim.x) {
+    for (int i = rank * 256 + threadIdx.x; i < N; i += 256 * kDynCtas) {
       const long long d = (long long)i * N + i;
       const int ipx = site_nn(L, i, 0);
       tr += gk[0][d] + gk[1][d];
@@ -1174,16 +1181,23 @@ __global__ void __launch_bounds__(256) dyn_measure_kernel(const WalkerDev* __res
       red[wid][3] = rcor;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (threadIdx.x < 4) {
+      double s = 0.0;
+      for (int k = 0; k < 8; ++k) s += red[k][threadIdx.x];
+      part[threadIdx.x] = s;
+    }
+    cl.sync();  // the parts, and dyn_vec
+    if (rank == 0 && threadIdx.x == 0) {
       double tot[4] = {0.0, 0.0, 0.0, 0.0};
-      for (int k = 0; k < 8; ++k)
-        for (int m = 0; m < 4; ++m) tot[m] += red[k][m];
+      for (int k = 0; k < kDynCtas; ++k)
+        for (int m = 0; m < 4; ++m) tot[m] += cl.map_shared_rank(part, k)[m];
       w.dyn_sum[slot] += sg * 0.5 * tot[0] / N;
       w.dyn_cnt[slot] += 1;
       w.dyn_obs[slot * 3 + 0] += sg * 0.5 * tot[1] / N;
       w.dyn_part[slot * 2 + 0] = tot[2];
       w.dyn_part[slot * 2 + 1] = tot[3];
     }
+    cl.sync();  // the parts stay until rank 0 has read them
   }
   if (phase != 2) return;
   // end of the half-sweep: g00 = G(beta,beta) completes the spin susceptibility and the
@@ -1200,7 +1214,7 @@ __global__ void __launch_bounds__(256) dyn_measure_kernel(const WalkerDev* __res
     B[i] = (g0[(long long)ipx * N + i] - g0[(long long)i * N + ipx]) + (g1[(long long)ipx * N + i] - g1[(long long)i * N + ipx]);
   }
   __syncthreads();
-  for (int k = 0; k < w.dyn_ntau; ++k) {
+  for (int k = rank; k < w.dyn_ntau; k += kDynCtas) {
     const double* dv = w.dyn_vec + (long long)k * 2 * N;
     double ch = 0.0, un = 0.0;
     for (int i = threadIdx.x; i < N; i += blockDim.x) ch += dv[i] * e[i];
@@ -1314,7 +1328,7 @@ void general_dynamic_prop(const WalkerDev* W, int nw, int j, int q, int maxN, bo
     launch_kin(W, nw, maxN, KIN_D0T, MODE_FWD, j, q, st);
   }
   if (any_dense && mixed) mixed_dynamic_prop(W, nw, maxN, j, q, st);
-  dyn_measure_kernel<<<nw, 256, sizeof(double) * 32, st>>>(W, j, q, 0);
+  dyn_measure_kernel<<<dim3(kDynCtas, nw), 256, sizeof(double) * 32, st>>>(W, j, q, 0);
 }
 
 void general_dynamic_chain(const WalkerDev* W, int nw, int j, int q, int maxN, bool mixed, bool any_dense,
@@ -1334,14 +1348,14 @@ void general_dynamic_stab(const WalkerDev* W, int nw, int j, int maxN, cudaStrea
 }
 // G(k,tau) measurement at the stabilization slice of forward step j (after both paths)
 void general_dynamic_stab_measure(const WalkerDev* W, int nw, int j, cudaStream_t st) {
-  dyn_measure_kernel<<<nw, 256, sizeof(double) * 32, st>>>(W, j, 0, 1);
+  dyn_measure_kernel<<<dim3(kDynCtas, nw), 256, sizeof(double) * 32, st>>>(W, j, 0, 1);
 }
 
 void general_dynamic_begin(const WalkerDev* W, int nw, cudaStream_t st) {
   dyn_init_kernel<<<dim3(64, 2 * nw), 256, 0, st>>>(W);
 }
 void general_dynamic_end(const WalkerDev* W, int nw, int maxN, cudaStream_t st) {
-  dyn_measure_kernel<<<nw, 256, sizeof(double) * (32 + 2 * maxN), st>>>(W, 0, 0, 2);
+  dyn_measure_kernel<<<dim3(kDynCtas, nw), 256, sizeof(double) * (32 + 2 * maxN), st>>>(W, 0, 0, 2);
 }
 
 void general_chain_init(int mode, const WalkerDev* W, int nw, int j, cudaStream_t st) {
