@@ -1089,19 +1089,20 @@ static void zgemm(const WalkerDev* W, int nw, StabSizes zs, int op, int mode, in
                                                                                              trace_slot, parts);
   }
   if (!zs.tc) return;
-  const int maxN = zs.tc, rows_max = rows ? rows : maxN, cols_max = cols ? cols : maxN;
-  // the walkers' K: a panel's width, what is left from panel p on, or N; each configuration is
-  // launched only where some walker's K takes it (at N = 576 half of the launches had no work)
+  const int rows_max = rows ? rows : zs.tc, cols_max = cols ? cols : zs.tc;
+  // the walkers' contraction lengths, minN to maxN: a panel's width, what is left from panel p
+  // on, or N; each configuration is launched only where some walker's length takes it (at
+  // N = 576 half of the launches had no work)
   const bool width = op == Z_QR_UPD || op == Z_Q_UPD || op == Z_VT;
   const bool rest = op == Z_QR_W || op == Z_Q_W || op == Z_GRAM || op == Z_TR_UPD;
   const int off = rest ? p * TB + (op == Z_TR_UPD ? TB : 0) : 0;
-  const bool k56 = width || zs.tc_min - off <= 256, k54 = !width && maxN - off > 256;
+  const int minN = width ? TB : zs.tc_min - off, maxN = width ? TB : zs.tc - off;
   const dim3 gs((std::max(rows_max, cols_max) + 31) / 32, 1 + parts, 2 * nw);
   const dim3 g(parts * ((cols_max + 31) / 32), (rows_max + 127) / 128, 2 * nw);
-  if (k56) zslice_kernel<8, 7><<<gs, 256, 0, st>>>(W, op, mode, j, p);
-  if (k54) zslice_kernel<9, 6><<<gs, 256, 0, st>>>(W, op, mode, j, p);
-  if (k56) ZGEMM56<<<g, 256, ztc_smem(8, 32, 2), st>>>(W, op, mode, j, p, trace_slot, parts);
-  if (k54) ZGEMM54<<<g, 256, ztc_smem(9, 32, 4), st>>>(W, op, mode, j, p, trace_slot, parts);
+  if (minN <= 256) zslice_kernel<8, 7><<<gs, 256, 0, st>>>(W, op, mode, j, p);
+  if (maxN > 256) zslice_kernel<9, 6><<<gs, 256, 0, st>>>(W, op, mode, j, p);
+  if (minN <= 256) ZGEMM56<<<g, 256, ztc_smem(8, 32, 2), st>>>(W, op, mode, j, p, trace_slot, parts);
+  if (maxN > 256) ZGEMM54<<<g, 256, ztc_smem(9, 32, 4), st>>>(W, op, mode, j, p, trace_slot, parts);
 }
 
 // Householder panel p: the FP64 column factorization, then its Gram matrix, T factor and
