@@ -272,11 +272,8 @@ int set_last_error(int code, const char* msg) { return fail(code, "%s", msg); }
 struct dqmc_batch {
   int nw = 0, maxN = 0, maxNs = 0, maxLt = 0;
   // walkers split by kernel family: N <= 64 (SMEM-resident) and N > 64 (general)
-  int maxN_small = 0, maxN_general = 0, maxPace_general = 0;
-  bool any_small = false, any_general = false, any_general_dense = false, any_general_cb = false;
-  bool any_ozstab = false;  // walkers stabilized by the blocked QR
-  bool any_qrp = false;     // HBM walkers stabilized by the column-pivoted QR and LU
-  StabSizes stab{};
+  int maxN_small = 0, maxN_general = 0;
+  bool any_small = false, any_general = false, any_general_dense = false;
   bool mixed = false;
   int kd = 0, smax = 1;  // flips a block update takes: delayed updates' k, 32 for submatrix updates
   // Metropolis of HBM walkers: 0 FP64 flush (FP64 walkers: submatrix updates; mixed: delayed), 1 delayed with tensor-core
@@ -427,16 +424,7 @@ int dqmc_batch_create(const dqmc_walker_desc* descs, int n, const dqmc_batch_opt
     if (N > kMaxSmemN || o.precision == DQMC_MIXED || o.hbm) {
       b->any_general = true;
       b->maxN_general = std::max(b->maxN_general, N);
-      b->maxPace_general = std::max(b->maxPace_general, d.pace);
-      if (d.checkerboard) b->any_general_cb = true; else b->any_general_dense = true;
-      if (const int kind = stab_kind(N, o.precision, true)) {
-        b->any_ozstab = true;
-        int& n = (kind == 1) ? b->stab.tc : b->stab.f64;
-        n = std::max(n, N);
-        if (kind == 1) b->stab.tc_min = b->stab.tc_min ? std::min(b->stab.tc_min, N) : N;
-      } else {
-        b->any_qrp = true;
-      }
+      if (!d.checkerboard) b->any_general_dense = true;
     } else {
       b->any_small = true;
       b->maxN_small = std::max(b->maxN_small, N);
@@ -945,31 +933,60 @@ static int autotune_products(dqmc_batch* b) {
   return DQMC_OK;
 }
 
+// What the HBM kernels' launches for a range of walkers need to reach: the largest N, pace, number of
+// stack levels and spins, the kinds of exp(-dtau K) and of stabilization that occur.  Taken per
+// walker group, so that the groups of an uneven batch's small walkers skip the launches that only
+// its large ones need.
+struct LaunchShape {
+  int maxN = 0, maxPace = 0, maxNs = 0, smax = 1;
+  bool dense = false, cb = false, qrp = false;
+  StabSizes stab{};
+  bool oz() const { return stab.max() > 0; }
+};
+// all_hbm: shared-memory walkers too (the dynamic half-sweep runs them as HBM walkers)
+static LaunchShape launch_shape(const dqmc_batch* b, int w0, int w1, bool all_hbm) {
+  LaunchShape s;
+  for (int w = w0; w < w1; ++w) {
+    const WalkerDev& h = b->hw[w];
+    if (h.path == 0 && !all_hbm) continue;
+    s.maxN = std::max(s.maxN, h.N);
+    s.maxPace = std::max(s.maxPace, h.pace);
+    s.maxNs = std::max(s.maxNs, h.nstack);
+    s.smax = std::max(s.smax, h.S);
+    if (h.cb) s.cb = true; else s.dense = true;
+    if (h.ozstab == 0) s.qrp = true;
+    if (h.ozstab == 1) {
+      s.stab.tc = std::max(s.stab.tc, h.N);
+      s.stab.tc_min = s.stab.tc_min ? std::min(s.stab.tc_min, h.N) : h.N;
+    }
+    if (h.ozstab == 2) s.stab.f64 = std::max(s.stab.f64, h.N);
+  }
+  return s;
+}
+
 int dqmc_init_greens(dqmc_batch* b) {
   if (!b) return fail(DQMC_ERR_ARG, "null batch");
   oz_set_shape(b->oz_shape);
-  for (int j = 0; j < b->maxNs; ++j) {
-    if (b->any_small) {
+  if (b->any_small) {
+    for (int j = 0; j < b->maxNs; ++j) {
       launch_segment(MODE_INIT, b->dW, b->nw, j, 0, b->maxN_small, b->stream);
       launch_push(MODE_INIT, b->dW, b->nw, j, b->maxN_small, b->stream);
     }
-    if (b->any_general) {
-      general_chain_init(MODE_INIT, b->dW, b->nw, j, b->stream);
-      for (int q = 0; q < b->maxPace_general; ++q)
-        general_slice_post(MODE_INIT, b->dW, b->nw, j, q, b->maxN_general, b->any_general_dense, b->any_general_cb,
-                           b->mixed, b->stream);  // the transposed B-chain of the initial right stack
-      if (b->any_qrp) general_push(MODE_INIT, b->dW, b->nw, j, b->maxN_general, b->stream);
-      if (b->any_ozstab) oz_push(MODE_INIT, b->dW, b->nw, j, b->stab, b->stream);
-    }
-  }
-  if (b->any_small) {
     launch_greens(MODE_INIT, b->dW, b->nw, 0, 0, -1, b->maxN_small, b->stream);
     launch_sign(b->dW, b->nw, b->maxN_small, b->stream);
   }
   if (b->any_general) {
-    if (b->any_qrp) general_greens(MODE_INIT, b->dW, b->nw, 0, -1, b->maxN_general, b->stream);
-    if (b->any_ozstab) oz_greens(MODE_INIT, b->dW, b->nw, 0, -1, b->stab, b->stream);
-    general_sign(b->dW, b->nw, b->maxN_general, b->stream);
+    const LaunchShape s = launch_shape(b, 0, b->nw, false);
+    for (int j = 0; j < s.maxNs; ++j) {
+      general_chain_init(MODE_INIT, b->dW, b->nw, j, b->stream);
+      for (int q = 0; q < s.maxPace; ++q)  // the transposed B-chain of the initial right stack
+        general_slice_post(MODE_INIT, b->dW, b->nw, j, q, s.maxN, s.dense, s.cb, b->mixed, b->stream);
+      if (s.qrp) general_push(MODE_INIT, b->dW, b->nw, j, s.maxN, b->stream);
+      if (s.oz()) oz_push(MODE_INIT, b->dW, b->nw, j, s.stab, b->stream);
+    }
+    if (s.qrp) general_greens(MODE_INIT, b->dW, b->nw, 0, -1, s.maxN, b->stream);
+    if (s.oz()) oz_greens(MODE_INIT, b->dW, b->nw, 0, -1, s.stab, b->stream);
+    general_sign(b->dW, b->nw, s.maxN, b->stream);
   }
   if (int r = launch_check("init kernels")) return r;
   // wrap error and accumulators start from zero (DqmcWalker::initial, dqmc_walker.cpp:41-49)
@@ -990,29 +1007,29 @@ int dqmc_init_greens(dqmc_batch* b) {
 }
 
 // Level j of the general walkers W[0..nw) on stream st (kernel classes timed when profiling).
-static void issue_general_level(dqmc_batch* b, int mode, int measure, int j, int slot, const WalkerDev* W, int nw,
-                                cudaStream_t st) {
+static void issue_general_level(dqmc_batch* b, const LaunchShape& s, int mode, int measure, int j, int slot,
+                                const WalkerDev* W, int nw, cudaStream_t st) {
   b->timed(DQMC_KCLASS_SEGMENT, [&] { general_chain_init(mode, W, nw, j, st); });
-  for (int q = 0; q < b->maxPace_general; ++q) {
+  for (int q = 0; q < s.maxPace; ++q) {
     b->timed(DQMC_KCLASS_PRODUCT, [&] {
-      general_slice_pre(mode, W, nw, j, q, b->maxN_general, b->any_general_dense, b->any_general_cb, b->mixed, st);
+      general_slice_pre(mode, W, nw, j, q, s.maxN, s.dense, s.cb, b->mixed, st);
     });
     b->timed(DQMC_KCLASS_METROPOLIS, [&] {
-      general_slice_metro(mode, W, nw, j, q, b->maxN_general, measure, b->mixed, b->kd, b->smax, b->tc_flush, st);
+      general_slice_metro(mode, W, nw, j, q, s.maxN, measure, b->mixed, b->kd, s.smax, b->tc_flush, st);
     });
     b->timed(DQMC_KCLASS_PRODUCT, [&] {
-      general_slice_post(mode, W, nw, j, q, b->maxN_general, b->any_general_dense, b->any_general_cb, b->mixed, st);
+      general_slice_post(mode, W, nw, j, q, s.maxN, s.dense, s.cb, b->mixed, st);
     });
   }
   b->timed(DQMC_KCLASS_PUSH, [&] {
-    if (b->any_qrp) general_push(mode, W, nw, j, b->maxN_general, st);
-    if (b->any_ozstab) oz_push(mode, W, nw, j, b->stab, st);
+    if (s.qrp) general_push(mode, W, nw, j, s.maxN, st);
+    if (s.oz()) oz_push(mode, W, nw, j, s.stab, st);
   });
   b->timed(DQMC_KCLASS_GREENS, [&] {
-    if (b->any_qrp) general_greens(mode, W, nw, j, slot, b->maxN_general, st);
-    if (b->any_ozstab) oz_greens(mode, W, nw, j, slot, b->stab, st);
+    if (s.qrp) general_greens(mode, W, nw, j, slot, s.maxN, st);
+    if (s.oz()) oz_greens(mode, W, nw, j, slot, s.stab, st);
   });
-  if (measure) b->timed(DQMC_KCLASS_MEASURE, [&] { general_measure_after(mode, W, nw, j, b->maxN_general, st); });
+  if (measure) b->timed(DQMC_KCLASS_MEASURE, [&] { general_measure_after(mode, W, nw, j, s.maxN, st); });
 }
 
 static int trace_slot(const dqmc_batch* b, int j) {
@@ -1034,11 +1051,13 @@ static void issue_half_sweep(dqmc_batch* b, int mode, int measure) {
     for (int g = 0; g < ng; ++g) {
       const int w0 = (int)((long long)b->nw * g / ng), w1 = (int)((long long)b->nw * (g + 1) / ng);
       cudaStreamWaitEvent(b->gst[g], b->ev_fork, 0);
-      for (int j = 0; j < b->maxNs; ++j)
-        issue_general_level(b, mode, measure, j, trace_slot(b, j), b->dW + w0, w1 - w0, b->gst[g]);
+      const LaunchShape s = launch_shape(b, w0, w1, false);
+      for (int j = 0; j < s.maxNs; ++j)
+        issue_general_level(b, s, mode, measure, j, trace_slot(b, j), b->dW + w0, w1 - w0, b->gst[g]);
       cudaEventRecord(b->ev_join[g], b->gst[g]);
     }
   }
+  const LaunchShape all = launch_shape(b, 0, b->nw, false);
   for (int j = 0; j < b->maxNs; ++j) {
     const int slot = trace_slot(b, j);
     if (b->any_small) {
@@ -1050,7 +1069,7 @@ static void issue_half_sweep(dqmc_batch* b, int mode, int measure) {
       if (measure)
         b->timed(DQMC_KCLASS_MEASURE, [&] { launch_measure(mode, b->dW, b->nw, j, b->maxN_small, b->stream); });
     }
-    if (b->any_general && ng == 1) issue_general_level(b, mode, measure, j, slot, b->dW, b->nw, b->stream);
+    if (j < all.maxNs && ng == 1) issue_general_level(b, all, mode, measure, j, slot, b->dW, b->nw, b->stream);
   }
   if (ng > 1)
     for (int g = 0; g < ng; ++g) cudaStreamWaitEvent(b->stream, b->ev_join[g], 0);
@@ -1258,46 +1277,39 @@ int dqmc_clear_dynamic(dqmc_batch* b) {
   return DQMC_OK;
 }
 
-// The dynamic half-sweep's launch sequence: the walkers' largest N and pace, and which
-// kinds of exp(-dtau K) occur
-struct DynShape {
-  int maxN, maxPace;
-  bool any_dense, any_cb;
-};
-
 // Forward step j of the dynamic half-sweep for walkers W[0..nw) on stream st
-static void issue_dynamic_level(dqmc_batch* b, const DynShape& ds, int j, const WalkerDev* W, int nw,
+static void issue_dynamic_level(dqmc_batch* b, const LaunchShape& s, int j, const WalkerDev* W, int nw,
                                 cudaStream_t st) {
-  const int maxN = ds.maxN;
-  const bool qrp = b->any_qrp || b->any_small;  // shared-memory walkers run this half-sweep as HBM walkers
+  const int maxN = s.maxN;
   b->timed(DQMC_KCLASS_SEGMENT, [&] { general_chain_init(MODE_FWD, W, nw, j, st); });
-  for (int q = 0; q < ds.maxPace; ++q) {
+  for (int q = 0; q < s.maxPace; ++q) {
     b->timed(DQMC_KCLASS_PRODUCT,
-             [&] { general_dynamic_wrap(W, nw, j, q, maxN, b->mixed, ds.any_dense, ds.any_cb, st); });
+             [&] { general_dynamic_wrap(W, nw, j, q, maxN, b->mixed, s.dense, s.cb, st); });
     b->timed(DQMC_KCLASS_DYNAMIC,
-             [&] { general_dynamic_prop(W, nw, j, q, maxN, b->mixed, ds.any_dense, ds.any_cb, st); });
+             [&] { general_dynamic_prop(W, nw, j, q, maxN, b->mixed, s.dense, s.cb, st); });
     b->timed(DQMC_KCLASS_PRODUCT,
-             [&] { general_dynamic_chain(W, nw, j, q, maxN, b->mixed, ds.any_dense, ds.any_cb, st); });
+             [&] { general_dynamic_chain(W, nw, j, q, maxN, b->mixed, s.dense, s.cb, st); });
   }
   b->timed(DQMC_KCLASS_PUSH, [&] {
-    if (qrp) general_push(MODE_FWD, W, nw, j, maxN, st);
-    if (b->any_ozstab) oz_push(MODE_FWD, W, nw, j, b->stab, st);
+    if (s.qrp) general_push(MODE_FWD, W, nw, j, maxN, st);
+    if (s.oz()) oz_push(MODE_FWD, W, nw, j, s.stab, st);
   });
   b->timed(DQMC_KCLASS_GREENS, [&] {
-    if (qrp) general_greens(MODE_FWD, W, nw, j, -1, maxN, st);
+    if (s.qrp) general_greens(MODE_FWD, W, nw, j, -1, maxN, st);
   });
   // the tensor-core walkers' equal-time assembly and their G(t,0), G(0,t) come from one
   // oz_greens (one factorization of M), timed in this class
   b->timed(DQMC_KCLASS_DYN_STAB, [&] {
-    if (qrp) general_dynamic_stab(W, nw, j, maxN, st);
-    if (b->any_ozstab) oz_greens(MODE_FWD, W, nw, j, -1, b->stab, st, true);
+    if (s.qrp) general_dynamic_stab(W, nw, j, maxN, st);
+    if (s.oz()) oz_greens(MODE_FWD, W, nw, j, -1, s.stab, st, true);
     general_dynamic_stab_measure(W, nw, j, st);
   });
 }
 
 // All device work of one dynamic half-sweep: as the updating half-sweeps, walker groups
 // run as forked branches (one branch when profiling)
-static void issue_dynamic(dqmc_batch* b, const DynShape& ds) {
+static void issue_dynamic(dqmc_batch* b) {
+  const LaunchShape all = launch_shape(b, 0, b->nw, true);
   const int ng = b->prof ? 1 : std::min(b->ngroups, b->nw);
   b->timed(DQMC_KCLASS_DYNAMIC, [&] { general_dynamic_begin(b->dW, b->nw, b->stream); });
   if (ng > 1) {
@@ -1305,14 +1317,15 @@ static void issue_dynamic(dqmc_batch* b, const DynShape& ds) {
     for (int g = 0; g < ng; ++g) {
       const int w0 = (int)((long long)b->nw * g / ng), w1 = (int)((long long)b->nw * (g + 1) / ng);
       cudaStreamWaitEvent(b->gst[g], b->ev_fork, 0);
-      for (int j = 0; j < b->maxNs; ++j) issue_dynamic_level(b, ds, j, b->dW + w0, w1 - w0, b->gst[g]);
+      const LaunchShape s = launch_shape(b, w0, w1, true);
+      for (int j = 0; j < s.maxNs; ++j) issue_dynamic_level(b, s, j, b->dW + w0, w1 - w0, b->gst[g]);
       cudaEventRecord(b->ev_join[g], b->gst[g]);
     }
     for (int g = 0; g < ng; ++g) cudaStreamWaitEvent(b->stream, b->ev_join[g], 0);
   } else {
-    for (int j = 0; j < b->maxNs; ++j) issue_dynamic_level(b, ds, j, b->dW, b->nw, b->stream);
+    for (int j = 0; j < all.maxNs; ++j) issue_dynamic_level(b, all, j, b->dW, b->nw, b->stream);
   }
-  b->timed(DQMC_KCLASS_DYNAMIC, [&] { general_dynamic_end(b->dW, b->nw, ds.maxN, b->stream); });
+  b->timed(DQMC_KCLASS_DYNAMIC, [&] { general_dynamic_end(b->dW, b->nw, all.maxN, b->stream); });
 }
 
 int dqmc_sweep_dynamic(dqmc_batch* b, const int* taus, int ntau) {
@@ -1338,8 +1351,6 @@ int dqmc_sweep_dynamic(dqmc_batch* b, const int* taus, int ntau) {
   // shared-memory walkers run this half-sweep on the HBM path's kernels with their own
   // buffers (the stacks, G and the fields are laid out alike on both paths)
   std::vector<WalkerDev> hv = b->hw;
-  int maxN = 0, maxPace = 0;
-  bool any_dense = false, any_cb = false;
   for (int w = 0; w < b->nw; ++w) {
     WalkerDev& h = hv[w];
     if (h.path == 0) {
@@ -1348,19 +1359,15 @@ int dqmc_sweep_dynamic(dqmc_batch* b, const int* taus, int ntau) {
       h.work = b->dyn_gen[w].work;
       h.scr = b->dyn_gen[w].scr;
     }
-    maxN = std::max(maxN, h.N);
-    maxPace = std::max(maxPace, h.pace);
-    if (h.cb) any_cb = true; else any_dense = true;
   }
   CUDA_TRY(cudaMemcpyAsync(b->dW, hv.data(), sizeof(WalkerDev) * b->nw, cudaMemcpyHostToDevice, b->stream));
   oz_set_shape(b->oz_shape);
-  const DynShape ds{maxN, maxPace, any_dense, any_cb};
   if (b->opt.graphs && !b->prof) {
     // captured once (the tau list and the per-walker descriptors are read on the device)
     if (!b->dyn_exec) {
       GraphGuard g;
       CUDA_TRY(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
-      issue_dynamic(b, ds);
+      issue_dynamic(b);
       CUDA_TRY(cudaStreamEndCapture(b->stream, &g.g));
       size_t nn = 0;
       CUDA_TRY(cudaGraphGetNodes(g.g, nullptr, &nn));
@@ -1378,7 +1385,7 @@ int dqmc_sweep_dynamic(dqmc_batch* b, const int* taus, int ntau) {
     CUDA_TRY(cudaGraphLaunch(b->dyn_exec, b->stream));
     b->launches += b->dyn_nodes;
   } else {
-    issue_dynamic(b, ds);  // eager, one branch when profiling
+    issue_dynamic(b);  // eager, one branch when profiling
   }
   CUDA_TRY(cudaMemcpyAsync(b->dW, b->hw.data(), sizeof(WalkerDev) * b->nw, cudaMemcpyHostToDevice, b->stream));
   CUDA_TRY(cudaStreamSynchronize(b->stream));
