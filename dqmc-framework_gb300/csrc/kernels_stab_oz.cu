@@ -155,6 +155,13 @@ enum ZOp {
   Z_D0T_OUT,     // G(0,t) = -F_R^T Drmin X
 };
 
+// A launch's column tiles: `first` of part 0, then `rest` of each further part
+struct ZTiles {
+  int first, rest;
+  __device__ __forceinline__ int part(int x) const { return x < first ? 0 : 1 + (x - first) / rest; }
+  __device__ __forceinline__ int col(int x) const { return x < first ? x : (x - first) % rest; }
+};
+
 // the job of op's part (columns of the product; parts share the operand A)
 __device__ bool zjob(const WalkerDev& w, int op, int mode, int j, int p, int sp, int part, ZJob& jb) {
   if (j >= w.nstack) return false;
@@ -398,7 +405,7 @@ __global__ void __launch_bounds__(256) zslice_kernel(const WalkerDev* __restrict
 // --------------------------------------------------------------------------
 template <int S, int B, int NT, int NS, int MINB>
 __global__ void __launch_bounds__(256, MINB) zgemm_tc_kernel(const WalkerDev* __restrict__ W, int op, int mode, int j,
-                                                             int p, int trace_slot, int parts) {
+                                                             int p, int trace_slot, ZTiles tl) {
   constexpr int MT = 128;
   constexpr int CW = (MINB > 1) ? 8 : 16;  // TMEM columns per load in the epilogue
   constexpr unsigned TCOLS = (S * NT <= 256) ? 256u : 512u;
@@ -407,10 +414,10 @@ __global__ void __launch_bounds__(256, MINB) zgemm_tc_kernel(const WalkerDev* __
   const WalkerDev& w = W[wi];
   if (w.ozstab != 1 || sp >= w.S) return;
   ZJob jb;
-  const int part = blockIdx.x % parts;
+  const int part = tl.part(blockIdx.x);
   if (!zjob(w, op, mode, j, p, sp, part, jb)) return;
   if ((jb.K <= 256) != (B == 7)) return;
-  const int r0 = blockIdx.y * MT, c0 = blockIdx.x / parts * NT;
+  const int r0 = blockIdx.y * MT, c0 = tl.col(blockIdx.x) * NT;
   if (r0 >= jb.M || c0 >= jb.N) return;
   extern __shared__ __align__(1024) unsigned char tsm[];
   __shared__ int eA[MT], eB[NT];
@@ -535,13 +542,13 @@ __global__ void __launch_bounds__(256, MINB) zgemm_tc_kernel(const WalkerDev* __
 // reaches 32 SMs per matrix.
 // --------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) zgemm_f64_kernel(const WalkerDev* __restrict__ W, int op, int mode, int j, int p,
-                                                        int trace_slot, int parts) {
+                                                        int trace_slot, ZTiles tl) {
   const int wi = blockIdx.z >> 1, sp = blockIdx.z & 1;
   const WalkerDev& w = W[wi];
   if (w.ozstab != 2 || sp >= w.S) return;
   ZJob jb;
-  if (!zjob(w, op, mode, j, p, sp, blockIdx.x % parts, jb)) return;
-  const int r0 = blockIdx.y * 16, c0 = blockIdx.x / parts * 16;
+  if (!zjob(w, op, mode, j, p, sp, tl.part(blockIdx.x), jb)) return;
+  const int r0 = blockIdx.y * 16, c0 = tl.col(blockIdx.x) * 16;
   if (r0 >= jb.M || c0 >= jb.N) return;
   __shared__ double As[32][17], Bs[32][17];
   const int tid = threadIdx.x, lane = tid & 31;
@@ -1080,16 +1087,37 @@ size_t stab_scratch_elems(int N) {
   return 4ull * TB * N + (size_t)TB * TB * ((N + TB - 1) / TB) + 5ull * N + (5ull * N + 1) / 2;
 }
 
-// rows / cols: 0 the whole matrix (maxN), TB a panel's width
-static void zgemm(const WalkerDev* W, int nw, StabSizes zs, int op, int mode, int j, int p, int rows, int cols,
-                  int trace_slot, cudaStream_t st, int parts = 1) {
+// The largest output of an operation over walkers of up to n sites: rows, and columns of part 0
+// and of each further part (zjob).  The trailing matrix shrinks with the panels: in grids for the
+// whole matrix more than half of the factorization's CTAs had no work (N = 256), and each waited
+// for 80 KB of shared memory to start.  Grids of the extent: 128 walkers of 16 x 16 690 -> 680 ms
+// a sweep pair, 32 walkers of 9 x 9 in FP64 22.2 -> 21.8, set-up of 48 of 12 x 12 17.9 -> 17.5.
+struct ZExtent {
+  int rows, cols0, cols;
+};
+static ZExtent zextent(int op, int p, int n) {
+  const int m = std::max(n - p * TB, 0), pb = std::min(TB, m);
+  switch (op) {
+    case Z_QR_W: return {pb, m - pb, n};
+    case Z_QR_UPD: return {m, m - pb, n};
+    case Z_Q_W: return {pb, m, m};
+    case Z_Q_UPD: return {m, m, m};
+    case Z_TR_UPD: return {m > TB ? pb : 0, n, n};
+    case Z_GRAM: return {pb, pb, pb};
+    case Z_VT: return {m, pb, pb};
+    default: return {n, n, n};
+  }
+}
+
+static void zgemm(const WalkerDev* W, int nw, StabSizes zs, int op, int mode, int j, int p, int trace_slot,
+                  cudaStream_t st, int parts = 1) {
   if (zs.f64) {
-    const int rm = rows ? rows : zs.f64, cm = cols ? cols : zs.f64;
-    zgemm_f64_kernel<<<dim3(parts * ((cm + 15) / 16), (rm + 15) / 16, 2 * nw), 256, 0, st>>>(W, op, mode, j, p,
-                                                                                             trace_slot, parts);
+    const ZExtent x = zextent(op, p, zs.f64);
+    const ZTiles tl{(x.cols0 + 15) / 16, (x.cols + 15) / 16};
+    const dim3 g(tl.first + (parts - 1) * tl.rest, (x.rows + 15) / 16, 2 * nw);
+    if (g.x && g.y) zgemm_f64_kernel<<<g, 256, 0, st>>>(W, op, mode, j, p, trace_slot, tl);
   }
   if (!zs.tc) return;
-  const int rows_max = rows ? rows : zs.tc, cols_max = cols ? cols : zs.tc;
   // the walkers' contraction lengths, minN to maxN: a panel's width, what is left from panel p
   // on, or N; each configuration is launched only where some walker's length takes it (at
   // N = 576 half of the launches had no work)
@@ -1097,21 +1125,24 @@ static void zgemm(const WalkerDev* W, int nw, StabSizes zs, int op, int mode, in
   const bool rest = op == Z_QR_W || op == Z_Q_W || op == Z_GRAM || op == Z_TR_UPD;
   const int off = rest ? p * TB + (op == Z_TR_UPD ? TB : 0) : 0;
   const int minN = width ? TB : zs.tc_min - off, maxN = width ? TB : zs.tc - off;
-  const dim3 gs((std::max(rows_max, cols_max) + 31) / 32, 1 + parts, 2 * nw);
-  const dim3 g(parts * ((cols_max + 31) / 32), (rows_max + 127) / 128, 2 * nw);
+  const ZExtent x = zextent(op, p, zs.tc);
+  const ZTiles tl{(x.cols0 + 31) / 32, (x.cols + 31) / 32};
+  const dim3 g(tl.first + (parts - 1) * tl.rest, (x.rows + 127) / 128, 2 * nw);
+  const dim3 gs((std::max(x.rows, parts > 1 ? x.cols : x.cols0) + 31) / 32, 1 + parts, 2 * nw);
+  if (!g.x || !g.y) return;
   if (minN <= 256) zslice_kernel<8, 7><<<gs, 256, 0, st>>>(W, op, mode, j, p);
   if (maxN > 256) zslice_kernel<9, 6><<<gs, 256, 0, st>>>(W, op, mode, j, p);
-  if (minN <= 256) ZGEMM56<<<g, 256, ztc_smem(8, 32, 2), st>>>(W, op, mode, j, p, trace_slot, parts);
-  if (maxN > 256) ZGEMM54<<<g, 256, ztc_smem(9, 32, 4), st>>>(W, op, mode, j, p, trace_slot, parts);
+  if (minN <= 256) ZGEMM56<<<g, 256, ztc_smem(8, 32, 2), st>>>(W, op, mode, j, p, trace_slot, tl);
+  if (maxN > 256) ZGEMM54<<<g, 256, ztc_smem(9, 32, 4), st>>>(W, op, mode, j, p, trace_slot, tl);
 }
 
 // Householder panel p: the FP64 column factorization, then its Gram matrix, T factor and
 // Vt = V T (the block reflector in the form the trailing products apply)
 static void zpanel(const WalkerDev* W, int nw, StabSizes zs, int mode, int j, int p, int push, cudaStream_t st) {
   zqr_panel_kernel<<<2 * nw, 256, zpanel_smem(zs.max()), st>>>(W, mode, j, p, push);
-  zgemm(W, nw, zs, Z_GRAM, mode, j, p, TB, TB, -1, st);
+  zgemm(W, nw, zs, Z_GRAM, mode, j, p, -1, st);
   ztfac_kernel<<<2 * nw, 256, 0, st>>>(W, mode, j, p);
-  zgemm(W, nw, zs, Z_VT, mode, j, p, 0, TB, -1, st);
+  zgemm(W, nw, zs, Z_VT, mode, j, p, -1, st);
 }
 
 void oz_push(int mode, const WalkerDev* W, int nw, int j, StabSizes zs, cudaStream_t st) {
@@ -1119,15 +1150,15 @@ void oz_push(int mode, const WalkerDev* W, int nw, int j, StabSizes zs, cudaStre
   zpush_prep_kernel<<<2 * nw, 256, sizeof(long long) * maxN, st>>>(W, mode, j);
   for (int p = 0; p < np; ++p) {
     zpanel(W, nw, zs, mode, j, p, 1, st);
-    zgemm(W, nw, zs, Z_QR_W, mode, j, p, TB, 0, -1, st);
-    zgemm(W, nw, zs, Z_QR_UPD, mode, j, p, 0, 0, -1, st);
+    zgemm(W, nw, zs, Z_QR_W, mode, j, p, -1, st);
+    zgemm(W, nw, zs, Z_QR_UPD, mode, j, p, -1, st);
   }
   zpush_fin_kernel<<<dim3(64, 2 * nw), 256, 0, st>>>(W, mode, j);
-  zgemm(W, nw, zs, Z_F, mode, j, 0, 0, 0, -1, st);
+  zgemm(W, nw, zs, Z_F, mode, j, 0, -1, st);
   for (int p = np - 1; p >= 0; --p) {
     zvt_kernel<<<dim3((maxN + 31) / 32, 2 * nw), 256, 0, st>>>(W, mode, j, p);
-    zgemm(W, nw, zs, Z_Q_W, mode, j, p, TB, 0, -1, st);
-    zgemm(W, nw, zs, Z_Q_UPD, mode, j, p, 0, 0, -1, st);
+    zgemm(W, nw, zs, Z_Q_W, mode, j, p, -1, st);
+    zgemm(W, nw, zs, Z_Q_UPD, mode, j, p, -1, st);
   }
 }
 
@@ -1137,24 +1168,24 @@ void oz_greens(int mode, const WalkerDev* W, int nw, int j, int trace_slot, Stab
   const int maxN = zs.max(), np = (maxN + TB - 1) / TB;
   zgreens_prep_kernel<<<dim3(64, 2 * nw), 256, 0, st>>>(W, mode, j);
   if (dyn) zdyn_prep_kernel<<<dim3(64, 2 * nw), 256, 0, st>>>(W, j);
-  zgemm(W, nw, zs, Z_GA, mode, j, 0, 0, 0, -1, st);
-  zgemm(W, nw, zs, Z_GB, mode, j, 0, 0, 0, -1, st);
+  zgemm(W, nw, zs, Z_GA, mode, j, 0, -1, st);
+  zgemm(W, nw, zs, Z_GB, mode, j, 0, -1, st);
   // Q^T goes to the trailing columns and the right-hand sides in the same launches (8 walkers of
   // 24 x 24 with the dynamic half-sweep: 216 -> 206 ms a pass, 128 walkers of 16 x 16 767 -> 751)
   for (int p = 0; p < np; ++p) {
     zpanel(W, nw, zs, mode, j, p, 0, st);
-    zgemm(W, nw, zs, Z_QR_W, mode, j, p, TB, 0, -1, st, dyn ? 3 : 2);
-    zgemm(W, nw, zs, Z_QR_UPD, mode, j, p, 0, 0, -1, st, dyn ? 3 : 2);
+    zgemm(W, nw, zs, Z_QR_W, mode, j, p, -1, st, dyn ? 3 : 2);
+    zgemm(W, nw, zs, Z_QR_UPD, mode, j, p, -1, st, dyn ? 3 : 2);
   }
   for (int p = np - 1; p >= 0; --p) {
-    zgemm(W, nw, zs, Z_TR_UPD, mode, j, p, TB, 0, -1, st, dyn ? 2 : 1);
+    zgemm(W, nw, zs, Z_TR_UPD, mode, j, p, -1, st, dyn ? 2 : 1);
     ztrsm_diag_kernel<<<dim3((maxN + 127) / 128, 2 * nw, dyn ? 2 : 1), 128, 0, st>>>(W, mode, j, p);
   }
-  zgemm(W, nw, zs, Z_GG, mode, j, 0, 0, 0, trace_slot, st);
+  zgemm(W, nw, zs, Z_GG, mode, j, 0, trace_slot, st);
   zgreens_out_kernel<<<dim3(64, 2 * nw), 256, 0, st>>>(W, mode, j, trace_slot);
   if (dyn) {
-    zgemm(W, nw, zs, Z_DT0_OUT, mode, j, 0, 0, 0, -1, st);
-    zgemm(W, nw, zs, Z_D0T_OUT, mode, j, 0, 0, 0, -1, st);
+    zgemm(W, nw, zs, Z_DT0_OUT, mode, j, 0, -1, st);
+    zgemm(W, nw, zs, Z_D0T_OUT, mode, j, 0, -1, st);
     zdyn_boundary_kernel<<<dim3(64, 2 * nw), 256, 0, st>>>(W, j);
   }
 }
