@@ -655,17 +655,14 @@ __global__ void __launch_bounds__(256) zpush_prep_kernel(const WalkerDev* __rest
 // reflectors into X below the diagonal, R on and above, tau on the diagonal of the panel's T
 // slot; for the push also D = |diag R| into the stack level and 1/D.
 //
-// Column c takes two barriers.  After the first, warps 1-7 form the dot products of the column
-// with the remaining ones from the unscaled column x, while warp 0 reduces its norm and computes
-// tau and the scale of the reflector v = x scale (a square root and one division, the two
-// quotients on two lanes); after the second, warps 1-7 apply the reflector, A -= x (scale w), and
-// warp 0 does so for column c + 1 and accumulates its norm.  The columns' scales are applied when
-// the panel is written back.  The dot products of a warp's columns share their shuffle steps
-// (zsum4, zsum8): an FP64 add costs a warp 64 cycles whatever its lanes hold.  What bounds it: the
-// FP64 rate of one SM (2 m pb^2 operations) for long panels, warp 0's chain for short ones.
-// Average of the 8 panels at N = 256 (12 CTAs): 134 us; 185 with a norm pass, a scaling pass, serial
-// quotients and a shuffle reduction per column.  A pass of 6 walkers of 16 x 16 went from 59.8 to
-// 55.6 ms (with ztfac_kernel), of 128 walkers from 794 to 771.
+// Column c takes one barrier.  Warps 1-7 apply its reflector to columns c + 2 ..., at most five
+// each: the dot products of a warp's columns share their loads and their shuffle steps (zsum4,
+// zsum8).  Meanwhile warp 0 applies it to column c + 1 and forms that column's reflector (norm, a
+// square root, the two quotients on two lanes, the scaling).  Every sum keeps the order of one
+// column at a time (a norm over 256 threads, dot products over a warp): the 49-bit products of a
+// stabilization interval amplify a change of rounding here to 1e-6 of the s-wave sum at beta = 10.
+// What bounds it: the FP64 rate of one SM (2 m pb^2 operations) for long panels, warp 0's chain
+// for short ones.
 // --------------------------------------------------------------------------
 // Sums of 4 (8) values over the warp, value k left in lanes 8 k .. 8 k + 7 (4 k .. 4 k + 3)
 __device__ __forceinline__ double zsum4(double a0, double a1, double a2, double a3, int lane) {
@@ -698,35 +695,69 @@ __global__ void __launch_bounds__(256) zqr_panel_kernel(const WalkerDev* __restr
   const int m = N - j0, pb = min(TB, m);
   const ZScr z = zscr(w, sp);
   extern __shared__ double P[];  // [TB][m], P[c * m + r]
-  __shared__ double s_tau[TB], s_scal[TB], s_dot[TB];
+  __shared__ double s_tau[TB];
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   for (int c = wid; c < pb; c += 8)
     for (int r = lane; r < m; r += 32) P[c * m + r] = z.X[(long long)(j0 + c) * N + j0 + r];
   __syncthreads();
-  double xn2 = 0.0;  // warp 0: this lane's part of the squared norm of column c below the diagonal
-  if (wid == 0)
-    for (int r = 1 + lane; r < m; r += 32) xn2 = fma(P[r], P[r], xn2);
-  for (int c = 0; c < pb; ++c) {
-    const double* x = P + c * m;
-    const int nr = pb - 1 - c;  // columns after c
-    if (wid == 0) {
-      const double n2 = zwarp_sum(xn2), alpha = x[c];
-      const double nrm = sqrt(fma(alpha, alpha, n2));
-      const bool any = __double_as_longlong(n2) != 0;  // n2 >= 0; bit tests keep off the FP64 pipe
-      const double beta = __double_as_longlong(alpha) < 0 ? nrm : -nrm;
-      // lane 0: tau = (beta - alpha) / beta, lane 1: scale = 1 / (alpha - beta)
-      const double d = beta - alpha, quo = __ddiv_rn(lane == 1 ? 1.0 : d, lane == 1 ? -d : beta);
-      if (lane == 0) s_tau[c] = any ? quo : 0.0;
-      if (lane == 1) s_scal[c] = any ? quo : 1.0;
-      __syncwarp();
-      if (lane == 0) P[c * m + c] = any ? beta : alpha;
-    } else {
-      // columns c + 1 + (wid - 1) + 7 k, at most 5
-      double acc[8];
+  // warp 0: the reflector of column c (norm in 8 strided parts, added in their order)
+  auto reflector = [&](int c) {
+    double* x = P + c * m;
+    double s[8];
 #pragma unroll
-      for (int k = 0; k < 8; ++k) acc[k] = 0.0;
-      const int c0 = c + wid, nc = (c0 < pb) ? (pb - c0 + 6) / 7 : 0;
+    for (int q = 0; q < 8; ++q) s[q] = 0.0;
+    for (int r0 = c + 1; r0 < m; r0 += 256) {
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const int r = r0 + 32 * q + lane;
+        if (r < m) s[q] = fma(x[r], x[r], s[q]);
+      }
+    }
+    __syncwarp();
+    const double v = zsum8(s, lane);
+    const int nq = min(8, (m - c - 1 + 31) / 32);
+    double n2 = __shfl_sync(0xffffffffu, v, 0);
+    for (int q = 1; q < nq; ++q) n2 += __shfl_sync(0xffffffffu, v, 4 * q);
+    const double alpha = x[c];
+    const double nrm = sqrt(alpha * alpha + n2);
+    const bool any = n2 != 0.0;
+    const double beta = alpha >= 0 ? -nrm : nrm;
+    // lane 0: tau = (beta - alpha) / beta, lane 1: scale = 1 / (alpha - beta)
+    const double d = beta - alpha, quo = __ddiv_rn(lane == 1 ? 1.0 : d, lane == 1 ? -d : beta);
+    const double tau = __shfl_sync(0xffffffffu, quo, 0), scal = __shfl_sync(0xffffffffu, quo, 1);
+    if (lane == 0) {
+      s_tau[c] = any ? tau : 0.0;
+      x[c] = any ? beta : alpha;
+    }
+    if (any)
+      for (int r = c + 1 + lane; r < m; r += 32) x[r] *= scal;
+    __syncwarp();
+  };
+  if (wid == 0) reflector(0);
+  __syncthreads();
+  for (int c = 0; c + 1 < pb; ++c) {
+    const double* x = P + c * m;
+    const double tau = s_tau[c];
+    if (wid == 0) {
+      double* a = P + (c + 1) * m;
+      if (tau != 0.0) {
+        double d = 0.0;
+        for (int r = c + 1 + lane; r < m; r += 32) d = fma(x[r], a[r], d);
+        d = zwarp_sum(d) + a[c];
+        const double wv = tau * d;
+        __syncwarp();
+        if (lane == 0) a[c] -= wv;
+        for (int r = c + 1 + lane; r < m; r += 32) a[r] = fma(-wv, x[r], a[r]);
+        __syncwarp();
+      }
+      reflector(c + 1);
+    } else if (tau != 0.0) {
+      // columns c + 2 + (wid - 1) + 7 k, at most 5; lane k forms column k's factor
+      const int c0 = c + 1 + wid, nc = (c0 < pb) ? (pb - c0 + 6) / 7 : 0;
       if (nc > 0) {
+        double acc[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) acc[k] = 0.0;
         for (int r = c + 1 + lane; r < m; r += 32) {
           const double xr = x[r];
 #pragma unroll
@@ -734,65 +765,33 @@ __global__ void __launch_bounds__(256) zqr_panel_kernel(const WalkerDev* __restr
             if (k < nc) acc[k] = fma(xr, P[(c0 + 7 * k) * m + r], acc[k]);
         }
         __syncwarp();
-        if (nc <= 4) {
-          const double v = zsum4(acc[0], acc[1], acc[2], acc[3], lane);
-          if ((lane & 7) == 0 && (lane >> 3) < nc) s_dot[c0 + 7 * (lane >> 3)] = v;
-        } else {
-          const double v = zsum8(acc, lane);
-          if ((lane & 3) == 0 && (lane >> 2) < nc) s_dot[c0 + 7 * (lane >> 2)] = v;
-        }
-      }
-    }
-    __syncthreads();
-    const double tau = s_tau[c], scal = s_scal[c];
-    if (nr > 0) {
-      if (wid == 0) {
-        // column c + 1, and its norm below row c + 1
-        double* a = P + (c + 1) * m;
-        const double wv = tau * fma(scal, s_dot[c + 1], a[c]), ws = -(wv * scal);
-        __syncwarp();
-        if (lane == 0) a[c] -= wv;
-        xn2 = 0.0;
-        for (int r = c + 1 + lane; r < m; r += 32) {
-          const double v = fma(ws, x[r], a[r]);
-          a[r] = v;
-          if (r > c + 1) xn2 = fma(v, v, xn2);
-        }
-        __syncwarp();
-      } else {
-        // columns c + 2 + (wid - 1) + 7 k: lane k forms column k's factor
-        const int c0 = c + 1 + wid, nc = (c0 < pb) ? (pb - c0 + 6) / 7 : 0;
-        double ws = 0.0;
+        const bool four = nc <= 4;
+        const double v = four ? zsum4(acc[0], acc[1], acc[2], acc[3], lane) : zsum8(acc, lane);
+        double d = __shfl_sync(0xffffffffu, v, (four ? 8 : 4) * lane & 31), wv = 0.0;
         if (lane < nc) {
           double* a = P + (c0 + 7 * lane) * m;
-          const double wv = tau * fma(scal, s_dot[c0 + 7 * lane], a[c]);
+          d += a[c];
+          wv = tau * d;
           a[c] -= wv;
-          ws = -(wv * scal);
         }
         double f[5];
 #pragma unroll
-        for (int k = 0; k < 5; ++k) f[k] = __shfl_sync(0xffffffffu, ws, k);
-        if (nc > 0)
-          for (int r = c + 1 + lane; r < m; r += 32) {
-            const double xr = x[r];
-            double v[5];
+        for (int k = 0; k < 5; ++k) f[k] = -__shfl_sync(0xffffffffu, wv, k);
+        for (int r = c + 1 + lane; r < m; r += 32) {
+          const double xr = x[r];
+          double y[5];
 #pragma unroll
-            for (int k = 0; k < 5; ++k) v[k] = (k < nc) ? P[(c0 + 7 * k) * m + r] : 0.0;
+          for (int k = 0; k < 5; ++k) y[k] = (k < nc) ? P[(c0 + 7 * k) * m + r] : 0.0;
 #pragma unroll
-            for (int k = 0; k < 5; ++k)
-              if (k < nc) P[(c0 + 7 * k) * m + r] = fma(f[k], xr, v[k]);
-          }
+          for (int k = 0; k < 5; ++k)
+            if (k < nc) P[(c0 + 7 * k) * m + r] = fma(f[k], xr, y[k]);
+        }
       }
     }
     __syncthreads();
   }
-  for (int c = wid; c < pb; c += 8) {
-    const double scal = s_scal[c];
-    for (int r = lane; r < m; r += 32) {
-      const double v = P[c * m + r];
-      z.X[(long long)(j0 + c) * N + j0 + r] = (r > c) ? v * scal : v;
-    }
-  }
+  for (int c = wid; c < pb; c += 8)
+    for (int r = lane; r < m; r += 32) z.X[(long long)(j0 + c) * N + j0 + r] = P[c * m + r];
   // the Gram matrix V^T V, the T factor and Vt = V T follow on the tensor cores (Z_GRAM,
   // ztfac_kernel, Z_VT); the panel leaves tau on the diagonal of its T slot
   double* Tg = z.Tb + (long long)p * TB * TB;
@@ -810,11 +809,10 @@ __global__ void __launch_bounds__(256) zqr_panel_kernel(const WalkerDev* __restr
   }
 }
 
-// The T factor of panel p: T^-1 = diag(1 / tau) + the strict upper part of Zg = V^T V (the Z_GRAM
-// product, in Wb), so row i of T is tau_i (e_i - sum_{k > i} Zg(i, k) T(k, :)), rows from the last
-// up: when row k is known every warp adds its term to its own rows above (rows i = warp mod 8, lane
-// per column), two barriers apart at most 4 FMAs.  One warp adding the columns' terms one after the
-// other (LAPACK's dlarft) took 36 us, this 20.
+// The T factor of panel p (LAPACK dlarft, forward, columnwise): T(c, c) = tau_c and
+// T(i, c) = -tau_c sum_{i <= k < c} T(i, k) Zg(k, c), Zg = V^T V from the Z_GRAM product (in Wb).
+// Row i needs no other row: a warp takes rows i = warp mod 8, lane c holds the sum of column c, and
+// step k broadcasts T(i, k).  No barriers, four rows a warp in flight; the sums run in dlarft's order.
 __global__ void __launch_bounds__(256) ztfac_kernel(const WalkerDev* __restrict__ W, int mode, int j, int p) {
   const int wi = blockIdx.x >> 1, sp = blockIdx.x & 1;
   const WalkerDev& w = W[wi];
@@ -823,32 +821,31 @@ __global__ void __launch_bounds__(256) ztfac_kernel(const WalkerDev* __restrict_
   if (j0 >= N) return;
   const int pb = min(TB, N - j0), tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const ZScr z = zscr(w, sp);
-  __shared__ double Zg[TB][TB + 1], Tr[TB][TB];  // Zg[k][i] = Zg(i, k); Tr[k][j] = T(k, j)
-  __shared__ double tau[TB];
+  __shared__ double Zg[TB][TB + 1];  // Zg[k][c] = Zg(k, c), k < c
+  __shared__ double s_tau[TB];
   double* Tg = z.Tb + (long long)p * TB * TB;
   for (int e = tid; e < TB * TB; e += 256) {
-    const int i = e % TB, k = e / TB;
-    Zg[k][i] = (i < k && k < pb) ? z.Wb[(long long)k * TB + i] : 0.0;
-    if (i == k) tau[k] = (k < pb) ? Tg[e] : 0.0;
+    const int k = e % TB, c = e / TB;
+    Zg[k][c] = (k < c && c < pb) ? z.Wb[(long long)c * TB + k] : 0.0;
+    if (k == c) s_tau[c] = (c < pb) ? Tg[e] : 0.0;
   }
+  __syncthreads();
+  const double tau = s_tau[lane];
   double acc[4] = {0.0, 0.0, 0.0, 0.0};  // rows wid + 8 u
-  __syncthreads();
-  for (int k = pb - 1; k >= 0; --k) {
-    if (wid == (k & 7)) {
-      const int u = k >> 3;
-      const double a = (u == 0) ? acc[0] : (u == 1) ? acc[1] : (u == 2) ? acc[2] : acc[3];
-      Tr[k][lane] = tau[k] * (((lane == k) ? 1.0 : 0.0) - a);
-    }
-    __syncthreads();
-    const double t = Tr[k][lane];
+  for (int k = wid; k + 1 < pb; ++k) {
+    const double zk = Zg[k][lane];
 #pragma unroll
-    for (int u = 3; u >= 0; --u)
-      if (wid + 8 * u < k) acc[u] = fma(Zg[k][wid + 8 * u], t, acc[u]);  // uniform in the warp
+    for (int u = 0; u < 4; ++u) {
+      const int i = wid + 8 * u;
+      if (i > k) continue;  // uniform in the warp
+      const double t = __shfl_sync(0xffffffffu, (i == k) ? tau : -tau * acc[u], k);
+      if (lane > k) acc[u] = fma(t, zk, acc[u]);
+    }
   }
-  __syncthreads();
-  for (int e = tid; e < TB * TB; e += 256) {
-    const int i = e % TB, k = e / TB;  // T(i, k)
-    Tg[e] = (i <= k && k < pb) ? Tr[i][k] : 0.0;
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const int i = wid + 8 * u;
+    Tg[lane * TB + i] = (i < pb && lane < pb && lane >= i) ? (lane == i ? tau : -tau * acc[u]) : 0.0;
   }
 }
 
