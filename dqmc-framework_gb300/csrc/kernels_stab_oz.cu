@@ -663,6 +663,9 @@ __global__ void __launch_bounds__(256) zpush_prep_kernel(const WalkerDev* __rest
 // stabilization interval amplify a change of rounding here to 1e-6 of the s-wave sum at beta = 10.
 // What bounds it: the FP64 rate of one SM (2 m pb^2 operations) for long panels, warp 0's chain
 // for short ones.
+// A pass of 6 walkers of 16 x 16 (with ztfac_kernel): 59.8 ms with four barriers a column and
+// serial quotients, 55.6 with two barriers and reordered sums, the same with this form;
+// 128 walkers 794, 771, and 3 ms (of 683) more than the reordered sums.
 // --------------------------------------------------------------------------
 // Sums of 4 (8) values over the warp, value k left in lanes 8 k .. 8 k + 7 (4 k .. 4 k + 3)
 __device__ __forceinline__ double zsum4(double a0, double a1, double a2, double a3, int lane) {
