@@ -96,7 +96,8 @@ namespace {
 
 // HBM walkers with 32 < N <= 768 are stabilized by the blocked QR of kernels_stab_oz.cu (its
 // FP64 panel of 32 columns fits shared memory up to 768 rows; one panel or less gains nothing
-// from blocks): 1 with tensor-core products (mixed walkers of N >= 128), 2 with FP64 products.
+// from blocks): 1 with tensor-core products (mixed walkers of N >= 128), 2 with FP64 products and
+// a column-pivoted QR in the push.
 // The others keep the column-pivoted QR and the LU with one thread per column.
 constexpr int kMaxOzN = 768;
 int stab_kind(int N, int precision, bool general) {
@@ -961,6 +962,8 @@ static LaunchShape launch_shape(const dqmc_batch* b, int w0, int w1, bool all_hb
     }
     if (h.ozstab == 2) s.stab.f64 = std::max(s.stab.f64, h.N);
   }
+  for (const WalkerDev& h : b->hw)
+    if (h.ozstab == 2) s.stab.f64_mats += h.S;
   return s;
 }
 

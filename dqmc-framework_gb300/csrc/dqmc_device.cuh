@@ -115,9 +115,9 @@ struct WalkerDev {
 };
 
 // The largest N of a batch's walkers stabilized with tensor-core and with FP64 products (0: none),
-// and the smallest of the former
+// the smallest of the former, and the matrices (walkers times spins) of the latter in the whole batch
 struct StabSizes {
-  int tc, f64, tc_min;
+  int tc, f64, tc_min, f64_mats;
   __host__ __device__ int max() const { return tc > f64 ? tc : f64; }
 };
 

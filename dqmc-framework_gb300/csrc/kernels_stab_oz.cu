@@ -8,12 +8,14 @@
 // MKL dgesvd and compute_equaltime_greens (include/utils/numerical_stable.hpp:
 // 186-239) assembles G through an LU inverse.  The plain path restates them
 // with column-pivoted QR (kernels_general.cu), a latency-bound FP64 loop.  Here
-//   push:   the columns of the chain are ordered once by norm (pre-pivoting,
-//           Bai, Lee, Li and Xu, Linear Algebra Appl. 435 (2011) 659) and
-//           factored by blocked Householder QR with 32-column panels.  Each
-//           panel is factored in FP64 in shared memory (LAPACK dgeqr2 and
-//           dlarft order); the trailing update A -= V T^T (V^T A), the formation
-//           of Q and F = D^-1 R P^T F_prev are products.
+//   push:   with tensor-core products the columns of the chain are ordered
+//           once by norm (pre-pivoting, Bai, Lee, Li and Xu, Linear Algebra
+//           Appl. 435 (2011) 659) and factored by blocked Householder QR with
+//           32-column panels.  Each panel is factored in FP64 in shared memory
+//           (LAPACK dgeqr2 and dlarft order); the trailing update A -= V T^T
+//           (V^T A) is two products.  With FP64 products the QR pivots on every
+//           column (zqrp_kernel).  The formation of Q and F = D^-1 R P^T F_prev
+//           are products in both.
 //   greens: M = Dlmax^-1 U_L^T U_R Drmax^-1 + Dlmin F_L F_R^T Drmin and
 //           Y = Dlmax^-1 U_L^T; M = QR by the same blocked Householder; X =
 //           R^-1 Q^T Y by blocked reflector application and blocked back
@@ -33,10 +35,12 @@
 // so applying a block reflector is two products.  Panels, diagonal solves,
 // reflectors and reductions are native FP64.  G equals the pivoted-QR path's
 // mathematically; the UDT factors differ only in the column order of the QR.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <cstdint>
+#include <utility>
 
 #include "dqmc_device.cuh"
 #include "ozaki.cuh"
@@ -48,6 +52,7 @@ namespace dqmc {
 namespace {
 
 constexpr int TB = 32;           // Householder panel width
+constexpr int QW = 8;            // warps of a CTA of the column-pivoted QR
 
 __device__ __forceinline__ double zwarp_sum(double v) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -604,22 +609,23 @@ __global__ void __launch_bounds__(256) zgemm_f64_kernel(const WalkerDev* __restr
   }
 }
 
+// the B-chain of spin sp that the push of step j factors
+__device__ __forceinline__ const double* zchain(const WalkerDev& w, int mode, int j, int sp) {
+  const int k = (mode == MODE_FWD) ? j : (w.nstack - 1 - j);
+  const int nsl = min((k + 1) * w.pace, w.Lt) - k * w.pace;
+  return w.chain + (long long)((w.cb ? 0 : (nsl & 1)) * w.S + sp) * w.N * w.N;
+}
+
 // --------------------------------------------------------------------------
-// Push preparation: column norms of the chain, order by decreasing norm
+// Push preparation with tensor-core products: column norms of the chain, order by decreasing norm
 // (ties by index), X = chain(:, perm).  One CTA per (walker, spin).
 // --------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) zpush_prep_kernel(const WalkerDev* __restrict__ W, int mode, int j) {
   const int wi = blockIdx.x >> 1, sp = blockIdx.x & 1;
   const WalkerDev& w = W[wi];
-  if (!w.ozstab || sp >= w.S || j >= w.nstack) return;
+  if (w.ozstab != 1 || sp >= w.S || j >= w.nstack) return;
   const int N = w.N;
-  int nsl;
-  {
-    const int k = (mode == MODE_FWD) ? j : (w.nstack - 1 - j);
-    nsl = min((k + 1) * w.pace, w.Lt) - k * w.pace;
-  }
-  const long long NN = (long long)N * N;
-  const double* Cin = w.chain + (long long)((w.cb ? 0 : (nsl & 1)) * w.S + sp) * NN;
+  const double* Cin = zchain(w, mode, j, sp);
   const ZScr z = zscr(w, sp);
   extern __shared__ long long zkey[];  // [N] norm bit patterns
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -688,11 +694,12 @@ __device__ __forceinline__ double zsum8(const double (&a)[8], int lane) {
   return v;
 }
 
+// kinds: the kinds of walkers (WalkerDev::ozstab, a bit each) that take part
 __global__ void __launch_bounds__(256) zqr_panel_kernel(const WalkerDev* __restrict__ W, int mode, int j, int p,
-                                                        int push) {
+                                                        int push, int kinds) {
   const int wi = blockIdx.x >> 1, sp = blockIdx.x & 1;
   const WalkerDev& w = W[wi];
-  if (!w.ozstab || sp >= w.S || j >= w.nstack) return;
+  if (!(w.ozstab & kinds) || sp >= w.S || j >= w.nstack) return;
   const int N = w.N, j0 = p * TB;
   if (j0 >= N) return;
   const int m = N - j0, pb = min(TB, m);
@@ -812,27 +819,246 @@ __global__ void __launch_bounds__(256) zqr_panel_kernel(const WalkerDev* __restr
   }
 }
 
-// The T factor of panel p (LAPACK dlarft, forward, columnwise): T(c, c) = tau_c and
-// T(i, c) = -tau_c sum_{i <= k < c} T(i, k) Zg(k, c), Zg = V^T V from the Z_GRAM product (in Wb).
+// --------------------------------------------------------------------------
+// The push's factorization with FP64 products (ozstab 2): column-pivoted Householder QR of the
+// chain (LAPACK dlaqp2: partial norms downdated, and summed again once half of their digits are
+// gone).  An order fixed beforehand costs a graded chain its accuracy: at U = 6, beta = 6, pace 10
+// the assembled G of a 12 x 12 walker was 4e-10 off its long-double value with columns ordered once
+// by norm (10 x 10: 1.5e-11), 1.9e-12 (1.3e-12) with a pivot per column.
+//
+// A cluster of P CTAs per (walker, spin), a warp per column (column c: CTA c mod P, warp c / P mod
+// QW, its partial norm in lane c / (P QW)).  Columns stay where they are, in shared memory (SM) or
+// in Y, and column k of the result goes to X once it is chosen.  A step has two cluster barriers:
+// the warp of the chosen column writes the reflector to every CTA's shared memory; then each warp
+// takes the dot products of its columns, four at a time, and with row k their partial norms, sends
+// its largest one to all CTAs and updates rows k + 1 .. while that travels.  A column's sums are
+// one warp's whatever P is, so results do not depend on it.
+// What bounds it: the chain of a step (norm, square root, division, two barriers, two reductions:
+// 10 us at N = 256), then FP64 issue.  A push of 16 walkers of 16 x 16 2.4 ms (panels and products
+// without pivoting: 1.9); a pass of them 30.1 ms (29.2; 91 with a thread per column), of 32 walkers
+// of 9 x 9 22.2 (21.9; 26).  Columns in L2 instead of shared memory 32.6 and 22.9, 16 warps a CTA
+// 30.0 and 22.3 (9 x 9 at P = 4: 23.2).
+// --------------------------------------------------------------------------
+template <int P, bool SM>
+__global__ void __launch_bounds__(32 * QW) __cluster_dims__(P, 1, 1)
+    zqrp_kernel(const WalkerDev* __restrict__ W, int mode, int j) {
+  namespace cg = cooperative_groups;
+  const int wi = blockIdx.y >> 1, sp = blockIdx.y & 1, rank = blockIdx.x;
+  const WalkerDev& w = W[wi];
+  // the whole cluster leaves or stays
+  if (w.ozstab != 2 || sp >= w.S || j >= w.nstack) return;
+  cg::cluster_group cl = cg::this_cluster();
+  auto barrier = [&]() {
+    if (P > 1) cl.sync();
+    else __syncthreads();
+  };
+  const int N = w.N, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const double* Cin = zchain(w, mode, j, sp);
+  const ZScr z = zscr(w, sp);
+  double* Do = stack_level(w, (mode == MODE_FWD) ? 0 : 1, sp, j) + 2 * (long long)N * N;
+  extern __shared__ double vsh[];  // [2][N] the reflectors of steps k even and odd, then the CTA's columns
+  auto column = [&](int q) {       // of this warp
+    return SM ? vsh + (long long)(2 + wid + QW * q) * N : z.Y + (long long)(rank + P * (wid + QW * q)) * N;
+  };
+  __shared__ long long s_key[QW * P];
+  __shared__ int s_col[QW * P];
+  __shared__ double s_tau;
+  // lane q: column rank + P (wid + 8 q), its squared partial norm and the last one summed in full
+  const int mycol = rank + P * (wid + QW * lane);
+  bool active = mycol < N;
+  double n1 = 0.0, n2 = 0.0;
+  for (int q = 0, c = rank + P * wid; c < N; ++q, c += QW * P) {
+    double s = 0.0, *a = column(q);
+    for (int r = lane; r < N; r += 32) {
+      const double x = Cin[(long long)c * N + r];
+      a[r] = x;
+      s = fma(x, x, s);
+    }
+    s = zwarp_sum(s);
+    if (lane == q) n1 = n2 = s;
+  }
+  __syncwarp();
+  // (key, col) of the largest key in the warp, ties to the lowest column; key < 0: none
+  auto warp_best = [&](long long& key, int& col) {
+    const int hi = (int)(key >> 32), mh = __reduce_max_sync(0xffffffffu, hi);
+    const unsigned lo = (hi == mh) ? (unsigned)key : 0u, ml = __reduce_max_sync(0xffffffffu, lo);
+    col = __reduce_min_sync(0xffffffffu, (hi == mh && (unsigned)key == ml) ? col : 0x7fffffff);
+    key = ((long long)mh << 32) | ml;
+  };
+  auto send = [&](long long key, int col) {  // the warp's candidate, to every CTA
+    warp_best(key, col);
+    if (lane < P) {
+      *((P > 1) ? cl.map_shared_rank(&s_key[rank * QW + wid], lane) : &s_key[wid]) = key;
+      *((P > 1) ? cl.map_shared_rank(&s_col[rank * QW + wid], lane) : &s_col[wid]) = col;
+    }
+  };
+  auto norm_key = [&]() { return active ? (__double_as_longlong(n1) & 0x7fffffffffffffffLL) : -1LL; };
+  if (P > 1) cl.sync();  // every CTA runs before its shared memory is written
+  send(norm_key(), mycol);
+  barrier();
+  for (int k = 0; k < N; ++k) {
+    double* v = vsh + (k & 1) * N;  // rows k + 1 ..; a slow warp may still read the previous one
+    long long key = -1;
+    int pc = 0x7fffffff;
+#pragma unroll
+    for (int q = 0; q < (QW * P + 31) / 32; ++q) {
+      const int e = lane + 32 * q;
+      if (e < QW * P && (s_key[e] > key || (s_key[e] == key && s_col[e] < pc))) { key = s_key[e]; pc = s_col[e]; }
+    }
+    warp_best(key, pc);
+    const bool owner = pc % P == rank && pc / P % QW == wid;
+    double beta = 0.0, quo = 0.0;
+    if (owner) {
+      // its reflector: rows k + 1 .. scaled, to every CTA
+      const double* a = column(pc / P / QW);
+      double s0 = 0.0, s1 = 0.0;
+      int r = k + 1 + lane;
+      for (; r + 32 < N; r += 64) {
+        s0 = fma(a[r], a[r], s0);
+        s1 = fma(a[r + 32], a[r + 32], s1);
+      }
+      if (r < N) s0 = fma(a[r], a[r], s0);
+      const double xn2 = zwarp_sum(s0 + s1), alpha = a[k];
+      const bool any = xn2 != 0.0;
+      const double nrm = sqrt(alpha * alpha + xn2);
+      beta = any ? (alpha >= 0 ? -nrm : nrm) : alpha;
+      // lane 0: tau = (beta - alpha) / beta, lane 1: scale = 1 / (alpha - beta), lane 2: 1 / |beta|
+      const double d = beta - alpha;
+      quo = __ddiv_rn(lane == 0 ? d : 1.0, lane == 0 ? beta : lane == 1 ? -d : fabs(beta));
+      const double tau = any ? __shfl_sync(0xffffffffu, quo, 0) : 0.0;
+      const double scal = any ? __shfl_sync(0xffffffffu, quo, 1) : 1.0;
+      for (r = k + 1 + lane; r < N; r += 32) {
+        const double y = a[r] * scal;
+#pragma unroll
+        for (int p = 0; p < P; ++p) *((P > 1) ? cl.map_shared_rank(&v[r], p) : &v[r]) = y;
+      }
+      if (lane < P) *((P > 1) ? cl.map_shared_rank(&s_tau, lane) : &s_tau) = tau;
+      if (mycol == pc) active = false;
+    }
+    barrier();
+    const double tau = s_tau;
+    // column k of R and V to X, with what else the step settles (its stores are not waited for at a barrier)
+    auto settle = [&]() {
+      const double* a = column(pc / P / QW);
+      double* x = z.X + (long long)k * N;
+      for (int r = lane; r < k; r += 32) x[r] = a[r];
+      for (int r = k + 1 + lane; r < N; r += 32) x[r] = v[r];
+      const double inv = __shfl_sync(0xffffffffu, quo, 2), ab = fabs(beta);
+      if (lane == 0) {
+        x[k] = beta;
+        z.perm[k] = pc;
+        z.Tb[(long long)(k / TB) * TB * TB + (k % TB) * (TB + 1)] = tau;  // the diagonal of its T factor
+        Do[k] = ab;
+        z.invd[k] = (ab != 0.0) ? inv : 0.0;
+        if (ab == 0.0 || !isfinite(ab)) atomicOr(w.status, ST_SINGULAR);
+      }
+    };
+    if (k + 1 == N) {
+      if (owner) settle();
+      break;
+    }
+    // A(k:, c) -= tau v (v^T A(k:, c)), v = [1; v]: row k and with it the partial norms first, so that
+    // the next candidates travel while rows k + 1 .. are updated
+    const unsigned mine = __ballot_sync(0xffffffffu, active);
+    double fc = 0.0;  // lane q: -tau (v^T A(k:, c)) of its column
+    bool again = false;
+    for (unsigned todo = mine; todo;) {
+      int q[4], n = 0;
+      double* a[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        q[u] = todo ? __ffs(todo) - 1 : q[0];
+        if (todo) ++n;
+        todo &= todo - 1;
+        a[u] = column(q[u]);
+      }
+      double d[4] = {0.0, 0.0, 0.0, 0.0};
+      for (int r = k + 1 + lane; r < N; r += 32) {
+        const double vr = v[r];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (u < n) d[u] = fma(vr, a[u][r], d[u]);
+      }
+      // lanes 8 u .. 8 u + 7: column u
+      const double dot = zsum4(d[0], d[1], d[2], d[3], lane);
+      const int g = lane >> 3;
+      double* ag = (g & 2) ? ((g & 1) ? a[3] : a[2]) : ((g & 1) ? a[1] : a[0]);
+      const double top = ag[k], f = tau * (dot + top), rk = top - f;
+      __syncwarp();
+      if ((lane & 7) == 0 && g < n) ag[k] = rk;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const double fu = -__shfl_sync(0xffffffffu, f, 8 * u), ru = __shfl_sync(0xffffffffu, rk, 8 * u);
+        if (u < n && lane == q[u]) {
+          fc = fu;
+          n1 = fma(-ru, ru, n1);
+          again = n1 <= 1.4901161193847656e-08 * n2;
+        }
+      }
+    }
+    auto update = [&]() {
+      for (unsigned todo = mine; todo;) {
+        int n = 0;
+        double* a[4];
+        double f[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int q = todo ? __ffs(todo) - 1 : 0;
+          if (todo) ++n;
+          todo &= todo - 1;
+          a[u] = column(q);
+          f[u] = __shfl_sync(0xffffffffu, fc, q);
+        }
+        int r = k + 1 + lane;
+        for (; r + 32 < N; r += 64) {  // two rows' loads before their stores
+          const double v0 = v[r], v1 = v[r + 32];
+          double y[4], x[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            if (u < n) { y[u] = a[u][r]; x[u] = a[u][r + 32]; }
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            if (u < n) { a[u][r] = fma(f[u], v0, y[u]); a[u][r + 32] = fma(f[u], v1, x[u]); }
+        }
+        if (r < N) {
+          const double v0 = v[r];
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            if (u < n) a[u][r] = fma(f[u], v0, a[u][r]);
+        }
+      }
+      __syncwarp();
+    };
+    const unsigned full = __ballot_sync(0xffffffffu, again);
+    if (full) update();
+    for (unsigned m = full; m; m &= m - 1) {
+      const int q = __ffs(m) - 1;
+      const double* a = column(q);
+      double s = 0.0;
+      for (int r = k + 1 + lane; r < N; r += 32) s = fma(a[r], a[r], s);
+      s = zwarp_sum(s);
+      if (lane == q) n1 = n2 = s;
+    }
+    send(norm_key(), mycol);
+    if (P > 1) {
+      cg::cluster_group::arrival_token t = cl.barrier_arrive();
+      if (!full) update();
+      if (owner) settle();
+      cl.barrier_wait(std::move(t));
+    } else {
+      if (!full) update();
+      if (owner) settle();
+      __syncthreads();
+    }
+  }
+}
+
+// The T factor of a panel (LAPACK dlarft, forward, columnwise) from Zg = V^T V (Zg[k][c], k < c) and tau:
+// T(c, c) = tau_c, T(i, c) = -tau_c sum_{i <= k < c} T(i, k) Zg(k, c).
 // Row i needs no other row: a warp takes rows i = warp mod 8, lane c holds the sum of column c, and
 // step k broadcasts T(i, k).  No barriers, four rows a warp in flight; the sums run in dlarft's order.
-__global__ void __launch_bounds__(256) ztfac_kernel(const WalkerDev* __restrict__ W, int mode, int j, int p) {
-  const int wi = blockIdx.x >> 1, sp = blockIdx.x & 1;
-  const WalkerDev& w = W[wi];
-  if (!w.ozstab || sp >= w.S || j >= w.nstack) return;
-  const int N = w.N, j0 = p * TB;
-  if (j0 >= N) return;
-  const int pb = min(TB, N - j0), tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  const ZScr z = zscr(w, sp);
-  __shared__ double Zg[TB][TB + 1];  // Zg[k][c] = Zg(k, c), k < c
-  __shared__ double s_tau[TB];
-  double* Tg = z.Tb + (long long)p * TB * TB;
-  for (int e = tid; e < TB * TB; e += 256) {
-    const int k = e % TB, c = e / TB;
-    Zg[k][c] = (k < c && c < pb) ? z.Wb[(long long)c * TB + k] : 0.0;
-    if (k == c) s_tau[c] = (c < pb) ? Tg[e] : 0.0;
-  }
-  __syncthreads();
+__device__ __forceinline__ void zt_rows(const double (&Zg)[TB][TB + 1], const double* s_tau, int pb, double* Tg) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const double tau = s_tau[lane];
   double acc[4] = {0.0, 0.0, 0.0, 0.0};  // rows wid + 8 u
   for (int k = wid; k + 1 < pb; ++k) {
@@ -850,6 +1076,63 @@ __global__ void __launch_bounds__(256) ztfac_kernel(const WalkerDev* __restrict_
     const int i = wid + 8 * u;
     Tg[lane * TB + i] = (i < pb && lane < pb && lane >= i) ? (lane == i ? tau : -tau * acc[u]) : 0.0;
   }
+}
+
+// The T factor of panel p, its Gram matrix from the Z_GRAM product (in Wb), tau on the diagonal of its slot
+__global__ void __launch_bounds__(256) ztfac_kernel(const WalkerDev* __restrict__ W, int mode, int j, int p, int kinds) {
+  const int wi = blockIdx.x >> 1, sp = blockIdx.x & 1;
+  const WalkerDev& w = W[wi];
+  if (!(w.ozstab & kinds) || sp >= w.S || j >= w.nstack) return;
+  const int N = w.N, j0 = p * TB;
+  if (j0 >= N) return;
+  const int pb = min(TB, N - j0), tid = threadIdx.x;
+  const ZScr z = zscr(w, sp);
+  __shared__ double Zg[TB][TB + 1];
+  __shared__ double s_tau[TB];
+  double* Tg = z.Tb + (long long)p * TB * TB;
+  for (int e = tid; e < TB * TB; e += 256) {
+    const int k = e % TB, c = e / TB;
+    Zg[k][c] = (k < c && c < pb) ? z.Wb[(long long)c * TB + k] : 0.0;
+    if (k == c) s_tau[c] = (c < pb) ? Tg[e] : 0.0;
+  }
+  __syncthreads();
+  zt_rows(Zg, s_tau, pb, Tg);
+}
+
+// The T factors of zqrp_kernel's panels, all in one launch (a CTA per walker, spin and panel): with the
+// factorization behind them the panels do not wait for one another.  The Gram matrix of the
+// reflectors is summed here, 32 rows at a time, four sums of a column c a thread (k = warp + 8 u).
+__global__ void __launch_bounds__(256) zqrp_tfac_kernel(const WalkerDev* __restrict__ W, int mode, int j) {
+  const int wi = blockIdx.y >> 1, sp = blockIdx.y & 1, p = blockIdx.x;
+  const WalkerDev& w = W[wi];
+  if (w.ozstab != 2 || sp >= w.S || j >= w.nstack) return;
+  const int N = w.N, j0 = p * TB;
+  if (j0 >= N) return;
+  const int m = N - j0, pb = min(TB, m), tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const ZScr z = zscr(w, sp);
+  __shared__ double Zg[TB][TB + 1], V[TB][TB + 1];  // V[c][r]
+  __shared__ double s_tau[TB];
+  double* Tg = z.Tb + (long long)p * TB * TB;
+  if (tid < TB) s_tau[tid] = (tid < pb) ? Tg[tid * (TB + 1)] : 0.0;
+  double g[4] = {0.0, 0.0, 0.0, 0.0};
+  for (int r0 = 0; r0 < m; r0 += TB) {
+    __syncthreads();
+    for (int c = wid; c < TB; c += 8) {
+      const int r = r0 + lane;
+      V[c][lane] = (c >= pb || r >= m || r < c) ? 0.0 : (r == c) ? 1.0 : z.X[(long long)(j0 + c) * N + j0 + r];
+    }
+    __syncthreads();
+#pragma unroll 8
+    for (int r = 0; r < TB; ++r) {
+      const double vc = V[lane][r];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) g[u] = fma(V[wid + 8 * u][r], vc, g[u]);
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < 4; ++u) Zg[wid + 8 * u][lane] = (wid + 8 * u < lane) ? g[u] : 0.0;
+  __syncthreads();
+  zt_rows(Zg, s_tau, pb, Tg);
 }
 
 // Vt = V_p T_p^T (m x pb, ld N) for forming Q: Vt(r, c) = sum_{c <= q <= r} V(r, q) T(c, q).
@@ -1070,6 +1353,12 @@ __global__ void __launch_bounds__(256) zdyn_boundary_kernel(const WalkerDev* __r
 static size_t ztc_smem(int S, int NT, int NS) { return (size_t)NS * oztc::stage_bytes(S, 128, NT); }
 static size_t zpanel_smem(int maxN) { return sizeof(double) * (size_t)TB * maxN; }
 
+// dynamic shared memory: two reflectors, and the columns of a CTA where they fit
+static size_t zqrp_smem(int N, int P, bool sm) {
+  return sizeof(double) * (size_t)N * (2 + (sm ? ((N + P - 1) / P + QW - 1) / QW * QW : 0));
+}
+constexpr size_t kQrpSmem = 224 * 1024;
+
 cudaError_t configure_stab_oz_kernels(int maxN) {
   cudaError_t e;
   if ((e = cudaFuncSetAttribute(ZGEMM56, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ztc_smem(8, 32, 2))))
@@ -1079,6 +1368,10 @@ cudaError_t configure_stab_oz_kernels(int maxN) {
   if ((e = cudaFuncSetAttribute(zqr_panel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)zpanel_smem(maxN > 0 ? maxN : 1))))
     return e;
+  const void* qrp[4] = {(const void*)zqrp_kernel<1, true>, (const void*)zqrp_kernel<2, true>,
+                        (const void*)zqrp_kernel<4, true>, (const void*)zqrp_kernel<8, true>};
+  for (const void* f : qrp)
+    if ((e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kQrpSmem))) return e;
   return cudaSuccess;
 }
 
@@ -1136,23 +1429,53 @@ static void zgemm(const WalkerDev* W, int nw, StabSizes zs, int op, int mode, in
   if (maxN > 256) ZGEMM54<<<g, 256, ztc_smem(9, 32, 4), st>>>(W, op, mode, j, p, trace_slot, tl);
 }
 
+static int zkinds(StabSizes zs) { return (zs.tc ? 1 : 0) | (zs.f64 ? 2 : 0); }
+
 // Householder panel p: the FP64 column factorization, then its Gram matrix, T factor and
 // Vt = V T (the block reflector in the form the trailing products apply)
 static void zpanel(const WalkerDev* W, int nw, StabSizes zs, int mode, int j, int p, int push, cudaStream_t st) {
-  zqr_panel_kernel<<<2 * nw, 256, zpanel_smem(zs.max()), st>>>(W, mode, j, p, push);
+  zqr_panel_kernel<<<2 * nw, 256, zpanel_smem(zs.max()), st>>>(W, mode, j, p, push, zkinds(zs));
   zgemm(W, nw, zs, Z_GRAM, mode, j, p, -1, st);
-  ztfac_kernel<<<2 * nw, 256, 0, st>>>(W, mode, j, p);
+  ztfac_kernel<<<2 * nw, 256, 0, st>>>(W, mode, j, p, zkinds(zs));
   zgemm(W, nw, zs, Z_VT, mode, j, p, -1, st);
+}
+
+template <int P>
+static void launch_qrp_p(const WalkerDev* W, int nw, int N, int mode, int j, cudaStream_t st) {
+  const dim3 g(P, 2 * nw);
+  const size_t sm = zqrp_smem(N, P, true);
+  if (sm <= kQrpSmem) zqrp_kernel<P, true><<<g, 32 * QW, sm, st>>>(W, mode, j);
+  else zqrp_kernel<P, false><<<g, 32 * QW, zqrp_smem(N, P, false), st>>>(W, mode, j);
+}
+
+// CTAs per matrix: as many as shared memory needs for the columns (a lane per column and warp asks
+// for N <= 256 P), then twice as many while the batch's matrices have at most three CTAs an SM.
+// Measured at P = 1, 2, 4, 8: a pass of 16 walkers of 16 x 16 (one spin; 1 and 2 do not fit) 41.7,
+// 36.2, 30.1, 30.3 ms; of 32 of 9 x 9 (two spins) 22.4, 22.1, 22.3, 23.0; of a mixed batch of 112
+// walkers, 96 of them of 36 to 121 sites, 299, 300, 303, 310, its set-up 56, 54, 53, 56.
+static void launch_qrp(const WalkerDev* W, int nw, StabSizes zs, int mode, int j, cudaStream_t st) {
+  const int N = zs.f64;
+  int P = 1, dev = 0, sms = 152;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  while (P < 8 && (N > 32 * QW * P || zqrp_smem(N, P, true) > kQrpSmem || 2 * P * zs.f64_mats <= 3 * sms)) P *= 2;
+  if (P == 8) launch_qrp_p<8>(W, nw, N, mode, j, st);
+  else if (P == 4) launch_qrp_p<4>(W, nw, N, mode, j, st);
+  else if (P == 2) launch_qrp_p<2>(W, nw, N, mode, j, st);
+  else launch_qrp_p<1>(W, nw, N, mode, j, st);
 }
 
 void oz_push(int mode, const WalkerDev* W, int nw, int j, StabSizes zs, cudaStream_t st) {
   const int maxN = zs.max(), np = (maxN + TB - 1) / TB;
-  zpush_prep_kernel<<<2 * nw, 256, sizeof(long long) * maxN, st>>>(W, mode, j);
-  for (int p = 0; p < np; ++p) {
-    zpanel(W, nw, zs, mode, j, p, 1, st);
-    zgemm(W, nw, zs, Z_QR_W, mode, j, p, -1, st);
-    zgemm(W, nw, zs, Z_QR_UPD, mode, j, p, -1, st);
+  const StabSizes tc{zs.tc, 0, zs.tc_min, 0};
+  if (zs.tc) zpush_prep_kernel<<<2 * nw, 256, sizeof(long long) * zs.tc, st>>>(W, mode, j);
+  if (zs.f64) launch_qrp(W, nw, zs, mode, j, st);
+  for (int p = 0; p * TB < zs.tc; ++p) {
+    zpanel(W, nw, tc, mode, j, p, 1, st);
+    zgemm(W, nw, tc, Z_QR_W, mode, j, p, -1, st);
+    zgemm(W, nw, tc, Z_QR_UPD, mode, j, p, -1, st);
   }
+  if (zs.f64) zqrp_tfac_kernel<<<dim3((zs.f64 + TB - 1) / TB, 2 * nw), 256, 0, st>>>(W, mode, j);
   zpush_fin_kernel<<<dim3(64, 2 * nw), 256, 0, st>>>(W, mode, j);
   zgemm(W, nw, zs, Z_F, mode, j, 0, -1, st);
   for (int p = np - 1; p >= 0; --p) {
