@@ -658,7 +658,7 @@ __global__ void __launch_bounds__(kSubCTA, 1) metropolis_sub_kernel(const Walker
   int* s_eR = s_eT + Nu;
   int* etmp = s_eR + Nu;                                                // [2][256]
   int8_t* s_field = reinterpret_cast<int8_t*>(etmp + 2 * kSubThreads);  // [N]
-  __shared__ int s_pos[KB], s_m, s_eGm[2][KB];
+  __shared__ int s_pos[KB], s_m[2], s_eGm[2][KB];
   __shared__ SubAccept s_acc;
   __shared__ __align__(8) unsigned long long bar_ldA, bar_ldB[NBB], bar_mma[2], bar_bfree[NBB], bar_accfree[2];
   __shared__ unsigned s_tmem;
@@ -693,10 +693,12 @@ __global__ void __launch_bounds__(kSubCTA, 1) metropolis_sub_kernel(const Walker
       sub_load_block(st, G, S, N, i0, kb);
       wsync();
       const int mm = sub_decide(w, S, kb, uni + i0, s_field + i0, st, s_pos, s_acc, sign, acc_count);
-      if (tid == 0) s_m = mm;
+      // the next block's count goes to the other slot: after a block without accepts the producer warp
+      // may read this one late (only the workers meet before the next count is written)
+      if (tid == 0) s_m[(i0 / KB) & 1] = mm;
     }
     __syncthreads();
-    const int m = s_m;
+    const int m = s_m[(i0 / KB) & 1];
     if (m == 0) continue;
     if (worker) {
       int* xGm[2] = {s_eGm[0], s_eGm[1]};

@@ -50,3 +50,35 @@ def test_split_equals_fused(dq, monkeypatch, model, L, lattice):
         np.testing.assert_array_equal(a, c)
     assert fused[2] == split[2] == plain[2]
     assert fused[3] == split[3] == plain[3] == [0, 0]
+
+
+@pytest.mark.parametrize("model", [0, 1])
+def test_blocks_without_accepts(dq, monkeypatch, model):
+    """Strong coupling on fields that have settled: most 32-site blocks accept nothing, so the fused
+    kernel's warps go from block to block meeting at one barrier only, and the blocks that do accept
+    lie at every parity.  Equal to the split kernels to the bit."""
+    descs = [dq.WalkerDesc(model=model, L=12, U=10.0, beta=8.0, Lt=16, pace=1, seed=60 + w) for w in range(4)]
+    out = []
+    for kind in ("2", "3"):
+        monkeypatch.setenv("DQMC_METROPOLIS_KIND", kind)
+        b = dq.Batch(descs, rng=dq.RNG_PHILOX, precision=dq.MIXED)
+        r = np.random.default_rng(model)
+        for w, d in enumerate(descs):
+            b.set_fields(w, (2 * r.integers(0, 2, size=(d.Lt, d.N)) - 1).astype(np.int8))
+        b.init_greens()
+        accepts = []
+        for _ in range(6):
+            before = [b.accept_count(w) for w in range(4)]
+            b.sweep_0_to_beta()
+            b.sweep_beta_to_0()
+            accepts.append([b.accept_count(w) - x for w, x in enumerate(before)])
+        out.append(([b.fields(w) for w in range(4)], [b.green(w, 0) for w in range(4)], accepts,
+                    [b.status(w) for w in range(4)]))
+        b.close()
+    (f2, g2, a2, s2), (f3, g3, a3, s3) = out
+    # 160 blocks a walker and pair of half-sweeps, 154 to 177 accepts in the last pair of a chain of the
+    # oracle: every third block or so has none
+    assert min(a2[-1]) < 320
+    assert a2 == a3 and s2 == s3 == [0] * 4
+    for a, c in zip(f2 + g2, f3 + g3):
+        np.testing.assert_array_equal(a, c)
