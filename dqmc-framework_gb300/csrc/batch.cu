@@ -295,7 +295,7 @@ struct dqmc_batch {
   char* dyn_arena = nullptr;
   // shared-memory walkers (N <= 64) take the HBM path's kernels in the dynamic half-sweep:
   // their ping-pong chain, product temporary and stabilization scratch, per walker
-  struct DynGen { double* chain = nullptr; double* work = nullptr; double* scr = nullptr; };
+  struct DynGen { double* chain = nullptr; double* scr = nullptr; };
   std::vector<DynGen> dyn_gen;
   // the dynamic half-sweep captured once (walker-group branches) and its kernel nodes
   cudaGraphExec_t dyn_exec = nullptr;
@@ -466,21 +466,26 @@ int dqmc_batch_create(const dqmc_walker_desc* descs, int n, const dqmc_batch_opt
     off[w].sle = (o.precision == DQMC_MIXED) ? take(sizeof(int) * S * (size_t)N) : 0;
     off[w].G = take(sizeof(double) * 2 * N * N);
     off[w].chain = take(sizeof(double) * (general ? 2 : 1) * S * N * N);
-    off[w].work = general ? take(sizeof(double) * S * N * N) : 0;
     off[w].scr = general ? take(sizeof(double) * 2 * S * N * N) : 0;
     off[w].stack = take(sizeof(double) * 2 * S * ns * lvl);
     off[w].fields = take((size_t)d.Lt * N);
     off[w].trace = b->trace_cap ? take(sizeof(double) * (size_t)b->trace_cap * 2 * N * N) : 0;
-    off[w].msub = (o.precision == DQMC_MIXED) ? take((size_t)S * submatrix_scratch_bytes(N))
-                  : general                     ? take(submatrix64_scratch_bytes(N, S))
-                                                : 0;
-    // the blocked QR's scratch is the product temporary where that has room
-    off[w].zwk = off[w].work;
-    if (stab_kind(N, o.precision, general) && stab_scratch_elems(N) > (size_t)N * N)
-      off[w].zwk = take(sizeof(double) * S * stab_scratch_elems(N));
-    off[w].zsl = stab_kind(N, o.precision, general) == 1
-                     ? take(sizeof(unsigned short) * (size_t)S * 4 * 9 * ozaki::tc_lines(N) * (size_t)((N + 31) / 32 * 32))
-                     : 0;
+    // The product temporary, the Metropolis updates' scratch and the blocked QR's are not in use at the
+    // same time.  FP64 walkers have one buffer for the last two (and no product temporary); mixed ones
+    // keep the updates' slices apart and take the QR's from the temporary where that has room (N >= 105).
+    const int kind = stab_kind(N, o.precision, general);
+    const size_t zwk = kind ? sizeof(double) * S * stab_scratch_elems(N) : 0;
+    off[w].work = off[w].msub = off[w].zwk = 0;
+    if (o.precision == DQMC_MIXED) {
+      const size_t work = sizeof(double) * S * N * N;
+      off[w].work = off[w].zwk = take(std::max(work, zwk));
+      off[w].msub = take((size_t)S * submatrix_scratch_bytes(N));
+    } else if (general) {
+      off[w].msub = off[w].zwk = take(std::max(submatrix64_scratch_bytes(N, S), zwk));
+    }
+    off[w].zsl = kind == 1 ? take(sizeof(unsigned short) * (size_t)S * 2 * 9 * ozaki::tc_lines(N) *
+                                  (size_t)((N + 31) / 32 * 32))
+                           : 0;
     off[w].dense_id = -1;
     if (!d.checkerboard) {
       const int dim = d.lattice == DQMC_CUBIC ? 3 : 2;
@@ -643,12 +648,12 @@ int dqmc_batch_create(const dqmc_walker_desc* descs, int n, const dqmc_batch_opt
     h.chain = reinterpret_cast<double*>(base + off[w].chain);
     const bool gen = N > kMaxSmemN || o.precision == DQMC_MIXED || o.hbm;
     h.path = (o.precision == DQMC_MIXED) ? 2 : (gen ? 1 : 0);
-    h.work = gen ? reinterpret_cast<double*>(base + off[w].work) : nullptr;
+    h.work = (o.precision == DQMC_MIXED) ? reinterpret_cast<double*>(base + off[w].work) : nullptr;
     h.scr = gen ? reinterpret_cast<double*>(base + off[w].scr) : nullptr;
     h.msub = gen ? reinterpret_cast<unsigned char*>(base + off[w].msub) : nullptr;
     h.ozstab = stab_kind(N, o.precision, gen);
     h.zwk = gen ? reinterpret_cast<double*>(base + off[w].zwk) : nullptr;
-    h.zwk_stride = (off[w].zwk == off[w].work) ? (long long)N * N : (long long)stab_scratch_elems(N);
+    h.zwk_stride = (long long)stab_scratch_elems(N);
     h.zld = (N + 31) / 32 * 32;
     h.zsl = h.ozstab == 1 ? reinterpret_cast<unsigned short*>(base + off[w].zsl) : nullptr;
     if (o.precision == DQMC_MIXED) {
@@ -827,14 +832,15 @@ static int autotune_delayed(dqmc_batch* b) {
       if (c.second == kind) keep.push_back(c);
     if (!keep.empty()) cand = keep;
   }
-  // back up what one Metropolis slice changes: G (spins < S) into work, fields into scr
+  // back up what one Metropolis slice changes: G (spins < S) into the chain (rebuilt before it is read
+  // again), fields into scr
   std::vector<dqmc_batch::Scal> scal(b->nw);
   CUDA_TRY(cudaMemcpyAsync(scal.data(), b->d_scal, sizeof(dqmc_batch::Scal) * b->nw, cudaMemcpyDeviceToHost,
                            b->stream));
   for (int w = 0; w < b->nw; ++w) {
     const WalkerDev& h = b->hw[w];
     if (h.path == 0) continue;
-    CUDA_TRY(cudaMemcpyAsync(h.work, h.G, sizeof(double) * h.S * h.N * h.N, cudaMemcpyDeviceToDevice, b->stream));
+    CUDA_TRY(cudaMemcpyAsync(h.chain, h.G, sizeof(double) * h.S * h.N * h.N, cudaMemcpyDeviceToDevice, b->stream));
     CUDA_TRY(cudaMemcpyAsync(h.scr, h.fields, (size_t)h.Lt * h.N, cudaMemcpyDeviceToDevice, b->stream));
   }
   cudaEvent_t e0, e1;
@@ -861,7 +867,7 @@ static int autotune_delayed(dqmc_batch* b) {
       for (int w = 0; w < b->nw; ++w) {  // restore
         const WalkerDev& h = b->hw[w];
         if (h.path == 0) continue;
-        CUDA_TRY(cudaMemcpyAsync(h.G, h.work, sizeof(double) * h.S * h.N * h.N, cudaMemcpyDeviceToDevice, b->stream));
+        CUDA_TRY(cudaMemcpyAsync(h.G, h.chain, sizeof(double) * h.S * h.N * h.N, cudaMemcpyDeviceToDevice, b->stream));
         CUDA_TRY(cudaMemcpyAsync(h.fields, h.scr, (size_t)h.Lt * h.N, cudaMemcpyDeviceToDevice, b->stream));
       }
       if (rep == 1) {
@@ -1231,8 +1237,7 @@ static int dyn_alloc(dqmc_batch* b) {
     off[kOff * w + 9] = take(sizeof(double) * kMaxTau * h.N);        // per-displacement G sums
     if (h.path == 0) {  // HBM-path buffers of a shared-memory walker
       off[kOff * w + 10] = take(sizeof(double) * 2 * h.S * NN);  // chain (ping-pong)
-      off[kOff * w + 11] = take(sizeof(double) * h.S * NN);      // work
-      off[kOff * w + 12] = take(sizeof(double) * 2 * h.S * NN);  // scr
+      off[kOff * w + 11] = take(sizeof(double) * 2 * h.S * NN);  // scr
     }
   }
   cudaError_t e = cudaMalloc(&b->dyn_arena, cur);
@@ -1257,8 +1262,7 @@ static int dyn_alloc(dqmc_batch* b) {
     b->dyn_gen.resize(b->nw);
     if (h.path == 0) {
       b->dyn_gen[w].chain = reinterpret_cast<double*>(b->dyn_arena + off[kOff * w + 10]);
-      b->dyn_gen[w].work = reinterpret_cast<double*>(b->dyn_arena + off[kOff * w + 11]);
-      b->dyn_gen[w].scr = reinterpret_cast<double*>(b->dyn_arena + off[kOff * w + 12]);
+      b->dyn_gen[w].scr = reinterpret_cast<double*>(b->dyn_arena + off[kOff * w + 11]);
     }
     h.dyn_taus = b->d_taus;
     h.dyn_ntau = 0;
@@ -1359,7 +1363,6 @@ int dqmc_sweep_dynamic(dqmc_batch* b, const int* taus, int ntau) {
     if (h.path == 0) {
       h.path = 1;
       h.chain = b->dyn_gen[w].chain;
-      h.work = b->dyn_gen[w].work;
       h.scr = b->dyn_gen[w].scr;
     }
   }

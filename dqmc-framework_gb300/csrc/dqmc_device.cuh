@@ -51,7 +51,7 @@ struct WalkerDev {
   const double* kin;
   double* G;                 // [2][N*N]
   double* chain;             // [S][N*N] (general walkers: [2][S][N*N], ping-pong)
-  double* work;              // general walkers: GEMM temporary [S][N*N]
+  double* work;              // mixed walkers: product temporary [S][N*N]
   double* scr;               // general walkers: stabilization scratch [S][2][N*N]
   // mixed walkers, submatrix Metropolis: per spin T [N][32] FP64, then the BF16
   // slices of T and of G0(:, accepted sites) [2][6][N][40] and their exponents [2][N]
@@ -75,7 +75,7 @@ struct WalkerDev {
   double* dyn_r;  // [tau][N] sign * 0.5 sum_i (G_up + G_dn)(i + r, i) / N: G(k,tau) of any k
   int zld;                   // line stride of zsl (N rounded up to 32)
   // tensor-core stabilization: BF16 slices of the operands of the current product, A and up to
-  // three parts of B, [S][4][9 slices][N][zld]
+  // three parts of B, in the room of two N x N operands: [S][2][9 slices][N][zld]
   unsigned short* zsl;
   // mixed walkers: BF16 slices of the operand being multiplied, [S][slices][N][ldk]
   unsigned short* sl;

@@ -66,9 +66,9 @@ __device__ __forceinline__ void zstack_tops(const WalkerDev& w, int mode, int j,
 }
 
 // per-spin scratch: scr = X (matrix being factored) | Y (right-hand sides);
-// zwk = Wb [3][TB N] | W2 [TB N] | T factors [ceil(N/TB) TB TB] | invd | four
-// diagonal scale vectors | perm | line exponents of the two operands of the
-// current product (stab_scratch_elems; the product temporary `work` where it has room)
+// zwk = Wb [TB N] | W2 [TB N] | T factors [ceil(N/TB) TB TB] | invd | four
+// diagonal scale vectors | perm | line exponents of the operands of the
+// current product, A and up to three parts of B (stab_scratch_elems)
 struct ZScr {
   double *X, *Y, *Wb, *W2, *Tb, *invd, *dlmaxi, *drmaxi, *dlmin, *drmin;
   int *perm, *expA, *expB;
@@ -82,9 +82,9 @@ __device__ __forceinline__ ZScr zscr(const WalkerDev& w, int sp) {
   z.Y = z.X + NN;
   double* wk = w.zwk + sp * w.zwk_stride;
   z.Wb = wk;
-  z.W2 = wk + 3 * TN;
-  z.Tb = wk + 4 * TN;
-  z.invd = wk + 4 * TN + TT;
+  z.W2 = wk + TN;
+  z.Tb = wk + 2 * TN;
+  z.invd = wk + 2 * TN + TT;
   z.dlmaxi = z.invd + w.N;
   z.drmaxi = z.dlmaxi + w.N;
   z.dlmin = z.drmaxi + w.N;
@@ -93,6 +93,12 @@ __device__ __forceinline__ ZScr zscr(const WalkerDev& w, int sp) {
   z.expA = z.perm + w.N;
   z.expB = z.expA + w.N;
   return z;
+}
+
+// Wb of a product's part: the further parts occur in the Green's assembly only, where the chain's two
+// buffers are free (the push has factored it, the next step writes it anew)
+__device__ __forceinline__ double* zwb(const WalkerDev& w, const ZScr& z, int sp, int part) {
+  return part == 0 ? z.Wb : w.chain + ((long long)(part - 1) * w.S + sp) * w.N * w.N;
 }
 
 // An operand of C = op(A) op(B).  Element (row, col) of the stored block sits at
@@ -160,10 +166,10 @@ enum ZOp {
   Z_D0T_OUT,     // G(0,t) = -F_R^T Drmin X
 };
 
-// A launch's column tiles: `first` of part 0, then `rest` of each further part
+// A launch's column tiles: `first` of part p0, then `rest` of each further part
 struct ZTiles {
-  int first, rest;
-  __device__ __forceinline__ int part(int x) const { return x < first ? 0 : 1 + (x - first) / rest; }
+  int first, rest, p0;
+  __device__ __forceinline__ int part(int x) const { return p0 + (x < first ? 0 : 1 + (x - first) / rest); }
   __device__ __forceinline__ int col(int x) const { return x < first ? x : (x - first) % rest; }
 };
 
@@ -191,7 +197,7 @@ __device__ bool zjob(const WalkerDev& w, int op, int mode, int j, int p, int sp,
       const int nt = (part == 0) ? m - pb : N;
       if (nt <= 0) return false;
       double* C = (part == 0) ? z.X + (long long)(j0 + pb) * N + j0 : (part == 1 ? z.Y : w.dynx + sp * NN) + j0;
-      double* Wp = z.Wb + (long long)part * TB * N;
+      double* Wp = zwb(w, z, sp, part);
       if (op == Z_QR_W) {
         jb.a = VtT;
         jb.b = ZOpnd{C, N, 0, 0, nullptr, nullptr};
@@ -295,6 +301,40 @@ __device__ bool zjob(const WalkerDev& w, int op, int mode, int j, int p, int sp,
   return false;
 }
 
+// Where a product's slices lie in zsl: one image of the lines of A, then those of B's parts, each
+// rounded up to 32, and K rounded up to 32, so that a spin needs the room of two N x N operands
+// whatever the product (2 N lines of K = N; a panel's 32 lines beside its trailing columns and N
+// right-hand sides are no more).  A third part of K = m would need more: it takes the second one's
+// lines after that has been used (Z_QR_W of the dynamic half-sweep).  A tile reads 128 lines of A,
+// also past the image's last one: only where the image is far below the room, and what it reads
+// there ends in rows that are not stored.
+struct ZImage {
+  int line_b, nlb;  // the part's first line, 8-line blocks of the image
+  long long sst;    // elements of a slice
+};
+__device__ __forceinline__ ZImage zimage(const WalkerDev& w, int op, int p, const ZJob& jb, int part) {
+  const auto up = [](int x) { return (x + 31) / 32 * 32; };
+  const int nr = up(w.N), M = up(jb.M), Kp = up(jb.K);
+  ZImage im;
+  int lines;
+  if (op == Z_QR_W || op == Z_QR_UPD) {
+    const int rest = up(max(w.N - (p + 1) * TB, 0));  // part 0: the trailing columns
+    const int slot = (op == Z_QR_W) ? min(part, 1) : part;
+    im.line_b = M + (slot == 0 ? 0 : rest + (slot - 1) * nr);
+    lines = M + rest + (op == Z_QR_W ? 1 : 2) * nr;
+  } else {
+    im.line_b = M + part * up(jb.N);
+    lines = M + (op == Z_TR_UPD ? 2 : 1) * up(jb.N);
+  }
+  im.nlb = lines / 8;
+  im.sst = (long long)lines * Kp;
+  return im;
+}
+// the start of spin sp's slices (room for 9 slices of two N x N operands a spin)
+__device__ __forceinline__ unsigned short* zslices(const WalkerDev& w, int sp) {
+  return w.zsl + (long long)sp * 2 * 9 * ozaki::tc_lines(w.N) * w.zld;
+}
+
 // fixed-point magnitude |x| / 2^e with Q fraction bits (e >= exp_bound(x), Q <= 62)
 __device__ __forceinline__ unsigned long long zfixed(double x, int e, int Q, bool& neg) {
   const unsigned long long b = (unsigned long long)__double_as_longlong(x);
@@ -311,22 +351,24 @@ __device__ __forceinline__ unsigned long long zfixed(double x, int e, int Q, boo
 }  // namespace
 
 // --------------------------------------------------------------------------
-// Slicing of both operands of a product, once per product: blockIdx.y = 0 the
+// Slicing of both operands of a product, once per product: blockIdx.y + y0 = 0 the
 // rows of op(A), 1 + part the columns of op(B); 32 lines per CTA.  Pass 1: the line
 // exponents (8 k groups per line); pass 2: 32 x 32 tiles staged through
-// shared memory so that loads run along the stored matrix.  Output: per
-// operand S slices of tc_lines(N) x zld in the tensor core's shared-memory
-// image (ozaki::tc_index), zero past K up to a multiple of 32.
+// shared memory so that loads run along the stored matrix.  Output: S
+// slices in the tensor core's shared-memory image (ozaki::tc_index, zimage), zero
+// past K up to a multiple of 32.
 // --------------------------------------------------------------------------
 template <int S, int B>
-__global__ void __launch_bounds__(256) zslice_kernel(const WalkerDev* __restrict__ W, int op, int mode, int j, int p) {
+__global__ void __launch_bounds__(256) zslice_kernel(const WalkerDev* __restrict__ W, int op, int mode, int j, int p,
+                                                     int y0) {
   const int wi = blockIdx.z >> 1, sp = blockIdx.z & 1;
   const WalkerDev& w = W[wi];
   if (w.ozstab != 1 || sp >= w.S) return;
   ZJob jb;
-  const bool isB = blockIdx.y != 0;
+  const int y = blockIdx.y + y0;
+  const bool isB = y != 0;
   // A by the part that every step has
-  const int part = isB ? blockIdx.y - 1 : (gridDim.y > 2 && (op == Z_QR_W || op == Z_QR_UPD)) ? 1 : 0;
+  const int part = isB ? y - 1 : (gridDim.y > 2 && (op == Z_QR_W || op == Z_QR_UPD)) ? 1 : 0;
   if (!zjob(w, op, mode, j, p, sp, part, jb)) return;
   if ((jb.K <= 256) != (B == 7)) return;
   const ZOpnd& o = isB ? jb.b : jb.a;
@@ -334,10 +376,10 @@ __global__ void __launch_bounds__(256) zslice_kernel(const WalkerDev* __restrict
   const int l0 = blockIdx.x * 32;
   if (l0 >= nlines) return;
   constexpr int Q = S * B;
-  const int N = w.N, Kp = (jb.K + 31) / 32 * 32, nlb = ozaki::tc_lines(N) / 8;
-  const long long sst = (long long)ozaki::tc_lines(N) * w.zld;
+  const int N = w.N, Kp = (jb.K + 31) / 32 * 32;
   const ZScr z = zscr(w, sp);
-  unsigned short* out = w.zsl + ((long long)(sp * 4 + (isB ? 1 + part : 0)) * 9) * sst;
+  const ZImage im = zimage(w, op, p, jb, part);
+  unsigned short* out = zslices(w, sp) + (isB ? im.line_b / 8 * 128 : 0);
   // lines contiguous in memory when the stored row index runs along the line
   const bool line_fast = (o.tr == (int)isB);
   __shared__ int s_e[8][32];
@@ -383,7 +425,7 @@ __global__ void __launch_bounds__(256) zslice_kernel(const WalkerDev* __restrict
         bool ng[4];
 #pragma unroll
         for (int u = 0; u < 4; ++u) q[u] = zfixed(s_t[ll][kq * 4 + u], s_e[0][ll], Q, ng[u]);
-        unsigned short* o = out + ozaki::tc_index(line, k0 + kq * 4, nlb);
+        unsigned short* o = out + ozaki::tc_index(line, k0 + kq * 4, im.nlb);
 #pragma unroll
         for (int s2 = 0; s2 < S; ++s2) {
           ushort4 v;
@@ -391,7 +433,7 @@ __global__ void __launch_bounds__(256) zslice_kernel(const WalkerDev* __restrict
           v.y = ozaki::slice_bf16q(q[1], s2, B, Q, ng[1]);
           v.z = ozaki::slice_bf16q(q[2], s2, B, Q, ng[2]);
           v.w = ozaki::slice_bf16q(q[3], s2, B, Q, ng[3]);
-          *reinterpret_cast<ushort4*>(o + s2 * sst) = v;
+          *reinterpret_cast<ushort4*>(o + s2 * im.sst) = v;
         }
       }
     }
@@ -449,13 +491,12 @@ __global__ void __launch_bounds__(256, MINB) zgemm_tc_kernel(const WalkerDev* __
   tc::fence_after();
   const unsigned taddr = tbase;
   if (tid == 0) {
-    const long long sst = (long long)ozaki::tc_lines(N) * w.zld;
-    const unsigned short* zA = w.zsl + (long long)(sp * 4) * 9 * sst;
-    const unsigned short* zB = zA + (1 + part) * 9 * sst;
-    const long long cstep = (long long)(ozaki::tc_lines(N) / 8) * 128;
+    const ZImage im = zimage(w, op, p, jb, part);
+    const unsigned short* zA = zslices(w, sp);
     bool ok;
     s_last = oztc::mainloop<S, MT, NT, NS>(tsm, full, done, taddr, zA + (long long)(r0 / 8) * 128,
-                                            zB + (long long)(c0 / 8) * 128, sst, cstep, (jb.K + 15) / 16, ok);
+                                            zA + (long long)((im.line_b + c0) / 8) * 128, im.sst, im.nlb * 128LL,
+                                            (jb.K + 15) / 16, ok);
     s_fail = ok ? 0 : 1;
   }
   __syncthreads();
@@ -1377,7 +1418,7 @@ cudaError_t configure_stab_oz_kernels(int maxN) {
 
 // doubles of scratch a spin's stabilization takes in zwk
 size_t stab_scratch_elems(int N) {
-  return 4ull * TB * N + (size_t)TB * TB * ((N + TB - 1) / TB) + 5ull * N + (5ull * N + 1) / 2;
+  return 2ull * TB * N + (size_t)TB * TB * ((N + TB - 1) / TB) + 5ull * N + (5ull * N + 1) / 2;
 }
 
 // The largest output of an operation over walkers of up to n sites: rows, and columns of part 0
@@ -1402,15 +1443,9 @@ static ZExtent zextent(int op, int p, int n) {
   }
 }
 
-static void zgemm(const WalkerDev* W, int nw, StabSizes zs, int op, int mode, int j, int p, int trace_slot,
-                  cudaStream_t st, int parts = 1) {
-  if (zs.f64) {
-    const ZExtent x = zextent(op, p, zs.f64);
-    const ZTiles tl{(x.cols0 + 15) / 16, (x.cols + 15) / 16};
-    const dim3 g(tl.first + (parts - 1) * tl.rest, (x.rows + 15) / 16, 2 * nw);
-    if (g.x && g.y) zgemm_f64_kernel<<<g, 256, 0, st>>>(W, op, mode, j, p, trace_slot, tl);
-  }
-  if (!zs.tc) return;
+// The parts p0 .. p0 + parts - 1 of a product; slice_a: A too (else its slices are still there)
+static void zgemm_tc(const WalkerDev* W, int nw, StabSizes zs, int op, int mode, int j, int p, int trace_slot, int p0,
+                     int parts, bool slice_a, cudaStream_t st) {
   // the walkers' contraction lengths, minN to maxN: a panel's width, what is left from panel p
   // on, or N; each configuration is launched only where some walker's length takes it (at
   // N = 576 half of the launches had no work)
@@ -1419,14 +1454,30 @@ static void zgemm(const WalkerDev* W, int nw, StabSizes zs, int op, int mode, in
   const int off = rest ? p * TB + (op == Z_TR_UPD ? TB : 0) : 0;
   const int minN = width ? TB : zs.tc_min - off, maxN = width ? TB : zs.tc - off;
   const ZExtent x = zextent(op, p, zs.tc);
-  const ZTiles tl{(x.cols0 + 31) / 32, (x.cols + 31) / 32};
+  const int cols = p0 ? x.cols : x.cols0;  // of part p0
+  const ZTiles tl{(cols + 31) / 32, (x.cols + 31) / 32, p0};
   const dim3 g(tl.first + (parts - 1) * tl.rest, (x.rows + 127) / 128, 2 * nw);
-  const dim3 gs((std::max(x.rows, parts > 1 ? x.cols : x.cols0) + 31) / 32, 1 + parts, 2 * nw);
+  const dim3 gs((std::max(x.rows, parts > 1 ? x.cols : cols) + 31) / 32, parts + (slice_a ? 1 : 0), 2 * nw);
+  const int y0 = slice_a ? 0 : 1 + p0;
   if (!g.x || !g.y) return;
-  if (minN <= 256) zslice_kernel<8, 7><<<gs, 256, 0, st>>>(W, op, mode, j, p);
-  if (maxN > 256) zslice_kernel<9, 6><<<gs, 256, 0, st>>>(W, op, mode, j, p);
+  if (minN <= 256) zslice_kernel<8, 7><<<gs, 256, 0, st>>>(W, op, mode, j, p, y0);
+  if (maxN > 256) zslice_kernel<9, 6><<<gs, 256, 0, st>>>(W, op, mode, j, p, y0);
   if (minN <= 256) ZGEMM56<<<g, 256, ztc_smem(8, 32, 2), st>>>(W, op, mode, j, p, trace_slot, tl);
   if (maxN > 256) ZGEMM54<<<g, 256, ztc_smem(9, 32, 4), st>>>(W, op, mode, j, p, trace_slot, tl);
+}
+
+static void zgemm(const WalkerDev* W, int nw, StabSizes zs, int op, int mode, int j, int p, int trace_slot,
+                  cudaStream_t st, int parts = 1) {
+  if (zs.f64) {
+    const ZExtent x = zextent(op, p, zs.f64);
+    const ZTiles tl{(x.cols0 + 15) / 16, (x.cols + 15) / 16, 0};
+    const dim3 g(tl.first + (parts - 1) * tl.rest, (x.rows + 15) / 16, 2 * nw);
+    if (g.x && g.y) zgemm_f64_kernel<<<g, 256, 0, st>>>(W, op, mode, j, p, trace_slot, tl);
+  }
+  if (!zs.tc) return;
+  const bool apart = op == Z_QR_W && parts == 3;  // part 2 after part 1, in its lines (zimage)
+  zgemm_tc(W, nw, zs, op, mode, j, p, trace_slot, 0, apart ? 2 : parts, true, st);
+  if (apart) zgemm_tc(W, nw, zs, op, mode, j, p, trace_slot, 2, 1, false, st);
 }
 
 static int zkinds(StabSizes zs) { return (zs.tc ? 1 : 0) | (zs.f64 ? 2 : 0); }
