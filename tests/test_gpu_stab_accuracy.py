@@ -124,7 +124,7 @@ def test_pivoted_qr_does_not_depend_on_its_cluster(dq, L, model):  # noqa: F811
     """The CTAs of a matrix follow from the number of matrices and the size (one to eight, columns
     ragged over warps and CTAs); a column's sums are one warp's, so G is the same to the bit."""
     out = []
-    for n in (2, 36, 80, 120) if L < 13 else (2, 60):
+    for n in (2, 16, 36, 80) if L < 13 else (2, 60):
         b = dq.Batch([dq.WalkerDesc(model=model, L=L, U=5.0, mu=-0.2 if model else 0.0, beta=2.0, Lt=10, pace=5,
                                     seed=40 + w) for w in range(n)], rng=dq.RNG_PHILOX, hbm=True)
         for w in range(n):
