@@ -833,7 +833,7 @@ static int autotune_delayed(dqmc_batch* b) {
     if (!keep.empty()) cand = keep;
   }
   // back up what one Metropolis slice changes: G (spins < S) into the chain (rebuilt before it is read
-  // again), fields into scr
+  // again), the first slice's fields into scr (all of them need not fit there: Lt is any number)
   std::vector<dqmc_batch::Scal> scal(b->nw);
   CUDA_TRY(cudaMemcpyAsync(scal.data(), b->d_scal, sizeof(dqmc_batch::Scal) * b->nw, cudaMemcpyDeviceToHost,
                            b->stream));
@@ -841,7 +841,7 @@ static int autotune_delayed(dqmc_batch* b) {
     const WalkerDev& h = b->hw[w];
     if (h.path == 0) continue;
     CUDA_TRY(cudaMemcpyAsync(h.chain, h.G, sizeof(double) * h.S * h.N * h.N, cudaMemcpyDeviceToDevice, b->stream));
-    CUDA_TRY(cudaMemcpyAsync(h.scr, h.fields, (size_t)h.Lt * h.N, cudaMemcpyDeviceToDevice, b->stream));
+    CUDA_TRY(cudaMemcpyAsync(h.scr, h.fields, (size_t)h.N, cudaMemcpyDeviceToDevice, b->stream));
   }
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
@@ -868,7 +868,7 @@ static int autotune_delayed(dqmc_batch* b) {
         const WalkerDev& h = b->hw[w];
         if (h.path == 0) continue;
         CUDA_TRY(cudaMemcpyAsync(h.G, h.chain, sizeof(double) * h.S * h.N * h.N, cudaMemcpyDeviceToDevice, b->stream));
-        CUDA_TRY(cudaMemcpyAsync(h.fields, h.scr, (size_t)h.Lt * h.N, cudaMemcpyDeviceToDevice, b->stream));
+        CUDA_TRY(cudaMemcpyAsync(h.fields, h.scr, (size_t)h.N, cudaMemcpyDeviceToDevice, b->stream));
       }
       if (rep == 1) {
         b->tune_log.push_back({c, ms});

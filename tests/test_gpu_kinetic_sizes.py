@@ -42,3 +42,23 @@ def test_hbm_products_against_shared_memory(dq, L, cb, lattice):
         np.testing.assert_array_equal(a, c)
     for a, c in zip(small[1] + small[2], large[1] + large[2]):
         assert abs(a - c).max() <= 1e-10 * max(1.0, abs(a).max())
+
+
+@pytest.mark.parametrize("mixed", [False, True])
+def test_many_slices_on_few_sites(dq, mixed):
+    """Lt N bytes of fields are more than the scratch of a 2 x 2 walker's matrices holds: the set-up
+    trials of HBM walkers leave the stacks and the fields as they are."""
+    out = []
+    for hbm in (False, True):
+        b = dq.Batch([dq.WalkerDesc(model=1, L=2, U=4.0, mu=-0.3, beta=4.0, Lt=400, pace=200, seed=8)], rng=dq.RNG_MINSTD,
+                     hbm=hbm, precision=dq.MIXED if mixed and hbm else dq.FP64)
+        b.fields_random(0)
+        b.init_greens()
+        b.sweep_0_to_beta()
+        b.sweep_beta_to_0()
+        out.append((b.fields(0), b.green(0, 0), b.status(0), b.wrap_error(0)))
+        b.close()
+    np.testing.assert_array_equal(out[0][0], out[1][0])
+    assert out[0][2] == out[1][2] == 0
+    # two ways to wrap 200 slices: their distance from a fresh G bounds how far apart they may be
+    assert abs(out[0][1] - out[1][1]).max() <= 1e-10 + out[0][3] + out[1][3]
