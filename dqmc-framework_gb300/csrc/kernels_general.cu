@@ -387,6 +387,13 @@ __global__ void __launch_bounds__(256) chain_init_general_kernel(const WalkerDev
 // FP64 throughput of one SM and the strided reads of G(j, i) bounded the one-CTA form: 264 us a
 // slice for 6 walkers of two spins at N = 256, 222 us for 128 walkers of one.
 // --------------------------------------------------------------------------
+// CTAs that share a walker's tile pairs: by its own size, so that its sums are added in the same order
+// whatever else is in the launch (the cluster is the largest walker's)
+__host__ __device__ inline int measure_ctas(int N) {
+  const int nt = (N + 31) / 32, pairs = nt * (nt + 1) / 2;
+  return pairs >= 8 ? 8 : pairs >= 4 ? 4 : pairs >= 2 ? 2 : 1;
+}
+
 template <int P>
 __global__ void __launch_bounds__(256) __cluster_dims__(P, 1, 1)
     measure_general_kernel(const WalkerDev* __restrict__ W, int mode, int j, int q, int after_stab) {
@@ -446,12 +453,12 @@ __global__ void __launch_bounds__(256) __cluster_dims__(P, 1, 1)
   }
   __syncthreads();
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int nt = (N + 31) / 32;
+  const int nt = (N + 31) / 32, share = measure_ctas(N);
   double p4 = 0.0, p5 = 0.0, p6 = 0.0, p7 = 0.0;
   int k = 0;  // tile pairs, dealt to the CTAs in turn
   for (int tj = 0; tj < nt; ++tj)
     for (int ti = 0; ti <= tj; ++ti, ++k) {
-      if (k % P != rank) continue;
+      if (k % share != rank) continue;
       const int i0 = ti * 32, j0 = tj * 32, i = i0 + lane;
       __syncthreads();  // the previous tile's readers are done
 #pragma unroll
@@ -540,14 +547,14 @@ __global__ void __launch_bounds__(256) __cluster_dims__(P, 1, 1)
   if (P > 1) cl.sync();  // the parts stay until rank 0 has read them
 }
 
-// CTAs per walker: the tile pairs of the largest walker, at most a portable cluster of 8
+// CTAs per walker: the largest walker's, at most a portable cluster of 8
 static void launch_measure_general(const WalkerDev* W, int nw, int maxN, int mode, int j, int q, int after_stab,
                                    cudaStream_t st) {
-  const int nt = (maxN + 31) / 32, pairs = nt * (nt + 1) / 2;
+  const int P = measure_ctas(maxN);
   const size_t sm = (size_t)maxN * (3 * sizeof(double) + sizeof(int));
-  if (pairs >= 8) measure_general_kernel<8><<<dim3(8, nw), 256, sm, st>>>(W, mode, j, q, after_stab);
-  else if (pairs >= 4) measure_general_kernel<4><<<dim3(4, nw), 256, sm, st>>>(W, mode, j, q, after_stab);
-  else if (pairs >= 2) measure_general_kernel<2><<<dim3(2, nw), 256, sm, st>>>(W, mode, j, q, after_stab);
+  if (P == 8) measure_general_kernel<8><<<dim3(8, nw), 256, sm, st>>>(W, mode, j, q, after_stab);
+  else if (P == 4) measure_general_kernel<4><<<dim3(4, nw), 256, sm, st>>>(W, mode, j, q, after_stab);
+  else if (P == 2) measure_general_kernel<2><<<dim3(2, nw), 256, sm, st>>>(W, mode, j, q, after_stab);
   else measure_general_kernel<1><<<dim3(1, nw), 256, sm, st>>>(W, mode, j, q, after_stab);
 }
 

@@ -35,3 +35,22 @@ def test_hbm_measurement_against_oracle(dq, oracle_mod, model, L, lattice):  # n
     d = dq.WalkerDesc(model=model, L=L, U=4.0, mu=-0.3 if model else 0.0, beta=0.8, Lt=8, pace=4, seed=520 + L,
                       lattice=lattice)
     _run_pair(dq, oracle_mod, [d], sweeps=1)
+
+
+@pytest.mark.parametrize("L", [5, 7, 9])
+def test_measured_sums_do_not_depend_on_the_batch(dq, L):  # noqa: F811
+    """Beside a larger walker the cluster is that one's; a walker's sums stay the same to the bit."""
+    out = []
+    for others in ([], [12], [16]):
+        b = dq.Batch([dq.WalkerDesc(model=0, L=x, U=4.0, beta=1.0, Lt=10, pace=5, seed=560 + x) for x in [L, *others]],
+                     rng=dq.RNG_PHILOX, hbm=True)
+        for w in range(1 + len(others)):
+            b.fields_random(w)
+        b.init_greens()
+        b.sweep_0_to_beta(measure=True)
+        b.sweep_beta_to_0(measure=True)
+        out.append((b.fields(0), b.green(0, 0), *b.observables(0)))
+        b.close()
+    for o in out[1:]:
+        for a, c in zip(out[0], o):
+            np.testing.assert_array_equal(a, c)
