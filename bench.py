@@ -316,7 +316,9 @@ class Clocks:
 # ----------------------------------------------------------------------------
 def flops_model(wl, accepts_per_walker_per_half):
     """FP64 work of one walker's half-sweep (a workload dict or a walker descriptor), counted
-    as the reference's sweep executes it (dqmc_walker.cpp:246-412)."""
+    as the reference's sweep executes it (dqmc_walker.cpp:246-412): dense products, plaquette
+    matrices.  The rate it gives is the reference's equivalent, not the hardware's: what the
+    kernels execute is fp64_class_flops."""
     wl = _shape(wl)
     N, Lt, p = wl["L"] ** 2, wl["Lt"], wl["pace"]
     S = 1 if wl["model"] == 1 else 2
@@ -333,6 +335,31 @@ def flops_model(wl, accepts_per_walker_per_half):
     greens = S * ns * (4.0 + 2.0 / 3.0 + 2.0 + 2.0) * N ** 3
     nominal = S * Lt * (W + C) + S * accepts_per_walker_per_half * 2 * N * N + S * ns * 33 * N ** 3
     return {"segment": seg, "push": push, "greens": greens, "nominal_F": nominal}
+
+
+def fp64_class_flops(wl, accepts):
+    """FP64 flops that the FP64 kernels execute in one walker's half-sweep with `accepts` accepted
+    flips, by kernel class (square lattice).  A product with exp(-+dtau K) is two plaquette passes of
+    8 FMAs on 4 values (9 N^2 with the scaling) or one ring factor per direction (2 L flops an element
+    each, 4 L N^2 + N^2); a wrap is two of them.  Shared-memory walkers (N <= 64) run products, updates
+    and measurement in the segment class; above, the updates are blocks of up to 32 flips, and the
+    stabilization (N <= 768) solves with a blocked QR instead of the LU."""
+    wl = _shape(wl)
+    L, N, Lt = wl["L"], wl["L"] ** 2, wl["Lt"]
+    S = 1 if wl["model"] == 1 else 2
+    ns = -(-Lt // wl["pace"])
+    product = 9 * N * N if wl["checkerboard"] else 4 * L * N * N + N * N
+    products, updates = S * Lt * 3 * product, S * accepts * 2 * N * N
+    # push: QR 4/3 N^3, forming Q 4/3 N^3, triangular T F_prev N^3
+    push = S * ns * (8.0 / 3.0 + 1.0) * N ** 3
+    # greens: U_L^T U_R, F_L F_R^T and the last product (6 N^3); LU 2/3 N^3 and its solve 2 N^3, or
+    # QR 4/3 N^3, Q^T Y 2 N^3 and the back substitution N^3
+    greens = S * ns * (6.0 + (13.0 / 3.0 if 64 < N <= 768 else 8.0 / 3.0)) * N ** 3
+    if N <= 64:
+        return {"segment": products + updates, "push": push, "greens": greens}
+    nb, p_acc = -(-N // 32), accepts / (N * Lt)
+    updates += S * (2 * N * block_accepts_sq(p_acc) * nb * Lt + accepts * 2 * 32 * 32 / 3)  # T, diagonal blocks
+    return {"product": products, "metropolis": updates, "push": push, "greens": greens}
 
 
 def stab_tensor_flops(N, TB=32):
@@ -390,7 +417,7 @@ def metropolis_work(d, accepts: float, tc_flush: int, kd: int):
       submatrix (tc_flush 2, or 3 split per block): per 32-site block with m accepts, Gamma's m x m products and the
         rank-1 updates of the block in FP64, T = Gamma R_A (N x m x m) and the flush
         G -= G0(:, I_A) T (N x N x m) as 6 x 7-bit slice products (21 pairs);
-      delayed (tc_flush 0 / 1; FP64 walkers take submatrix updates with an FP64 flush of the same 2 N^2 per accept): the corrected diagonal and the u, w vectors per accept in FP64
+      delayed (tc_flush 0 / 1): the corrected diagonal and the u, w vectors per accept in FP64
         (about 4 N k), the flush G -= U V^T (N x N x k) in FP64 or as 21 slice pairs."""
     N, Lt = d.L ** 2, d.Lt
     S = 1 if d.model == 1 else 2
@@ -723,14 +750,12 @@ def run_gpu(args, wl, rank, world):
         extra["_fp64_met"] = fp_met
         extra["_ref_rank1"] = ref_rank1
     else:
-        tot = {"segment": 0.0, "push": 0.0, "greens": 0.0}
+        tot = {}
         for d, a in zip(descs, acc_w):
-            fm = flops_model(d, a)
-            for k in tot:
-                tot[k] += steps * fm[k]
-        for k in ("segment", "push", "greens"):
-            model[k] = ("fp64", tot[k], fp64_peak / 1e3,
-                        "FP64 flops of the class (flops_model: wraps, chain products, Green's assembly)")
+            for k, f in fp64_class_flops(d, a).items():
+                tot[k] = tot.get(k, 0.0) + steps * f
+        for k, f in tot.items():
+            model[k] = ("fp64", f, fp64_peak / 1e3, "FP64 flops that the class executes (fp64_class_flops)")
     timed_classes = [k for k in model if prof.get(k, (0, 0))[1] > 0 and model[k][1] > 0]
     dom = max(timed_classes, key=lambda k: prof[k][0]) if timed_classes else max(prof, key=lambda k: prof[k][0])
     classes = {k: {"bound": v[0], "achieved_tflops": v[1] / (prof[k][0] * 1e-3) / 1e12,
@@ -761,6 +786,7 @@ def run_gpu(args, wl, rank, world):
                 "classes": classes}
     if not mixed:
         nominal = sum(steps * flops_model(d, a)["nominal_F"] for d, a in zip(descs, acc_w))
+        # the reference's count over the sweep's time: an equivalent, not a rate of this hardware
         roofline["sweep_nominal_F_tflops"] = nominal / (ms * 1e-3) / 1e12
 
     # ---- e2e: reference RNG on the host, copies in and out every step

@@ -34,6 +34,23 @@ def test_flop_model_counts_the_reference_work(bench):
     assert cb["segment"] == 2 * 160 * (34 + 17) * 64 * 64  # checkerboard passes, no flips
 
 
+def test_fp64_classes_count_what_the_kernels_execute(bench):
+    """The FP64 roofline divides executed operations by time: plaquettes of 8 FMAs on 4 values, ring
+    factors instead of dense products; the reference's larger count stays with flops_model."""
+    cb = bench.WORKLOADS["fp64_batch_8x8_checkerboard"]  # N = 64, Lt = 160, both spins
+    assert bench.fp64_class_flops(cb, 0.0)["segment"] == 2 * 160 * 27 * 64 * 64
+    assert bench.fp64_class_flops(cb, 100.0)["segment"] == 2 * (160 * 27 + 200) * 64 * 64
+    one = bench.WORKLOADS["fp64_single_4x4_dense"]  # N = 16, Lt = 80
+    assert bench.fp64_class_flops(one, 0.0)["segment"] == 2 * 80 * 3 * (4 * 4 + 1) * 16 * 16
+    for wl in (cb, one):
+        a, r = bench.fp64_class_flops(wl, 500.0), bench.flops_model(wl, 500.0)
+        assert a["segment"] < r["segment"] and a["push"] == pytest.approx(r["push"])
+    big = bench.fp64_class_flops(bench.WORKLOADS["fp64_batch_16x16_attractive"], 1e4)  # N = 256, one spin
+    assert set(big) == {"product", "metropolis", "push", "greens"}
+    assert big["product"] == 100 * 3 * (4 * 16 + 1) * 256 ** 2
+    assert 2 * 1e4 * 256 ** 2 < big["metropolis"] < 1.1 * 2 * 1e4 * 256 ** 2
+
+
 def test_blocked_qr_products_flops(bench):
     """Each panel of the blocked QR costs its trailing update and the Q formation; the counts
     grow like N^3 and exceed the plain 2N^3 products they include."""
