@@ -46,3 +46,25 @@ def test_uneven_groups_give_identical_walkers(dq, monkeypatch, mixed):  # noqa: 
         np.testing.assert_allclose(d1[w], d4[w], rtol=1e-12, atol=1e-12)
     np.testing.assert_allclose(o1[0], o4[0], rtol=1e-12, atol=1e-12)
     np.testing.assert_array_equal(o1[1], o4[1])
+
+
+def test_uneven_groups_with_the_split_kernels(dq, monkeypatch):  # noqa: F811
+    """The split Metropolis kernels' grids (128-line blocks, column tiles, spins) follow the group's
+    largest walker: one group and four, to the bit."""
+    monkeypatch.setenv("DQMC_METROPOLIS_KIND", "3")
+    descs = [dq.WalkerDesc(model=m, L=L, U=4.0, mu=-0.4 * m, beta=0.1 * Lt, Lt=Lt, pace=pace, checkerboard=cb,
+                           seed=720 + i) for i, (m, L, Lt, pace, cb) in enumerate(SHAPES)]
+    res = []
+    for groups in ("1", "4"):
+        monkeypatch.setenv("DQMC_STREAM_GROUPS", groups)
+        b = dq.Batch(descs, rng=dq.RNG_PHILOX, precision=dq.MIXED)
+        for w in range(len(descs)):
+            b.fields_random(w)
+        b.init_greens()
+        assert b.tuning()["tc_flush"] == 3
+        b.sweep_0_to_beta(measure=True)
+        b.sweep_beta_to_0(measure=True)
+        res.append([x for w in range(len(descs)) for x in (b.fields(w), b.green(w, 0), b.status(w))])
+        b.close()
+    for a, c in zip(*res):
+        np.testing.assert_array_equal(a, c)
