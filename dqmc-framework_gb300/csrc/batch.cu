@@ -509,10 +509,10 @@ int dqmc_batch_create(const dqmc_walker_desc* descs, int n, const dqmc_batch_opt
   for (auto& kv : dense_ids) dense_n[kv.second] = lattice_sites(std::get<0>(kv.first), std::get<1>(kv.first));
   for (size_t i = 0; i < dense.size(); ++i) {
     const size_t nn = dense[i].first.size();
-    dense_off[i] = take(sizeof(double) * 2 * nn);
     dense_kin[i] = take(sizeof(double) * rings[i].size());
-    if (o.precision == DQMC_MIXED) {  // 4 sliced copies: expK (A, B roles), invK (A, B roles)
+    if (o.precision == DQMC_MIXED) {  // the pair and 4 sliced copies: expK (A, B roles), invK (A, B roles)
       const int N = dense_n[i], ldk = (N + 15) / 16 * 16;
+      dense_off[i] = take(sizeof(double) * 2 * nn);
       dense_sl[i] = take(sizeof(unsigned short) * 4 * ozaki::kMaxSlices * ozaki::tc_slice_elems(N, ldk));
       dense_sle[i] = take(sizeof(int) * 4 * (size_t)N);
     }
@@ -572,12 +572,13 @@ int dqmc_batch_create(const dqmc_walker_desc* descs, int n, const dqmc_batch_opt
   // upload dense matrices and Fourier tables
   for (size_t i = 0; i < dense.size(); ++i) {
     const size_t nn = dense[i].first.size();
-    cudaMemcpyAsync(base + dense_off[i], dense[i].first.data(), sizeof(double) * nn, cudaMemcpyHostToDevice, b->stream);
-    cudaMemcpyAsync(base + dense_off[i] + sizeof(double) * nn, dense[i].second.data(), sizeof(double) * nn,
-                    cudaMemcpyHostToDevice, b->stream);
     cudaMemcpyAsync(base + dense_kin[i], rings[i].data(), sizeof(double) * rings[i].size(), cudaMemcpyHostToDevice,
                     b->stream);
     if (o.precision == DQMC_MIXED) {
+      cudaMemcpyAsync(base + dense_off[i], dense[i].first.data(), sizeof(double) * nn, cudaMemcpyHostToDevice,
+                      b->stream);
+      cudaMemcpyAsync(base + dense_off[i] + sizeof(double) * nn, dense[i].second.data(), sizeof(double) * nn,
+                      cudaMemcpyHostToDevice, b->stream);
       const int N = dense_n[i], ldk = (N + 15) / 16 * 16;
       const auto c = ozaki::cfg_for_k(N);
       const auto cfg = std::make_pair(c.bits, c.slices);
@@ -676,8 +677,6 @@ int dqmc_batch_create(const dqmc_walker_desc* descs, int n, const dqmc_batch_opt
     h.side_stride = (long long)h.S * h.nstack * h.lvl_stride;
     h.fields = reinterpret_cast<int8_t*>(base + off[w].fields);
     if (off[w].dense_id >= 0) {
-      h.expK = reinterpret_cast<const double*>(base + dense_off[off[w].dense_id]);
-      h.invK = h.expK + (size_t)N * N;
       h.kin = reinterpret_cast<const double*>(base + dense_kin[off[w].dense_id]);
     }
     h.ff = reinterpret_cast<const double*>(base + off[w].ff);

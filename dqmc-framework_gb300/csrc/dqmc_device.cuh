@@ -89,8 +89,6 @@ struct WalkerDev {
   long long lvl_stride;      // doubles per stack level (2 N^2 + N, padded)
   long long side_stride;     // doubles per side (S * nstack * lvl_stride)
   int8_t* fields;            // [Lt][N]
-  const double* expK;        // dense exp(-dtau K)  (N*N) or null
-  const double* invK;        // dense exp(+dtau K)
   const double* ff;          // Fourier factor per displacement index, measured k
   double* obs;               // [kNumObs] sums of sign * O
   long long* obs_cnt;        // [kNumObs]

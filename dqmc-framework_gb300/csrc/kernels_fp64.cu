@@ -1021,7 +1021,6 @@ __global__ void __launch_bounds__(kThreads, 2) greens_kernel(const WalkerDev* __
     for (int i = threadIdx.x; i < N; i += kThreads) dr_min[i] = 1.0 / dr_max[i];
     __syncthreads();
     // G = (U_R Drmax^-1) Y; the product is formed in registers, compared, stored
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
     block_gemm(N, [&](int r, int k) { return __ldg(UR + (long long)k * N + r) * dr_min[k]; },
                [&](int k, int c) { return at(Ys, ld, k, c); },
                [&](int r, int c, double v) {
@@ -1031,7 +1030,6 @@ __global__ void __launch_bounds__(kThreads, 2) greens_kernel(const WalkerDev* __
                  G[o] = v;
                  if (tr) tr[o] = v;
                });
-    (void)tx; (void)ty;
   } else {
     for (int e = threadIdx.x; e < N * N; e += kThreads) {
       const int r = e % N, c = e / N;
