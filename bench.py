@@ -91,7 +91,8 @@ METRIC = "HS-field updates/s (walkers*N*Lt / half-sweep time)"
 # kernel of a class on the tensor-core path, from one ncu --set full capture each of an
 # 8-walker launch of the 16x16, beta = 10 configuration.  ncu replays a kernel with L2
 # flushed, and each walker's G, chain and slices are its own, so this cold-cache traffic
-# grows in proportion to the walkers a launch covers.
+# grows in proportion to the walkers a launch covers.  Captures of the kernels after their later
+# rework moved the same bytes to 1 % (4.42 and 8.31 MB).
 NCU_TRAFFIC_8_WALKERS = {
     "metropolis": ("metropolis_sub_kernel", 4379392 + 0),
     "product": ("oz_prod_tc_kernel<3,7>", 8307200 + 0),

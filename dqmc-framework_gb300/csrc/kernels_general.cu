@@ -6,9 +6,11 @@
 //   wrap (two products in the factors of exp(-dtau K), the diagonal
 //   exp(+/-alpha s) fused) -> Metropolis (submatrix updates, kernels_submatrix.cu)
 //   -> measurement -> B-chain step (one product).
-// Stabilization: column-pivoted QR with one thread per column (row-major copy,
-// coalesced across threads), Green's assembly by batched GEMMs and an LU solve
-// with one thread per column of [M | Y].
+// Stabilization: of walkers of 33 to 768 sites in kernels_stab_oz.cu; of the
+// others, and of shared-memory walkers in the dynamic half-sweep, here:
+// column-pivoted QR with one thread per column (row-major copy, coalesced across
+// threads), Green's assembly by batched GEMMs and an LU solve with one thread
+// per column of [M | Y].
 //
 // Reference behaviour is the same as kernels_fp64.cu (src/dqmc_walker.cpp,
 // src/model/*.cpp, src/svd_stack.cpp, include/utils/numerical_stable.hpp,

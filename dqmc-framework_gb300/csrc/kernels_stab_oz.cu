@@ -1,5 +1,5 @@
 // kernels_stab_oz.cu — stabilization of HBM walkers (32 < N <= 768): the UDT
-// push and the Green's assembly as blocked Householder factorizations whose
+// push and the Green's assembly as Householder factorizations whose blocked
 // matrix products run on the BF16 tensor cores at FP64 accuracy (mixed walkers
 // with N >= 128, WalkerDev::ozstab 1) or in FP64 (FP64 walkers, and mixed ones
 // below 128 sites, where a product does not fill the tensor core's tiles; 2).
@@ -843,7 +843,7 @@ __global__ void __launch_bounds__(256) zqr_panel_kernel(const WalkerDev* __restr
   }
   for (int c = wid; c < pb; c += 8)
     for (int r = lane; r < m; r += 32) z.X[(long long)(j0 + c) * N + j0 + r] = P[c * m + r];
-  // the Gram matrix V^T V, the T factor and Vt = V T follow on the tensor cores (Z_GRAM,
+  // the Gram matrix V^T V, the T factor and Vt = V T follow as products (Z_GRAM,
   // ztfac_kernel, Z_VT); the panel leaves tau on the diagonal of its T slot
   double* Tg = z.Tb + (long long)p * TB * TB;
   for (int e = tid; e < TB * TB; e += 256) {

@@ -1,5 +1,6 @@
-// kernels_submatrix.cu — Metropolis of one time slice for walkers on the
-// tensor-core path, by submatrix updates.
+// kernels_submatrix.cu — Metropolis of one time slice for HBM walkers, by
+// submatrix updates: fused or split per block with tensor-core products
+// (mixed walkers), split with FP64 products (FP64 walkers).
 //
 // The reference visits the N sites of slice t in order (metropolis_update,
 // src/dqmc_walker.cpp:173-197) and applies every accepted flip at once to the
@@ -16,15 +17,16 @@
 // where u~_p, w~_p are u_p, w_p on the block and R_A = E_A^T - G0(I_A,:).
 // After the block
 //     G = G0 - G0(:,I_A) Gamma R_A,   Gamma = sum_q a_q b_q^T   (m x m),
-// the Sherman-Morrison-Woodbury form of the m flips, applied as two products
-// on the 5th-generation tensor cores through exact 42-bit integer slices
-// (ozaki.cuh; K <= 32 per flush): T = Gamma R_A (m x N), then
-// G -= G0(:,I_A) T (N x N, K = m).  Both run as a pipelined tile loop: one
-// thread stages the slices (bulk copies into shared memory, B tiles two
-// ahead) and issues the MMAs of tile t+1 into one of two TMEM accumulators
-// while all warps run the epilogue of tile t from the other.  The epilogue of
-// T slices T directly (per-column exponents by warp reductions), so T never
-// exists in FP64 outside registers.
+// the Sherman-Morrison-Woodbury form of the m flips, applied as two products:
+// T = Gamma R_A (m x N), then G -= G0(:,I_A) T (N x N, K = m).  FP64 walkers
+// run them in FP64 over tiles of G.  Mixed walkers run them on the
+// 5th-generation tensor cores through exact 42-bit integer slices (ozaki.cuh;
+// K <= 32 per flush), as a pipelined tile loop: a producer warp's thread stages
+// the slices (bulk copies into shared memory, B tiles two ahead) and issues the
+// MMAs of tile t+1 into one of two TMEM accumulators while eight worker warps
+// run the epilogue of tile t from the other.  The epilogue of T slices T
+// directly (a column's exponent is the maximum of two threads' halves), so T
+// never exists in FP64 outside registers.
 //
 // The decisions use the reference's ratio formula, evaluated with the same
 // rounded operations, and the same uniform per site; G reaches them through
@@ -467,8 +469,8 @@ __device__ __forceinline__ void sub_slice_gamma(const WalkerDev& w, int S, int N
 
 // Spin sp of a block with m accepts at sites i0 + s_pos[q], Gamma's slices made: the row blocks
 // rb0 .. rb0 + nrb - 1 (128 lines) of the slices of G0(:, I_A) and R_A = E_A^T - G0(I_A, :) (taken
-// before G changes), then of T^T = R_A^T Gamma^T on the tensor cores: warp w and w + 4 share TMEM lanes 32 (w & 3).. (columns c) and take x in [0, 16) and
-// [16, 32); the column exponent max over x goes through etmp, and the epilogue slices T straight
+// before G changes), then of T^T = R_A^T Gamma^T on the tensor cores: warp w and w + 4 share TMEM
+// lanes 32 (w & 3).. (columns c) and take x in [0, 16) and [16, 32); the column exponent max over x goes through etmp, and the epilogue slices T straight
 // into the B image of the flush (line c, k = x).  Line exponents: eGm [KB] of Gamma, eG [N] of
 // G0(:, I_A), eR [N] of R_A, eT [N] of T (shared or global memory); etmp: [2][256] scratch.
 // Called by all kSubCTA threads; the workers slice.
@@ -737,8 +739,8 @@ __global__ void __launch_bounds__(kSubCTA, 1) metropolis_sub_kernel(const Walker
 
 // dynamic shared memory of the decision kernel: the block's uniforms, the FP64 block state, the
 // exponent scratch [2][256] and the block's fields; of the preparation kernel: the operand
-// buffers, the exponent scratch and eR of one row block; of the flush kernel: the operand
-// buffers, the G staging and the line exponents eG, eT [N]
+// buffers and the exponent scratch (the line exponents stay in msub); of the flush kernel: the
+// operand buffers, the G staging and the line exponents eG, eT [N]
 size_t submatrix_block_smem_bytes(int S) {
   return sizeof(double) * (KB + (size_t)S * (GBS + 5 * KK)) + 2 * kSubThreads * sizeof(int) + KB;
 }

@@ -12,8 +12,9 @@
 // The array is shared by all calls on a device and keeps the last call's
 // contents.  Nothing in it has to start at zero: every call rewrites all the
 // slices and exponents it reads (the slicing kernel also writes the zero
-// padding of each line; the lines past n only reach outputs past n).  Calls that overlap on the GPU (concurrent streams,
-// or several host threads) race on it; the caller serialises them.
+// padding of each line; the lines past n only reach outputs past n).  Calls that
+// overlap on the GPU (concurrent streams, or several host threads) race on it;
+// the caller serialises them.
 #include <cuda_runtime.h>
 
 #include <mutex>
