@@ -70,7 +70,7 @@ void general_dynamic_stab(const WalkerDev* W, int nw, int j, int maxN, cudaStrea
 void general_dynamic_stab_measure(const WalkerDev* W, int nw, int j, cudaStream_t st);
 void general_dynamic_begin(const WalkerDev* W, int nw, cudaStream_t st);
 void general_dynamic_end(const WalkerDev* W, int nw, int maxN, cudaStream_t st);
-void oz_push(int mode, const WalkerDev* W, int nw, int j, StabSizes zs, cudaStream_t st);
+void oz_push(int mode, const WalkerDev* W, int nw, int j, StabSizes zs, SideStream side, cudaStream_t st);
 void oz_greens(int mode, const WalkerDev* W, int nw, int j, int trace_slot, StabSizes zs, cudaStream_t st,
                bool dyn = false);
 size_t stab_scratch_elems(int N);
@@ -313,6 +313,7 @@ struct dqmc_batch {
   static constexpr int kMaxGroups = 16;
   int ngroups = 1;
   cudaStream_t gst[kMaxGroups] = {};
+  SideStream side[kMaxGroups] = {};  // per group, in batches with both kinds of stabilization (oz_push)
   cudaEvent_t ev_fork = nullptr, ev_join[kMaxGroups] = {};
   std::vector<std::minstd_rand0> eng;
   double* h_uni = nullptr;          // pinned [nw][maxLt*maxN]
@@ -548,6 +549,15 @@ int dqmc_batch_create(const dqmc_walker_desc* descs, int n, const dqmc_batch_opt
       if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->ev_join[g], cudaEventDisableTiming);
     }
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->ev_fork, cudaEventDisableTiming);
+    bool kinds[3] = {false, false, false};
+    for (const auto& d : b->desc)
+      kinds[stab_kind(desc_sites(d), o.precision, desc_sites(d) > kMaxSmemN || o.precision == DQMC_MIXED || o.hbm)] = true;
+    for (int g = 0; kinds[1] && kinds[2] && g < b->ngroups && e == cudaSuccess; ++g) {
+      SideStream& s = b->side[g];
+      e = cudaStreamCreateWithFlags(&s.st, cudaStreamNonBlocking);
+      if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s.fork, cudaEventDisableTiming);
+      if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s.join, cudaEventDisableTiming);
+    }
     if (e != cudaSuccess) {
       dqmc_batch_destroy(b);
       return fail(DQMC_ERR_CUDA, "stream groups: %s", cudaGetErrorString(e));
@@ -734,6 +744,9 @@ int dqmc_batch_destroy(dqmc_batch* b) {
   if (b->dyn_arena) cudaFree(b->dyn_arena);
   for (int g = 0; g < dqmc_batch::kMaxGroups; ++g) {
     if (b->gst[g]) cudaStreamDestroy(b->gst[g]);
+    if (b->side[g].st) cudaStreamDestroy(b->side[g].st);
+    if (b->side[g].fork) cudaEventDestroy(b->side[g].fork);
+    if (b->side[g].join) cudaEventDestroy(b->side[g].join);
     if (b->ev_join[g]) cudaEventDestroy(b->ev_join[g]);
   }
   if (b->ev_fork) cudaEventDestroy(b->ev_fork);
@@ -947,11 +960,13 @@ struct LaunchShape {
   int maxN = 0, maxPace = 0, maxNs = 0, smax = 1;
   bool dense = false, cb = false, qrp = false;
   StabSizes stab{};
+  SideStream side{};
   bool oz() const { return stab.max() > 0; }
 };
-// all_hbm: shared-memory walkers too (the dynamic half-sweep runs them as HBM walkers)
-static LaunchShape launch_shape(const dqmc_batch* b, int w0, int w1, bool all_hbm) {
+// all_hbm: shared-memory walkers too (the dynamic half-sweep runs them as HBM walkers); g: the group
+static LaunchShape launch_shape(const dqmc_batch* b, int w0, int w1, bool all_hbm, int g = 0) {
   LaunchShape s;
+  s.side = b->side[g];
   for (int w = w0; w < w1; ++w) {
     const WalkerDev& h = b->hw[w];
     if (h.path == 0 && !all_hbm) continue;
@@ -990,7 +1005,7 @@ int dqmc_init_greens(dqmc_batch* b) {
       for (int q = 0; q < s.maxPace; ++q)  // the transposed B-chain of the initial right stack
         general_slice_post(MODE_INIT, b->dW, b->nw, j, q, s.maxN, s.dense, s.cb, b->mixed, b->stream);
       if (s.qrp) general_push(MODE_INIT, b->dW, b->nw, j, s.maxN, b->stream);
-      if (s.oz()) oz_push(MODE_INIT, b->dW, b->nw, j, s.stab, b->stream);
+      if (s.oz()) oz_push(MODE_INIT, b->dW, b->nw, j, s.stab, s.side, b->stream);
     }
     if (s.qrp) general_greens(MODE_INIT, b->dW, b->nw, 0, -1, s.maxN, b->stream);
     if (s.oz()) oz_greens(MODE_INIT, b->dW, b->nw, 0, -1, s.stab, b->stream);
@@ -1031,7 +1046,7 @@ static void issue_general_level(dqmc_batch* b, const LaunchShape& s, int mode, i
   }
   b->timed(DQMC_KCLASS_PUSH, [&] {
     if (s.qrp) general_push(mode, W, nw, j, s.maxN, st);
-    if (s.oz()) oz_push(mode, W, nw, j, s.stab, st);
+    if (s.oz()) oz_push(mode, W, nw, j, s.stab, s.side, st);
   });
   b->timed(DQMC_KCLASS_GREENS, [&] {
     if (s.qrp) general_greens(mode, W, nw, j, slot, s.maxN, st);
@@ -1059,7 +1074,7 @@ static void issue_half_sweep(dqmc_batch* b, int mode, int measure) {
     for (int g = 0; g < ng; ++g) {
       const int w0 = (int)((long long)b->nw * g / ng), w1 = (int)((long long)b->nw * (g + 1) / ng);
       cudaStreamWaitEvent(b->gst[g], b->ev_fork, 0);
-      const LaunchShape s = launch_shape(b, w0, w1, false);
+      const LaunchShape s = launch_shape(b, w0, w1, false, g);
       for (int j = 0; j < s.maxNs; ++j)
         issue_general_level(b, s, mode, measure, j, trace_slot(b, j), b->dW + w0, w1 - w0, b->gst[g]);
       cudaEventRecord(b->ev_join[g], b->gst[g]);
@@ -1298,7 +1313,7 @@ static void issue_dynamic_level(dqmc_batch* b, const LaunchShape& s, int j, cons
   }
   b->timed(DQMC_KCLASS_PUSH, [&] {
     if (s.qrp) general_push(MODE_FWD, W, nw, j, maxN, st);
-    if (s.oz()) oz_push(MODE_FWD, W, nw, j, s.stab, st);
+    if (s.oz()) oz_push(MODE_FWD, W, nw, j, s.stab, s.side, st);
   });
   b->timed(DQMC_KCLASS_GREENS, [&] {
     if (s.qrp) general_greens(MODE_FWD, W, nw, j, -1, maxN, st);
@@ -1323,7 +1338,7 @@ static void issue_dynamic(dqmc_batch* b) {
     for (int g = 0; g < ng; ++g) {
       const int w0 = (int)((long long)b->nw * g / ng), w1 = (int)((long long)b->nw * (g + 1) / ng);
       cudaStreamWaitEvent(b->gst[g], b->ev_fork, 0);
-      const LaunchShape s = launch_shape(b, w0, w1, true);
+      const LaunchShape s = launch_shape(b, w0, w1, true, g);
       for (int j = 0; j < s.maxNs; ++j) issue_dynamic_level(b, s, j, b->dW + w0, w1 - w0, b->gst[g]);
       cudaEventRecord(b->ev_join[g], b->gst[g]);
     }

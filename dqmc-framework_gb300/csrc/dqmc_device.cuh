@@ -119,6 +119,12 @@ struct StabSizes {
   __host__ __device__ int max() const { return tc > f64 ? tc : f64; }
 };
 
+// A stream beside the launch's own, with the events that fork it off and join it; null: none
+struct SideStream {
+  cudaStream_t st;
+  cudaEvent_t fork, join;
+};
+
 constexpr int kDefaultWaitLimit = 1 << 24;
 
 // Philox4x32-10 (Salmon, Moraes, Dror, Shaw, SC'11): uniform double in [0,1)
