@@ -1502,8 +1502,8 @@ static void launch_qrp_p(const WalkerDev* W, int nw, int N, int mode, int j, cud
 // CTAs per matrix: as many as shared memory needs for the columns (a lane per column and warp asks
 // for N <= 256 P), then twice as many while every CTA of the batch's matrices still has an SM of its own.
 // Measured at P = 1, 2, 4, 8: a pass of 16 walkers of 16 x 16 (one spin; 1 and 2 do not fit) 41.7,
-// 36.2, 30.1, 30.3 ms; of 32 of 9 x 9 (two spins) 22.4, 22.1, 22.3, 23.0; of a mixed batch of 112
-// walkers, 96 of them of 36 to 121 sites, 299, 300, 303, 310, its set-up 56, 54, 53, 56.
+// 36.2, 30.1, 30.3 ms; of 32 of 9 x 9 (two spins) 22.4, 22.1, 22.3, 23.0; of a mixed batch of 64
+// walkers, 48 of them of 36 to 100 sites, 299, 300, 303, 310, its set-up 56, 54, 53, 56.
 static void launch_qrp(const WalkerDev* W, int nw, StabSizes zs, int mode, int j, cudaStream_t st) {
   const int N = zs.f64;
   int P = 1, dev = 0, sms = 152;
